@@ -173,6 +173,14 @@ _SIGS = {
                                  _vp]),
     "ds_col2im_bf16": (C.c_int, [_vp, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, _vp,
                                  _vp, _vp]),
+    "ds_conv3x3_forward": (C.c_int, [_vp, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, _vp,
+                                     C.c_int, C.c_int, _vp, _vp, _vp, _vp, _vp, _vp]),
+    "ds_conv3x3_dgrad": (C.c_int, [_vp, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, _vp,
+                                   C.c_int, C.c_int, _vp, _vp, _vp, _vp]),
+    "ds_conv3x3_wgrad_workspace": (C.c_int64, [C.c_int, C.c_int, C.c_int, C.c_int, C.c_int,
+                                               C.c_int, C.c_int]),
+    "ds_conv3x3_wgrad": (C.c_int, [_vp, _vp, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int,
+                                   C.c_int, C.c_int, _vp, _vp, _vp, _vp]),
     "ds_transpose_bf16": (C.c_int, [_vp, C.c_int, C.c_int, _vp, _vp]),
     "ds_colsum_bf16": (C.c_int, [_vp, C.c_int64, C.c_int, _vp, C.c_int, _vp, _vp]),
     "ds_adamw": (C.c_int, [_vp, _vp, _vp, _vp, C.c_int64, C.c_float, C.c_float, C.c_float,

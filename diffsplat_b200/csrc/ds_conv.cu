@@ -1,0 +1,708 @@
+// 3x3 convolution (padding 1, stride 1 or 2) of NHWC BF16 tensors on tcgen05
+// tensor cores, forward, input gradient and weight gradient, as implicit
+// GEMMs: the taps are TMA boxes of the tensors themselves, so no im2col matrix,
+// transpose or per-tap gradient reaches HBM.  No reference counterpart.
+//
+//   forward  out[m][n]      = sum_{tap, c} x(m, tap)[c] w[n][tap C + c]
+//   dgrad    dx[p][c]       = sum_{tap, n} dz(p, tap)[n] w[n][tap C + c]
+//   wgrad    gw[n][tap C+c] = sum_m dz[m][n] x(m, tap)[c]
+//
+// An output pixel m = (b, oy, ox) reads x at (oy s - 1 + ky, ox s - 1 + kx).
+// For each tap one 4-D tensor map covers exactly the elements of x that the
+// tap reads, in output-pixel coordinates (strides s C and s W C), so a box of
+// output pixels is one TMA load and what lies in the padding is zero-filled.
+// With stride 2 the input gradient splits into the four parities of (iy, ix),
+// each a dense sum over 4, 2, 2 or 1 taps of dz.
+//
+// One persistent CTA per SM, 6 warps: warp 0 issues the TMA loads of a ring of
+// stages, warp 1 issues tcgen05.mma into one of two TMEM accumulators, warps
+// 2-5 read the other one back, so a tile's epilogue runs beside the next
+// tile's MMAs.  Operand layouts: what is contiguous along K in HBM is loaded
+// K-major, what is contiguous along M or N (the weights in dgrad, both operands
+// in wgrad) MN-major, so nothing is transposed.  The K order of the forward is
+// that of the im2col matrix, hence its results too, bit for bit.
+//
+// Every mbarrier wait is bounded as in ds_gemm.cu: on a timeout the CTA sets the
+// error word, lets what it issued land, frees its TMEM and returns.
+#include <algorithm>
+#include <mutex>
+
+#include "ds_common.cuh"
+#include "ds_internal.h"
+#include "ds_umma.cuh"
+
+namespace ds {
+namespace {
+
+enum ConvMode : int { kConvFwd = 0, kConvDgrad = 1, kConvWgrad = 2 };
+enum ConvEpi : int { kConvGelu = 0, kConvF32 = 1 };  // forward only
+
+constexpr int kConvThreads = 192;
+constexpr int kWgradPixels = 64;  // K block of the weight gradient
+// Pixels summed by one accumulation chain of the weight gradient: the tensor
+// cores' FP32 sums lose precision with the chain's length (relative error
+// 4.6e-6 at 4096 products, the length the im2col path used), so longer
+// reductions are split and their partials added in order.
+constexpr int kWgradChain = 4096;
+
+// A rectangle of pixels per tile: bw x bh of each of bb images (powers of two),
+// and the number of such tiles along x, y and the images.
+struct PixelTiles {
+  int lw, lh;      // log2 of bw, bh
+  int bb;
+  int tx, ty, tb;
+};
+
+struct ConvArgs {
+  int B, H, W, C, Ho, Wo, N, stride;
+  int kp;                       // row pitch of the weights
+  int tiles_n;                  // column tiles (forward: of N, dgrad: of C, wgrad: of 9C)
+  PixelTiles pt[4];             // dgrad: one per parity class
+  int first[5];                 // first work item of each class; [classes] = all items
+  int classes;
+  int splits, kb_per_split;     // wgrad
+  int off_x[9], off_y[9];       // forward / wgrad: coordinate of output pixel 0 in the tap's map
+  const float* bias;
+  const __nv_bfloat16* zprev;   // dgrad: pre-activation below, or null
+  __nv_bfloat16 *y, *z;         // forward outputs; dgrad writes y
+  float* d;                     // forward FP32 output; wgrad [splits][N][kp]
+  uint32_t* err;
+  uint32_t spin;
+};
+
+struct ConvMaps {
+  CUtensorMap x[9];  // the taps of x (forward, wgrad)
+  CUtensorMap w;     // the weights (forward, dgrad)
+  CUtensorMap dz;    // the output gradient (dgrad, wgrad)
+};
+
+template <int BN, int MODE, int G>
+struct ConvShape {
+  // forward: K block of G channels; dgrad: 64 output channels; wgrad: 64 pixels
+  static constexpr int kBK = MODE == kConvFwd ? G : 64;
+  static constexpr int kNB = MODE == kConvFwd ? BN : (BN < 64 ? 64 : BN);  // columns staged of B
+  static constexpr uint32_t kBytesA = 128 * kBK * 2;
+  static constexpr uint32_t kBytesB = kNB * kBK * 2;
+  static constexpr uint32_t kStage = kBytesA + kBytesB;
+  static constexpr int kStages = 196608 / kStage < 8 ? 196608 / kStage : 8;
+  static constexpr size_t kSmem = 1024 + (size_t)kStages * kStage + 256;
+  static constexpr uint32_t kCols = 2 * BN;  // two accumulators (32 .. 512 columns)
+};
+
+struct Item {
+  int x0, y0, b0;  // first pixel of the tile
+  int n0;          // first column
+  int cls;         // dgrad: parity class
+  int kb0, kb1;    // wgrad: pixel blocks of the split
+  int split;
+};
+
+template <int MODE>
+__device__ __forceinline__ Item item_of(const ConvArgs& g, int it, int bn) {
+  Item r;
+  r.cls = 0;
+  r.kb0 = r.kb1 = r.split = 0;
+  if (MODE == kConvWgrad) {
+    // tile of 128 columns of gw innermost: concurrent CTAs share the pixels
+    const int jt = (g.kp + 127) / 128, per = jt * g.tiles_n;
+    r.split = it / per;
+    const int t = it - r.split * per;
+    r.x0 = (t % jt) * 128;  // first column of gw
+    r.n0 = (t / jt) * bn;   // first output channel
+    r.y0 = r.b0 = 0;
+    const int total = g.pt[0].tx * g.pt[0].ty * g.pt[0].tb;
+    r.kb0 = r.split * g.kb_per_split;
+    r.kb1 = min(total, r.kb0 + g.kb_per_split);
+    return r;
+  }
+  if (MODE == kConvDgrad) {
+    while (r.cls + 1 < g.classes && it >= g.first[r.cls + 1]) ++r.cls;
+    it -= g.first[r.cls];
+  }
+  const PixelTiles& p = g.pt[MODE == kConvDgrad ? r.cls : 0];
+  const int m = it / g.tiles_n;
+  r.n0 = (it - m * g.tiles_n) * bn;
+  const int row = m / p.tx;
+  r.x0 = (m - row * p.tx) << p.lw;
+  r.b0 = row / p.ty * p.bb;
+  r.y0 = (row % p.ty) << p.lh;
+  return r;
+}
+
+// dgrad with stride 2: class k covers the pixels of parity (py, px), heaviest
+// class (four taps) first.
+__device__ __forceinline__ int class_py(int cls) { return cls < 2 ? 1 : 0; }
+__device__ __forceinline__ int class_px(int cls) { return (cls & 1) ^ 1; }
+
+template <int BN, int MODE, int G, int EPI>
+__global__ void __launch_bounds__(kConvThreads, 1)
+    conv3x3_kernel(const __grid_constant__ ConvMaps maps, const __grid_constant__ ConvArgs g) {
+  using S = ConvShape<BN, MODE, G>;
+  constexpr int kStages = S::kStages;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  uint64_t* full = (uint64_t*)(smem + (size_t)kStages * S::kStage);
+  uint64_t* empty = full + kStages;
+  uint64_t* acc_full = empty + kStages;
+  uint64_t* acc_empty = acc_full + 2;
+  uint64_t* drained = acc_empty + 2;
+  uint32_t* tmem_slot = (uint32_t*)(drained + 1);
+  __shared__ int failed;
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int items = g.first[g.classes];
+
+  if (threadIdx.x == 0) {
+    failed = 0;
+    for (int s = 0; s < kStages; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    for (int a = 0; a < 2; ++a) {
+      mbar_init(&acc_full[a], 1);
+      mbar_init(&acc_empty[a], 4);
+    }
+    mbar_init(drained, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     smem_u32(tmem_slot)),
+                 "r"(S::kCols));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tmem_slot;
+
+  // K blocks of a work item
+  auto blocks_of = [&](const Item& t) {
+    if (MODE == kConvFwd) return 9 * (g.C / G);
+    if (MODE == kConvWgrad) return t.kb1 - t.kb0;
+    const int nb = (g.N + 63) / 64;
+    if (g.stride == 1) return 9 * nb;
+    return (class_py(t.cls) ? 2 : 1) * (class_px(t.cls) ? 2 : 1) * nb;
+  };
+
+  int issued = 0;
+  if (warp == 0 && lane == 0) {
+    bool ok = true;
+    for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
+      const Item t = item_of<MODE>(g, it, BN);
+      const int nkb = blocks_of(t);
+      for (int i = 0; i < nkb; ++i) {
+        const int s = issued % kStages;
+        if (!mbar_wait(&empty[s], ((uint32_t)(issued / kStages) & 1u) ^ 1u, g.spin)) {
+          atomicExch(&failed, 1);
+          ok = false;
+          break;
+        }
+        mbar_expect_tx(&full[s], S::kStage);
+        uint8_t* a = smem + (size_t)s * S::kStage;
+        uint8_t* b = a + S::kBytesA;
+        if (MODE == kConvFwd) {
+          const int cpb = g.C / G, tap = i / cpb, c = (i - tap * cpb) * G;
+          tma_load_4d(a, &maps.x[tap], &full[s], c, t.x0 + g.off_x[tap], t.y0 + g.off_y[tap],
+                      t.b0);
+          tma_load_2d(b, &maps.w, &full[s], tap * g.C + c, t.n0);
+        } else if (MODE == kConvDgrad) {
+          const int nb = (g.N + 63) / 64, k = i / nb, n = (i - k * nb) * 64;
+          int ky, kx, oy, ox;
+          if (g.stride == 1) {
+            ky = k / 3, kx = k - 3 * ky;
+            oy = t.y0 + 1 - ky, ox = t.x0 + 1 - kx;
+          } else {
+            // iy = 2 y + py reads oy = (iy + 1 - ky) / 2: ky = 1 for even rows, 0 and 2 for odd
+            const int py = class_py(t.cls), px = class_px(t.cls);
+            const int iy = px ? k >> 1 : k, ix = px ? k & 1 : 0;
+            ky = py ? 2 * iy : 1, kx = px ? 2 * ix : 1;
+            oy = t.y0 + (py && ky == 0 ? 1 : 0), ox = t.x0 + (px && kx == 0 ? 1 : 0);
+          }
+          tma_load_4d(a, &maps.dz, &full[s], n, ox, oy, t.b0);
+          const int c = (ky * 3 + kx) * g.C + t.n0;
+#pragma unroll
+          for (int j = 0; j < S::kNB / 64; ++j)
+            tma_load_2d(b + j * 8192, &maps.w, &full[s], c + 64 * j, n);
+        } else {
+          const PixelTiles& p = g.pt[0];
+          const int m = t.kb0 + i, row = m / p.tx;
+          const int x0 = (m - row * p.tx) << p.lw, y0 = (row % p.ty) << p.lh,
+                    b0 = row / p.ty * p.bb;
+#pragma unroll
+          for (int j = 0; j < 128 / G; ++j) {
+            // columns past 9C load from past the images: zeros
+            const int col = t.x0 + j * G, tap = min(col / g.C, 8), c = col - tap * g.C;
+            const bool in = col < 9 * g.C;
+            tma_load_4d(a + j * G * 128, &maps.x[tap], &full[s], in ? c : 0,
+                        x0 + g.off_x[tap], y0 + g.off_y[tap], in ? b0 : g.B);
+          }
+#pragma unroll
+          for (int j = 0; j < S::kNB / 64; ++j)
+            tma_load_4d(b + j * 8192, &maps.dz, &full[s], t.n0 + 64 * j, x0, y0, b0);
+        }
+        ++issued;
+      }
+    }
+  } else if (warp == 1 && lane == 0) {
+    constexpr uint32_t idesc =
+        instr_desc_bf16(128, BN, MODE == kConvWgrad, MODE != kConvFwd);
+    bool ok = true;
+    int n = 0, li = 0;
+    for (int it = blockIdx.x; it < items && ok; it += gridDim.x, ++li) {
+      const Item t = item_of<MODE>(g, it, BN);
+      const int nkb = blocks_of(t), acc = li & 1;
+      if (!mbar_wait(&acc_empty[acc], ((uint32_t)(li >> 1) & 1u) ^ 1u, g.spin)) {
+        atomicExch(&failed, 1);
+        break;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      for (int i = 0; i < nkb; ++i, ++n) {
+        const int s = n % kStages;
+        if (!mbar_wait(&full[s], (uint32_t)(n / kStages) & 1u, g.spin)) {
+          atomicExch(&failed, 1);
+          ok = false;
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t a = smem_u32(smem + (size_t)s * S::kStage), b = a + S::kBytesA;
+#pragma unroll
+        for (int kk = 0; kk < S::kBK / 16; ++kk) {
+          // K-major rows of G (64) channels: 16 channels further are 32 bytes.
+          // MN-major: 8-row groups of 128 (64) bytes, 16 rows further two groups,
+          // the next 64 (32) columns a whole K block further.
+          const uint64_t da =
+              MODE == kConvWgrad
+                  ? smem_desc(a + kk * G * 32, G * 128, G * 16, G == 64 ? 2u : 4u)
+                  : smem_desc(a + kk * 32, 16, S::kBK * 16, S::kBK == 64 ? 2u : 4u);
+          const uint64_t db =
+              MODE == kConvFwd ? smem_desc(b + kk * 32, 16, G * 16, G == 64 ? 2u : 4u)
+                               : smem_desc(b + kk * 2048, 8192, 1024, 2u);
+          umma_bf16(tmem + (uint32_t)(acc * BN), da, db, idesc, (i > 0 || kk > 0) ? 1u : 0u);
+        }
+        umma_commit(&empty[s]);
+      }
+      umma_commit(&acc_full[acc]);
+    }
+    umma_commit(drained);
+  } else if (warp >= 2) {
+    const int quad = warp & 3;  // the TMEM lanes this warp may read: 32 quad ..
+    const int row = quad * 32 + lane;
+    int li = 0;
+    for (int it = blockIdx.x; it < items; it += gridDim.x, ++li) {
+      const Item t = item_of<MODE>(g, it, BN);
+      const int acc = li & 1;
+      if (!__all_sync(0xffffffffu,
+                      mbar_wait(&acc_full[acc], (uint32_t)(li >> 1) & 1u, g.spin))) {
+        atomicExch(&failed, 1);
+        break;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint32_t ta = tmem + (uint32_t)(acc * BN) + ((uint32_t)(quad * 32) << 16);
+      bool valid = false;
+      size_t pix = 0;
+      if (MODE != kConvWgrad) {
+        const PixelTiles& p = g.pt[MODE == kConvDgrad ? t.cls : 0];
+        int x = t.x0 + (row & ((1 << p.lw) - 1));
+        int y = t.y0 + ((row >> p.lw) & ((1 << p.lh) - 1));
+        const int b = t.b0 + (row >> (p.lw + p.lh));
+        if (MODE == kConvFwd) {
+          valid = x < g.Wo && y < g.Ho && b < g.B;
+          pix = ((size_t)b * g.Ho + y) * g.Wo + x;
+        } else {
+          if (g.stride == 2) {
+            x = 2 * x + class_px(t.cls);
+            y = 2 * y + class_py(t.cls);
+          }
+          valid = x < g.W && y < g.H && b < g.B;
+          pix = ((size_t)b * g.H + y) * g.W + x;
+        }
+      }
+#pragma unroll 1
+      for (int c0 = 0; c0 < BN; c0 += 32) {
+        uint32_t r[32];
+        tmem_ld32(ta + (uint32_t)c0, r);
+        if (MODE == kConvWgrad) {
+          // rows are columns of gw: the lanes write 128 contiguous bytes
+          const int j = t.x0 + row;
+          float* dst = g.d + ((size_t)t.split * g.N + t.n0 + c0) * g.kp + j;
+          if (j < g.kp) {
+#pragma unroll
+            for (int q = 0; q < 32; ++q)
+              if (t.n0 + c0 + q < g.N) dst[(size_t)q * g.kp] = __uint_as_float(r[q]);
+          }
+        } else if (valid) {
+          const int width = MODE == kConvFwd ? g.N : g.C;  // a multiple of 8
+          const size_t base = pix * width + t.n0 + c0;
+#pragma unroll
+          for (int q = 0; q < 32; q += 8) {
+            if (t.n0 + c0 + q >= width) break;
+            float v[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v[k] = __uint_as_float(r[q + k]);
+            if (MODE == kConvFwd) {
+              const float4* bias = reinterpret_cast<const float4*>(g.bias + t.n0 + c0 + q);
+              const float4 b0 = bias[0], b1 = bias[1];
+              v[0] += b0.x, v[1] += b0.y, v[2] += b0.z, v[3] += b0.w;
+              v[4] += b1.x, v[5] += b1.y, v[6] += b1.z, v[7] += b1.w;
+              if (EPI == kConvF32) {
+                float4* d = reinterpret_cast<float4*>(g.d + base + q);
+                d[0] = make_float4(v[0], v[1], v[2], v[3]);
+                d[1] = make_float4(v[4], v[5], v[6], v[7]);
+              } else {
+                __align__(16) __nv_bfloat162 z2[4], y2[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                  z2[k] = __floats2bfloat162_rn(v[2 * k], v[2 * k + 1]);
+                  y2[k] = __floats2bfloat162_rn(gelu(v[2 * k]), gelu(v[2 * k + 1]));
+                }
+                *reinterpret_cast<uint4*>(g.z + base + q) = *reinterpret_cast<uint4*>(z2);
+                *reinterpret_cast<uint4*>(g.y + base + q) = *reinterpret_cast<uint4*>(y2);
+              }
+            } else {
+              if (g.zprev) {
+                __align__(16) __nv_bfloat162 z2[4];
+                *reinterpret_cast<uint4*>(z2) =
+                    *reinterpret_cast<const uint4*>(g.zprev + base + q);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                  const float2 zf = __bfloat1622float2(z2[k]);
+                  v[2 * k] *= gelu_grad(zf.x);
+                  v[2 * k + 1] *= gelu_grad(zf.y);
+                }
+              }
+              __align__(16) __nv_bfloat162 y2[4];
+#pragma unroll
+              for (int k = 0; k < 4; ++k) y2[k] = __floats2bfloat162_rn(v[2 * k], v[2 * k + 1]);
+              *reinterpret_cast<uint4*>(g.y + base + q) = *reinterpret_cast<uint4*>(y2);
+            }
+          }
+        }
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0)
+        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[acc]))
+                     : "memory");
+    }
+  }
+  __syncwarp();
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (failed) {
+    // Drain before freeing TMEM and shared memory: the copies still in flight
+    // (at most the last kStages issued: a stage is reused only once its copy
+    // has landed and been consumed) and every MMA, committed to `drained`.
+    if (warp == 0 && lane == 0) {
+      for (int i = max(0, issued - kStages); i < issued; ++i)
+        mbar_wait(&full[i % kStages], (uint32_t)(i / kStages) & 1u, kSpinLimit);
+      mbar_wait(drained, 0, kSpinLimit);
+      atomicOr(g.err, 1u);
+    }
+    __syncthreads();
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
+                 "r"(S::kCols));
+  }
+}
+
+// gw = sum of the split partials in split order, four values per thread, eight
+// partials in flight.
+__global__ void __launch_bounds__(256)
+    conv_reduce_kernel(const float4* __restrict__ p, float4* __restrict__ out, int n4,
+                       int splits) {
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i >= n4) return;
+  float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+  for (int k = 0; k < splits; ++k) {
+    const float4 v = p[(size_t)k * n4 + i];
+    s.x += v.x, s.y += v.y, s.z += v.z, s.w += v.w;
+  }
+  out[i] = s;
+}
+
+// ---- host side ----------------------------------------------------------------
+
+// The rectangle of `pixels` (a power of two) pixels over B images of W x H that
+// needs the fewest tiles; among equals the widest.
+PixelTiles pick_tiles(int pixels, int W, int H, int B) {
+  PixelTiles best{};
+  int64_t fewest = INT64_MAX;
+  int total = 0;
+  while ((1 << total) < pixels) ++total;
+  for (int lw = total; lw >= 0; --lw)
+    for (int lh = total - lw; lh >= 0; --lh) {
+      const int bw = 1 << lw, bh = 1 << lh, bb = pixels >> (lw + lh);
+      PixelTiles p{lw, lh, bb, (W + bw - 1) / bw, (H + bh - 1) / bh, (B + bb - 1) / bb};
+      const int64_t n = (int64_t)p.tx * p.ty * p.tb;
+      if (n < fewest) {
+        fewest = n;
+        best = p;
+      }
+    }
+  return best;
+}
+
+int64_t count_of(const PixelTiles& p) { return (int64_t)p.tx * p.ty * p.tb; }
+
+int encode(CUtensorMap* map, int rank, const void* base, const cuuint64_t* dims,
+           const cuuint64_t* strides, const cuuint32_t* box, CUtensorMapSwizzle swizzle) {
+  EncodeFn fn = encode_fn();
+  if (!fn) return DS_ERR_CUDA;
+  const cuuint32_t one[4] = {1, 1, 1, 1};
+  const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank,
+                        const_cast<void*>(base), dims, strides, box, one,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? DS_OK : DS_ERR_ARG;
+}
+
+// Box of `group` channels over a rectangle of pixels of an NHWC view.
+int map_pixels(CUtensorMap* map, const __nv_bfloat16* base, int C, int W, int H, int B,
+               int64_t sx, int64_t sy, int64_t sb, int group, const PixelTiles& p) {
+  const cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)B};
+  const cuuint64_t strides[3] = {(cuuint64_t)sx * 2, (cuuint64_t)sy * 2, (cuuint64_t)sb * 2};
+  const cuuint32_t box[4] = {(cuuint32_t)group, 1u << p.lw, 1u << p.lh, (cuuint32_t)p.bb};
+  return encode(map, 4, base, dims, strides, box,
+                group == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B);
+}
+
+// The nine taps of x in output-pixel coordinates (see the file's head).
+int map_taps(ConvMaps& maps, ConvArgs& g, const __nv_bfloat16* x, int group,
+             const PixelTiles& p) {
+  const int s = g.stride;
+  for (int tap = 0; tap < 9; ++tap) {
+    const int ky = tap / 3, kx = tap - 3 * ky;
+    // output rows whose input row oy s - 1 + ky lies inside: [oy0, oy1)
+    const int oy0 = ky == 0 ? 1 : 0, ox0 = kx == 0 ? 1 : 0;
+    const int oy1 = std::min(g.Ho, (g.H - ky) / s + 1), ox1 = std::min(g.Wo, (g.W - kx) / s + 1);
+    const bool none = oy1 <= oy0 || ox1 <= ox0 || g.H < ky || g.W < kx;
+    const int iy = oy0 * s - 1 + ky, ix = ox0 * s - 1 + kx;
+    const __nv_bfloat16* base = none ? x : x + ((int64_t)iy * g.W + ix) * g.C;
+    // a tap that reads nothing gets coordinates outside of a one-pixel map
+    g.off_x[tap] = none ? 1 << 24 : -ox0;
+    g.off_y[tap] = none ? 1 << 24 : -oy0;
+    DS_TRY(map_pixels(&maps.x[tap], base, g.C, none ? 1 : ox1 - ox0, none ? 1 : oy1 - oy0, g.B,
+                      (int64_t)s * g.C, (int64_t)s * g.W * g.C, (int64_t)g.H * g.W * g.C, group,
+                      p));
+  }
+  return DS_OK;
+}
+
+int map_matrix(CUtensorMap* map, const void* base, int rows, int cols, int ld, int box_cols,
+               int box_rows) {
+  const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+  const cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
+  const cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
+  return encode(map, 2, base, dims, strides, box,
+                box_cols == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B);
+}
+
+int sm_count() {
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) == cudaSuccess)
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
+}
+
+template <int BN, int MODE, int G, int EPI>
+int launch_conv(const ConvMaps& maps, const ConvArgs& g, cudaStream_t s) {
+  using S = ConvShape<BN, MODE, G>;
+  static std::once_flag once;
+  static cudaError_t attr = cudaSuccess;
+  std::call_once(once, [] {
+    attr = cudaFuncSetAttribute(conv3x3_kernel<BN, MODE, G, EPI>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::kSmem);
+  });
+  DS_CUDA(attr);
+  const int grid = std::min(g.first[g.classes], sm_count());
+  conv3x3_kernel<BN, MODE, G, EPI><<<grid, kConvThreads, S::kSmem, s>>>(maps, g);
+  return cuda_status(cudaGetLastError());
+}
+
+template <int MODE, int G, int EPI>
+int dispatch_bn(int bn, const ConvMaps& maps, const ConvArgs& g, cudaStream_t s) {
+  switch (bn) {
+    case 32: return launch_conv<32, MODE, G, EPI>(maps, g, s);
+    case 64: return launch_conv<64, MODE, G, EPI>(maps, g, s);
+    case 128: return launch_conv<128, MODE, G, EPI>(maps, g, s);
+    default: return launch_conv<256, MODE, G, EPI>(maps, g, s);
+  }
+}
+
+// Tile width for n columns over `tiles` row tiles: the widest that n fills,
+// narrowed while SMs would stay idle.
+int pick_bn(int n, int64_t tiles, int least = 32) {
+  int bn = n <= 32 ? 32 : n <= 64 ? 64 : n <= 128 ? 128 : 256;
+  bn = std::max(bn, least);
+  while (bn > 64 && tiles * ((n + bn - 1) / bn) < sm_count()) bn /= 2;
+  return bn;
+}
+
+bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
+
+// Shapes and addresses the tensor maps and the vector accesses take.
+bool conv_ok(int B, int H, int W, int C, int N, int stride, int kp) {
+  if (B <= 0 || H <= 0 || W <= 0 || N <= 0 || (stride != 1 && stride != 2)) return false;
+  if (!(C == 32 || (C > 0 && C % 64 == 0)) || N % 8 != 0) return false;
+  if (kp < 9 * C || kp % 8 != 0) return false;
+  // items and pixel tiles are counted in 32 bits
+  return (int64_t)B * H * W < ((int64_t)1 << 30) && C <= (1 << 16) && N <= (1 << 16);
+}
+
+ConvArgs base_args(int B, int H, int W, int C, int N, int stride, int kp, uint32_t* err) {
+  ConvArgs g{};
+  g.B = B, g.H = H, g.W = W, g.C = C, g.N = N, g.stride = stride, g.kp = kp;
+  g.Ho = (H - 1) / stride + 1, g.Wo = (W - 1) / stride + 1;
+  g.classes = 1;
+  g.err = err;
+  g.spin = gemm_spin_limit();
+  return g;
+}
+
+// Splits of the weight gradient: chains of at most kWgradChain pixels, and
+// enough splits that every SM gets a tile.
+void pick_splits(ConvArgs& g, int64_t blocks, int tiles) {
+  int64_t per = kWgradChain / kWgradPixels;
+  const int64_t want = (sm_count() + tiles - 1) / tiles;
+  per = std::min(per, std::max<int64_t>(4, (blocks + want - 1) / want));
+  // the partials stay within 512 of them
+  per = std::max(per, (blocks + 511) / 512);
+  g.kb_per_split = (int)per;
+  g.splits = (int)((blocks + per - 1) / per);
+}
+
+int wgrad_plan(ConvArgs& g, int& bn) {
+  g.pt[0] = pick_tiles(kWgradPixels, g.Wo, g.Ho, g.B);
+  const int jt = (g.kp + 127) / 128;
+  bn = g.N <= 32 ? 32 : g.N <= 64 ? 64 : g.N <= 128 ? 128 : 256;
+  g.tiles_n = (g.N + bn - 1) / bn;
+  const int64_t blocks = count_of(g.pt[0]);
+  if (blocks > INT32_MAX / 2) return DS_ERR_ARG;
+  pick_splits(g, blocks, jt * g.tiles_n);
+  g.first[1] = jt * g.tiles_n * g.splits;
+  return DS_OK;
+}
+
+}  // namespace
+}  // namespace ds
+
+extern "C" {
+
+int ds_conv3x3_forward(const void* x, int B, int H, int W, int C, int stride, const void* w,
+                       int Kp, int N, const float* bias, void* z, void* y, float* d,
+                       uint32_t* err, ds_stream stream) {
+  using namespace ds;
+  if (!x || !w || !bias || !err || (!d && (!z || !y))) return DS_ERR_ARG;
+  if (!conv_ok(B, H, W, C, N, stride, Kp)) return DS_ERR_ARG;
+  if (!aligned16(x) || !aligned16(w) || !aligned16(bias) || !aligned16(z) || !aligned16(y) ||
+      !aligned16(d))
+    return DS_ERR_ARG;
+  ConvArgs g = base_args(B, H, W, C, N, stride, Kp, err);
+  const int G = C == 32 ? 32 : 64;
+  g.pt[0] = pick_tiles(128, g.Wo, g.Ho, B);
+  const int64_t tiles = count_of(g.pt[0]);
+  const int bn = pick_bn(N, tiles);
+  g.tiles_n = (N + bn - 1) / bn;
+  if (tiles * g.tiles_n > INT32_MAX) return DS_ERR_ARG;
+  g.first[1] = (int)(tiles * g.tiles_n);
+  g.bias = bias;
+  g.z = (__nv_bfloat16*)z;
+  g.y = (__nv_bfloat16*)y;
+  g.d = d;
+  ConvMaps maps;
+  DS_TRY(map_taps(maps, g, (const __nv_bfloat16*)x, G, g.pt[0]));
+  DS_TRY(map_matrix(&maps.w, w, N, Kp, Kp, G, bn));
+  maps.dz = maps.w;  // not read
+  cudaStream_t s = (cudaStream_t)stream;
+  if (G == 32)
+    return d ? dispatch_bn<kConvFwd, 32, kConvF32>(bn, maps, g, s)
+             : dispatch_bn<kConvFwd, 32, kConvGelu>(bn, maps, g, s);
+  return d ? dispatch_bn<kConvFwd, 64, kConvF32>(bn, maps, g, s)
+           : dispatch_bn<kConvFwd, 64, kConvGelu>(bn, maps, g, s);
+}
+
+int ds_conv3x3_dgrad(const void* dz, int B, int H, int W, int C, int stride, const void* w,
+                     int Kp, int N, const void* zprev, void* dx, uint32_t* err,
+                     ds_stream stream) {
+  using namespace ds;
+  if (!dz || !w || !dx || !err) return DS_ERR_ARG;
+  if (!conv_ok(B, H, W, C, N, stride, Kp)) return DS_ERR_ARG;
+  if (!aligned16(dz) || !aligned16(w) || !aligned16(zprev) || !aligned16(dx)) return DS_ERR_ARG;
+  ConvArgs g = base_args(B, H, W, C, N, stride, Kp, err);
+  g.zprev = (const __nv_bfloat16*)zprev;
+  g.y = (__nv_bfloat16*)dx;
+  int64_t tiles = 0;
+  // All classes use one rectangle (the box of the dz map), picked for the
+  // largest class: the even rows and columns.
+  const int Wc = (W + stride - 1) / stride, Hc = (H + stride - 1) / stride;
+  const PixelTiles p = pick_tiles(128, Wc, Hc, B);
+  const int bn = pick_bn(C, count_of(p) * stride * stride);
+  g.tiles_n = (C + bn - 1) / bn;
+  g.classes = stride * stride;
+  for (int k = 0; k < g.classes; ++k) {
+    const int py = stride == 2 ? (k < 2 ? 1 : 0) : 0, px = stride == 2 ? (k & 1) ^ 1 : 0;
+    const int wk = (W - px + stride - 1) / stride, hk = (H - py + stride - 1) / stride;
+    g.pt[k] = p;
+    g.pt[k].tx = (wk + (1 << p.lw) - 1) >> p.lw;
+    g.pt[k].ty = (hk + (1 << p.lh) - 1) >> p.lh;
+    g.first[k] = (int)tiles;
+    tiles += count_of(g.pt[k]) * g.tiles_n;
+  }
+  if (tiles > INT32_MAX) return DS_ERR_ARG;
+  g.first[g.classes] = (int)tiles;
+  ConvMaps maps;
+  DS_TRY(map_pixels(&maps.dz, (const __nv_bfloat16*)dz, N, g.Wo, g.Ho, B, N, (int64_t)g.Wo * N,
+                    (int64_t)g.Ho * g.Wo * N, 64, p));
+  DS_TRY(map_matrix(&maps.w, w, N, Kp, Kp, 64, 64));
+  for (int t = 0; t < 9; ++t) maps.x[t] = maps.dz;  // not read
+  return dispatch_bn<kConvDgrad, 64, 0>(bn, maps, g, (cudaStream_t)stream);
+}
+
+int64_t ds_conv3x3_wgrad_workspace(int B, int H, int W, int C, int stride, int Kp, int N) {
+  using namespace ds;
+  if (!conv_ok(B, H, W, C, N, stride, Kp)) return -1;
+  ConvArgs g = base_args(B, H, W, C, N, stride, Kp, nullptr);
+  int bn;
+  if (wgrad_plan(g, bn) != DS_OK) return -1;
+  return g.splits > 1 ? (int64_t)g.splits * N * Kp : 0;
+}
+
+int ds_conv3x3_wgrad(const void* x, const void* dz, int B, int H, int W, int C, int stride,
+                     int Kp, int N, float* gw, float* workspace, uint32_t* err,
+                     ds_stream stream) {
+  using namespace ds;
+  if (!x || !dz || !gw || !err) return DS_ERR_ARG;
+  if (!conv_ok(B, H, W, C, N, stride, Kp)) return DS_ERR_ARG;
+  if (!aligned16(x) || !aligned16(dz) || !aligned16(gw) || !aligned16(workspace))
+    return DS_ERR_ARG;
+  ConvArgs g = base_args(B, H, W, C, N, stride, Kp, err);
+  // like the GEMM over pixels that this replaces: its rows are 16-byte aligned
+  if (((int64_t)B * g.Ho * g.Wo) % 8 != 0) return DS_ERR_ARG;
+  int bn;
+  DS_TRY(wgrad_plan(g, bn));
+  if (g.splits > 1 && !workspace) return DS_ERR_ARG;
+  g.d = g.splits > 1 ? workspace : gw;
+  const int G = C == 32 ? 32 : 64;
+  ConvMaps maps;
+  DS_TRY(map_taps(maps, g, (const __nv_bfloat16*)x, G, g.pt[0]));
+  DS_TRY(map_pixels(&maps.dz, (const __nv_bfloat16*)dz, N, g.Wo, g.Ho, B, N, (int64_t)g.Wo * N,
+                    (int64_t)g.Ho * g.Wo * N, 64, g.pt[0]));
+  maps.w = maps.dz;  // not read
+  cudaStream_t s = (cudaStream_t)stream;
+  if (G == 32) DS_TRY((dispatch_bn<kConvWgrad, 32, 0>(bn, maps, g, s)));
+  else DS_TRY((dispatch_bn<kConvWgrad, 64, 0>(bn, maps, g, s)));
+  if (g.splits > 1) {
+    const int64_t n4 = (int64_t)N * Kp / 4;
+    if (n4 > INT32_MAX) return DS_ERR_ARG;
+    conv_reduce_kernel<<<(unsigned)((n4 + 255) / 256), 256, 0, s>>>(
+        (const float4*)workspace, (float4*)gw, (int)n4, g.splits);
+    DS_CUDA(cudaGetLastError());
+  }
+  return DS_OK;
+}
+
+}  // extern "C"

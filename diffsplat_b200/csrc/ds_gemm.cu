@@ -29,12 +29,12 @@
 
 #include "ds_common.cuh"
 #include "ds_internal.h"
+#include "ds_umma.cuh"
 
 namespace ds {
 namespace {
 
 constexpr int kBM = 128, kBK = 64, kStages = 4, kGemmThreads = 128;
-constexpr uint32_t kSpinLimit = 1u << 24;  // default pipeline limit and the drain's limit
 uint32_t g_spin_limit = kSpinLimit;
 
 enum Epilogue : int { kEpiF32 = 0, kEpiBiasGeluBf16 = 1, kEpiBiasF32 = 2 };
@@ -51,110 +51,6 @@ struct GemmArgs {
   uint32_t* err;      // set non-zero when a wait times out
   uint32_t spin;      // polls per pipeline wait
 };
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
-
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
-}
-
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)),
-               "r"(bytes)
-               : "memory");
-}
-
-// Bounded wait for the phase with the given parity; false on timeout.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
-                                          uint32_t limit = kSpinLimit) {
-  const uint32_t a = smem_u32(bar);
-  for (uint32_t it = 0; it < limit; ++it) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(a), "r"(parity)
-        : "memory");
-    if (ok) return true;
-  }
-  return false;
-}
-
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, uint64_t* bar,
-                                            int x, int y) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, "
-      "{%3, %4}], [%2];" ::"r"(smem_u32(dst)),
-      "l"((uint64_t)map), "r"(smem_u32(bar)), "r"(x), "r"(y)
-      : "memory");
-}
-
-// K-major operand tile in shared memory, 128-byte swizzle: rows of 64 BF16
-// (128 B), 8-row groups 1024 B apart.
-__device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t addr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((addr >> 4) & 0x3FFFu);        // start address
-  d |= (uint64_t)1u << 16;                        // leading byte offset (16 B, unused)
-  d |= (uint64_t)(1024u >> 4) << 32;              // stride byte offset
-  d |= (uint64_t)1u << 46;                        // descriptor version (sm_100)
-  d |= (uint64_t)2u << 61;                        // 128-byte swizzle
-  return d;
-}
-
-// kind::f16 instruction descriptor: BF16 A and B, FP32 D, both K-major.
-__host__ __device__ constexpr uint32_t instr_desc_bf16(int m, int n) {
-  return (1u << 4)                     // D format F32
-         | (1u << 7)                   // A format BF16
-         | (1u << 10)                  // B format BF16
-         | ((uint32_t)(n >> 3) << 17)  // N
-         | ((uint32_t)(m >> 4) << 24); // M
-}
-
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc,
-                                          uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-      "l"(da), "l"(db), "r"(idesc), "r"(accumulate));
-}
-
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                   smem_u32(bar))
-               : "memory");
-}
-
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, "
-      "%12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, "
-      "%30, %31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-        "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]),
-        "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]),
-        "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
-// GELU with the tanh form: 0.5 x (1 + tanh(sqrt(2/pi) (x + 0.044715 x^3))).
-__device__ __forceinline__ float gelu(float x) {
-  const float u = 0.7978845608f * (x + 0.044715f * x * x * x);
-  return 0.5f * x * (1.f + tanhf(u));
-}
-
-__device__ __forceinline__ float gelu_grad(float x) {
-  const float u = 0.7978845608f * (x + 0.044715f * x * x * x);
-  const float t = tanhf(u);
-  const float du = 0.7978845608f * (1.f + 3.f * 0.044715f * x * x);
-  return 0.5f * (1.f + t) + 0.5f * x * (1.f - t * t) * du;
-}
 
 template <int BN, int EPI>
 __global__ void __launch_bounds__(kGemmThreads, 1)
@@ -318,25 +214,6 @@ __global__ void gemm_reduce_splits(const float* __restrict__ P, float* __restric
     for (int k = 0; k < splits; ++k) s += P[((int64_t)k * M + r) * ldd + c];
     D[r * ldd + c] = s;
   }
-}
-
-using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
-                              const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                              const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                              CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeFn encode_fn() {
-  static EncodeFn fn = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) ==
-            cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = (EncodeFn)p;
-  });
-  return fn;
 }
 
 // 2-D BF16 tensor map of a row-major [rows][cols] matrix with leading dimension
@@ -569,6 +446,10 @@ unsigned grid_for(int64_t n) {
 }
 
 }  // namespace
+}  // namespace ds
+
+namespace ds {
+uint32_t gemm_spin_limit() { return g_spin_limit; }
 }  // namespace ds
 
 extern "C" {

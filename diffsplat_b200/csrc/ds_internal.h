@@ -341,6 +341,9 @@ int raster_reduce_grads(RasterBuffers& rb, const ds_splat2d& gin, int n, cudaStr
 // itself from grad_segments(rb).
 int raster_reduce_long_grads(RasterBuffers& rb, int n, cudaStream_t s);
 
+// Polls per pipeline wait of the tensor-core kernels (ds_gemm_set_spin_limit).
+uint32_t gemm_spin_limit();
+
 // Losses and Adam (ds_loss_adam.cu)
 int launch_mse_forward(const float* px, const float* tgt, int64_t npix, float* loss,
                        float* partials, uint32_t* ticket, cudaStream_t s);

@@ -74,9 +74,9 @@ class Initializer:
         x = nn.cast_bf16(images)
         self.zs = []
         for layer in self.layers:
-            z, x = layer.forward(self.gemm, x)
+            z, x = layer.forward(self.gemm, x, keep=True)  # x stays as it is
             self.zs.append(z)
-        out, _ = self.head.forward(self.gemm, x)
+        out, _ = self.head.forward(self.gemm, x, keep=True)
         self.batch = images.shape[0]
         return out.reshape(-1, 56)
 

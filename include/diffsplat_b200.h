@@ -396,6 +396,25 @@ int ds_im2col_bf16(const void *x, int B, int H, int W, int C, int stride, int Kp
                    ds_stream stream);
 int ds_col2im_bf16(const float *dcol, int B, int H, int W, int C, int stride, int Kp,
                    const void *z, void *dx, ds_stream stream);
+/* The same convolution without the im2col matrix (implicit GEMM on tcgen05):
+ * C == 32 or a multiple of 64, N (output channels) a multiple of 8, all
+ * pointers 16-byte aligned, else DS_ERR_ARG.  w is BF16 [N][Kp] in im2col
+ * order.  Forward: z = BF16(conv + bias) and y = BF16(gelu(conv + bias))
+ * [B*Ho*Wo][N], or FP32 d = conv + bias when d is given; equal to im2col +
+ * ds_gemm_bf16_tn bit for bit.  dgrad: dx [B][H][W][C] BF16, times gelu'(zprev)
+ * when given.  wgrad: gw [N][Kp] FP32 (B*Ho*Wo a multiple of 8); workspace holds
+ * the floats that ds_conv3x3_wgrad_workspace returns (0: none; negative: a
+ * shape it does not take).  *err as for ds_gemm_bf16_tn. */
+int ds_conv3x3_forward(const void *x, int B, int H, int W, int C, int stride, const void *w,
+                       int Kp, int N, const float *bias, void *z, void *y, float *d,
+                       uint32_t *err, ds_stream stream);
+int ds_conv3x3_dgrad(const void *dz, int B, int H, int W, int C, int stride, const void *w,
+                     int Kp, int N, const void *zprev, void *dx, uint32_t *err,
+                     ds_stream stream);
+int64_t ds_conv3x3_wgrad_workspace(int B, int H, int W, int C, int stride, int Kp, int N);
+int ds_conv3x3_wgrad(const void *x, const void *dz, int B, int H, int W, int C, int stride,
+                     int Kp, int N, float *gw, float *workspace, uint32_t *err,
+                     ds_stream stream);
 int ds_transpose_bf16(const void *in, int rows, int cols, void *out, ds_stream stream);
 /* out[c] = sum_m a[m][c]; workspace holds max_parts * C floats. */
 int ds_colsum_bf16(const void *a, int64_t M, int C, float *workspace, int max_parts, float *out,

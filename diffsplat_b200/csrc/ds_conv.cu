@@ -22,6 +22,9 @@
 // in wgrad) MN-major, so nothing is transposed.  The K order of the forward is
 // that of the im2col matrix, hence its results too, bit for bit.
 //
+// An RGB input (the first layer) has rows of 27 products, too short and too
+// unaligned for TMA: conv3x3_rgb_kernel gathers them into shared memory itself.
+//
 // Every mbarrier wait is bounded as in ds_gemm.cu: on a timeout the CTA sets the
 // error word, lets what it issued land, frees its TMEM and returns.
 #include <algorithm>
@@ -127,6 +130,26 @@ __device__ __forceinline__ Item item_of(const ConvArgs& g, int it, int bn) {
   r.b0 = row / p.ty * p.bb;
   r.y0 = (row % p.ty) << p.lh;
   return r;
+}
+
+// Eight neighbouring outputs of the forward (bias added): FP32, or z and gelu(z).
+template <int EPI>
+__device__ __forceinline__ void store_outputs(float* d, __nv_bfloat16* z, __nv_bfloat16* y,
+                                              size_t at, const float (&v)[8]) {
+  if (EPI == kConvF32) {
+    float4* o = reinterpret_cast<float4*>(d + at);
+    o[0] = make_float4(v[0], v[1], v[2], v[3]);
+    o[1] = make_float4(v[4], v[5], v[6], v[7]);
+  } else {
+    __align__(16) __nv_bfloat162 z2[4], y2[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      z2[k] = __floats2bfloat162_rn(v[2 * k], v[2 * k + 1]);
+      y2[k] = __floats2bfloat162_rn(gelu(v[2 * k]), gelu(v[2 * k + 1]));
+    }
+    *reinterpret_cast<uint4*>(z + at) = *reinterpret_cast<uint4*>(z2);
+    *reinterpret_cast<uint4*>(y + at) = *reinterpret_cast<uint4*>(y2);
+  }
 }
 
 // dgrad with stride 2: class k covers the pixels of parity (py, px), heaviest
@@ -345,20 +368,7 @@ __global__ void __launch_bounds__(kConvThreads, 1)
               const float4 b0 = bias[0], b1 = bias[1];
               v[0] += b0.x, v[1] += b0.y, v[2] += b0.z, v[3] += b0.w;
               v[4] += b1.x, v[5] += b1.y, v[6] += b1.z, v[7] += b1.w;
-              if (EPI == kConvF32) {
-                float4* d = reinterpret_cast<float4*>(g.d + base + q);
-                d[0] = make_float4(v[0], v[1], v[2], v[3]);
-                d[1] = make_float4(v[4], v[5], v[6], v[7]);
-              } else {
-                __align__(16) __nv_bfloat162 z2[4], y2[4];
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                  z2[k] = __floats2bfloat162_rn(v[2 * k], v[2 * k + 1]);
-                  y2[k] = __floats2bfloat162_rn(gelu(v[2 * k]), gelu(v[2 * k + 1]));
-                }
-                *reinterpret_cast<uint4*>(g.z + base + q) = *reinterpret_cast<uint4*>(z2);
-                *reinterpret_cast<uint4*>(g.y + base + q) = *reinterpret_cast<uint4*>(y2);
-              }
+              store_outputs<EPI>(g.d, g.z, g.y, base + q, v);
             } else {
               if (g.zprev) {
                 __align__(16) __nv_bfloat162 z2[4];
@@ -405,6 +415,153 @@ __global__ void __launch_bounds__(kConvThreads, 1)
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
                  "r"(S::kCols));
+  }
+}
+
+// First layer, three input channels: out = x * w + bias with the 27 products of a
+// pixel padded to one K block of 32.  Each thread gathers its pixel's row (nine
+// taps of three channels) into the swizzled A tile, two tcgen05.mma make the
+// 128 x BN tile, and the same threads write z and gelu(z).  Bound by the output
+// (2 x 2 BN bytes a pixel): an im2col matrix of 64 columns would move 128 bytes
+// a pixel twice more.  Many small CTAs per SM (8 of 128 threads at BN = 32)
+// overlap one another's gather, MMA and epilogue, so no warp is specialised.
+// The initializer's forward on 16 images of 512 x 512 went from 2.92 ms with
+// im2col + GEMM in this layer to 0.81 ms (B200).
+constexpr int kRgbThreads = 128;
+
+struct RgbArgs {
+  const __nv_bfloat16 *x, *w;
+  int B, H, W, Ho, Wo, N, stride, kp;
+  uint32_t pixels;
+  const float* bias;
+  __nv_bfloat16 *z, *y;
+  float* d;
+  uint32_t* err;
+  uint32_t spin;
+};
+
+template <int BN, int EPI>
+__global__ void __launch_bounds__(kRgbThreads) conv3x3_rgb_kernel(const RgbArgs g) {
+  constexpr int kK = 32;  // 27 products and five zeros
+  __shared__ __align__(1024) uint8_t sA[128 * kK * 2];
+  __shared__ __align__(1024) uint8_t sB[BN * kK * 2];
+  __shared__ uint64_t done;
+  __shared__ uint32_t tmem_slot;
+  __shared__ __align__(16) float sBias[BN];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int n0 = blockIdx.y * BN;
+  if (threadIdx.x == 0) {
+    mbar_init(&done, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     smem_u32(&tmem_slot)),
+                 "r"((uint32_t)BN));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  // rows of 32 BF16 (64 B), 64-byte swizzle: 16-byte chunk q of row r at q ^ (r >> 1 & 3)
+  auto chunk = [](uint8_t* tile, int r, int q) {
+    return reinterpret_cast<uint4*>(tile + r * 64 + ((q ^ ((r >> 1) & 3)) << 4));
+  };
+  auto pack = [](uint32_t lo, uint32_t hi) { return lo | (hi << 16); };
+  for (int r = threadIdx.x; r < BN; r += kRgbThreads) {
+    uint32_t v[kK];
+    const unsigned short* w = reinterpret_cast<const unsigned short*>(g.w) +
+                              (size_t)min(n0 + r, g.N - 1) * g.kp;
+#pragma unroll
+    for (int k = 0; k < kK; ++k) v[k] = n0 + r < g.N && k < 27 ? w[k] : 0u;
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      *chunk(sB, r, q) = make_uint4(pack(v[8 * q], v[8 * q + 1]), pack(v[8 * q + 2], v[8 * q + 3]),
+                                    pack(v[8 * q + 4], v[8 * q + 5]),
+                                    pack(v[8 * q + 6], v[8 * q + 7]));
+    sBias[r] = n0 + r < g.N ? g.bias[n0 + r] : 0.f;
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = tmem_slot;
+  const uint32_t tiles = (g.pixels + 127) / 128;
+  const unsigned short* x = reinterpret_cast<const unsigned short*>(g.x);
+  uint32_t phase = 0;
+  bool ok = true;
+  for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x) {
+    const uint32_t m = t * 128 + threadIdx.x;
+    uint32_t v[kK];
+#pragma unroll
+    for (int k = 0; k < kK; ++k) v[k] = 0u;
+    if (m < g.pixels) {
+      const uint32_t row = m / (uint32_t)g.Wo;
+      const int ox = (int)(m - row * (uint32_t)g.Wo);
+      const uint32_t b = row / (uint32_t)g.Ho;
+      const int oy = (int)(row - b * (uint32_t)g.Ho);
+      const int iy0 = oy * g.stride - 1, ix0 = ox * g.stride - 1;
+#pragma unroll
+      for (int ky = 0; ky < 3; ++ky) {
+        const int iy = iy0 + ky;
+        const unsigned short* line = x + (((int64_t)b * g.H + iy) * g.W + ix0) * 3;
+#pragma unroll
+        for (int kx = 0; kx < 3; ++kx)
+          if (iy >= 0 && iy < g.H && ix0 + kx >= 0 && ix0 + kx < g.W) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) v[(ky * 3 + kx) * 3 + c] = line[kx * 3 + c];
+          }
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      *chunk(sA, threadIdx.x, q) =
+          make_uint4(pack(v[8 * q], v[8 * q + 1]), pack(v[8 * q + 2], v[8 * q + 3]),
+                     pack(v[8 * q + 4], v[8 * q + 5]), pack(v[8 * q + 6], v[8 * q + 7]));
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+      for (int kk = 0; kk < kK / 16; ++kk)
+        umma_bf16(tmem, smem_desc(smem_u32(sA) + kk * 32, 16, 512, 4u),
+                  smem_desc(smem_u32(sB) + kk * 32, 16, 512, 4u), instr_desc_bf16(128, BN),
+                  kk > 0 ? 1u : 0u);
+      umma_commit(&done);
+    }
+    __syncwarp();
+    // Every thread polls to the same limit; a timeout is voted on, so that the
+    // whole CTA leaves together.
+    ok = mbar_wait(&done, phase, g.spin);
+    ok = __syncthreads_and(ok);
+    if (!ok) break;
+    phase ^= 1u;
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll 1
+    for (int c0 = 0; c0 < BN; c0 += 32) {
+      uint32_t r[32];
+      tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, r);
+      if (m < g.pixels) {
+        const size_t base = (size_t)m * g.N + n0 + c0;
+#pragma unroll
+        for (int q = 0; q < 32; q += 8) {
+          if (n0 + c0 + q >= g.N) break;
+          float f[8];
+#pragma unroll
+          for (int k = 0; k < 8; ++k) f[k] = __uint_as_float(r[q + k]) + sBias[c0 + q + k];
+          store_outputs<EPI>(g.d, g.z, g.y, base + q, f);
+        }
+      }
+    }
+    // the accumulator and the A tile are free again once every thread has read
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+  }
+  if (!ok && threadIdx.x == 0) {
+    mbar_wait(&done, phase, kSpinLimit);  // the MMAs land before TMEM is freed
+    atomicOr(g.err, 1u);
+  }
+  __syncthreads();
+  if (warp == 0) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
+                 "r"((uint32_t)BN));
   }
 }
 
@@ -553,6 +710,16 @@ bool conv_ok(int B, int H, int W, int C, int N, int stride, int kp) {
   return (int64_t)B * H * W < ((int64_t)1 << 30) && C <= (1 << 16) && N <= (1 << 16);
 }
 
+template <int BN, int EPI>
+int launch_rgb(const RgbArgs& g, cudaStream_t s) {
+  // TMEM holds 512 / BN accumulators per SM; 8 CTAs are what the registers allow
+  const int per_sm = std::min(8, 512 / BN);
+  const int tiles = (int)((g.pixels + 127) / 128), ny = (g.N + BN - 1) / BN;
+  const dim3 grid(std::max(1, std::min(tiles, sm_count() * per_sm / ny)), ny);
+  conv3x3_rgb_kernel<BN, EPI><<<grid, kRgbThreads, 0, s>>>(g);
+  return cuda_status(cudaGetLastError());
+}
+
 ConvArgs base_args(int B, int H, int W, int C, int N, int stride, int kp, uint32_t* err) {
   ConvArgs g{};
   g.B = B, g.H = H, g.W = W, g.C = C, g.N = N, g.stride = stride, g.kp = kp;
@@ -597,6 +764,23 @@ int ds_conv3x3_forward(const void* x, int B, int H, int W, int C, int stride, co
                        uint32_t* err, ds_stream stream) {
   using namespace ds;
   if (!x || !w || !bias || !err || (!d && (!z || !y))) return DS_ERR_ARG;
+  if (C == 3) {
+    if (!conv_ok(B, H, W, 32, N, stride, 288) || Kp < 27) return DS_ERR_ARG;
+    if (!aligned16(z) || !aligned16(y) || !aligned16(d)) return DS_ERR_ARG;
+    RgbArgs g{};
+    g.x = (const __nv_bfloat16*)x, g.w = (const __nv_bfloat16*)w;
+    g.B = B, g.H = H, g.W = W, g.N = N, g.stride = stride, g.kp = Kp;
+    g.Ho = (H - 1) / stride + 1, g.Wo = (W - 1) / stride + 1;
+    g.pixels = (uint32_t)B * g.Ho * g.Wo;
+    g.bias = bias;
+    g.z = (__nv_bfloat16*)z, g.y = (__nv_bfloat16*)y, g.d = d;
+    g.err = err;
+    g.spin = gemm_spin_limit();
+    cudaStream_t s = (cudaStream_t)stream;
+    if (N <= 32)
+      return d ? launch_rgb<32, kConvF32>(g, s) : launch_rgb<32, kConvGelu>(g, s);
+    return d ? launch_rgb<64, kConvF32>(g, s) : launch_rgb<64, kConvGelu>(g, s);
+  }
   if (!conv_ok(B, H, W, C, N, stride, Kp)) return DS_ERR_ARG;
   if (!aligned16(x) || !aligned16(w) || !aligned16(bias) || !aligned16(z) || !aligned16(y) ||
       !aligned16(d))

@@ -150,16 +150,16 @@ class Conv3x3:
     def params(self):
         return [(self.w, self.gw, self.w16), (self.b, self.gb, None)]
 
-    def _implicit(self, *tensors):
+    def _implicit(self, *tensors, rgb=False):
         """Whether the convolution runs without an im2col matrix (ds_conv3x3_*):
-        whole 64-channel blocks (or 32 channels), 16-byte rows and addresses,
-        counts that fit 32 bits.  Measured against im2col + GEMM (B200, forward +
-        backward): 64 -> 128 channels, stride 2, 8 x 256 x 256: 2.03 -> 0.31 ms;
+        whole 64-channel blocks (or 32 channels; with `rgb` also 3), 16-byte
+        rows and addresses, counts that fit 32 bits.  Measured against im2col +
+        GEMM (B200, forward + backward): 64 -> 128 channels, stride 2, 8 x 256 x 256: 2.03 -> 0.31 ms;
         256 -> 256, 32 x 64 x 64: 6.16 -> 0.58 ms.  What it does not take (the
-        3-channel first layer above all) goes through im2col."""
+        weight gradient of a 3-channel layer above all) goes through im2col."""
         x = tensors[0]
-        return ((self.cin == 32 or self.cin % 64 == 0) and self.cout % 8 == 0
-                and max(self.cin, self.cout) <= 1 << 16 and x[..., 0].numel() < 1 << 30
+        return ((self.cin == 32 or self.cin % 64 == 0 or (rgb and self.cin == 3))
+                and self.cout % 8 == 0 and max(self.cin, self.cout) <= 1 << 16 and x[..., 0].numel() < 1 << 30
                 and all(t is None or (t.data_ptr() % 16 == 0 and t.is_contiguous())
                         for t in (self.w16, self.b, self.gw, *tensors)))
 
@@ -168,7 +168,7 @@ class Conv3x3:
         z only as FP32 when the layer has no GELU).  The backward needs the
         input as it is now: it is copied unless the caller says with `keep`
         that x will not change before the backward."""
-        if self._implicit(x):
+        if self._implicit(x, rgb=True):
             B, H, W, _ = self.in_shape = tuple(x.shape)
             Ho, Wo = (H - 1) // self.stride + 1, (W - 1) // self.stride + 1
             self.x, self.col = x if keep else x.clone(), None
@@ -213,7 +213,7 @@ class Conv3x3:
                    self.cout, _p(z_prev), dx.data_ptr(), gemm.err.data_ptr(), _s())
             return dx
         col = self.col
-        if col is None:  # a gradient at an address the tensor maps do not take
+        if col is None:  # three channels, or an address the tensor maps do not take
             col, _ = im2col(self.x, self.stride, self.kp)
         dzt = transpose(dz2)              # [Cout, M]
         colt = transpose(col)             # [Kp, M]

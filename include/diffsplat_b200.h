@@ -397,8 +397,8 @@ int ds_im2col_bf16(const void *x, int B, int H, int W, int C, int stride, int Kp
 int ds_col2im_bf16(const float *dcol, int B, int H, int W, int C, int stride, int Kp,
                    const void *z, void *dx, ds_stream stream);
 /* The same convolution without the im2col matrix (implicit GEMM on tcgen05):
- * C == 32 or a multiple of 64, N (output channels) a multiple of 8, all
- * pointers 16-byte aligned, else DS_ERR_ARG.  w is BF16 [N][Kp] in im2col
+ * C == 32 or a multiple of 64 (the forward also takes C == 3), N (output
+ * channels) a multiple of 8, all pointers 16-byte aligned, else DS_ERR_ARG.  w is BF16 [N][Kp] in im2col
  * order.  Forward: z = BF16(conv + bias) and y = BF16(gelu(conv + bias))
  * [B*Ho*Wo][N], or FP32 d = conv + bias when d is given; equal to im2col +
  * ds_gemm_bf16_tn bit for bit.  dgrad: dx [B][H][W][C] BF16, times gelu'(zprev)

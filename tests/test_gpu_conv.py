@@ -68,6 +68,31 @@ def test_conv_matches_im2col_and_fp64(cuda_lib, B, H, W, cin, cout, stride, act)
     assert _rel(dx, gx * slope) < 4e-3
 
 
+@pytest.mark.parametrize("B,H,W,cout", [(1, 1, 1, 8), (3, 7, 5, 32), (2, 40, 33, 56),
+                                        (1, 130, 300, 72), (64, 9, 9, 32)])
+@pytest.mark.parametrize("stride", [1, 2])
+@pytest.mark.parametrize("act", [True, False])
+def test_rgb_layer_equals_im2col(cuda_lib, B, H, W, cout, stride, act):
+    import torch
+    from diffsplat_b200 import nn
+    gen = torch.Generator().manual_seed(cout + H)
+    conv = nn.Conv3x3(3, cout, stride, gelu=act, gen=gen)
+    conv.b.copy_(torch.randn(cout, generator=gen))
+    x = torch.randn(B, H, W, 3, generator=gen).to(torch.bfloat16).cuda()
+    gemm = nn.Gemm()
+    got = conv.forward(gemm, x)
+    assert conv.col is None
+    col, _ = nn.im2col(x, stride, conv.kp)
+    torch.cuda.synchronize()
+    gemm.check()
+    if act:
+        z, y = gemm(col, conv.w16, nn.EPI_BIAS_GELU, bias=conv.b)
+        assert torch.equal(got[0].view(z.shape), z) and torch.equal(got[1].view(y.shape), y)
+    else:
+        d = gemm(col, conv.w16, nn.EPI_BIAS_F32, bias=conv.b)
+        assert torch.equal(got[0].view(-1, cout), d)
+
+
 def test_conv_timeout_is_reported_and_device_stays_usable(cuda_lib):
     """Pipeline waits limited to one poll: the waits run out, what was issued
     lands, TMEM is freed and the error word is set; then a normal call works."""

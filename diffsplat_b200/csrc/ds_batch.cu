@@ -31,15 +31,15 @@ namespace {
 
 // One warp per instance: sum of its tiles' loss partials in tile order.
 __global__ void batch_loss_kernel(const float* __restrict__ partials,
-                                  const InstGeom* __restrict__ geom, int instances,
+                                  const InstGeom* __restrict__ geom, int instances, int parts,
                                   float* __restrict__ losses) {
   const int k = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
   if (k >= instances) return;
   const InstGeom g = geom[k];
-  const int tiles = g.ntx * g.nty;
+  const int n = g.ntx * g.nty * parts;
   float s = 0.f;
-  for (int t = lane; t < tiles; t += 32) s += partials[g.tile_off + t];
+  for (int t = lane; t < n; t += 32) s += partials[(size_t)g.tile_off * parts + t];
   s = warp_sum(s);
   if (lane == 0) losses[k] = s;
 }
@@ -88,7 +88,7 @@ static void launch_batch_preprocess(ds_batch* b, const Soa<T>& R, cudaStream_t s
   RasterBuffers& rb = b->rb;
   const unsigned blocks = (unsigned)((b->total_splats + kPreThreads - 1) / kPreThreads);
   fit_preprocess_kernel<T, TS, true><<<blocks, kPreThreads, 0, s>>>(
-      b->P, R, b->cfg.sh_degree, b->cams, 0, 0, 0, 0, rb.rec_a, rb.rec_b, rb.rec_c, rb.rec_idet,
+      b->P, R, b->cfg.sh_degree, b->cams, 0, 0, 0, 0, rb.rec_a, rb.rec_b, rb.rec_c,
       rb.rect, rb.counts, rb.depth_keys, rb.scalars, b->inst_of_splat, b->geom_dev);
 }
 
@@ -113,7 +113,7 @@ static int batch_enqueue(ds_batch* b, cudaStream_t s) {
   DS_TRY(raster_build_lists(rb, n, s, nullptr, true));
   DS_TRY(raster_composite_forward(rb, b->images, b->targets, s));
   batch_loss_kernel<<<(b->instances * 32 + 255) / 256, 256, 0, s>>>(
-      rb.loss_partials, b->geom_dev, b->instances, b->losses);
+      rb.loss_partials, b->geom_dev, b->instances, loss_parts(rb.tile_size), b->losses);
   DS_CUDA(cudaGetLastError());
   DS_TRY(raster_composite_backward(rb, b->images, nullptr, b->targets, s));
   DS_TRY(raster_reduce_long_grads(rb, n, s));
@@ -280,8 +280,6 @@ int ds_batch_create(const ds_batch_config* cfg, const ds_batch_instance* inst, d
     return fail(st);
   b->rb.grad_mode = cfg->grad_mode;
   b->rb.schedule = cfg->schedule;
-  b->rb.ppt = cfg->pixels_per_thread;
-  b->rb.ppt_bwd = cfg->pixels_per_thread;
   b->rb.inst_of_splat = b->inst_of_splat;
   b->rb.tile_inst = b->tile_inst;
   b->rb.geom = b->geom_dev;

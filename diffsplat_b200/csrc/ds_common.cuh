@@ -304,7 +304,6 @@ __device__ __forceinline__ uint32_t depth_bits(float depth) {
 //   A = {ndc x, ndc y, cull half-width x, cull half-width y}
 //   B = {conic xx, conic xy, conic yy, opacity}
 //   C = {r, g, b, sigma cut}
-// plus idet (1/det of Cov2D) used only by the backward.
 // The conic is computed with the reference's formula (tile_rasterize_layer.cu:
 // 260-272) so the per-pixel Gaussian value is bit-identical.  The culling box
 // and sigma cut are conservative bounds of the region where the reference's
@@ -313,7 +312,6 @@ __device__ __forceinline__ uint32_t depth_bits(float depth) {
 // ---------------------------------------------------------------------------
 struct Record {
   float4 a, b, c;
-  float idet;
 };
 
 __device__ __forceinline__ Record make_record(float x, float y, float cxx, float cxy, float cyy,
@@ -324,7 +322,6 @@ __device__ __forceinline__ Record make_record(float x, float y, float cxx, float
   float icxx = cyy * idet;
   float icxy = -cxy * idet;
   float icyy = cxx * idet;
-  rec.idet = idet;
   // alpha = min(0.99, o*exp(-sigma)) >= 1/255 needs sigma <= ln(255 o); 0.01 of slack
   // in sigma covers the approximate exp and every rounding step.
   float cut = logf(255.f * opac) + 0.01f;
@@ -356,6 +353,39 @@ __device__ __forceinline__ Record make_record(float x, float y, float cxx, float
   rec.c = make_float4(r, g, b, cut);
   return rec;
 }
+
+// ---------------------------------------------------------------------------
+// Two FP32 lanes per instruction (sm_100 packed arithmetic): each half rounds
+// like the scalar operation, flushing denormals like the rest of this build.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ unsigned long long bits2(float2 v) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(v.x), "f"(v.y));
+  return r;
+}
+__device__ __forceinline__ float2 float2_of(unsigned long long b) {
+  float2 v;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(b));
+  return v;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  unsigned long long r;
+  asm("add.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(bits2(a)), "l"(bits2(b)));
+  return float2_of(r);
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  unsigned long long r;
+  asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(bits2(a)), "l"(bits2(b)));
+  return float2_of(r);
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  unsigned long long r;
+  asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;"
+      : "=l"(r)
+      : "l"(bits2(a)), "l"(bits2(b)), "l"(bits2(c)));
+  return float2_of(r);
+}
+__device__ __forceinline__ float2 both(float v) { return make_float2(v, v); }
 
 // ---------------------------------------------------------------------------
 // Warp helpers

@@ -8,20 +8,21 @@
 // T_before = T / max(1 - alpha, 1e-6).
 //
 // Layout: tiles are TS x TS pixels (16, the reference's TILE_SIZE; batches may
-// use 8 or 32); each thread owns PPT pixels of one column (PPT = 1, 2 or 4); a
-// warp covers a BW x BH block (8x4, 8x8 or 16x8 pixels).  When a batch of
-// splats is staged in shared memory, each splat's acceptance box is tested
-// once against every warp's block; each warp then walks only its own hits
-// (ballot words of the per-splat warp masks), so shared-memory reads and
-// (backward) the warp reduction are shared by 32 * PPT pixels and misses cost
-// nothing in the inner loop.  The backward keeps one gradient partial per warp
-// and splat in shared memory and sums the warps in a fixed order: gradients
-// are deterministic run to run.
+// use 8 or 32), cut into 8x8-pixel blocks of one warp each.  A lane owns two
+// pixels of one column, four rows apart, and works on both with packed FP32
+// instructions.  A splat is tested once against each warp's block; the warp then
+// walks only its own hits, so misses cost nothing in the inner loop.  One warp
+// per block at every tile size and in batches, so each pixel's result and each
+// splat's gradient sums are the same whatever the launch.  Gradients are summed
+// in a fixed order: they are deterministic run to run.
 //
 // Batch mode (kBatch): tile indices are batch-wide; tile_inst / geom give each
 // tile's instance, image size, tile grid and first pixel.
 #include <stdlib.h>
 #include <string.h>
+
+#include <atomic>
+#include <type_traits>
 
 #include "ds_common.cuh"
 #include "ds_internal.h"
@@ -30,58 +31,29 @@ namespace ds {
 
 namespace {
 
-constexpr int kFwdBatch = 256;  // splats staged in shared memory per forward batch
 #ifndef DS_FWD_GROUP
-#define DS_FWD_GROUP 4
+#define DS_FWD_GROUP 2
 #endif
-constexpr int kFwdGroupPpt1 = DS_FWD_GROUP;  // forward hits evaluated together at 1 px/thread
-#ifndef DS_BWD_GROUP
-#define DS_BWD_GROUP 2
-#endif
-constexpr int kBwdGroupPpt1 = DS_BWD_GROUP;  // backward hits evaluated together at 1 px/thread
 #ifndef DS_FWD_MIN_BLOCKS
-#define DS_FWD_MIN_BLOCKS 4
+#define DS_FWD_MIN_BLOCKS 6
 #endif
 #ifndef DS_BWD_MIN_BLOCKS
-#define DS_BWD_MIN_BLOCKS 3
+#define DS_BWD_MIN_BLOCKS 5
 #endif
+constexpr int kFwdGroup = DS_FWD_GROUP;  // forward hits whose alphas are computed together
+constexpr int kBwdHits = 8;  // hits whose gradients a warp sums at once, four lanes each
 
-// Backward layout chosen per forward when ppt_bwd is 0: two pixels per thread
-// (8x8-pixel warp blocks, one warp reduction per 64 pixels) when the
-// forward's hits had at least 24.7 contributing pixels of the 32 of an 8x4
-// block on average, one otherwise.  Measured on the 1280x720 / 60000-splat fit
-// at steps 25-4000: the two-pixel backward is faster down to about 24.7 (0.49
-// vs 0.63 ms at 26.6, early in the fit), equal there and slower below (0.64
-// vs 0.48 ms at 21.9, late).  Chosen for a whole frame: a per-tile choice
-// (two launches splitting the tiles) measured slower than either layout alone.
-constexpr uint32_t kDenseLanesX10 = 247;
-
-template <int PPT, int TS>
+// Backward CTA of one tile: a warp per 8x8 block.
+template <int TS>
 struct Lay {
-  static constexpr int kThreads = TS * TS / PPT;
-  static constexpr int kWarps = kThreads / 32;
-  static constexpr int BW = PPT == 4 ? 16 : 8;  // warp block width
-  static constexpr int BH = 32 * PPT / BW;      // warp block height
-  static constexpr int kLaneRows = 32 / BW;     // rows between a thread's pixels
-  static constexpr int kWarpsX = TS / BW;
-  // backward batch: the per-warp partials (kWarps x kBwdBatch x 36 B) stay within 36 KB
-  static constexpr int kBwdBatch = 1024 / kWarps < 128 ? 1024 / kWarps : 128;
-  // resident CTAs per SM the register allocation must allow (256-thread CTAs)
-  static constexpr int kMinBlocksFwd = kThreads == 256 ? DS_FWD_MIN_BLOCKS : 1;
-  // 128-thread backward (two pixels per thread): 7 CTAs per SM caps it at 70
-  // registers with no spills (93 unbounded, 5 CTAs; bwd 0.488 -> 0.471 ms on
-  // the 1280x720 fit at step 25, B200); 8 CTAs (64 registers) measured slower.
-  // 256-thread backward (one pixel per thread): 3 CTAs per SM (up to 85
-  // registers); at 4 (64 registers) it spills, 0.479 -> 0.503 ms at step 1010
-  static constexpr int kMinBlocksBwd = kThreads == 256 ? DS_BWD_MIN_BLOCKS
-                                                        : (kThreads == 128 ? 7 : 1);
-  // hits evaluated together: only at 1 pixel per thread; with more pixels the
-  // per-pixel state already fills the registers (batch64, B200: grouping
-  // at 2 pixels per thread cost 0.6% there and 5% before the backward
-  // was limited to one hit per group)
-  static constexpr int kFwdGroup = PPT == 1 ? kFwdGroupPpt1 : 1;
-  static constexpr int kBwdGroup = PPT == 1 ? kBwdGroupPpt1 : 1;
-  static_assert(kThreads % 32 == 0 && BW <= TS && kWarps <= 32, "unsupported tile layout");
+  static constexpr int kWarps = (TS / 8) * (TS / 8);
+  static constexpr int kThreads = 32 * kWarps;
+  // backward batch: the per-warp partials (kWarps x kBwdBatch x 36 B) stay within
+  // 9 KB up to 16-pixel tiles, 18 KB at 32
+  static constexpr int kBwdBatch = kWarps <= 1 ? 128 : kWarps <= 4 ? 64 : 32;
+  // 16-pixel tiles: 5 CTAs per SM (96 registers); 4 and 6 measured 0.307 and
+  // 0.326 ms against 0.301 on the 1280x720 fit at step 25 (B200)
+  static constexpr int kMinBlocksBwd = kWarps == 4 ? DS_BWD_MIN_BLOCKS : 1;
 };
 
 // Where a tile lies: its image size, its tile grid, its index in that grid and
@@ -99,36 +71,31 @@ __device__ __forceinline__ TileGeo tile_geo(int tile, int W, int H, int ntx,
   return TileGeo{g.width, g.height, g.ntx, tile - g.tile_off, g.pix_off};
 }
 
-template <int PPT>
+// The two pixels of a lane in block `blk` of a tile.
 struct Pixels {
-  int j;       // column
-  int i[PPT];  // rows
-  bool inside[PPT];
+  int j;     // column
+  int i[2];  // rows
+  bool inside[2];
   float px;
-  float py[PPT];
+  float py[2];
   float wx_lo, wx_hi, wy_lo, wy_hi;  // extremes of the warp's pixel centres (NDC)
 };
 
-template <int PPT, int TS>
-__device__ __forceinline__ Pixels<PPT> pixels(int tile, int ntx, int W, int H) {
-  using Lc = Lay<PPT, TS>;
-  Pixels<PPT> m;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+template <int TS>
+__device__ __forceinline__ Pixels pixels(int tile, int ntx, int W, int H, int blk) {
+  Pixels m;
+  const int lane = threadIdx.x & 31;
   const int trow = tile / ntx, tcol = tile - trow * ntx;
-  const int lx = lane % Lc::BW, ly = lane / Lc::BW;
-  const int wx = w % Lc::kWarpsX, wy = w / Lc::kWarpsX;
-  m.j = tcol * TS + wx * Lc::BW + lx;
+  m.j = tcol * TS + blk % (TS / 8) * 8 + lane % 8;
   m.px = 2.f * (m.j + 0.5f) / W - 1.f;
-  float yl = 3.0e38f, yh = -3.0e38f;
 #pragma unroll
-  for (int k = 0; k < PPT; ++k) {
-    m.i[k] = trow * TS + wy * Lc::BH + ly + k * Lc::kLaneRows;
+  for (int k = 0; k < 2; ++k) {
+    m.i[k] = trow * TS + blk / (TS / 8) * 8 + lane / 8 + 4 * k;
     m.inside[k] = m.i[k] < H && m.j < W;
     m.py[k] = 1.f - 2.f * (m.i[k] + 0.5f) / H;
-    yl = fminf(yl, m.py[k]);
-    yh = fmaxf(yh, m.py[k]);
   }
   float xl = m.px, xh = m.px;
+  float yl = fminf(m.py[0], m.py[1]), yh = fmaxf(m.py[0], m.py[1]);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     xl = fminf(xl, __shfl_xor_sync(0xffffffffu, xl, o));
@@ -180,25 +147,72 @@ __device__ __forceinline__ bool ellipse_hits(const float4& a, const float4& b, f
   return 0.5f * m <= cut;
 }
 
-// Forward alpha of a splat at a pixel (0 when the splat is skipped there):
-// sigma < 0, or alpha below 1/255.  Beyond the cut (ln(255 o) + 0.01, used by
-// the warp-block tests) alpha is below 0.99 / 255 and fails the threshold test
-// by itself, so the pixel loop does not test sigma against the cut.
-__device__ __forceinline__ float splat_alpha(float dx, float dy, const float4& b, float cut) {
-  (void)cut;
-  const float sigma = 0.5f * conic_dist2(dx, dy, b.x, b.y, b.z);
-  if (sigma < 0.f) return 0.f;
-  const float alpha = fminf(kMaxAlpha, b.w * __expf(-sigma));
-  return alpha < kAlphaThres ? 0.f : alpha;
-}
-
 // One splat of a batch, loaded into registers a batch ahead of its use so the
 // gathers overlap the current batch's compositing.
 struct Staged {
   float4 a, b, c;
-  float idet;
   bool ok;
 };
+
+// A splat as the pixel loops read it: every value twice, so that it loads as a
+// packed operand.
+struct SplatRec {
+  float4 pos;     // x, x, y, y
+  float4 ab;      // conic a, a, b, b
+  float4 co;      // conic c, c, opacity, opacity
+  float4 rg;      // r, r, g, g
+  float4 blue;    // b, b, -, - (forward: the splat's sorted index as bits)
+  __device__ __forceinline__ void set(const float4& a, const float4& b, const float4& c,
+                                      int index) {
+    pos = make_float4(a.x, a.x, a.y, a.y);
+    ab = make_float4(b.x, b.x, b.y, b.y);
+    co = make_float4(b.z, b.z, b.w, b.w);
+    rg = make_float4(c.x, c.x, c.y, c.y);
+    blue = make_float4(c.z, c.z, __int_as_float(index), 0.f);
+  }
+  // opacity 0: skipped at every pixel
+  __device__ __forceinline__ void set_none() {
+    pos = ab = co = rg = blue = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  __device__ __forceinline__ float2 conic_a() const { return make_float2(ab.x, ab.y); }
+  __device__ __forceinline__ float2 conic_b() const { return make_float2(ab.z, ab.w); }
+  __device__ __forceinline__ float2 conic_c() const { return make_float2(co.x, co.y); }
+  __device__ __forceinline__ float2 x() const { return make_float2(pos.x, pos.y); }
+  __device__ __forceinline__ float2 y() const { return make_float2(pos.z, pos.w); }
+  __device__ __forceinline__ float2 red() const { return make_float2(rg.x, rg.y); }
+  __device__ __forceinline__ float2 green() const { return make_float2(rg.z, rg.w); }
+  __device__ __forceinline__ float opacity() const { return co.z; }
+};
+
+// opacity exp(-sigma) of a splat at a pair of pixels (conic_dist2 in its
+// rounding) and whether sigma >= 0 there; dx, dxx = dx dx and dx2 = 2 dx.
+__device__ __forceinline__ float2 pair_opacity(float2 dx2, float2 dxx, float2 dy,
+                                               const SplatRec& r, bool& ok0, bool& ok1) {
+  const float2 dist2 = fma2(mul2(dy, dy), r.conic_c(),
+                            fma2(dxx, r.conic_a(), mul2(mul2(dx2, dy), r.conic_b())));
+  const float2 sigma = mul2(both(0.5f), dist2);
+  ok0 = !(sigma.x < 0.f);
+  ok1 = !(sigma.y < 0.f);
+  return mul2(make_float2(r.co.z, r.co.w), make_float2(__expf(-sigma.x), __expf(-sigma.y)));
+}
+
+// A warp's hits of a staged batch, listed in order: the splats l of [from, n)
+// whose mask has the warp's bit.  Padded with `none` to an even count; returns
+// the count before padding.
+__device__ __forceinline__ int list_hits(const uint32_t* mask, int w, int lane, int from, int n,
+                                         int none, int* list) {
+  int count = 0;
+  for (int k = 0; k < n; k += 32) {
+    const int l = k + lane;
+    const bool hit = l >= from && l < n && ((mask[l] >> w) & 1u);
+    const uint32_t word = __ballot_sync(0xffffffffu, hit);
+    if (hit) list[count + __popc(word & ((1u << lane) - 1u))] = l;
+    count += __popc(word);
+  }
+  if (lane == 0) list[count] = none;
+  __syncwarp();
+  return count;
+}
 
 // Bit w set: the splat can reach warp w's pixel block.
 template <int NW>
@@ -210,229 +224,205 @@ __device__ __forceinline__ uint32_t warp_hits(const float4& a, const float4& b, 
   return mk;
 }
 
-template <int PPT, int TS, bool kLoss, bool kCount, bool kBatch>
-__global__ void __launch_bounds__(Lay<PPT, TS>::kThreads, Lay<PPT, TS>::kMinBlocksFwd)
+// Forward of a tile's 8x8-pixel blocks, one warp each, two pixels per lane (the
+// same column, four rows apart) handled by packed instructions.  Bound by
+// instruction issue, so the warps share nothing that would make one wait for
+// another: each walks its tile's list by itself, 32 splats at a time (one
+// test of one splat against the warp's block per lane, the next 32 records in
+// flight), compacts the records of its hits into its own shared memory and
+// composites them.  Staging a tile's batch once for all its warps saves
+// three of four loads of a record (they hit L1 here) but made the warps of a
+// tile wait for the one with the most hits in every batch.  Against that, with
+// one pixel per lane and 8x4 blocks (B200): 1280x720 fit of 60000 splats at step
+// 25 0.231 -> 0.119 ms, at step 400 0.359 -> 0.189; a million splats at
+// 1920x1080 0.320 -> 0.235.  6 CTAs per SM and two hits at a time: 8 CTAs took
+// 0.122 / 0.199 / 0.268, 5 CTAs and four hits 0.122 / 0.195 / 0.231.
+//
+// A pixel that is done (T <= 1e-4), outside the image or not reached by the
+// splat composites alpha = 0, which changes neither its colour nor its T; only
+// colours that are not finite need the guarded variant.
+constexpr int kFwdWarps = 4;
+
+struct FwdShared {
+  SplatRec hit[kFwdWarps][32 + kFwdGroup];
+  float red[kFwdWarps];
+  bool last;
+};
+
+template <int TS, bool kLoss, bool kCount, bool kBatch>
+__global__ void __launch_bounds__(32 * kFwdWarps, DS_FWD_MIN_BLOCKS)
     composite_fwd_kernel(const float4* __restrict__ ra, const float4* __restrict__ rb,
                          const float4* __restrict__ rc, const uint32_t* __restrict__ sorted_splat,
                          const int2* __restrict__ ranges, const int32_t* __restrict__ order,
                          float* __restrict__ out_rgb, float* __restrict__ out_alpha,
-                         int32_t* __restrict__ last_ids, int W_, int H_, int ntx_,
+                         int32_t* __restrict__ last_ids, int tiles, int W_, int H_, int ntx_,
                          const uint16_t* __restrict__ tile_inst, const InstGeom* __restrict__ geom,
                          const float* __restrict__ target, float* __restrict__ loss_partials,
-                         DevScalars* __restrict__ sc, DevScalars* __restrict__ mode_sc) {
+                         DevScalars* __restrict__ sc) {
   pdl_wait();
-  using Lc = Lay<PPT, TS>;
-  constexpr int NT = Lc::kThreads;
-  constexpr int NW = Lc::kWarps;
-  __shared__ float4 sA[kFwdBatch], sB[kFwdBatch], sC[kFwdBatch];
-  __shared__ uint32_t sHits[NW], sLanes[NW];
-  __shared__ uint32_t sMask[kFwdBatch];
-  __shared__ float4 sBox[NW];
-  __shared__ float red[NW];
-  __shared__ bool last;
-  const int tile = order ? order[blockIdx.x] : (int)blockIdx.x;
+  constexpr int kBlocks = (TS / 8) * (TS / 8);  // warp blocks of a tile
+  constexpr int G = kFwdGroup;
+  __shared__ FwdShared sm;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int at = blockIdx.x * kFwdWarps + w;
+  const int blk = at % kBlocks;
+  const bool real = at / kBlocks < tiles;  // 8-pixel tiles: the last CTA may be ragged
+  const int slot = real ? at / kBlocks : 0;
+  const int tile = order ? order[slot] : slot;
   const TileGeo tg = tile_geo<kBatch>(tile, W_, H_, ntx_, tile_inst, geom);
   const int W = tg.W, H = tg.H;
-  const Pixels<PPT> m = pixels<PPT, TS>(tg.local, tg.ntx, W, H);
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  if (lane == 0) sBox[w] = make_float4(m.wx_lo, m.wx_hi, m.wy_lo, m.wy_hi);
-  const int2 range = ranges[tile];
-  const int start = range.x, end = range.y;
-  float T[PPT], Cr[PPT], Cg[PPT], Cb[PPT];
-  uint32_t cur[PPT];
-  bool done[PPT];
-  bool all_done = true;
+  const Pixels m = pixels<TS>(tg.local, tg.ntx, W, H, blk);
+  const float4 box = make_float4(m.wx_lo, m.wx_hi, m.wy_lo, m.wy_hi);
+  const int2 range = real ? ranges[tile] : make_int2(0, 0);
+  const int end = range.y;
+  const float2 npx = both(-m.px), npy = make_float2(-m.py[0], -m.py[1]);
+  // T = 0: never composited
+  float2 T = make_float2(m.inside[0] ? 1.f : 0.f, m.inside[1] ? 1.f : 0.f);
+  float2 Cr = both(0.f), Cg = both(0.f), Cb = both(0.f);
+  int cur0 = 0, cur1 = 0;
   uint32_t n_contrib = 0, n_tested = 0;
-  uint32_t n_hits = 0, n_lanes = 0;  // this warp's hits and their contributing lanes
+  SplatRec* const hit = sm.hit[w];
+
+  auto composite = [&](auto guarded, int n) {
+    for (int i = 0; i < n; i += G) {
+      float2 al[G];
+      bool ok0[G], ok1[G];
 #pragma unroll
-  for (int k = 0; k < PPT; ++k) {
-    T[k] = 1.f;
-    Cr[k] = Cg[k] = Cb[k] = 0.f;
-    cur[k] = 0;
-    done[k] = !m.inside[k];
-    all_done = all_done && done[k];
-  }
-  constexpr int R = (kFwdBatch + NT - 1) / NT;  // splats each thread stages
-  Staged pf[R];
-  auto prefetch = [&](int b0) {
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int l = threadIdx.x + r * NT, idx = b0 + l;
-      pf[r].ok = l < kFwdBatch && idx < end;
-      if (pf[r].ok) {
-        const uint32_t g = sorted_splat[idx];
-        pf[r].a = ra[g];
-        pf[r].b = rb[g];
-        pf[r].c = rc[g];
+      for (int g = 0; g < G; ++g) {
+        const SplatRec& r = hit[i + g];
+        const float2 dx = add2(r.x(), npx);
+        al[g] = pair_opacity(add2(dx, dx), mul2(dx, dx), add2(r.y(), npy), r, ok0[g], ok1[g]);
+        al[g] = make_float2(fminf(kMaxAlpha, al[g].x), fminf(kMaxAlpha, al[g].y));
+        ok0[g] = ok0[g] && !(al[g].x < kAlphaThres);
+        ok1[g] = ok1[g] && !(al[g].y < kAlphaThres);
       }
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+        const SplatRec& r = hit[i + g];
+        const float4 blue = r.blue;
+        const int id = __float_as_int(blue.z);
+        const bool p0 = ok0[g] && T.x > kTThres, p1 = ok1[g] && T.y > kTThres;
+        if (kCount) {
+          n_tested += (T.x > kTThres) + (T.y > kTThres);
+          n_contrib += p0 + p1;
+        }
+        const float2 a = make_float2(p0 ? al[g].x : 0.f, p1 ? al[g].y : 0.f);
+        cur0 = p0 ? id : cur0;
+        cur1 = p1 ? id : cur1;
+        const float2 vis = mul2(a, T);
+        const float2 r1 = fma2(r.red(), vis, Cr);
+        const float2 g1 = fma2(r.green(), vis, Cg);
+        const float2 b1 = fma2(make_float2(blue.x, blue.y), vis, Cb);
+        if (decltype(guarded)::value) {
+          Cr = make_float2(p0 ? r1.x : Cr.x, p1 ? r1.y : Cr.y);
+          Cg = make_float2(p0 ? g1.x : Cg.x, p1 ? g1.y : Cg.y);
+          Cb = make_float2(p0 ? b1.x : Cb.x, p1 ? b1.y : Cb.y);
+        } else {
+          Cr = r1, Cg = g1, Cb = b1;
+        }
+        T = mul2(T, fma2(a, both(-1.f), both(1.f)));
+      }
+      if (!__any_sync(0xffffffffu, T.x > kTThres || T.y > kTThres)) return;
     }
   };
-  prefetch(start);
-  for (int b0 = start; b0 < end; b0 += kFwdBatch) {
-    if (__syncthreads_count(all_done) >= NT) break;
-    // Stage the batch; each splat's warp-overlap mask is computed once here
-    // so that every warp walks only the splats that can touch its pixels.
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int l = threadIdx.x + r * NT;
-      if (l < kFwdBatch) {
-        uint32_t mk = 0u;
-        if (pf[r].ok) {
-          sA[l] = pf[r].a;
-          sB[l] = pf[r].b;
-          sC[l] = pf[r].c;
-          mk = warp_hits<NW>(pf[r].a, pf[r].b, pf[r].c.w, sBox);
-        }
-        sMask[l] = mk;
-      }
+
+  // records of the first 32 splats, ids of the next 32
+  Staged pf;
+  uint32_t next = 0;
+  pf.ok = range.x + lane < end;
+  if (pf.ok) {
+    const uint32_t g = sorted_splat[range.x + lane];
+    pf.a = ra[g];
+    pf.b = rb[g];
+    pf.c = rc[g];
+  }
+  if (range.x + 32 + lane < end) next = sorted_splat[range.x + 32 + lane];
+  for (int b0 = range.x; b0 < end; b0 += 32) {
+    const bool mine = pf.ok && ellipse_hits(pf.a, pf.b, pf.c.w, box);
+    const uint32_t word = __ballot_sync(0xffffffffu, mine);
+    const int n = __popc(word);
+    bool odd = false;  // a colour that is not finite
+    if (mine) {
+      hit[__popc(word & ((1u << lane) - 1u))].set(pf.a, pf.b, pf.c, b0 + lane);
+      odd = !(fabsf(pf.c.x) <= 3.0e38f && fabsf(pf.c.y) <= 3.0e38f && fabsf(pf.c.z) <= 3.0e38f);
     }
-    if (b0 + kFwdBatch < end) prefetch(b0 + kFwdBatch);
-    __syncthreads();
-    const int bs = min(kFwdBatch, end - b0);
-    bool stop = !__any_sync(0xffffffffu, !all_done);
-    for (int kw = 0; kw * 32 < bs && !stop; ++kw) {
-      const int l = kw * 32 + lane;
-      uint32_t word = __ballot_sync(0xffffffffu, l < bs && ((sMask[l] >> w) & 1u));
-      // Hits are taken Lc::kFwdGroup at a time: all their alphas are computed
-      // before any is composited (front to back), so the conic / exp chains of
-      // the group overlap.
-      while (word) {
-        int tg[Lc::kFwdGroup];
-        int ng = 0;
-#pragma unroll
-        for (int g = 0; g < Lc::kFwdGroup; ++g) {
-          tg[g] = word ? kw * 32 + __ffs(word) - 1 : tg[0];  // word is warp-uniform
-          ng += word ? 1 : 0;
-          word &= word - 1u;
-        }
-        n_hits += (uint32_t)ng;
-        float4 ag[Lc::kFwdGroup], bg[Lc::kFwdGroup], cg[Lc::kFwdGroup];
-#pragma unroll
-        for (int g = 0; g < Lc::kFwdGroup; ++g) {
-          ag[g] = sA[tg[g]];
-          bg[g] = sB[tg[g]];
-          cg[g] = sC[tg[g]];
-        }
-#pragma unroll
-        for (int k = 0; k < PPT; ++k) {
-          if (done[k]) continue;
-          float al[Lc::kFwdGroup];
-#pragma unroll
-          for (int g = 0; g < Lc::kFwdGroup; ++g)
-            al[g] = splat_alpha(ag[g].x - m.px, ag[g].y - m.py[k], bg[g], cg[g].w);
-#pragma unroll
-          for (int g = 0; g < Lc::kFwdGroup; ++g) {
-            if (g >= ng || done[k]) break;
-            if (kCount) ++n_tested;
-            if (al[g] > 0.f) {
-              if (kCount) ++n_contrib;
-              ++n_lanes;
-              const float vis = al[g] * T[k];
-              Cr[k] = __fmaf_rn(cg[g].x, vis, Cr[k]);
-              Cg[k] = __fmaf_rn(cg[g].y, vis, Cg[k]);
-              Cb[k] = __fmaf_rn(cg[g].z, vis, Cb[k]);
-              cur[k] = (uint32_t)(b0 + tg[g]);
-              T[k] = T[k] * (1.f - al[g]);
-              if (T[k] <= kTThres) done[k] = true;
-            }
-          }
-        }
-        all_done = true;
-#pragma unroll
-        for (int k = 0; k < PPT; ++k) all_done = all_done && done[k];
-        if (!__any_sync(0xffffffffu, !all_done)) {
-          stop = true;
-          break;
-        }
-      }
+    // the last group is filled with splats of opacity 0
+    if (lane < G && n + lane < (n + G - 1) / G * G) hit[n + lane].set_none();
+    pf.ok = b0 + 32 + lane < end;
+    if (pf.ok) {
+      pf.a = ra[next];
+      pf.b = rb[next];
+      pf.c = rc[next];
     }
+    if (b0 + 64 + lane < end) next = sorted_splat[b0 + 64 + lane];
+    odd = __any_sync(0xffffffffu, odd);
+    __syncwarp();
+    if (odd) composite(std::true_type{}, n);
+    else composite(std::false_type{}, n);
+    if (!__any_sync(0xffffffffu, T.x > kTThres || T.y > kTThres)) break;
+    __syncwarp();
   }
   if (kCount) {
-    uint32_t a = n_contrib, t = n_tested;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      a += __shfl_xor_sync(0xffffffffu, a, o);
-      t += __shfl_xor_sync(0xffffffffu, t, o);
-    }
-    if ((threadIdx.x & 31) == 0) {
-      atomicAdd(&sc->pairs[0], (unsigned long long)a);
-      atomicAdd(&sc->pairs[1], (unsigned long long)t);
-    }
-  }
-  if (mode_sc) {
-    const uint32_t lanes = warp_sum_u32(n_lanes);
+    n_contrib = warp_sum_u32(n_contrib);
+    n_tested = warp_sum_u32(n_tested);
     if (lane == 0) {
-      sHits[w] = n_hits;
-      sLanes[w] = lanes;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      unsigned long long h = 0, c = 0;
-#pragma unroll
-      for (int k = 0; k < NW; ++k) {
-        h += sHits[k];
-        c += sLanes[k];
-      }
-      atomicAdd(&mode_sc->mode_hits, h);
-      atomicAdd(&mode_sc->mode_lanes, c);
-      __threadfence();
-      if (atomicAdd(&mode_sc->mode_ticket, 1u) == gridDim.x - 1) {
-        // the last CTA decides for the frame and clears the sums
-        __threadfence();
-        const unsigned long long th = atomicAdd(&mode_sc->mode_hits, 0ull);
-        const unsigned long long tc = atomicAdd(&mode_sc->mode_lanes, 0ull);
-        mode_sc->bwd_ppt = (th > 0ull && 10ull * tc >= kDenseLanesX10 * th) ? 2u : 1u;
-        mode_sc->mode_hits = 0ull;
-        mode_sc->mode_lanes = 0ull;
-        mode_sc->mode_ticket = 0u;
-      }
+      atomicAdd(&sc->pairs[0], (unsigned long long)n_contrib);
+      atomicAdd(&sc->pairs[1], (unsigned long long)n_tested);
     }
   }
   float l = 0.f;
 #pragma unroll
-  for (int k = 0; k < PPT; ++k) {
-    if (!m.inside[k]) continue;
+  for (int k = 0; k < 2; ++k) {
+    if (!m.inside[k] || !real) continue;
     const int pix = tg.pix_off + m.i[k] * W + m.j;
-    out_rgb[pix * 3 + 0] = Cr[k];
-    out_rgb[pix * 3 + 1] = Cg[k];
-    out_rgb[pix * 3 + 2] = Cb[k];
-    out_alpha[pix] = 1.f - T[k];
-    last_ids[pix] = (int32_t)cur[k];
+    const float r = k ? Cr.y : Cr.x, g = k ? Cg.y : Cg.x, b = k ? Cb.y : Cb.x;
+    out_rgb[pix * 3 + 0] = r;
+    out_rgb[pix * 3 + 1] = g;
+    out_rgb[pix * 3 + 2] = b;
+    out_alpha[pix] = 1.f - (k ? T.y : T.x);
+    last_ids[pix] = k ? cur1 : cur0;
     if (kLoss) {
       const float scale = 1.f / (float)(W * H);
-      const float dR = Cr[k] - target[pix * 3 + 0];
-      const float dG = Cg[k] - target[pix * 3 + 1];
-      const float dB = Cb[k] - target[pix * 3 + 2];
+      const float dR = r - target[pix * 3 + 0];
+      const float dG = g - target[pix * 3 + 1];
+      const float dB = b - target[pix * 3 + 2];
       l += (dR * dR + dG * dG + dB * dB) * scale;
     }
   }
   if (kLoss) {
     l = warp_sum(l);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = l;
+    if (kBlocks < kFwdWarps) {  // 8-pixel tiles: one warp each
+      if (lane == 0 && real) loss_partials[tile] = l;
+      return;
+    }
+    // one partial per CTA: kBlocks / kFwdWarps of them per tile
+    if (lane == 0) sm.red[w] = l;
     __syncthreads();
     if (threadIdx.x == 0) {
       float s = 0.f;
-      for (int k = 0; k < Lc::kWarps; ++k) s += red[k];
-      loss_partials[tile] = s;
+#pragma unroll
+      for (int k = 0; k < kFwdWarps; ++k) s += sm.red[k];
+      loss_partials[tile * (kBlocks / kFwdWarps) + blk / kFwdWarps] = s;
       if (!kBatch) {
         __threadfence();
-        last = atomicAdd(&sc->ticket, 1u) == gridDim.x - 1;
+        sm.last = atomicAdd(&sc->ticket, 1u) == gridDim.x - 1;
       }
     }
-    __syncthreads();
     // Batches sum their per-instance losses in batch_loss_kernel instead.
-    if (!kBatch && last) {
+    if (kBatch) return;
+    __syncthreads();
+    if (sm.last) {
       // The last CTA to finish sums the per-tile partials in tile order.
       __threadfence();
       float s = 0.f;
-      for (int k = threadIdx.x; k < (int)gridDim.x; k += NT)
+      for (int k = threadIdx.x; k < (int)gridDim.x; k += 32 * kFwdWarps)
         s += ((volatile float*)loss_partials)[k];
       s = warp_sum(s);
-      if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+      if (lane == 0) sm.red[w] = s;
       __syncthreads();
       if (threadIdx.x == 0) {
         float tot = 0.f;
-        for (int k = 0; k < Lc::kWarps; ++k) tot += red[k];
+        for (int k = 0; k < kFwdWarps; ++k) tot += sm.red[k];
         sc->loss = tot;
         sc->ticket = 0u;
       }
@@ -440,10 +430,127 @@ __global__ void __launch_bounds__(Lay<PPT, TS>::kThreads, Lay<PPT, TS>::kMinBloc
   }
 }
 
-template <int PPT, int TS, bool kFusedLoss, bool kExact, bool kBatch>
-__global__ void __launch_bounds__(Lay<PPT, TS>::kThreads, Lay<PPT, TS>::kMinBlocksBwd)
+// Shared memory of one backward CTA (dynamic: up to 120 KB for 32-pixel tiles).
+template <int TS>
+struct BwdShared {
+  using Lc = Lay<TS>;
+  static constexpr int B = Lc::kBwdBatch, NW = Lc::kWarps;
+  // Row of a hit's per-pixel values: 4 floats past the pixels of a warp, so
+  // that the eight lanes of a 16-byte shared-memory phase (two hits, four
+  // lanes each, 8 floats apart) fall on distinct banks.
+  static constexpr int kPitch = 64 + 4;
+  SplatRec splat[B + 1];       // the last one reaches nothing
+  float4 box[NW];
+  float4 npx[NW][16];     // per pixel of a warp: -x, -y (NDC) and dL/dpixel
+  float4 npy[NW][16];
+  float4 gr[NW][16], gg[NW][16], gb[NW][16];
+  float4 s[NW][kBwdHits * kPitch / 4];    // per (hit, pixel): opacity exp() dL/dalpha
+  float4 fac[NW][kBwdHits * kPitch / 4];  // per (hit, pixel): alpha T
+  float part[NW][B * 9];       // per-warp gradient of each batch splat
+  uint32_t rec[B];             // record index of each batch splat
+  uint32_t mask[B];            // warps whose block the splat can reach
+  uint32_t got[NW][B / 32];    // batch splats with a partial from the warp
+  int2 list[NW][B / 2 + 1];    // the warp's hits of the batch
+  int32_t final_id[NW];
+};
+
+// The gradients of up to kBwdHits hits of a warp from their per-pixel values:
+// four lanes per hit, each over a quarter of the warp's pixels, two pixels per
+// instruction.  With u = a dx + b dy and w = b dx + c dy,
+//   d dist2 / d(ndc x, ndc y) = (2u, 2w)
+//   d dist2 / d(cov xx, xy, yy) = -u^2, -2uw, -w^2
+// (uw = b dist2 + dx dy / det written without the cancelling difference), and s
+// = -2 dL/d(dist2).  kSafe leaves out what s = 0 or fac = 0 multiplies, as it
+// may be infinite or NaN.
+template <bool kSafe, int TS>
+__device__ __forceinline__ void reduce_hits(BwdShared<TS>& sm, int w, int lane, int count,
+                                            int slot) {
+  using Sh = BwdShared<TS>;
+  const int h = lane >> 2, q = lane & 3;
+  const SplatRec& hit = sm.splat[slot];
+  const float2 x = hit.x(), y = hit.y();
+  const float2 ca = hit.conic_a(), cb = hit.conic_b(), cc = hit.conic_c();
+  float2 v[9];
+#pragma unroll
+  for (int k = 0; k < 9; ++k) v[k] = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int at = (k >> 1) * 8 + q * 2 + (k & 1);  // group of four pixels
+    const float4 s4 = sm.s[w][h * (Sh::kPitch / 4) + at];
+    const float4 f4 = sm.fac[w][h * (Sh::kPitch / 4) + at];
+    const float4 x4 = sm.npx[w][at], y4 = sm.npy[w][at];
+    const float4 r4 = sm.gr[w][at], g4 = sm.gg[w][at], b4 = sm.gb[w][at];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const float2 s = e ? make_float2(s4.z, s4.w) : make_float2(s4.x, s4.y);
+      const float2 f = e ? make_float2(f4.z, f4.w) : make_float2(f4.x, f4.y);
+      float2 gr = e ? make_float2(r4.z, r4.w) : make_float2(r4.x, r4.y);
+      float2 gg = e ? make_float2(g4.z, g4.w) : make_float2(g4.x, g4.y);
+      float2 gb = e ? make_float2(b4.z, b4.w) : make_float2(b4.x, b4.y);
+      const float2 dx = add2(x, e ? make_float2(x4.z, x4.w) : make_float2(x4.x, x4.y));
+      const float2 dy = add2(y, e ? make_float2(y4.z, y4.w) : make_float2(y4.x, y4.y));
+      float2 u = fma2(dx, ca, mul2(dy, cb));
+      float2 t = fma2(dx, cb, mul2(dy, cc));
+      if (kSafe) {
+        u.x = s.x != 0.f ? u.x : 0.f, u.y = s.y != 0.f ? u.y : 0.f;
+        t.x = s.x != 0.f ? t.x : 0.f, t.y = s.y != 0.f ? t.y : 0.f;
+        gr.x = f.x != 0.f ? gr.x : 0.f, gr.y = f.y != 0.f ? gr.y : 0.f;
+        gg.x = f.x != 0.f ? gg.x : 0.f, gg.y = f.y != 0.f ? gg.y : 0.f;
+        gb.x = f.x != 0.f ? gb.x : 0.f, gb.y = f.y != 0.f ? gb.y : 0.f;
+      }
+      const float2 su = mul2(s, u), st = mul2(s, t);
+      v[0] = fma2(f, gr, v[0]);
+      v[1] = fma2(f, gg, v[1]);
+      v[2] = fma2(f, gb, v[2]);
+      v[3] = add2(v[3], su);
+      v[4] = add2(v[4], st);
+      v[5] = fma2(su, u, v[5]);
+      v[6] = fma2(su, t, v[6]);
+      v[7] = fma2(st, t, v[7]);
+      v[8] = add2(v[8], s);
+    }
+  }
+  float r[9];
+#pragma unroll
+  for (int k = 0; k < 9; ++k) r[k] = v[k].x + v[k].y;
+  r[3] = -r[3];
+  r[4] = -r[4];
+  r[5] *= 0.5f;
+  r[7] *= 0.5f;
+  // sum over the hit's four lanes: lane q ends with values 4 (q & 1) + (q & 2) + {0, 1}
+  const bool b0 = q & 1, b1 = q & 2;
+  float t4[4], t2[2];
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    t4[k] = (b0 ? r[k + 4] : r[k]) + __shfl_xor_sync(0xffffffffu, b0 ? r[k] : r[k + 4], 1);
+#pragma unroll
+  for (int k = 0; k < 2; ++k)
+    t2[k] = (b1 ? t4[k + 2] : t4[k]) + __shfl_xor_sync(0xffffffffu, b1 ? t4[k] : t4[k + 2], 2);
+  float o = r[8] + __shfl_xor_sync(0xffffffffu, r[8], 1);
+  o += __shfl_xor_sync(0xffffffffu, o, 2);
+  if (h < count) {
+    float* dst = &sm.part[w][slot * 9];
+    const int k = (b0 ? 4 : 0) + (b1 ? 2 : 0);
+    dst[k] = t2[0];
+    dst[k + 1] = t2[1];
+    if (q == 0) dst[8] = o == 0.f ? 0.f : o / hit.opacity();  // s carries the opacity
+  }
+}
+
+// Backward of one tile per CTA.  Bound by instruction issue.  Each (hit, pixel)
+// yields two numbers, s (for position, covariance and opacity) and fac (for the
+// colour); the nine gradients of a hit are sums of products of these with
+// values that depend on the pixel or on the splat alone.  So the pixel loop
+// (lane = pixel) only stores s and fac to shared memory, and for every
+// kBwdHits hits the lanes regroup, four to a hit, and form the sums over the
+// pixels (reduce_hits), which costs about 25 issue slots a hit where the
+// nine-value butterfly over the warp took about 60.  Against the butterfly
+// (B200): 1280x720 fit of 60000 splats at step 25 0.366 -> 0.301 ms,
+// at step 400 0.828 -> 0.504; a million splats at 1920x1080 0.656 -> 0.600.
+template <int TS, bool kFusedLoss, bool kExact, bool kBatch>
+__global__ void __launch_bounds__(Lay<TS>::kThreads, Lay<TS>::kMinBlocksBwd)
     composite_bwd_kernel(const float4* __restrict__ ra, const float4* __restrict__ rb,
-                         const float4* __restrict__ rc, const float* __restrict__ ridet,
+                         const float4* __restrict__ rc,
                          const uint32_t* __restrict__ sorted_splat,
                          const uint32_t* __restrict__ seg_start,
                          const ushort4* __restrict__ rect, const int2* __restrict__ ranges,
@@ -454,25 +561,16 @@ __global__ void __launch_bounds__(Lay<PPT, TS>::kThreads, Lay<PPT, TS>::kMinBloc
                          const uint16_t* __restrict__ tile_inst,
                          const InstGeom* __restrict__ geom,
                          const uint32_t* __restrict__ depth_keys,
-                         unsigned long long* __restrict__ tile_bound,
-                         const DevScalars* __restrict__ mode_sc) {
+                         unsigned long long* __restrict__ tile_bound) {
   pdl_wait();
-  using Lc = Lay<PPT, TS>;
+  using Lc = Lay<TS>;
+  using Sh = BwdShared<TS>;
   constexpr int NT = Lc::kThreads;
   constexpr int NW = Lc::kWarps;
   constexpr int B = Lc::kBwdBatch;
-  __shared__ float4 sA[B], sB[B], sC[B];
-  __shared__ float sI[B];
-  __shared__ uint32_t sG[2][B];  // splat ids of the staged batch and the next
-  __shared__ int sRC[2];
-  __shared__ uint32_t sMask[B];
-  __shared__ float4 sBox[NW];
-  __shared__ __align__(16) float part[NW][B * 9];  // per-warp partial of each batch splat
-  __shared__ int32_t sFinal[NW];
+  extern __shared__ __align__(16) unsigned char bwd_smem[];
+  Sh& sm = *reinterpret_cast<Sh*>(bwd_smem);
   const int tile = order ? order[blockIdx.x] : (int)blockIdx.x;
-  // ppt_bwd == 0: the forward chose the layout for this frame; the other
-  // layout's launch returns at once
-  if (mode_sc && (PPT == 2) != (mode_sc->bwd_ppt == 2u)) return;
   const int2 range = ranges[tile];
   const int start = range.x;
   if (range.y <= start) {
@@ -481,47 +579,58 @@ __global__ void __launch_bounds__(Lay<PPT, TS>::kThreads, Lay<PPT, TS>::kMinBloc
   }
   const TileGeo tg = tile_geo<kBatch>(tile, W_, H_, ntx_, tile_inst, geom);
   const int W = tg.W, H = tg.H;
-  const Pixels<PPT> m = pixels<PPT, TS>(tg.local, tg.ntx, W, H);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  if (threadIdx.x == 0) {  // the tile's row and column in its grid, for the record indices
-    sRC[0] = tg.local / tg.ntx;
-    sRC[1] = tg.local - sRC[0] * tg.ntx;
-  }
-  if (lane == 0) sBox[w] = make_float4(m.wx_lo, m.wx_hi, m.wy_lo, m.wy_hi);
-  // acc[k]: over the splats behind (already visited), weight x (colour . dL/dpixel)
-  float T[PPT], gr[PPT], gg[PPT], gb[PPT], acc[PPT];
-  int32_t fin[PPT];
+  const Pixels m = pixels<TS>(tg.local, tg.ntx, W, H, w);
+  // the tile's row and column in its grid, for the record indices
+  const int trow = tg.local / tg.ntx, tcol = tg.local - trow * tg.ntx;
+  if (lane == 0) sm.box[w] = make_float4(m.wx_lo, m.wx_hi, m.wy_lo, m.wy_hi);
+  // acc: over the splats behind (already visited), weight x (colour . dL/dpixel)
+  float2 T, gr, gg, gb, acc = both(0.f);
+  const float2 npx = both(-m.px), npy = make_float2(-m.py[0], -m.py[1]);
+  int32_t fin[2];
   int32_t my_final = -1;
+  bool finite = true;
 #pragma unroll
-  for (int k = 0; k < PPT; ++k) {
+  for (int k = 0; k < 2; ++k) {
     const int pix = tg.pix_off + min(m.i[k] * W + m.j, W * H - 1);
-    T[k] = 1.f - alphas[pix];
+    const float t = 1.f - alphas[pix];
     fin[k] = m.inside[k] ? last_ids[pix] : -1;
     my_final = max(my_final, fin[k]);
-    gr[k] = gg[k] = gb[k] = 0.f;
+    float r = 0.f, g = 0.f, b = 0.f;
     if (m.inside[k]) {
       if (kFusedLoss) {
         const float scale = 2.f / (float)(W * H);
-        gr[k] = scale * (grad_or_image[pix * 3 + 0] - target[pix * 3 + 0]);
-        gg[k] = scale * (grad_or_image[pix * 3 + 1] - target[pix * 3 + 1]);
-        gb[k] = scale * (grad_or_image[pix * 3 + 2] - target[pix * 3 + 2]);
+        r = scale * (grad_or_image[pix * 3 + 0] - target[pix * 3 + 0]);
+        g = scale * (grad_or_image[pix * 3 + 1] - target[pix * 3 + 1]);
+        b = scale * (grad_or_image[pix * 3 + 2] - target[pix * 3 + 2]);
       } else {
-        gr[k] = grad_or_image[pix * 3 + 0];
-        gg[k] = grad_or_image[pix * 3 + 1];
-        gb[k] = grad_or_image[pix * 3 + 2];
+        r = grad_or_image[pix * 3 + 0];
+        g = grad_or_image[pix * 3 + 1];
+        b = grad_or_image[pix * 3 + 2];
       }
+      finite = finite && fabsf(r) <= 3.0e38f && fabsf(g) <= 3.0e38f && fabsf(b) <= 3.0e38f;
     }
-    acc[k] = 0.f;
+    (k ? T.y : T.x) = t;
+    (k ? gr.y : gr.x) = r;
+    (k ? gg.y : gg.x) = g;
+    (k ? gb.y : gb.x) = b;
   }
+  // pixel k of lane l is value 2 l + k of the warp's tables
+  reinterpret_cast<float2*>(sm.npx[w])[lane] = npx;
+  reinterpret_cast<float2*>(sm.npy[w])[lane] = npy;
+  reinterpret_cast<float2*>(sm.gr[w])[lane] = gr;
+  reinterpret_cast<float2*>(sm.gg[w])[lane] = gg;
+  reinterpret_cast<float2*>(sm.gb[w])[lane] = gb;
+  const bool safe_pixels = __all_sync(0xffffffffu, finite);
   const int32_t warp_final = warp_max(my_final);
   // Pairs after the tile's last contributing splat reach no pixel: the list
   // ends there for the backward, and no record is written for them (their
   // consumers skip them by tile_bound).
-  if (lane == 0) sFinal[w] = warp_final;
+  if (lane == 0) sm.final_id[w] = warp_final;
   __syncthreads();
-  int32_t tile_final = sFinal[0];
+  int32_t tile_final = sm.final_id[0];
 #pragma unroll
-  for (int k = 1; k < NW; ++k) tile_final = max(tile_final, sFinal[k]);
+  for (int k = 1; k < NW; ++k) tile_final = max(tile_final, sm.final_id[k]);
   const int end = min(range.y, tile_final + 1);
   if (threadIdx.x == 0) {
     unsigned long long bound = 0ull;
@@ -538,6 +647,7 @@ __global__ void __launch_bounds__(Lay<PPT, TS>::kThreads, Lay<PPT, TS>::kMinBloc
   constexpr int kSplit = NT >= 2 * B ? 2 : 1;
   constexpr int R = (B * kSplit + NT - 1) / NT;  // splats each thread stages
   Staged pf[R];
+  uint32_t pf_rec[R];
   // batch bi holds sorted indices end - 1 - B bi down to end - B (bi + 1)
   auto prefetch = [&](int bi) {
     const int batch_end = end - 1 - B * bi;
@@ -550,11 +660,19 @@ __global__ void __launch_bounds__(Lay<PPT, TS>::kThreads, Lay<PPT, TS>::kMinBloc
         pf[r].a = ra[g];
         pf[r].b = rb[g];
         pf[r].c = rc[g];
-        pf[r].idet = ridet[g];
-        if ((threadIdx.x + r * NT) % kSplit == 0) sG[bi & 1][l] = g;
+        if ((threadIdx.x + r * NT) % kSplit == 0) {
+          // the pair's emission index: the splat's first one plus the tile's
+          // row-major index in the splat's tile rectangle
+          const ushort4 t = rect[g];
+          pf_rec[r] = seg_start[g] + (uint32_t)(trow - t.z) * (uint32_t)(t.y - t.x + 1) +
+                      (uint32_t)(tcol - t.x);
+        }
       }
     }
   };
+  if (threadIdx.x == 0) sm.splat[B].set_none();
+  float* const my_s = reinterpret_cast<float*>(sm.s[w]) + 2 * lane;
+  float* const my_f = reinterpret_cast<float*>(sm.fac[w]) + 2 * lane;
   prefetch(0);
   for (int bi = 0; bi < nb; ++bi) {
     const int batch_end = end - 1 - B * bi;  // farthest splat of the batch
@@ -566,206 +684,168 @@ __global__ void __launch_bounds__(Lay<PPT, TS>::kThreads, Lay<PPT, TS>::kMinBloc
       const int slot = threadIdx.x + r * NT, l = slot / kSplit, h = slot % kSplit;
       uint32_t mk = 0u;
       if (l < B && pf[r].ok) {
+        const float4 a = pf[r].a, b = pf[r].b, c = pf[r].c;
         if (kSplit == 1) {
-          mk = warp_hits<NW>(pf[r].a, pf[r].b, pf[r].c.w, sBox);
+          mk = warp_hits<NW>(a, b, c.w, sm.box);
         } else {
           // this thread tests half of the warp blocks
 #pragma unroll
           for (int k = 0; k < NW / 2; ++k) {
             const int wb = h * (NW / 2) + k;
-            mk |= ellipse_hits(pf[r].a, pf[r].b, pf[r].c.w, sBox[wb]) ? (1u << wb) : 0u;
+            mk |= ellipse_hits(a, b, c.w, sm.box[wb]) ? (1u << wb) : 0u;
           }
         }
         if (h == 0) {
-          sA[l] = pf[r].a;
-          sB[l] = pf[r].b;
-          sC[l] = pf[r].c;
-          sI[l] = pf[r].idet;
+          sm.splat[l].set(a, b, c, 0);
+          sm.rec[l] = pf_rec[r];
         }
       }
       if (kSplit == 2) mk |= __shfl_xor_sync(0xffffffffu, mk, 1);  // pairs are adjacent lanes
-      if (l < B && h == 0) sMask[l] = mk;
+      if (l < B && h == 0) sm.mask[l] = mk;
     }
     if (bi + 1 < nb) prefetch(bi + 1);
-    {
-      float4* p4 = reinterpret_cast<float4*>(&part[0][0]);
-      for (int q = threadIdx.x; q < NW * B * 9 / 4; q += NT) p4[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
     __syncthreads();
     const int t_start = max(0, batch_end - warp_final);
-    for (int kw = 0; kw * 32 < bs; ++kw) {
-      const int l = kw * 32 + lane;
-      uint32_t word =
-          __ballot_sync(0xffffffffu, l >= t_start && l < bs && ((sMask[l] >> w) & 1u));
-      // Hits are taken Lc::kBwdGroup at a time: the conic / exp / alpha of all of
-      // them first (independent of T), then the recurrence back to front, then
-      // the warp reductions, which overlap.
-      while (word) {
-        int tg[Lc::kBwdGroup];
-        int ng = 0;
+    int* const list = reinterpret_cast<int*>(sm.list[w]);
+    const int hits = list_hits(sm.mask, w, lane, t_start, bs, B, list);
+    if (lane < B / 32) sm.got[w][lane] = 0u;
+    __syncwarp();
+    int count = 0, slot = 0;  // hits stored; the slot of this lane's hit (lane / 4)
+    auto flush = [&] {
+      __syncwarp();
+      bool tame = true;
+      if ((lane >> 2) < count) {
+        const SplatRec& r = sm.splat[slot];
+        tame = fabsf(r.conic_a().x) <= 1e30f && fabsf(r.conic_b().x) <= 1e30f &&
+               fabsf(r.conic_c().x) <= 1e30f;
+        if ((lane & 3) == 0) atomicOr(&sm.got[w][slot >> 5], 1u << (slot & 31));
+      }
+      if (safe_pixels && __all_sync(0xffffffffu, tame))
+        reduce_hits<false, TS>(sm, w, lane, count, slot);
+      else
+        reduce_hits<true, TS>(sm, w, lane, count, slot);
+      count = 0;
+      __syncwarp();
+    };
+    // The hits two at a time: conic, exp and alpha of both first (independent of
+    // T), then the recurrence back to front.
+    for (int i = 0; i < hits; i += 2) {
+      const int2 pair = sm.list[w][i >> 1];
+      float2 oe[2], al[2];
+      bool any[2];
 #pragma unroll
-        for (int g = 0; g < Lc::kBwdGroup; ++g) {
-          tg[g] = word ? kw * 32 + __ffs(word) - 1 : tg[0];  // word is warp-uniform
-          ng += word ? 1 : 0;
-          word &= word - 1u;
-        }
-        float4 ag[Lc::kBwdGroup], bg[Lc::kBwdGroup], cg[Lc::kBwdGroup];
-        float ig[Lc::kBwdGroup];
+      for (int g = 0; g < 2; ++g) {
+        const int t = g ? pair.y : pair.x, id = batch_end - t;
+        const SplatRec& r = sm.splat[t];
+        const float2 dx = add2(r.x(), npx);
+        bool o0, o1;
+        oe[g] = pair_opacity(add2(dx, dx), mul2(dx, dx), add2(r.y(), npy), r, o0, o1);
+        const float a0 = fminf(kMaxAlpha, oe[g].x), a1 = fminf(kMaxAlpha, oe[g].y);
+        o0 = o0 && id <= fin[0] && !(a0 < kAlphaThres);
+        o1 = o1 && id <= fin[1] && !(a1 < kAlphaThres);
+        // alpha 0: the splat is skipped at that pixel
+        al[g] = make_float2(o0 ? a0 : 0.f, o1 ? a1 : 0.f);
+        any[g] = o0 || o1;
+      }
 #pragma unroll
-        for (int g = 0; g < Lc::kBwdGroup; ++g) {
-          ag[g] = sA[tg[g]];
-          bg[g] = sB[tg[g]];
-          cg[g] = sC[tg[g]];
-          ig[g] = sI[tg[g]];
-        }
-        float v[Lc::kBwdGroup][8], va[Lc::kBwdGroup];
-        bool any[Lc::kBwdGroup];
-#pragma unroll
-        for (int g = 0; g < Lc::kBwdGroup; ++g) {
-#pragma unroll
-          for (int q = 0; q < 8; ++q) v[g][q] = 0.f;
-          va[g] = 0.f;
-          any[g] = false;
-        }
-#pragma unroll
-        for (int k = 0; k < PPT; ++k) {
-          if (!m.inside[k]) continue;
-          float dxg[Lc::kBwdGroup], dyg[Lc::kBwdGroup], d2g[Lc::kBwdGroup], eg[Lc::kBwdGroup], alg[Lc::kBwdGroup];
-          bool pg[Lc::kBwdGroup];
-#pragma unroll
-          for (int g = 0; g < Lc::kBwdGroup; ++g) {
-            dxg[g] = ag[g].x - m.px;
-            dyg[g] = ag[g].y - m.py[k];
-            d2g[g] = conic_dist2(dxg[g], dyg[g], bg[g].x, bg[g].y, bg[g].z);
-            const float sigma = 0.5f * d2g[g];
-            eg[g] = __expf(-sigma);
-            alg[g] = fminf(kMaxAlpha, bg[g].w * eg[g]);
-            pg[g] = g < ng && batch_end - tg[g] <= fin[k] && !(sigma < 0.f) &&
-                    !(alg[g] < kAlphaThres);
-          }
-#pragma unroll
-          for (int g = 0; g < Lc::kBwdGroup; ++g) {
-            if (!pg[g]) continue;
-            const float4 b = bg[g], c = cg[g];
-            const float dx = dxg[g], dy = dyg[g], dist2 = d2g[g], g_exp = eg[g], alpha = alg[g];
-            const float opac = b.w;
-            any[g] = true;
-            const float T_before = T[k] / fmaxf(1.f - alpha, 1e-6f);
-            const float fac = alpha * T_before;
-            v[g][0] += fac * gr[k];
-            v[g][1] += fac * gg[k];
-            v[g][2] += fac * gb[k];
-            // Reference recurrence (tile_rasterize_layer.cu:518-521) weighs the
-            // colour behind (absolute weights c_j alpha_j T_j) by T_before; the
-            // exact derivative divides it by T_after instead.  The three
-            // colour channels enter only through their dot product with
-            // dL/dpixel.
-            const float cg_k = c.x * gr[k] + c.y * gg[k] + c.z * gb[k];
-            const float ia = kExact ? 1.f / T[k] : 1.f;
-            const float v_alpha = T_before * (cg_k - acc[k] * ia);
-            if (opac * g_exp <= kMaxAlpha) {
-              va[g] += g_exp * v_alpha;
-              // s = -2 dL/d(dist2).  With u = dx bx + dy by and w = dx by + dy
-              // bz, d dist2 / d(ndc x, ndc y) = (2u, 2w) and d dist2 / d(conic)
-              // gives the Cov2D terms -u^2, -w^2 and -2 (by dist2 + dx dy idet).
-              const float s = opac * g_exp * v_alpha;
-              const float u = dx * b.x + dy * b.y;
-              const float wv = dx * b.y + dy * b.z;
-              v[g][3] -= s * u;
-              v[g][4] -= s * wv;
-              const float hs = 0.5f * s;
-              v[g][5] += hs * u * u;
-              v[g][7] += hs * wv * wv;
-              v[g][6] += s * (b.y * dist2 + dx * dy * ig[g]);
-            }
-            acc[k] += cg_k * fac;
-            T[k] = T_before;
-          }
-        }
-        bool hit_any[Lc::kBwdGroup];
-#pragma unroll
-        for (int g = 0; g < Lc::kBwdGroup; ++g) hit_any[g] = __any_sync(0xffffffffu, any[g]);
-        if (Lc::kBwdGroup == 2 && hit_any[0] && hit_any[Lc::kBwdGroup - 1]) {
-          // both hits contributed: one butterfly for their 2 x 9 sums
-          const float s16 = warp_sum16_transposed(v[0], v[Lc::kBwdGroup - 1], lane);
-          const float s2 = warp_sum2_transposed(va[0], va[Lc::kBwdGroup - 1], lane);
-          const int gh = lane >> 4;
-          if ((lane & 1) == 0) part[w][tg[gh] * 9 + ((lane >> 1) & 7)] = s16;
-          if ((lane & 15) == 0) part[w][tg[gh] * 9 + 8] = s2;
-        } else {
-#pragma unroll
-          for (int g = 0; g < Lc::kBwdGroup; ++g) {
-            if (!hit_any[g]) continue;
-            // lane 4q ends up with the warp sum of v[q]
-            const float s8 = warp_sum8_transposed(v[g], lane);
-            const float sa = warp_sum(va[g]);
-            if ((lane & 3) == 0) part[w][tg[g] * 9 + (lane >> 2)] = s8;
-            if (lane == 0) part[w][tg[g] * 9 + 8] = sa;
-          }
-        }
+      for (int g = 0; g < 2; ++g) {
+        if (!__any_sync(0xffffffffu, any[g])) continue;
+        const int t = g ? pair.y : pair.x;
+        const SplatRec& r = sm.splat[t];
+        const float2 blue = *reinterpret_cast<const float2*>(&r.blue);
+        const bool o0 = al[g].x > 0.f, o1 = al[g].y > 0.f;
+        const float2 om = fma2(al[g], both(-1.f), both(1.f));  // >= 0.01
+        const float2 Tb = mul2(T, make_float2(__fdividef(1.f, om.x), __fdividef(1.f, om.y)));
+        const float2 fac = mul2(al[g], Tb);
+        // Reference recurrence (tile_rasterize_layer.cu:518-521) weighs the
+        // colour behind (absolute weights c_j alpha_j T_j) by T_before; the
+        // exact derivative divides it by T_after instead.  The three colour
+        // channels enter only through their dot product with dL/dpixel.
+        const float2 lit = fma2(blue, gb, fma2(r.red(), gr, mul2(r.green(), gg)));
+        const float2 nia = kExact ? make_float2(-1.f / T.x, -1.f / T.y) : both(-1.f);
+        const float2 s2 = mul2(oe[g], mul2(Tb, fma2(acc, nia, lit)));
+        const float2 next = fma2(lit, fac, acc);
+        float2 s;
+        s.x = o0 && oe[g].x <= kMaxAlpha ? s2.x : 0.f;
+        s.y = o1 && oe[g].y <= kMaxAlpha ? s2.y : 0.f;
+        acc = make_float2(o0 ? next.x : acc.x, o1 ? next.y : acc.y);
+        T = make_float2(o0 ? Tb.x : T.x, o1 ? Tb.y : T.y);
+        *reinterpret_cast<float2*>(my_s + count * Sh::kPitch) = s;
+        *reinterpret_cast<float2*>(my_f + count * Sh::kPitch) = fac;
+        if ((lane >> 2) == count) slot = t;
+        if (++count == kBwdHits) flush();
       }
     }
+    if (count > 0) flush();
     __syncthreads();
-    const int trow = sRC[0], tcol = sRC[1];
-    for (int slot = threadIdx.x; slot < bs * kSplit; slot += NT) {
-      const int l = slot / kSplit, h = slot % kSplit;
-      // the pair's emission index: the splat's first one plus the tile's
-      // row-major index in the splat's tile rectangle
-      const uint32_t g = sG[bi & 1][l];
-      const ushort4 r = rect[g];
-      const uint32_t e = seg_start[g] + (uint32_t)(trow - r.z) * (uint32_t)(r.y - r.x + 1) +
-                         (uint32_t)(tcol - r.x);
-      float* dst = isect_grad + (size_t)e * 9;
+    for (int slot2 = threadIdx.x; slot2 < bs * kSplit; slot2 += NT) {
+      const int l = slot2 / kSplit, h = slot2 % kSplit;
+      float* dst = isect_grad + (size_t)sm.rec[l] * 9;
+      float v[(9 + kSplit - 1) / kSplit];
 #pragma unroll
-      for (int q = h; q < 9; q += kSplit) {
-        float s = 0.f;
+      for (int q = 0; q < (9 + kSplit - 1) / kSplit; ++q) v[q] = 0.f;
 #pragma unroll
-        for (int ww = 0; ww < NW; ++ww) s += part[ww][l * 9 + q];
-        dst[q] = s;
+      for (int ww = 0; ww < NW; ++ww) {
+        if (!(sm.got[ww][l >> 5] >> (l & 31) & 1u)) continue;
+#pragma unroll
+        for (int q = h; q < 9; q += kSplit) v[q / kSplit] += sm.part[ww][l * 9 + q];
       }
+#pragma unroll
+      for (int q = h; q < 9; q += kSplit) dst[q] = v[q / kSplit];
     }
   }
+}
+
+// Lets a kernel use `bytes` of dynamic shared memory, once per device (`set`: the
+// devices done).
+template <class K>
+void allow_smem(K kernel, int bytes, std::atomic<uint64_t>& set) {
+  int dev = 0;
+  if (bytes <= 48 * 1024 || cudaGetDevice(&dev) != cudaSuccess) return;
+  if (dev < 64 && (set.load() >> dev & 1u)) return;
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (dev < 64) set.fetch_or(1ull << dev);
 }
 
 const int32_t* schedule(const RasterBuffers& rb) {
   return rb.schedule == DS_SCHEDULE_LONGEST_FIRST ? rb.tile_order : nullptr;
 }
 
-// Whether the forward chooses the backward's layout (see kDenseLanesX10).
-bool adaptive_bwd(const RasterBuffers& rb) {
-  return rb.ppt_bwd == 0 && rb.ppt == 1 && !rb.geom;
-}
-
-template <int PPT, int TS, bool kBatch>
+template <int TS, bool kBatch>
 void launch_fwd(RasterBuffers& rb, float* out_rgb, const float* target, bool count,
                 cudaStream_t s) {
-  constexpr int NT = Lay<PPT, TS>::kThreads;
+  constexpr int kBlocks = (TS / 8) * (TS / 8);
   const int32_t* order = schedule(rb);
-  DevScalars* mode = (!count && PPT == 1 && adaptive_bwd(rb)) ? rb.scalars : nullptr;
+  const dim3 grid((unsigned)(((int64_t)rb.tiles * kBlocks + kFwdWarps - 1) / kFwdWarps));
 #define DS_FWD(L, C)                                                                         \
-  launch_pdl(composite_fwd_kernel<PPT, TS, L, C, kBatch>, dim3(rb.tiles), dim3(NT), 0, s,     \
+  launch_pdl(composite_fwd_kernel<TS, L, C, kBatch>, grid, dim3(32 * kFwdWarps), 0, s,       \
              rb.rec_a, rb.rec_b, rb.rec_c, rb.sorted_splat, rb.ranges, order, out_rgb,        \
-             rb.alphas, rb.last_ids, rb.width, rb.height, rb.ntx, rb.tile_inst, rb.geom,      \
-             L ? target : nullptr, L ? rb.loss_partials : nullptr, rb.scalars, mode)
+             rb.alphas, rb.last_ids, rb.tiles, rb.width, rb.height, rb.ntx, rb.tile_inst,     \
+             rb.geom, L ? target : nullptr, L ? rb.loss_partials : nullptr, rb.scalars)
   if (count) DS_FWD(false, true);
   else if (target) DS_FWD(true, false);
   else DS_FWD(false, false);
 #undef DS_FWD
 }
 
-template <int PPT, int TS, bool kBatch>
+template <int TS, bool kBatch>
 void launch_bwd(RasterBuffers& rb, const float* image, const float* grad_rgb, const float* target,
-                cudaStream_t s, const DevScalars* mode = nullptr) {
-  constexpr int NT = Lay<PPT, TS>::kThreads;
+                cudaStream_t s) {
+  constexpr int NT = Lay<TS>::kThreads;
   const float* g = grad_rgb ? grad_rgb : image;
   const float* t = grad_rgb ? nullptr : target;
   const bool exact = rb.grad_mode == DS_GRAD_EXACT;
   const int32_t* order = schedule(rb);
+  constexpr int smem = (int)sizeof(BwdShared<TS>);
 #define DS_BWD(F, E)                                                                         \
-  launch_pdl(composite_bwd_kernel<PPT, TS, F, E, kBatch>, dim3(rb.tiles), dim3(NT), 0, s,     \
-             rb.rec_a, rb.rec_b, rb.rec_c, rb.rec_idet, rb.sorted_splat, rb.seg_start, rb.rect,\
-             rb.ranges, order, rb.alphas, rb.last_ids, g, t, rb.isect_grad, rb.width,         \
-             rb.height, rb.ntx, rb.tile_inst, rb.geom, rb.depth_keys, rb.tile_bound, mode)
+  do {                                                                                       \
+    static std::atomic<uint64_t> set{0};                                                     \
+    allow_smem(composite_bwd_kernel<TS, F, E, kBatch>, smem, set);                           \
+    launch_pdl(composite_bwd_kernel<TS, F, E, kBatch>, dim3(rb.tiles), dim3(NT), smem, s,    \
+               rb.rec_a, rb.rec_b, rb.rec_c, rb.sorted_splat, rb.seg_start, rb.rect,         \
+               rb.ranges, order, rb.alphas, rb.last_ids, g, t, rb.isect_grad, rb.width,      \
+               rb.height, rb.ntx, rb.tile_inst, rb.geom, rb.depth_keys, rb.tile_bound);      \
+  } while (0)
   if (grad_rgb) {
     if (exact) DS_BWD(false, true);
     else DS_BWD(false, false);
@@ -776,81 +856,16 @@ void launch_bwd(RasterBuffers& rb, const float* image, const float* grad_rgb, co
 #undef DS_BWD
 }
 
-struct FwdOp {
-  RasterBuffers& rb;
-  float* out_rgb;
-  const float* target;
-  bool count;
-  cudaStream_t s;
-  template <int P, int T, bool B>
-  void run() const {
-    launch_fwd<P, T, B>(rb, out_rgb, target, count, s);
-  }
-};
-
-struct BwdOp {
-  RasterBuffers& rb;
-  const float* image;
-  const float* grad_rgb;
-  const float* target;
-  cudaStream_t s;
-  template <int P, int T, bool B>
-  void run() const {
-    launch_bwd<P, T, B>(rb, image, grad_rgb, target, s);
-  }
-};
-
-// Single instance: 16x16 tiles, PPT 1, 2 or 4.  Batch: tiles of 8, 16 or 32
-// pixels with PPT 1 or 2.
-template <class F>
-int dispatch(const RasterBuffers& rb, const F& f, bool backward = false) {
-  const int ppt = (backward && rb.ppt_bwd != 0) ? rb.ppt_bwd : rb.ppt;
-  if (!rb.geom) {
-    switch (ppt) {
-      case 4: f.template run<4, 16, false>(); return DS_OK;
-      case 2: f.template run<2, 16, false>(); return DS_OK;
-      default: f.template run<1, 16, false>(); return DS_OK;
-    }
-  }
-  const bool two = ppt == 2;
-  switch (rb.tile_size) {
-    case 8:
-      if (two) f.template run<2, 8, true>();
-      else f.template run<1, 8, true>();
-      return DS_OK;
-    case 32:
-      if (two) f.template run<2, 32, true>();
-      else f.template run<1, 32, true>();
-      return DS_OK;
-    default:
-      if (two) f.template run<2, 16, true>();
-      else f.template run<1, 16, true>();
-      return DS_OK;
-  }
+// Single instance: 16-pixel tiles.  Batch: tiles of 8, 16 or 32 pixels.
+void forward(RasterBuffers& rb, float* out_rgb, const float* target, bool count,
+             cudaStream_t s) {
+  if (!rb.geom) launch_fwd<16, false>(rb, out_rgb, target, count, s);
+  else if (rb.tile_size == 8) launch_fwd<8, true>(rb, out_rgb, target, count, s);
+  else if (rb.tile_size == 32) launch_fwd<32, true>(rb, out_rgb, target, count, s);
+  else launch_fwd<16, true>(rb, out_rgb, target, count, s);
 }
 
 }  // namespace
-
-int composite_default_ppt() {
-  const char* e = getenv("DS_COMPOSITE_PPT");
-  if (e) {
-    int v = atoi(e);
-    if (v == 1 || v == 2 || v == 4) return v;
-  }
-  // Fastest on the 1280x720 / 60000-splat fitter with the longest-first tile
-  // schedule (B200, 1000 steps: 1 -> 688, 2 -> 631, 4 -> 454 steps/s).
-  return 1;
-}
-
-int composite_default_ppt_bwd() {
-  const char* e = getenv("DS_COMPOSITE_PPT_BWD");
-  if (e) {
-    int v = atoi(e);
-    if (v == 1 || v == 2 || v == 4) return v;
-  }
-  // chosen per forward (kDenseLanesX10) behind a one-pixel-per-thread forward
-  return composite_default_ppt() == 1 ? 0 : composite_default_ppt();
-}
 
 bool composite_longest_first() {
   static const bool on = [] {
@@ -862,25 +877,22 @@ bool composite_longest_first() {
 
 int raster_composite_forward(RasterBuffers& rb, float* out_rgb, const float* target,
                              cudaStream_t s) {
-  dispatch(rb, FwdOp{rb, out_rgb, target, false, s});
+  forward(rb, out_rgb, target, false, s);
   return cuda_status(cudaGetLastError());
 }
 
 int raster_composite_count(RasterBuffers& rb, float* out_rgb, cudaStream_t s) {
   DS_CUDA(cudaMemsetAsync(rb.scalars->pairs, 0, sizeof(rb.scalars->pairs), s));
-  dispatch(rb, FwdOp{rb, out_rgb, nullptr, true, s});
+  forward(rb, out_rgb, nullptr, true, s);
   return cuda_status(cudaGetLastError());
 }
 
 int raster_composite_backward(RasterBuffers& rb, const float* image, const float* grad_rgb,
                               const float* target, cudaStream_t s) {
-  if (adaptive_bwd(rb)) {
-    // the launch of the layout the forward chose does the work
-    launch_bwd<2, 16, false>(rb, image, grad_rgb, target, s, rb.scalars);
-    launch_bwd<1, 16, false>(rb, image, grad_rgb, target, s, rb.scalars);
-  } else {
-    dispatch(rb, BwdOp{rb, image, grad_rgb, target, s}, true);
-  }
+  if (!rb.geom) launch_bwd<16, false>(rb, image, grad_rgb, target, s);
+  else if (rb.tile_size == 8) launch_bwd<8, true>(rb, image, grad_rgb, target, s);
+  else if (rb.tile_size == 32) launch_bwd<32, true>(rb, image, grad_rgb, target, s);
+  else launch_bwd<16, true>(rb, image, grad_rgb, target, s);
   return cuda_status(cudaGetLastError());
 }
 

@@ -158,11 +158,6 @@ struct DevScalars {
   float loss;
   float pad2;
   unsigned long long pairs[2];  // counting forward: contributing, tested (pixel, splat) pairs
-  // Backward layout of the last forward (ppt_bwd == 0): its hits and their
-  // contributing lanes summed over the CTAs, the last CTA's decision
-  unsigned long long mode_hits, mode_lanes;
-  uint32_t mode_ticket;
-  uint32_t bwd_ppt;  // 2: two pixels per thread; otherwise one
 };
 
 // ---------------------------------------------------------------------------
@@ -175,16 +170,14 @@ struct InstGeom {
   int tile_off, pix_off, splat_off, count;
 };
 
+// Loss partials of a tile: one per four 8x8 blocks of its composite forward.
+constexpr int loss_parts(int tile_size) { return tile_size == 32 ? 4 : 1; }
+
 struct RasterBuffers {
   int width = 0, height = 0, ntx = 0, nty = 0, tiles = 0;
   int max_splats = 0;
   int64_t cap = 0;  // intersection capacity
   int grad_mode = DS_GRAD_REFERENCE;
-  int ppt = 2;      // pixels per thread of the composite forward (1, 2 or 4)
-  // pixels per thread of the composite backward (1, 2 or 4), or 0: chosen
-  // per forward, 2 when its hits covered the warps' pixel blocks densely and 1
-  // otherwise (single-instance 16-pixel tiles; DevScalars::bwd_ppt)
-  int ppt_bwd = 2;
   int schedule = DS_SCHEDULE_LONGEST_FIRST;  // composite tile order
   int tile_size = 16;  // pixels per tile edge: 16 (reference); batches may use 8 or 32
 
@@ -200,7 +193,6 @@ struct RasterBuffers {
   float4* rec_a = nullptr;
   float4* rec_b = nullptr;
   float4* rec_c = nullptr;
-  float* rec_idet = nullptr;
   ushort4* rect = nullptr;     // tile rectangle {x0, x1, y0, y1}
   uint32_t* counts = nullptr;  // tiles per splat (0 = invisible)
   uint32_t* seg_start = nullptr;  // first emission index of each splat
@@ -241,7 +233,7 @@ struct RasterBuffers {
   int32_t* tile_order = nullptr;  // composite schedule: tiles by descending list length
   float* alphas = nullptr;
   int32_t* last_ids = nullptr;
-  float* loss_partials = nullptr;  // [tiles]
+  float* loss_partials = nullptr;  // [tiles * loss_parts(tile_size)]
 
   DevScalars* scalars = nullptr;
 
@@ -292,10 +284,6 @@ __device__ __forceinline__ void seg_origin(const GradSegments& g, uint32_t i, co
 #endif
 
 int raster_alloc(RasterBuffers& rb, int width, int height, int max_splats, int64_t cap);
-// Pixels per thread of the composite kernels; DS_COMPOSITE_PPT=1|2|4 overrides
-// the default (a tuning knob: results are identical for every value).
-int composite_default_ppt();
-int composite_default_ppt_bwd();
 // Composite CTA schedule: longest tile lists first (default) or raster order
 // (DS_TILE_SCHEDULE=raster).
 bool composite_longest_first();

@@ -39,12 +39,12 @@ constexpr int kMaxDevices = 64;
 
 constexpr size_t up256(size_t b) { return (b + 255) / 256 * 256; }
 
-// Sub-buffers, in carving order: 13 per-splat arrays (16 B per splat each,
+// Sub-buffers, in carving order: 12 per-splat arrays (16 B per splat each,
 // enough for the widest), 6 per-pair arrays, 2 per-pixel arrays, tile ranges,
-// sort histogram, scan partials and the device scalars: about 5.7 MB.
+// sort histogram, scan partials and the device scalars: about 5.6 MB.
 constexpr size_t kIsectBytes = 4 * (size_t)kMaxIsects;  // each of 6 pair arrays
 constexpr size_t kTotalBytes =
-    13 * up256(16 * (size_t)kMaxSplats) +
+    12 * up256(16 * (size_t)kMaxSplats) +
     6 * up256(kIsectBytes) + 2 * up256(4 * (size_t)kMaxPixels) + up256(8 * (size_t)kMaxTiles) +
     up256(4 * 256 * ((size_t)kSortBlocks + 1)) + up256(8 * ((size_t)kSortBlocks + 1)) +
     up256(sizeof(DevScalars));
@@ -150,13 +150,10 @@ extern "C" int ds_raster_forward_noalloc(const ds_splat2d* in, int width, int he
   rb.tiles = ntx * nty;
   rb.max_splats = kMaxSplats;
   rb.cap = kMaxIsects;
-  rb.ppt = composite_default_ppt();
-  rb.ppt_bwd = rb.ppt;  // forward only: no backward layout to choose
   const size_t n = kMaxSplats;
   rb.rec_a = c.take<float4>(16 * n);
   rb.rec_b = c.take<float4>(16 * n);
   rb.rec_c = c.take<float4>(16 * n);
-  rb.rec_idet = c.take<float>(16 * n);
   rb.rect = c.take<ushort4>(16 * n);
   rb.counts = c.take<uint32_t>(16 * n);
   rb.seg_start = c.take<uint32_t>(16 * n);

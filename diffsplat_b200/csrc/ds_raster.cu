@@ -38,7 +38,7 @@ __device__ __forceinline__ void count_visible(bool vis, uint32_t* visible) {
 // Splat2D SoA -> records / rectangles / counts / depth keys (layer-API path).
 __global__ void __launch_bounds__(kThreads)
     prep_splat2d_kernel(ds_splat2d in, int n, int W, int H, int ntx, int nty, float4* ra,
-                        float4* rb, float4* rc, float* ridet, ushort4* rect, uint32_t* counts,
+                        float4* rb, float4* rc, ushort4* rect, uint32_t* counts,
                         uint32_t* depth_keys, DevScalars* sc) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i == 0) sc->n_splats = (uint32_t)n;
@@ -54,7 +54,6 @@ __global__ void __launch_bounds__(kThreads)
       ra[i] = rec.a;
       rb[i] = rec.b;
       rc[i] = rec.c;
-      ridet[i] = rec.idet;
       rect[i] = make_ushort4(r.x0, r.x1, r.y0, r.y1);
       counts[i] = (uint32_t)((r.x1 - r.x0 + 1) * (r.y1 - r.y0 + 1));
       depth_keys[i] = depth_bits(z);
@@ -668,14 +667,11 @@ static int raster_alloc_splats(RasterBuffers& rb, int max_splats, int64_t cap) {
   if (cap > ((int64_t)1 << 31)) return DS_ERR_ARG;
   rb.max_splats = max_splats;
   rb.cap = cap;
-  rb.ppt = composite_default_ppt();
-  rb.ppt_bwd = composite_default_ppt_bwd();
   rb.schedule = composite_longest_first() ? DS_SCHEDULE_LONGEST_FIRST : DS_SCHEDULE_RASTER;
   const size_t n = (size_t)max_splats;
   DS_TRY(alloc(&rb.rec_a, n));
   DS_TRY(alloc(&rb.rec_b, n));
   DS_TRY(alloc(&rb.rec_c, n));
-  DS_TRY(alloc(&rb.rec_idet, n));
   DS_TRY(alloc(&rb.rect, n));
   DS_TRY(alloc(&rb.counts, n));
   DS_TRY(alloc(&rb.seg_start, n));
@@ -755,7 +751,7 @@ int raster_alloc_batch(RasterBuffers& rb, int64_t pixels, int tiles, int tile_si
   DS_TRY(alloc(&rb.tile_order, (size_t)tiles));
   DS_TRY(alloc(&rb.alphas, (size_t)pixels));
   DS_TRY(alloc(&rb.last_ids, (size_t)pixels));
-  DS_TRY(alloc(&rb.loss_partials, (size_t)tiles));
+  DS_TRY(alloc(&rb.loss_partials, (size_t)tiles * loss_parts(tile_size)));
   DS_CUDA(cudaMemset(rb.ranges, 0, tiles * sizeof(int2)));
   return alloc_count_sort(rb);
 }
@@ -790,7 +786,6 @@ void raster_free(RasterBuffers& rb) {
   release(rb.rec_a);
   release(rb.rec_b);
   release(rb.rec_c);
-  release(rb.rec_idet);
   release(rb.rect);
   release(rb.counts);
   release(rb.seg_start);
@@ -830,7 +825,7 @@ int raster_prepare_from_splat2d(RasterBuffers& rb, const ds_splat2d& in, cudaStr
   DS_CUDA(cudaMemsetAsync(&rb.scalars->visible, 0, sizeof(uint32_t), s));
   const int blocks = n > 0 ? (n + kThreads - 1) / kThreads : 1;
   prep_splat2d_kernel<<<blocks, kThreads, 0, s>>>(in, n, rb.width, rb.height, rb.ntx, rb.nty,
-                                                  rb.rec_a, rb.rec_b, rb.rec_c, rb.rec_idet,
+                                                  rb.rec_a, rb.rec_b, rb.rec_c,
                                                   rb.rect, rb.counts, rb.depth_keys, rb.scalars);
   return cuda_status(cudaGetLastError());
 }

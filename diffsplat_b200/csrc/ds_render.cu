@@ -130,12 +130,12 @@ int ds_renderer_render(ds_renderer* r, const float pv[16], const float cam_pos[3
     if (r->storage == DS_STORAGE_BF16)
       ds::fit_preprocess_kernel<<<blocks, ds::kPreThreads, 0, s>>>(
           r->P, r->R16, r->active_degree, r->cam_dev, rb.width, rb.height, rb.ntx, rb.nty,
-          rb.rec_a, rb.rec_b, rb.rec_c, rb.rec_idet, rb.rect, rb.counts, rb.depth_keys,
+          rb.rec_a, rb.rec_b, rb.rec_c, rb.rect, rb.counts, rb.depth_keys,
           rb.scalars);
     else
       ds::fit_preprocess_kernel<<<blocks, ds::kPreThreads, 0, s>>>(
           r->P, ds::soa_of(r->P), r->active_degree, r->cam_dev, rb.width, rb.height, rb.ntx,
-          rb.nty, rb.rec_a, rb.rec_b, rb.rec_c, rb.rec_idet, rb.rect, rb.counts, rb.depth_keys,
+          rb.nty, rb.rec_a, rb.rec_b, rb.rec_c, rb.rect, rb.counts, rb.depth_keys,
           rb.scalars);
     DS_CUDA(cudaGetLastError());
   }

@@ -186,7 +186,7 @@ int ds_raster_destroy(ds_raster *r);
  * application whose own pool allocator owns all device memory, or a per-frame
  * loop in which cudaMalloc / cudaFree would synchronise the device.  Same
  * kernels and same image as ds_raster_create + ds_raster_forward, with every
- * intermediate buffer in one ~5.7 MB __device__ array of the library that each
+ * intermediate buffer in one ~5.6 MB __device__ array of the library that each
  * GPU holds until the process exits.  Limits: count <= 8192 splats,
  * width * height <= 65536 pixels, at most 1024 16x16 tiles (DS_ERR_ARG
  * beyond); (tile, splat) pairs beyond 131072 are dropped, the deepest first,

@@ -386,6 +386,12 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
   return float2_of(r);
 }
 __device__ __forceinline__ float2 both(float v) { return make_float2(v, v); }
+// 1 / x to the hardware's reciprocal (1 ulp; exact for powers of two).
+__device__ __forceinline__ float rcp(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
 
 // ---------------------------------------------------------------------------
 // Warp helpers

@@ -155,17 +155,18 @@ struct Staged {
 };
 
 // A splat as the pixel loops read it: every value twice, so that it loads as a
-// packed operand.
+// packed operand.  The conic's off-diagonal is held doubled: (dx dy) 2b rounds
+// like (2 dx dy) b.
 struct SplatRec {
   float4 pos;     // x, x, y, y
-  float4 ab;      // conic a, a, b, b
+  float4 ab;      // conic a, a, 2b, 2b
   float4 co;      // conic c, c, opacity, opacity
   float4 rg;      // r, r, g, g
   float4 blue;    // b, b, -, - (forward: the splat's sorted index as bits)
   __device__ __forceinline__ void set(const float4& a, const float4& b, const float4& c,
                                       int index) {
     pos = make_float4(a.x, a.x, a.y, a.y);
-    ab = make_float4(b.x, b.x, b.y, b.y);
+    ab = make_float4(b.x, b.x, 2.f * b.y, 2.f * b.y);
     co = make_float4(b.z, b.z, b.w, b.w);
     rg = make_float4(c.x, c.x, c.y, c.y);
     blue = make_float4(c.z, c.z, __int_as_float(index), 0.f);
@@ -175,7 +176,7 @@ struct SplatRec {
     pos = ab = co = rg = blue = make_float4(0.f, 0.f, 0.f, 0.f);
   }
   __device__ __forceinline__ float2 conic_a() const { return make_float2(ab.x, ab.y); }
-  __device__ __forceinline__ float2 conic_b() const { return make_float2(ab.z, ab.w); }
+  __device__ __forceinline__ float2 conic_2b() const { return make_float2(ab.z, ab.w); }
   __device__ __forceinline__ float2 conic_c() const { return make_float2(co.x, co.y); }
   __device__ __forceinline__ float2 x() const { return make_float2(pos.x, pos.y); }
   __device__ __forceinline__ float2 y() const { return make_float2(pos.z, pos.w); }
@@ -184,29 +185,44 @@ struct SplatRec {
   __device__ __forceinline__ float opacity() const { return co.z; }
 };
 
-// opacity exp(-sigma) of a splat at a pair of pixels (conic_dist2 in its
-// rounding) and whether sigma >= 0 there; dx, dxx = dx dx and dx2 = 2 dx.
-__device__ __forceinline__ float2 pair_opacity(float2 dx2, float2 dxx, float2 dy,
-                                               const SplatRec& r, bool& ok0, bool& ok1) {
-  const float2 dist2 = fma2(mul2(dy, dy), r.conic_c(),
-                            fma2(dxx, r.conic_a(), mul2(mul2(dx2, dy), r.conic_b())));
-  const float2 sigma = mul2(both(0.5f), dist2);
-  ok0 = !(sigma.x < 0.f);
-  ok1 = !(sigma.y < 0.f);
-  return mul2(make_float2(r.co.z, r.co.w), make_float2(__expf(-sigma.x), __expf(-sigma.y)));
+// Whether the computed quadratic form of a conic can nowhere be negative (or
+// NaN): it rounds to within 4 eps (a dx^2 + 2 |b dx dy| + c dy^2), and is at least
+// (1 - |b| / sqrt(a c)) (a dx^2 + c dy^2), so b^2 <= 0.9999 a c leaves a margin of
+// two orders of magnitude.  Holds for splats up to about 100 times longer than
+// wide; the pixel loops then need no test of sigma's sign.
+__device__ __forceinline__ bool definite(const float4& b) {
+  return b.x >= 1e-12f && b.z >= 1e-12f && b.x <= 1e18f && b.z <= 1e18f &&
+         b.y * b.y <= 0.9999f * b.x * b.z;
+}
+__device__ __forceinline__ bool finite3(float r, float g, float b) {
+  return fabsf(r) <= 3.0e38f && fabsf(g) <= 3.0e38f && fabsf(b) <= 3.0e38f;
+}
+
+// Mahalanobis distances (conic_dist2 in its rounding) of a splat at a pair of
+// pixels and opacity exp(-dist2 / 2) there, exp as 2^(dist2 (-log2(e) / 2)); dxx =
+// dx dx.
+__device__ __forceinline__ float2 pair_dist2(float2 dx, float2 dxx, float2 dy,
+                                             const SplatRec& r) {
+  return fma2(mul2(dy, dy), r.conic_c(),
+              fma2(dxx, r.conic_a(), mul2(mul2(dx, dy), r.conic_2b())));
+}
+__device__ __forceinline__ float2 pair_opacity(float2 dist2, const SplatRec& r) {
+  const float2 p = mul2(both(-0.72134752f), dist2);
+  return mul2(make_float2(r.co.z, r.co.w), make_float2(exp2f(p.x), exp2f(p.y)));
 }
 
 // A warp's hits of a staged batch, listed in order: the splats l of [from, n)
-// whose mask has the warp's bit.  Padded with `none` to an even count; returns
-// the count before padding.
+// whose mask has the warp's bit, with the mask's sign bit.  Padded with `none` to an
+// even count; returns the count before padding.
 __device__ __forceinline__ int list_hits(const uint32_t* mask, int w, int lane, int from, int n,
                                          int none, int* list) {
   int count = 0;
   for (int k = 0; k < n; k += 32) {
     const int l = k + lane;
-    const bool hit = l >= from && l < n && ((mask[l] >> w) & 1u);
+    const uint32_t mk = l >= from && l < n ? mask[l] : 0u;
+    const bool hit = (mk >> w) & 1u;
     const uint32_t word = __ballot_sync(0xffffffffu, hit);
-    if (hit) list[count + __popc(word & ((1u << lane) - 1u))] = l;
+    if (hit) list[count + __popc(word & ((1u << lane) - 1u))] = l | (int)(mk & 0x80000000u);
     count += __popc(word);
   }
   if (lane == 0) list[count] = none;
@@ -240,7 +256,10 @@ __device__ __forceinline__ uint32_t warp_hits(const float4& a, const float4& b, 
 //
 // A pixel that is done (T <= 1e-4), outside the image or not reached by the
 // splat composites alpha = 0, which changes neither its colour nor its T; only
-// colours that are not finite need the guarded variant.
+// colours that are not finite and conics that are nearly singular (whose sigma may
+// come out negative) need the guarded variant.  Without the sign test of the others,
+// and with the two constants of exp folded into one packed product, the two scenes
+// above went from 0.103 to 0.099 and from 0.217 to 0.209 ms.
 constexpr int kFwdWarps = 4;
 
 struct FwdShared {
@@ -249,7 +268,7 @@ struct FwdShared {
   bool last;
 };
 
-template <int TS, bool kLoss, bool kCount, bool kBatch>
+template <int TS, bool kLoss, bool kCount, bool kBatch, bool kIds>
 __global__ void __launch_bounds__(32 * kFwdWarps, DS_FWD_MIN_BLOCKS)
     composite_fwd_kernel(const float4* __restrict__ ra, const float4* __restrict__ rb,
                          const float4* __restrict__ rc, const uint32_t* __restrict__ sorted_splat,
@@ -291,10 +310,15 @@ __global__ void __launch_bounds__(32 * kFwdWarps, DS_FWD_MIN_BLOCKS)
       for (int g = 0; g < G; ++g) {
         const SplatRec& r = hit[i + g];
         const float2 dx = add2(r.x(), npx);
-        al[g] = pair_opacity(add2(dx, dx), mul2(dx, dx), add2(r.y(), npy), r, ok0[g], ok1[g]);
+        const float2 d2 = pair_dist2(dx, mul2(dx, dx), add2(r.y(), npy), r);
+        al[g] = pair_opacity(d2, r);
         al[g] = make_float2(fminf(kMaxAlpha, al[g].x), fminf(kMaxAlpha, al[g].y));
-        ok0[g] = ok0[g] && !(al[g].x < kAlphaThres);
-        ok1[g] = ok1[g] && !(al[g].y < kAlphaThres);
+        ok0[g] = !(al[g].x < kAlphaThres);
+        ok1[g] = !(al[g].y < kAlphaThres);
+        if (decltype(guarded)::value) {
+          ok0[g] = ok0[g] && !(d2.x < 0.f);
+          ok1[g] = ok1[g] && !(d2.y < 0.f);
+        }
       }
 #pragma unroll
       for (int g = 0; g < G; ++g) {
@@ -307,8 +331,10 @@ __global__ void __launch_bounds__(32 * kFwdWarps, DS_FWD_MIN_BLOCKS)
           n_contrib += p0 + p1;
         }
         const float2 a = make_float2(p0 ? al[g].x : 0.f, p1 ? al[g].y : 0.f);
-        cur0 = p0 ? id : cur0;
-        cur1 = p1 ? id : cur1;
+        if (kIds) {
+          cur0 = p0 ? id : cur0;
+          cur1 = p1 ? id : cur1;
+        }
         const float2 vis = mul2(a, T);
         const float2 r1 = fma2(r.red(), vis, Cr);
         const float2 g1 = fma2(r.green(), vis, Cg);
@@ -341,10 +367,10 @@ __global__ void __launch_bounds__(32 * kFwdWarps, DS_FWD_MIN_BLOCKS)
     const bool mine = pf.ok && ellipse_hits(pf.a, pf.b, pf.c.w, box);
     const uint32_t word = __ballot_sync(0xffffffffu, mine);
     const int n = __popc(word);
-    bool odd = false;  // a colour that is not finite
+    bool odd = false;  // a colour that is not finite, a conic that may go negative
     if (mine) {
       hit[__popc(word & ((1u << lane) - 1u))].set(pf.a, pf.b, pf.c, b0 + lane);
-      odd = !(fabsf(pf.c.x) <= 3.0e38f && fabsf(pf.c.y) <= 3.0e38f && fabsf(pf.c.z) <= 3.0e38f);
+      odd = !(finite3(pf.c.x, pf.c.y, pf.c.z) && definite(pf.b));
     }
     // the last group is filled with splats of opacity 0
     if (lane < G && n + lane < (n + G - 1) / G * G) hit[n + lane].set_none();
@@ -379,8 +405,10 @@ __global__ void __launch_bounds__(32 * kFwdWarps, DS_FWD_MIN_BLOCKS)
     out_rgb[pix * 3 + 0] = r;
     out_rgb[pix * 3 + 1] = g;
     out_rgb[pix * 3 + 2] = b;
-    out_alpha[pix] = 1.f - (k ? T.y : T.x);
-    last_ids[pix] = k ? cur1 : cur0;
+    if (kIds) {
+      out_alpha[pix] = 1.f - (k ? T.y : T.x);
+      last_ids[pix] = k ? cur1 : cur0;
+    }
     if (kLoss) {
       const float scale = 1.f / (float)(W * H);
       const float dR = r - target[pix * 3 + 0];
@@ -441,73 +469,112 @@ struct BwdShared {
   static constexpr int kPitch = 64 + 4;
   SplatRec splat[B + 1];       // the last one reaches nothing
   float4 box[NW];
-  float4 npx[NW][16];     // per pixel of a warp: -x, -y (NDC) and dL/dpixel
-  float4 npy[NW][16];
-  float4 gr[NW][16], gg[NW][16], gb[NW][16];
+  float4 gr[NW][16], gg[NW][16], gb[NW][16];  // per pixel of a warp: dL/dpixel
+  float2 nx[NW][4];    // -x (NDC) of a warp's columns 2q and 2q + 1
+  float2 ny[NW];       // -y of its rows 1 and 5,
+  float2 row[NW][4];   // and what rows r and r + 4 add to that
   float4 s[NW][kBwdHits * kPitch / 4];    // per (hit, pixel): opacity exp() dL/dalpha
   float4 fac[NW][kBwdHits * kPitch / 4];  // per (hit, pixel): alpha T
   float part[NW][B * 9];       // per-warp gradient of each batch splat
   uint32_t rec[B];             // record index of each batch splat
-  uint32_t mask[B];            // warps whose block the splat can reach
+  uint32_t mask[B];            // warps whose block the splat can reach; bit 31: not plain
   uint32_t got[NW][B / 32];    // batch splats with a partial from the warp
   int2 list[NW][B / 2 + 1];    // the warp's hits of the batch
   int32_t final_id[NW];
 };
 
+// Slot of lane l's pixel pair (column l % 8, rows l / 8 and l / 8 + 4) in a hit's row
+// of per-pixel values, in floats.  Row r's columns 2q and 2q + 1 are the 16-byte word
+// at_word(r, q): for a fixed r, the four q of two hits fall on distinct banks.
+__device__ __forceinline__ int at_word(int r, int q) { return (r >> 1) * 8 + q * 2 + (r & 1); }
+__device__ __forceinline__ int pixel_slot(int lane) {
+  return 4 * at_word(lane >> 3, (lane & 7) >> 1) + 2 * (lane & 1);
+}
+
 // The gradients of up to kBwdHits hits of a warp from their per-pixel values:
-// four lanes per hit, each over a quarter of the warp's pixels, two pixels per
-// instruction.  With u = a dx + b dy and w = b dx + c dy,
+// four lanes per hit, each over two columns of the warp's block, the upper and the
+// lower four rows in the halves of an instruction.  With u = a dx + b dy and
+// w = b dx + c dy,
 //   d dist2 / d(ndc x, ndc y) = (2u, 2w)
 //   d dist2 / d(cov xx, xy, yy) = -u^2, -2uw, -w^2
 // (uw = b dist2 + dx dy / det written without the cancelling difference), and s
-// = -2 dL/d(dist2).  kSafe leaves out what s = 0 or fac = 0 multiplies, as it
-// may be infinite or NaN.
+// = -2 dL/d(dist2).  In a column u and w are linear in y, so the sums of s u, s w,
+// s u^2, s u w and s w^2 over four rows follow from three moments of s about one of
+// them (from the rows' own y, which are not quite evenly spaced in FP32).  kSafe
+// forms them pixel by pixel instead and leaves out what s = 0 or fac = 0 multiplies,
+// as it may be infinite or NaN.
 template <bool kSafe, int TS>
 __device__ __forceinline__ void reduce_hits(BwdShared<TS>& sm, int w, int lane, int count,
                                             int slot) {
   using Sh = BwdShared<TS>;
   const int h = lane >> 2, q = lane & 3;
   const SplatRec& hit = sm.splat[slot];
-  const float2 x = hit.x(), y = hit.y();
-  const float2 ca = hit.conic_a(), cb = hit.conic_b(), cc = hit.conic_c();
+  const float2 ca = hit.conic_a(), cb = mul2(hit.conic_2b(), both(0.5f)), cc = hit.conic_c();
+  const float2 dyc = add2(hit.y(), sm.ny[w]);  // dy in rows 1 and 5
+  const float2 nx = sm.nx[w][q];
   float2 v[9];
 #pragma unroll
   for (int k = 0; k < 9; ++k) v[k] = make_float2(0.f, 0.f);
+  float2 s[4][2];
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const int at = (k >> 1) * 8 + q * 2 + (k & 1);  // group of four pixels
+  for (int r = 0; r < 4; ++r) {
+    const int at = at_word(r, q);
     const float4 s4 = sm.s[w][h * (Sh::kPitch / 4) + at];
     const float4 f4 = sm.fac[w][h * (Sh::kPitch / 4) + at];
-    const float4 x4 = sm.npx[w][at], y4 = sm.npy[w][at];
     const float4 r4 = sm.gr[w][at], g4 = sm.gg[w][at], b4 = sm.gb[w][at];
+    s[r][0] = make_float2(s4.x, s4.y), s[r][1] = make_float2(s4.z, s4.w);
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
-      const float2 s = e ? make_float2(s4.z, s4.w) : make_float2(s4.x, s4.y);
       const float2 f = e ? make_float2(f4.z, f4.w) : make_float2(f4.x, f4.y);
       float2 gr = e ? make_float2(r4.z, r4.w) : make_float2(r4.x, r4.y);
       float2 gg = e ? make_float2(g4.z, g4.w) : make_float2(g4.x, g4.y);
       float2 gb = e ? make_float2(b4.z, b4.w) : make_float2(b4.x, b4.y);
-      const float2 dx = add2(x, e ? make_float2(x4.z, x4.w) : make_float2(x4.x, x4.y));
-      const float2 dy = add2(y, e ? make_float2(y4.z, y4.w) : make_float2(y4.x, y4.y));
-      float2 u = fma2(dx, ca, mul2(dy, cb));
-      float2 t = fma2(dx, cb, mul2(dy, cc));
       if (kSafe) {
-        u.x = s.x != 0.f ? u.x : 0.f, u.y = s.y != 0.f ? u.y : 0.f;
-        t.x = s.x != 0.f ? t.x : 0.f, t.y = s.y != 0.f ? t.y : 0.f;
         gr.x = f.x != 0.f ? gr.x : 0.f, gr.y = f.y != 0.f ? gr.y : 0.f;
         gg.x = f.x != 0.f ? gg.x : 0.f, gg.y = f.y != 0.f ? gg.y : 0.f;
         gb.x = f.x != 0.f ? gb.x : 0.f, gb.y = f.y != 0.f ? gb.y : 0.f;
       }
-      const float2 su = mul2(s, u), st = mul2(s, t);
       v[0] = fma2(f, gr, v[0]);
       v[1] = fma2(f, gg, v[1]);
       v[2] = fma2(f, gb, v[2]);
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    const float2 dx = add2(hit.x(), both(e ? nx.y : nx.x));
+    if (kSafe) {
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const float2 dy = add2(dyc, sm.row[w][r]);
+        float2 u = fma2(dx, ca, mul2(dy, cb));
+        float2 t = fma2(dx, cb, mul2(dy, cc));
+        const float2 z = s[r][e];
+        u.x = z.x != 0.f ? u.x : 0.f, u.y = z.y != 0.f ? u.y : 0.f;
+        t.x = z.x != 0.f ? t.x : 0.f, t.y = z.y != 0.f ? t.y : 0.f;
+        const float2 su = mul2(z, u), st = mul2(z, t);
+        v[3] = add2(v[3], su);
+        v[4] = add2(v[4], st);
+        v[5] = fma2(su, u, v[5]);
+        v[6] = fma2(su, t, v[6]);
+        v[7] = fma2(st, t, v[7]);
+        v[8] = add2(v[8], z);
+      }
+    } else {
+      const float2 d0 = sm.row[w][0], d2 = sm.row[w][2], d3 = sm.row[w][3];
+      const float2 z0 = mul2(s[0][e], d0), z2 = mul2(s[2][e], d2), z3 = mul2(s[3][e], d3);
+      const float2 m0 = add2(add2(s[0][e], s[1][e]), add2(s[2][e], s[3][e]));
+      const float2 m1 = add2(add2(z0, z2), z3);
+      const float2 m2 = fma2(z3, d3, fma2(z2, d2, mul2(z0, d0)));
+      // in row 1 (5): u and t
+      const float2 u = fma2(dx, ca, mul2(dyc, cb)), t = fma2(dx, cb, mul2(dyc, cc));
+      const float2 su = fma2(u, m0, mul2(cb, m1)), ru = fma2(u, m1, mul2(cb, m2));
+      const float2 st = fma2(t, m0, mul2(cc, m1)), rt = fma2(t, m1, mul2(cc, m2));
       v[3] = add2(v[3], su);
       v[4] = add2(v[4], st);
-      v[5] = fma2(su, u, v[5]);
-      v[6] = fma2(su, t, v[6]);
-      v[7] = fma2(st, t, v[7]);
-      v[8] = add2(v[8], s);
+      v[5] = fma2(u, su, fma2(cb, ru, v[5]));
+      v[6] = fma2(t, su, fma2(cc, ru, v[6]));
+      v[7] = fma2(t, st, fma2(cc, rt, v[7]));
+      v[8] = add2(v[8], m0);
     }
   }
   float r[9];
@@ -542,11 +609,19 @@ __device__ __forceinline__ void reduce_hits(BwdShared<TS>& sm, int w, int lane, 
 // colour); the nine gradients of a hit are sums of products of these with
 // values that depend on the pixel or on the splat alone.  So the pixel loop
 // (lane = pixel) only stores s and fac to shared memory, and for every
-// kBwdHits hits the lanes regroup, four to a hit, and form the sums over the
-// pixels (reduce_hits), which costs about 25 issue slots a hit where the
-// nine-value butterfly over the warp took about 60.  Against the butterfly
-// (B200): 1280x720 fit of 60000 splats at step 25 0.366 -> 0.301 ms,
-// at step 400 0.828 -> 0.504; a million splats at 1920x1080 0.656 -> 0.600.
+// kBwdHits hits (or one fewer, so that the loop has a single place to do it) the
+// lanes regroup, four to a hit, and form the sums over the pixels (reduce_hits),
+// which costs about 18 issue slots a hit where the nine-value butterfly over the
+// warp took about 60.  Against the butterfly (B200): 1280x720 fit of 60000 splats at
+// step 25 0.366 -> 0.301 ms, at step 400 0.828 -> 0.504; a million splats at
+// 1920x1080 0.656 -> 0.600.
+//
+// The pixel loop was next: of some 70 issue slots a hit, half went to tests and
+// selects on the ALU pipe, which issues at half rate.  Splats that cannot reach alpha
+// 0.99, whose conic is not nearly singular and behind which every pixel's list has
+// begun ("plain", nearly all) need one test of alpha and no select.  With the moments
+// of reduce_hits: step 4 of the 1280x720 fit 0.258 -> 0.214 ms, the million splats
+// 0.525 -> 0.511 (there the warps of a tile wait for one another at every batch).
 template <int TS, bool kFusedLoss, bool kExact, bool kBatch>
 __global__ void __launch_bounds__(Lay<TS>::kThreads, Lay<TS>::kMinBlocksBwd)
     composite_bwd_kernel(const float4* __restrict__ ra, const float4* __restrict__ rb,
@@ -586,9 +661,17 @@ __global__ void __launch_bounds__(Lay<TS>::kThreads, Lay<TS>::kMinBlocksBwd)
   if (lane == 0) sm.box[w] = make_float4(m.wx_lo, m.wx_hi, m.wy_lo, m.wy_hi);
   // acc: over the splats behind (already visited), weight x (colour . dL/dpixel)
   float2 T, gr, gg, gb, acc = both(0.f);
-  const float2 npx = both(-m.px), npy = make_float2(-m.py[0], -m.py[1]);
+  // NaN outside the image: no splat reaches it there
+  const float nan = __int_as_float(0x7fffffff);
+  const float2 npx = both(-m.px);
+  const float2 npy = make_float2(m.inside[0] ? -m.py[0] : nan, m.inside[1] ? -m.py[1] : nan);
   int32_t fin[2];
   int32_t my_final = -1;
+  // The splats from which on no pixel's last contributor needs a look: behind the
+  // last contributor of a pixel that did not end opaque nothing passes the alpha
+  // test (the forward's arithmetic), so only opaque ones count.  1% above kTThres for
+  // the rounding of 1 - alpha.
+  int32_t first_plain = 0x7fffffff;
   bool finite = true;
 #pragma unroll
   for (int k = 0; k < 2; ++k) {
@@ -596,6 +679,7 @@ __global__ void __launch_bounds__(Lay<TS>::kThreads, Lay<TS>::kMinBlocksBwd)
     const float t = 1.f - alphas[pix];
     fin[k] = m.inside[k] ? last_ids[pix] : -1;
     my_final = max(my_final, fin[k]);
+    if (m.inside[k] && !(t > 1.01f * kTThres)) first_plain = min(first_plain, fin[k]);
     float r = 0.f, g = 0.f, b = 0.f;
     if (m.inside[k]) {
       if (kFusedLoss) {
@@ -608,20 +692,25 @@ __global__ void __launch_bounds__(Lay<TS>::kThreads, Lay<TS>::kMinBlocksBwd)
         g = grad_or_image[pix * 3 + 1];
         b = grad_or_image[pix * 3 + 2];
       }
-      finite = finite && fabsf(r) <= 3.0e38f && fabsf(g) <= 3.0e38f && fabsf(b) <= 3.0e38f;
+      finite = finite && fabsf(r) <= 1e15f && fabsf(g) <= 1e15f && fabsf(b) <= 1e15f;
     }
     (k ? T.y : T.x) = t;
     (k ? gr.y : gr.x) = r;
     (k ? gg.y : gg.x) = g;
     (k ? gb.y : gb.x) = b;
   }
-  // pixel k of lane l is value 2 l + k of the warp's tables
-  reinterpret_cast<float2*>(sm.npx[w])[lane] = npx;
-  reinterpret_cast<float2*>(sm.npy[w])[lane] = npy;
-  reinterpret_cast<float2*>(sm.gr[w])[lane] = gr;
-  reinterpret_cast<float2*>(sm.gg[w])[lane] = gg;
-  reinterpret_cast<float2*>(sm.gb[w])[lane] = gb;
+  reinterpret_cast<float2*>(sm.gr[w])[pixel_slot(lane) / 2] = gr;
+  reinterpret_cast<float2*>(sm.gg[w])[pixel_slot(lane) / 2] = gg;
+  reinterpret_cast<float2*>(sm.gb[w])[pixel_slot(lane) / 2] = gb;
   const bool safe_pixels = __all_sync(0xffffffffu, finite);
+  first_plain = safe_pixels ? __reduce_min_sync(0xffffffffu, first_plain) : -1;
+  {
+    const float y1 = __shfl_sync(0xffffffffu, m.py[0], 8);
+    const float y5 = __shfl_sync(0xffffffffu, m.py[1], 8);
+    if (lane < 8) reinterpret_cast<float*>(sm.nx[w])[lane] = -m.px;
+    if ((lane & 7) == 0) sm.row[w][lane >> 3] = make_float2(y1 - m.py[0], y5 - m.py[1]);
+    if (lane == 0) sm.ny[w] = make_float2(-y1, -y5);
+  }
   const int32_t warp_final = warp_max(my_final);
   // Pairs after the tile's last contributing splat reach no pixel: the list
   // ends there for the backward, and no record is written for them (their
@@ -671,8 +760,8 @@ __global__ void __launch_bounds__(Lay<TS>::kThreads, Lay<TS>::kMinBlocksBwd)
     }
   };
   if (threadIdx.x == 0) sm.splat[B].set_none();
-  float* const my_s = reinterpret_cast<float*>(sm.s[w]) + 2 * lane;
-  float* const my_f = reinterpret_cast<float*>(sm.fac[w]) + 2 * lane;
+  float* const my_s = reinterpret_cast<float*>(sm.s[w]) + pixel_slot(lane);
+  float* const my_f = reinterpret_cast<float*>(sm.fac[w]) + pixel_slot(lane);
   prefetch(0);
   for (int bi = 0; bi < nb; ++bi) {
     const int batch_end = end - 1 - B * bi;  // farthest splat of the batch
@@ -698,6 +787,10 @@ __global__ void __launch_bounds__(Lay<TS>::kThreads, Lay<TS>::kMinBlocksBwd)
         if (h == 0) {
           sm.splat[l].set(a, b, c, 0);
           sm.rec[l] = pf_rec[r];
+          // plain: cannot reach alpha 0.99, and nothing about it overflows
+          const bool plain = definite(b) && b.w <= kMaxAlpha && fabsf(c.x) <= 1e15f &&
+                             fabsf(c.y) <= 1e15f && fabsf(c.z) <= 1e15f;
+          if (!plain) mk |= 0x80000000u;
         }
       }
       if (kSplit == 2) mk |= __shfl_xor_sync(0xffffffffu, mk, 1);  // pairs are adjacent lanes
@@ -716,8 +809,8 @@ __global__ void __launch_bounds__(Lay<TS>::kThreads, Lay<TS>::kMinBlocksBwd)
       bool tame = true;
       if ((lane >> 2) < count) {
         const SplatRec& r = sm.splat[slot];
-        tame = fabsf(r.conic_a().x) <= 1e30f && fabsf(r.conic_b().x) <= 1e30f &&
-               fabsf(r.conic_c().x) <= 1e30f;
+        tame = fabsf(r.conic_a().x) <= 1e15f && fabsf(r.conic_2b().x) <= 1e15f &&
+               fabsf(r.conic_c().x) <= 1e15f;
         if ((lane & 3) == 0) atomicOr(&sm.got[w][slot >> 5], 1u << (slot & 31));
       }
       if (safe_pixels && __all_sync(0xffffffffu, tame))
@@ -727,56 +820,93 @@ __global__ void __launch_bounds__(Lay<TS>::kThreads, Lay<TS>::kMinBlocksBwd)
       count = 0;
       __syncwarp();
     };
+    auto store = [&](float2 s, float2 fac, int t) {
+      *reinterpret_cast<float2*>(my_s + count * Sh::kPitch) = s;
+      *reinterpret_cast<float2*>(my_f + count * Sh::kPitch) = fac;
+      if ((lane >> 2) == count) slot = t;
+      ++count;
+    };
+    // lit: the splat's colour . dL/dpixel.  Reference recurrence
+    // (tile_rasterize_layer.cu:518-521) weighs the colour behind (absolute weights
+    // c_j alpha_j T_j) by T_before; the exact derivative divides it by T_after
+    // instead.  The three colour channels enter only through their dot product with
+    // dL/dpixel.
+    auto lit_of = [&](const SplatRec& r) {
+      const float2 blue = *reinterpret_cast<const float2*>(&r.blue);
+      return fma2(blue, gb, fma2(r.red(), gr, mul2(r.green(), gg)));
+    };
+    auto weigh = [&](float2 lit) {
+      const float2 nia = kExact ? make_float2(-1.f / T.x, -1.f / T.y) : both(-1.f);
+      return fma2(acc, nia, lit);
+    };
+    // from this slot on every pixel's list has begun
+    const int t_plain = max(0, batch_end - first_plain);
     // The hits two at a time: conic, exp and alpha of both first (independent of
     // T), then the recurrence back to front.
     for (int i = 0; i < hits; i += 2) {
       const int2 pair = sm.list[w][i >> 1];
       float2 oe[2], al[2];
       bool any[2];
+      if (pair.x >= t_plain && pair.y >= 0) {
+        // Plain splats: alpha = opacity exp() where it passes, 0 elsewhere, which
+        // leaves T and acc as they are.
 #pragma unroll
-      for (int g = 0; g < 2; ++g) {
-        const int t = g ? pair.y : pair.x, id = batch_end - t;
-        const SplatRec& r = sm.splat[t];
-        const float2 dx = add2(r.x(), npx);
-        bool o0, o1;
-        oe[g] = pair_opacity(add2(dx, dx), mul2(dx, dx), add2(r.y(), npy), r, o0, o1);
-        const float a0 = fminf(kMaxAlpha, oe[g].x), a1 = fminf(kMaxAlpha, oe[g].y);
-        o0 = o0 && id <= fin[0] && !(a0 < kAlphaThres);
-        o1 = o1 && id <= fin[1] && !(a1 < kAlphaThres);
-        // alpha 0: the splat is skipped at that pixel
-        al[g] = make_float2(o0 ? a0 : 0.f, o1 ? a1 : 0.f);
-        any[g] = o0 || o1;
-      }
+        for (int g = 0; g < 2; ++g) {
+          const SplatRec& r = sm.splat[g ? pair.y : pair.x];
+          const float2 dx = add2(r.x(), npx);
+          oe[g] = pair_opacity(pair_dist2(dx, mul2(dx, dx), add2(r.y(), npy), r), r);
+          const bool o0 = oe[g].x >= kAlphaThres, o1 = oe[g].y >= kAlphaThres;
+          al[g] = make_float2(o0 ? oe[g].x : 0.f, o1 ? oe[g].y : 0.f);
+          any[g] = o0 || o1;
+        }
 #pragma unroll
-      for (int g = 0; g < 2; ++g) {
-        if (!__any_sync(0xffffffffu, any[g])) continue;
-        const int t = g ? pair.y : pair.x;
-        const SplatRec& r = sm.splat[t];
-        const float2 blue = *reinterpret_cast<const float2*>(&r.blue);
-        const bool o0 = al[g].x > 0.f, o1 = al[g].y > 0.f;
-        const float2 om = fma2(al[g], both(-1.f), both(1.f));  // >= 0.01
-        const float2 Tb = mul2(T, make_float2(__fdividef(1.f, om.x), __fdividef(1.f, om.y)));
-        const float2 fac = mul2(al[g], Tb);
-        // Reference recurrence (tile_rasterize_layer.cu:518-521) weighs the
-        // colour behind (absolute weights c_j alpha_j T_j) by T_before; the
-        // exact derivative divides it by T_after instead.  The three colour
-        // channels enter only through their dot product with dL/dpixel.
-        const float2 lit = fma2(blue, gb, fma2(r.red(), gr, mul2(r.green(), gg)));
-        const float2 nia = kExact ? make_float2(-1.f / T.x, -1.f / T.y) : both(-1.f);
-        const float2 s2 = mul2(oe[g], mul2(Tb, fma2(acc, nia, lit)));
-        const float2 next = fma2(lit, fac, acc);
-        float2 s;
-        s.x = o0 && oe[g].x <= kMaxAlpha ? s2.x : 0.f;
-        s.y = o1 && oe[g].y <= kMaxAlpha ? s2.y : 0.f;
-        acc = make_float2(o0 ? next.x : acc.x, o1 ? next.y : acc.y);
-        T = make_float2(o0 ? Tb.x : T.x, o1 ? Tb.y : T.y);
-        *reinterpret_cast<float2*>(my_s + count * Sh::kPitch) = s;
-        *reinterpret_cast<float2*>(my_f + count * Sh::kPitch) = fac;
-        if ((lane >> 2) == count) slot = t;
-        if (++count == kBwdHits) flush();
+        for (int g = 0; g < 2; ++g) {
+          if (!__any_sync(0xffffffffu, any[g])) continue;
+          const int t = g ? pair.y : pair.x;
+          const float2 om = fma2(al[g], both(-1.f), both(1.f));  // >= 0.01
+          const float2 lit = lit_of(sm.splat[t]);
+          const float2 in = weigh(lit);
+          T = mul2(T, make_float2(rcp(om.x), rcp(om.y)));
+          const float2 fac = mul2(al[g], T);
+          acc = fma2(lit, fac, acc);
+          store(mul2(fac, in), fac, t);
+        }
+      } else {
+#pragma unroll
+        for (int g = 0; g < 2; ++g) {
+          const int t = (g ? pair.y : pair.x) & 0x7fffffff, id = batch_end - t;
+          const SplatRec& r = sm.splat[t];
+          const float2 dx = add2(r.x(), npx);
+          const float2 d2 = pair_dist2(dx, mul2(dx, dx), add2(r.y(), npy), r);
+          oe[g] = pair_opacity(d2, r);
+          const float a0 = fminf(kMaxAlpha, oe[g].x), a1 = fminf(kMaxAlpha, oe[g].y);
+          const bool o0 = !(d2.x < 0.f) && id <= fin[0] && !(a0 < kAlphaThres);
+          const bool o1 = !(d2.y < 0.f) && id <= fin[1] && !(a1 < kAlphaThres);
+          // alpha 0: the splat is skipped at that pixel
+          al[g] = make_float2(o0 ? a0 : 0.f, o1 ? a1 : 0.f);
+          any[g] = o0 || o1;
+        }
+#pragma unroll
+        for (int g = 0; g < 2; ++g) {
+          if (!__any_sync(0xffffffffu, any[g])) continue;
+          const int t = (g ? pair.y : pair.x) & 0x7fffffff;
+          const bool o0 = al[g].x > 0.f, o1 = al[g].y > 0.f;
+          const float2 om = fma2(al[g], both(-1.f), both(1.f));  // >= 0.01
+          const float2 Tb = mul2(T, make_float2(rcp(om.x), rcp(om.y)));
+          const float2 fac = mul2(al[g], Tb);
+          const float2 lit = lit_of(sm.splat[t]);
+          const float2 s2 = mul2(oe[g], mul2(Tb, weigh(lit)));
+          const float2 next = fma2(lit, fac, acc);
+          float2 s;
+          s.x = o0 && oe[g].x <= kMaxAlpha ? s2.x : 0.f;
+          s.y = o1 && oe[g].y <= kMaxAlpha ? s2.y : 0.f;
+          acc = make_float2(o0 ? next.x : acc.x, o1 ? next.y : acc.y);
+          T = make_float2(o0 ? Tb.x : T.x, o1 ? Tb.y : T.y);
+          store(s, fac, t);
+        }
       }
+      if (count >= kBwdHits - 1 || (i + 2 >= hits && count > 0)) flush();
     }
-    if (count > 0) flush();
     __syncthreads();
     for (int slot2 = threadIdx.x; slot2 < bs * kSplit; slot2 += NT) {
       const int l = slot2 / kSplit, h = slot2 % kSplit;
@@ -817,14 +947,15 @@ void launch_fwd(RasterBuffers& rb, float* out_rgb, const float* target, bool cou
   constexpr int kBlocks = (TS / 8) * (TS / 8);
   const int32_t* order = schedule(rb);
   const dim3 grid((unsigned)(((int64_t)rb.tiles * kBlocks + kFwdWarps - 1) / kFwdWarps));
-#define DS_FWD(L, C)                                                                         \
-  launch_pdl(composite_fwd_kernel<TS, L, C, kBatch>, grid, dim3(32 * kFwdWarps), 0, s,       \
+#define DS_FWD(L, C, I)                                                                      \
+  launch_pdl(composite_fwd_kernel<TS, L, C, kBatch, I>, grid, dim3(32 * kFwdWarps), 0, s,    \
              rb.rec_a, rb.rec_b, rb.rec_c, rb.sorted_splat, rb.ranges, order, out_rgb,        \
              rb.alphas, rb.last_ids, rb.tiles, rb.width, rb.height, rb.ntx, rb.tile_inst,     \
              rb.geom, L ? target : nullptr, L ? rb.loss_partials : nullptr, rb.scalars)
-  if (count) DS_FWD(false, true);
-  else if (target) DS_FWD(true, false);
-  else DS_FWD(false, false);
+  if (count) DS_FWD(false, true, true);
+  else if (target) DS_FWD(true, false, true);
+  else if (kBatch || !rb.image_only) DS_FWD(false, false, true);
+  else DS_FWD(false, false, false);
 #undef DS_FWD
 }
 

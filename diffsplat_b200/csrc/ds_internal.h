@@ -180,6 +180,7 @@ struct RasterBuffers {
   int grad_mode = DS_GRAD_REFERENCE;
   int schedule = DS_SCHEDULE_LONGEST_FIRST;  // composite tile order
   int tile_size = 16;  // pixels per tile edge: 16 (reference); batches may use 8 or 32
+  bool image_only = false;  // no backward follows: alphas and last_ids are not written
 
   // Batch mode (several independent instances in one set of buffers): set
   // together, null for a single instance.  Tiles and pixels are the

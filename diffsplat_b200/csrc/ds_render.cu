@@ -56,6 +56,7 @@ int ds_renderer_create(int width, int height, int max_splats, int sh_degree, int
   r->bands = ds::sh_bands(sh_degree);
   int st;
   if ((st = ds::raster_alloc(r->rb, width, height, max_splats, max_isects))) return fail(st);
+  r->rb.image_only = true;
   if ((st = ds::cuda_status(ds::device_alloc(&r->cam_dev, sizeof(ds::Camera))))) return fail(st);
   cudaMemset(r->cam_dev, 0, sizeof(ds::Camera));
   if ((st = ds::cuda_status(ds::device_alloc(&r->image, image_floats(width, height) * 4))))

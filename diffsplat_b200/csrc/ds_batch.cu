@@ -123,14 +123,19 @@ static int batch_enqueue(ds_batch* b, cudaStream_t s) {
   const int blocks = (n + kThreads - 1) / kThreads;
   const int exact = b->cfg.grad_mode == DS_GRAD_EXACT ? 1 : 0;
   ds_gaussian3d G = b->P;  // unused: keep_grads == 0
+  auto backward_adam = [&](auto kernel, auto r, auto m, auto v) {
+    kernel<<<blocks, kThreads, 0, s>>>(b->P, r, m, v, G, 0, exact, b->cfg.sh_degree, b->cams, rb.g2,
+                                       grad_segments(rb), rb.rec_c, b->bc_cur, rb.scalars, lr, h,
+                                       b->inst_of_splat, nullptr, nullptr, nullptr);
+  };
   if (bf16)
-    fit_backward_adam_kernel<__nv_bfloat16, true><<<blocks, kThreads, 0, s>>>(
-        b->P, b->R16, b->M16, b->V16, G, 0, exact, b->cfg.sh_degree, b->cams, rb.g2,
-        grad_segments(rb), b->bc_cur, rb.scalars, lr, h, b->inst_of_splat);
+    backward_adam(b->bands > 0 ? fit_backward_adam_kernel<__nv_bfloat16, true, true>
+                               : fit_backward_adam_kernel<__nv_bfloat16, false, true>,
+                  b->R16, b->M16, b->V16);
   else
-    fit_backward_adam_kernel<float, true><<<blocks, kThreads, 0, s>>>(
-        b->P, soa_of(b->P), soa_of(b->M), soa_of(b->V), G, 0, exact, b->cfg.sh_degree, b->cams,
-        rb.g2, grad_segments(rb), b->bc_cur, rb.scalars, lr, h, b->inst_of_splat);
+    backward_adam(b->bands > 0 ? fit_backward_adam_kernel<float, true, true>
+                               : fit_backward_adam_kernel<float, false, true>,
+                  soa_of(b->P), soa_of(b->M), soa_of(b->V));
   return cuda_status(cudaGetLastError());
 }
 

@@ -97,16 +97,19 @@ static int fitter_enqueue(ds_fitter* f, cudaStream_t s, cudaEvent_t* ev = nullpt
          f->cfg.lr_opacity};
   AdamHyper h{f->cfg.beta1, f->cfg.beta2, f->cfg.epsilon};
   const int keep = f->g_mem ? 1 : 0, exact = f->cfg.grad_mode == DS_GRAD_EXACT ? 1 : 0;
+  auto backward_adam = [&](auto kernel, auto r, auto m, auto v) {
+    return launch_pdl(kernel, dim3(blocks), dim3(kThreads), 0, s, f->P, r, m, v, f->G, keep, exact,
+                      f->cfg.sh_degree, f->cam_dev, rb.g2, grad_segments(rb), rb.rec_c, f->bc_cur,
+                      rb.scalars, lr, h, nullptr, rb.counts, f->grad_accum, f->grad_count);
+  };
   if (bf16)
-    DS_CUDA(launch_pdl(fit_backward_adam_kernel<__nv_bfloat16>, dim3(blocks), dim3(kThreads), 0,
-                       s, f->P, f->R16, f->M16, f->V16, f->G, keep, exact, f->cfg.sh_degree,
-                       f->cam_dev, rb.g2, grad_segments(rb), f->bc_cur, rb.scalars, lr, h,
-                       nullptr, rb.counts, f->grad_accum, f->grad_count));
+    DS_CUDA(backward_adam(f->bands > 0 ? fit_backward_adam_kernel<__nv_bfloat16, true>
+                                       : fit_backward_adam_kernel<__nv_bfloat16, false>,
+                          f->R16, f->M16, f->V16));
   else
-    DS_CUDA(launch_pdl(fit_backward_adam_kernel<float>, dim3(blocks), dim3(kThreads), 0, s, f->P,
-                       soa_of(f->P), soa_of(f->M), soa_of(f->V), f->G, keep, exact,
-                       f->cfg.sh_degree, f->cam_dev, rb.g2, grad_segments(rb), f->bc_cur,
-                       rb.scalars, lr, h, nullptr, rb.counts, f->grad_accum, f->grad_count));
+    DS_CUDA(backward_adam(f->bands > 0 ? fit_backward_adam_kernel<float, true>
+                                       : fit_backward_adam_kernel<float, false>,
+                          soa_of(f->P), soa_of(f->M), soa_of(f->V)));
   if (ev) DS_CUDA(cudaEventRecord(ev[7], s));
   return DS_OK;
 }

@@ -281,14 +281,15 @@ int ds_batch_create(const ds_batch_config* cfg, const ds_batch_instance* inst, d
   cudaMemcpy(b->geom_dev, b->geom.data(), (size_t)I * sizeof(ds::InstGeom),
              cudaMemcpyHostToDevice);
   cudaMemset(b->cams, 0, (size_t)I * sizeof(ds::Camera));
-  if ((st = ds::raster_alloc_batch(b->rb, pixels, (int)tiles, TS, n, cfg->max_isects)))
-    return fail(st);
-  b->rb.grad_mode = cfg->grad_mode;
-  b->rb.schedule = cfg->schedule;
   b->rb.inst_of_splat = b->inst_of_splat;
   b->rb.tile_inst = b->tile_inst;
   b->rb.geom = b->geom_dev;
   b->rb.instances = I;
+  if ((st = ds::raster_alloc_batch(b->rb, pixels, (int)tiles, TS, n, cfg->max_isects,
+                                   b->geom.data())))
+    return fail(st);
+  b->rb.grad_mode = cfg->grad_mode;
+  b->rb.schedule = cfg->schedule;
   if ((st = ds::make_bc_table(cfg->beta1, cfg->beta2, &b->bc_table, &b->bc_len))) return fail(st);
   if ((st = ds::cuda_status(ds::device_alloc(&b->bc_cur, sizeof(float2))))) return fail(st);
   uint32_t nn = (uint32_t)n;

@@ -100,8 +100,8 @@ int launch_project_backward(const ds_splat3d& in, const float pv[16], const ds_s
 // captured into a CUDA graph.  Fixed grid of kSortBlocks CTAs.
 // ---------------------------------------------------------------------------
 constexpr int kSortBlocks = 296;    // 2 x 148 SMs
-// Tile grids up to this size sort their pairs by a single stable counting
-// pass (ds_raster.cu); larger ones by radix passes over the tile id.
+// Tile grids up to this size sort their pairs, where they have any, by a single stable
+// counting pass (ds_raster.cu); larger ones by radix passes over the tile id.
 constexpr int kCountSortMaxTiles = 8192;
 constexpr int kSortTileItems = 2048;  // items per CTA iteration (8 warps x 32 lanes x 8)
 
@@ -114,11 +114,15 @@ struct SortScratch {
 // kb may alias kin (the input is consumed by pass 0); ka may not.  *out_k /
 // *out_v receive the buffers holding the result.  vin == nullptr means the
 // input values are 0..n-1.  When gather_src != nullptr, the last pass also
-// writes gather_dst[q] = gather_src[value[q]].
+// writes gather_dst[q] = gather_src[value[q]].  With group set, `group_bits` bits of
+// group[value] are the most significant digits (more passes; the sorted keys are then
+// the groups).
+template <typename G>
 int radix_sort_pairs(const uint32_t* kin, const uint32_t* vin, uint32_t* ka, uint32_t* va,
                      uint32_t* kb, uint32_t* vb, uint32_t** out_k, uint32_t** out_v,
-                     const uint32_t* n_dev, uint32_t cap, int bits, const uint32_t* gather_src,
-                     uint32_t* gather_dst, SortScratch& scratch, cudaStream_t s);
+                     const uint32_t* n_dev, uint32_t cap, int bits, const G* gather_src,
+                     G* gather_dst, SortScratch& scratch, cudaStream_t s,
+                     const uint16_t* group = nullptr, int group_bits = 0);
 
 // Exclusive scan of counts gathered through a permutation:
 //   offsets[p] = sum_{q < p} counts[perm[q]]   (64-bit),
@@ -137,12 +141,18 @@ struct ScanScratch {
 // offsets[p] = exclusive sum of counts[perm[q]], q < p.  With long_list set,
 // also long_list[0 .. *n_long) = {perm[p], offsets[p], offsets[p] +
 // counts[perm[p]]} (offsets clamped to cap) for the positions p with
-// counts[perm[p]] > kSerialRecords, ascending in p.
+// counts[perm[p]] > kSerialRecords, ascending in p.  With rect_sorted set (the tile
+// rectangles in order of p), counts[perm[p]] is the rectangle's area, and also
+//   seg_start[perm[p]] = min(offsets[p], cap) where it is not empty,
+//   sc->last_p, last_m: the last p of which any pair fits cap, and how many of its
+//   pairs do (last_p = 0xffffffff: all pairs fit).
+struct DevScalars;
 int scan_counts_permuted(const uint32_t* counts, const uint32_t* perm, uint32_t n,
                          unsigned long long* offsets, uint32_t* n_clamped,
                          unsigned long long* raw_total, uint32_t cap, uint32_t* status,
                          ScanScratch& scratch, cudaStream_t s, uint4* long_list = nullptr,
-                         uint32_t* n_long = nullptr);
+                         uint32_t* n_long = nullptr, const ushort4* rect_sorted = nullptr,
+                         uint32_t* seg_start = nullptr, DevScalars* sc = nullptr);
 
 // Device-resident scalars of one rasterizer / fitter.
 struct DevScalars {
@@ -158,6 +168,7 @@ struct DevScalars {
   float loss;
   float pad2;
   unsigned long long pairs[2];  // counting forward: contributing, tested (pixel, splat) pairs
+  uint32_t last_p, last_m;      // see scan_counts_permuted
 };
 
 // ---------------------------------------------------------------------------
@@ -194,7 +205,8 @@ struct RasterBuffers {
   float4* rec_a = nullptr;
   float4* rec_b = nullptr;
   float4* rec_c = nullptr;
-  ushort4* rect = nullptr;     // tile rectangle {x0, x1, y0, y1}
+  ushort4* rect = nullptr;     // tile rectangle {x0, x1, y0, y1}; {1, 0, 1, 0} when invisible
+  ushort4* rect_sorted = nullptr;  // in depth order (tile lists by bins; else null)
   uint32_t* counts = nullptr;  // tiles per splat (0 = invisible)
   uint32_t* seg_start = nullptr;  // first emission index of each splat
   uint4* long_list = nullptr;  // {splat, first record, record end} of splats with long segments
@@ -206,7 +218,7 @@ struct RasterBuffers {
   unsigned long long* emit_offsets = nullptr;  // exclusive scan of counts in depth order
   float* g2 = nullptr;  // [9][max_splats] per-splat Splat2D gradient sums (fitter path)
 
-  // per intersection
+  // per intersection (all but sorted_splat and isect_grad: where pairs are sorted)
   uint32_t* tile_k0 = nullptr;
   uint32_t* tile_k1 = nullptr;
   uint32_t* tile_v0 = nullptr;
@@ -221,13 +233,17 @@ struct RasterBuffers {
   uint32_t* depth_perm = nullptr;         // depth-sorted splat ids
   uint32_t* depth_sorted_keys = nullptr;  // their depth keys
 
-  // Counting sort of the pairs by tile (grids of at most kCountSortMaxTiles
-  // tiles; null: the radix path): per-chunk tile counts, then their column
-  // prefix [count_chunks][tiles], and the per-tile totals.
+  // Per-chunk tile counts, then their column prefix, and the per-tile totals, of
+  // the tile lists by bins (ds_tiles.cu) or of the counting sort of the pairs (grids of
+  // at most kCountSortMaxTiles tiles; null: the radix path).
   uint32_t* tile_hist = nullptr;
   uint32_t* tile_totals = nullptr;
   int count_chunks = 0;
-
+  // Batches, by bins: chunks {first splat, end, instance, first of tile_hist} and per
+  // instance {first of tile_hist, chunks}
+  int4* bin_chunks = nullptr;
+  int2* inst_hist = nullptr;
+  int bin_chunk_count = 0, bin_per = 0, bin_most = 0;
   // per tile / pixel
   unsigned long long* tile_bound = nullptr;  // see GradSegments
   int2* ranges = nullptr;
@@ -290,10 +306,10 @@ int raster_alloc(RasterBuffers& rb, int width, int height, int max_splats, int64
 bool composite_longest_first();
 int raster_resize(RasterBuffers& rb, int width, int height);
 // Batch-mode allocation: `tiles` tiles of tile_size^2 pixels over `pixels`
-// pixels in all (the concatenated instance grids); the geometry arrays are set
-// by the caller.
+// pixels in all (the concatenated instance grids); inst: the instances, whose device
+// arrays (geom, tile_inst, inst_of_splat) the caller has set.
 int raster_alloc_batch(RasterBuffers& rb, int64_t pixels, int tiles, int tile_size,
-                       int max_splats, int64_t cap);
+                       int max_splats, int64_t cap, const InstGeom* inst);
 void raster_free(RasterBuffers& rb);
 
 // Everything after the per-splat records exist: depth sort, emission, tile
@@ -302,6 +318,17 @@ void raster_free(RasterBuffers& rb);
 // reduce gradients afterwards).
 int raster_build_lists(RasterBuffers& rb, int n, cudaStream_t s, cudaEvent_t* ev = nullptr,
                        bool with_long_list = false);
+
+// Tile lists by bins (ds_tiles.cu): ranges, sorted_splat and the composite schedule
+// from rect_sorted and depth_perm.  tile_bins_pay: whether they are the faster way
+// for this grid and max_splats; inst: the instances of a batch.
+bool tile_bins_pay(const RasterBuffers& rb, const InstGeom* inst);
+int tile_bins_alloc(RasterBuffers& rb, const InstGeom* inst);
+int tile_bins(RasterBuffers& rb, int n, cudaStream_t s);
+// Column prefix of the per-chunk counts, ranges and schedule (single instance).
+int tile_offsets(RasterBuffers& rb, int chunks, cudaStream_t s);
+// The composite schedule alone, from the ranges.
+int tile_order(RasterBuffers& rb, cudaStream_t s);
 
 // Copies the state of the last forward to host memory (synchronises the
 // device); `what` is one of DS_RASTER_KEYS .. DS_RASTER_COUNTS and n_splats the

@@ -125,6 +125,7 @@ __global__ void __launch_bounds__(kPreThreads)
       }
     }
     if (!vis) {
+      rect[i] = make_ushort4(1, 0, 1, 0);
       counts[i] = 0u;
       depth_keys[i] = 0xffffffffu;
     }

@@ -58,6 +58,7 @@ __global__ void __launch_bounds__(kThreads)
       counts[i] = (uint32_t)((r.x1 - r.x0 + 1) * (r.y1 - r.y0 + 1));
       depth_keys[i] = depth_bits(z);
     } else {
+      rect[i] = make_ushort4(1, 0, 1, 0);
       counts[i] = 0u;
       depth_keys[i] = 0xffffffffu;
     }
@@ -336,8 +337,6 @@ __global__ void __launch_bounds__(kThreads)
 //                       the tile's place in its rectangle, so none is stored.)
 // One pass over the pairs instead of ceil(log2 T / 8) radix passes, and the
 // ranges come out of the scan.
-constexpr int kOffsetThreads = 1024;  // 32 tiles x 32 slices of the chunk column
-
 __device__ __forceinline__ void chunk_of(uint32_t n, uint32_t chunks, uint32_t c, uint32_t& lo,
                                          uint32_t& hi) {
   const uint32_t per = (n + chunks - 1) / chunks;
@@ -373,83 +372,6 @@ __global__ void __launch_bounds__(kThreads)
   __syncthreads();
   uint32_t* row = hist + (size_t)blockIdx.x * tiles;
   for (int t = threadIdx.x; t < tiles; t += kThreads) row[t] = cnt[t];
-}
-
-__device__ void order_tiles(const int2* __restrict__ ranges, int tiles, int32_t* __restrict__ order);
-
-__global__ void __launch_bounds__(kOffsetThreads)
-    tile_offsets_kernel(uint32_t* __restrict__ hist, int chunks, int tiles,
-                        uint32_t* __restrict__ totals, int2* __restrict__ ranges,
-                        DevScalars* __restrict__ sc, int32_t* __restrict__ order) {
-  pdl_wait();
-  constexpr int kSlices = kOffsetThreads / 32;
-  __shared__ uint32_t part[kSlices][33];
-  __shared__ uint32_t wsum[kSlices];
-  __shared__ bool last;
-  const int lane = threadIdx.x & 31, s = threadIdx.x >> 5;
-  const int t = blockIdx.x * 32 + lane;
-  const int r0 = s * chunks / kSlices, r1 = (s + 1) * chunks / kSlices;
-  uint32_t sum = 0;
-  if (t < tiles) {
-#pragma unroll 4
-    for (int r = r0; r < r1; ++r) sum += hist[(size_t)r * tiles + t];
-  }
-  part[s][lane] = sum;
-  __syncthreads();
-  uint32_t run = 0;
-  for (int k = 0; k < s; ++k) run += part[k][lane];
-  if (t < tiles) {
-    for (int r = r0; r < r1; ++r) {
-      const size_t q = (size_t)r * tiles + t;
-      const uint32_t v = hist[q];
-      hist[q] = run;
-      run += v;
-    }
-    if (s == kSlices - 1) totals[t] = run;
-  }
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) last = atomicAdd(&sc->sort_ticket, 1u) == gridDim.x - 1;
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  // Last CTA: exclusive scan of the totals into the ranges; each thread takes
-  // a contiguous run of tiles.
-  const int per = (tiles + kOffsetThreads - 1) / kOffsetThreads;
-  const int a = min(tiles, threadIdx.x * per), b = min(tiles, a + per);
-  uint32_t mine = 0;
-  for (int k = a; k < b; ++k) mine += ((volatile uint32_t*)totals)[k];
-  uint32_t incl = mine;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += v;
-  }
-  if (lane == 31) wsum[s] = incl;
-  __syncthreads();
-  if (s == 0) {
-    const uint32_t w = wsum[lane];
-    uint32_t wi = w;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t v = __shfl_up_sync(0xffffffffu, wi, o);
-      if (lane >= o) wi += v;
-    }
-    wsum[lane] = wi - w;  // exclusive over the warps
-  }
-  __syncthreads();
-  uint32_t base = incl - mine + wsum[s];
-  for (int k = a; k < b; ++k) {
-    const uint32_t c = ((volatile uint32_t*)totals)[k];
-    ranges[k] = c ? make_int2((int)base, (int)(base + c)) : make_int2(0, 0);
-    base += c;
-  }
-  if (threadIdx.x == 0) sc->sort_ticket = 0u;
-  if (order) {
-    // the longest-first composite schedule from the ranges just written
-    __syncthreads();
-    order_tiles(ranges, tiles, order);
-  }
 }
 
 // kScatterWarps warps per CTA; dynamic shared memory 4 tiles + 2 kScatterWarps
@@ -579,68 +501,6 @@ __global__ void __launch_bounds__(32 * kScatterWarps)
   }
 }
 
-// Longest-first schedule of the composite CTAs: tiles bucketed by their list
-// length (quarter-octave buckets), buckets in descending order.  The heaviest
-// tiles start in the first wave, so they no longer set the kernel's tail.  The
-// order inside a bucket is arbitrary (plain shared atomics hand out the
-// slots); every tile's result is independent of it.
-constexpr int kOrderBuckets = 128;
-
-__device__ __forceinline__ int work_bucket(int2 r) {
-  const uint32_t len = (uint32_t)max(r.y - r.x, 0);
-  if (len == 0) return 0;
-  const int l = 31 - __clz(len);
-  const uint32_t sub = l >= 2 ? (len >> (l - 2)) & 3u : (len << (2 - l)) & 3u;
-  return min(kOrderBuckets - 1, 1 + 4 * l + (int)sub);
-}
-
-// The schedule of tiles [0, tiles) from their ranges, by one 1024-thread CTA.
-__device__ void order_tiles(const int2* __restrict__ ranges, int tiles, int32_t* __restrict__ order) {
-  __shared__ uint32_t cnt[kOrderBuckets];
-  __shared__ uint32_t off[kOrderBuckets];
-  for (int b = threadIdx.x; b < kOrderBuckets; b += blockDim.x) cnt[b] = 0u;
-  __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const int rounds = (tiles + (int)blockDim.x - 1) / (int)blockDim.x;
-  for (int r = 0; r < rounds; ++r) {
-    const int t = r * blockDim.x + threadIdx.x;
-    if (t < tiles) atomicAdd(&cnt[work_bucket(ranges[t])], 1u);
-  }
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    // lane l owns buckets 127-4l .. 124-4l (descending); exclusive scan over lanes
-    uint32_t v[4], s = 0;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      v[k] = cnt[kOrderBuckets - 1 - 4 * lane - k];
-      s += v[k];
-    }
-    uint32_t incl = s;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += t;
-    }
-    uint32_t run = incl - s;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      off[kOrderBuckets - 1 - 4 * lane - k] = run;
-      run += v[k];
-    }
-  }
-  __syncthreads();
-  for (int r = 0; r < rounds; ++r) {
-    const int t = r * blockDim.x + threadIdx.x;
-    if (t < tiles) order[atomicAdd(&off[work_bucket(ranges[t])], 1u)] = t;
-  }
-}
-
-__global__ void __launch_bounds__(1024)
-    tile_order_kernel(const int2* __restrict__ ranges, int tiles, int32_t* __restrict__ order) {
-  pdl_wait();
-  order_tiles(ranges, tiles, order);
-}
-
 template <typename T>
 int alloc(T** p, size_t n) {
   *p = nullptr;
@@ -684,11 +544,6 @@ static int raster_alloc_splats(RasterBuffers& rb, int max_splats, int64_t cap) {
   DS_TRY(alloc(&rb.emit_offsets, n));
   DS_TRY(alloc(&rb.g2, n * 9));
   const size_t c = (size_t)cap;
-  DS_TRY(alloc(&rb.tile_k0, c));
-  DS_TRY(alloc(&rb.tile_k1, c));
-  DS_TRY(alloc(&rb.tile_v0, c));
-  DS_TRY(alloc(&rb.tile_v1, c));
-  DS_TRY(alloc(&rb.emit_splat, c));
   DS_TRY(alloc(&rb.sorted_splat, c));
   DS_TRY(alloc(&rb.isect_grad, c * 9));
   DS_TRY(alloc(&rb.sort.hist, (size_t)256 * (kSortBlocks + 1)));
@@ -701,9 +556,9 @@ static int raster_alloc_splats(RasterBuffers& rb, int max_splats, int64_t cap) {
   return DS_OK;
 }
 
-// Scratch of the counting sort for a grid of rb.tiles tiles (none beyond
-// kCountSortMaxTiles, or with DS_TILE_SORT=radix: the radix path then runs).
-static int alloc_count_sort(RasterBuffers& rb) {
+// Buffers of the tile lists for a grid of rb.tiles tiles: those of ds_tiles.cu, the
+// counting sort's or the radix passes' (see the choice in raster_build_lists).
+static int alloc_tile_lists(RasterBuffers& rb, const InstGeom* inst = nullptr) {
   release(rb.tile_hist);
   release(rb.tile_totals);
   rb.count_chunks = 0;
@@ -711,6 +566,19 @@ static int alloc_count_sort(RasterBuffers& rb) {
     const char* e = getenv("DS_TILE_SORT");
     return e && strcmp(e, "radix") == 0;
   }();
+  if (!radix_only && tile_bins_pay(rb, inst)) {
+    if (!rb.rect_sorted) DS_TRY(alloc(&rb.rect_sorted, (size_t)rb.max_splats));
+    return tile_bins_alloc(rb, inst);
+  }
+  release(rb.rect_sorted);
+  if (!rb.tile_k0) {
+    const size_t c = (size_t)rb.cap;
+    DS_TRY(alloc(&rb.tile_k0, c));
+    DS_TRY(alloc(&rb.tile_k1, c));
+    DS_TRY(alloc(&rb.tile_v0, c));
+    DS_TRY(alloc(&rb.tile_v1, c));
+    DS_TRY(alloc(&rb.emit_splat, c));
+  }
   if (radix_only || rb.tiles <= 0 || rb.tiles > kCountSortMaxTiles) return DS_OK;
   // one chunk per 2 x 148 SMs, at least 512 pairs each
   rb.count_chunks = (int)std::max<int64_t>(1, std::min<int64_t>(kSortBlocks, (rb.cap + 511) / 512));
@@ -736,7 +604,7 @@ int raster_alloc(RasterBuffers& rb, int width, int height, int max_splats, int64
 }
 
 int raster_alloc_batch(RasterBuffers& rb, int64_t pixels, int tiles, int tile_size,
-                       int max_splats, int64_t cap) {
+                       int max_splats, int64_t cap, const InstGeom* inst) {
   if (pixels <= 0 || tiles <= 0 || max_splats < 0) return DS_ERR_ARG;
   if (tile_size != 8 && tile_size != 16 && tile_size != 32) return DS_ERR_ARG;
   DS_TRY(raster_alloc_splats(rb, max_splats, cap));
@@ -753,7 +621,7 @@ int raster_alloc_batch(RasterBuffers& rb, int64_t pixels, int tiles, int tile_si
   DS_TRY(alloc(&rb.last_ids, (size_t)pixels));
   DS_TRY(alloc(&rb.loss_partials, (size_t)tiles * loss_parts(tile_size)));
   DS_CUDA(cudaMemset(rb.ranges, 0, tiles * sizeof(int2)));
-  return alloc_count_sort(rb);
+  return alloc_tile_lists(rb, inst);
 }
 
 int raster_resize(RasterBuffers& rb, int width, int height) {
@@ -779,7 +647,7 @@ int raster_resize(RasterBuffers& rb, int width, int height) {
   DS_TRY(alloc(&rb.last_ids, px));
   DS_TRY(alloc(&rb.loss_partials, (size_t)rb.tiles));
   DS_CUDA(cudaMemset(rb.ranges, 0, rb.tiles * sizeof(int2)));
-  return alloc_count_sort(rb);
+  return alloc_tile_lists(rb);
 }
 
 void raster_free(RasterBuffers& rb) {
@@ -814,8 +682,11 @@ void raster_free(RasterBuffers& rb) {
   release(rb.alphas);
   release(rb.last_ids);
   release(rb.loss_partials);
+  release(rb.rect_sorted);
   release(rb.tile_hist);
   release(rb.tile_totals);
+  release(rb.bin_chunks);
+  release(rb.inst_hist);
   rb.width = rb.height = 0;
 }
 
@@ -834,15 +705,30 @@ int raster_build_lists(RasterBuffers& rb, int n, cudaStream_t s, cudaEvent_t* ev
                        bool with_long_list) {
   DevScalars* sc = rb.scalars;
   if (n > 0) {
-    // 1) depth order of the splats: stable sort of (depth bits, id)
+    // 1) depth order of the splats: stable sort of (depth bits, id); batches that list
+    //    their tiles by bins: within each instance
+    const bool bins = rb.rect_sorted != nullptr;
+    const bool by_instance = bins && rb.geom && rb.instances > 1;
     DS_TRY(radix_sort_pairs(rb.depth_keys, nullptr, rb.depth_k0, rb.depth_v0, rb.depth_k1,
                             rb.depth_v1, &rb.depth_sorted_keys, &rb.depth_perm, &sc->n_splats,
-                            (uint32_t)rb.max_splats, 32, nullptr, nullptr, rb.sort, s));
+                            (uint32_t)rb.max_splats, 32, bins ? rb.rect : nullptr, rb.rect_sorted,
+                            rb.sort, s, by_instance ? rb.inst_of_splat : nullptr,
+                            by_instance ? ceil_log2(rb.instances) : 0));
     if (ev) DS_CUDA(cudaEventRecord(ev[0], s));
-    // 2) emission offsets in depth order
+    // 2) offsets of the splats' pairs (and gradient records) in depth order
     DS_TRY(scan_counts_permuted(rb.counts, rb.depth_perm, (uint32_t)n, rb.emit_offsets,
                                 &sc->n_isects, &sc->n_isects_raw, (uint32_t)rb.cap, &sc->status,
-                                rb.scan, s, with_long_list ? rb.long_list : nullptr, &sc->n_long));
+                                rb.scan, s, with_long_list ? rb.long_list : nullptr, &sc->n_long,
+                                bins ? rb.rect_sorted : nullptr, bins ? rb.seg_start : nullptr,
+                                sc));
+    if (bins) {
+      // 3) tile lists
+      if (ev) DS_CUDA(cudaEventRecord(ev[1], s));
+      DS_TRY(tile_bins(rb, n, s));
+      rb.sorted_tile = nullptr;
+      if (ev) DS_CUDA(cudaEventRecord(ev[2], s));
+      return DS_OK;
+    }
     // 3) emit (tile, emission index) pairs grouped by splat in depth order
     const dim3 emit_grid((unsigned)(((int64_t)n * 4 + kThreads - 1) / kThreads));
     static_assert(kCountSortMaxTiles <= 65536, "counting-path tile ids are 16-bit");
@@ -866,10 +752,7 @@ int raster_build_lists(RasterBuffers& rb, int n, cudaStream_t s, cudaEvent_t* ev
       const size_t sct_smem = (size_t)T * 4 + (size_t)((T + 1) & ~1) * 2 * kScatterWarps;
       DS_CUDA(launch_pdl(tile_count_kernel, dim3(G), dim3(kThreads), cnt_smem, s, tile16,
                          &sc->n_isects, T, rb.tile_hist, &sc->status));
-      int32_t* order = (rb.tile_order && rb.schedule == DS_SCHEDULE_LONGEST_FIRST)
-                           ? rb.tile_order : nullptr;
-      DS_CUDA(launch_pdl(tile_offsets_kernel, dim3((T + 31) / 32), dim3(kOffsetThreads), 0, s,
-                         rb.tile_hist, G, T, rb.tile_totals, rb.ranges, sc, order));
+      DS_TRY(tile_offsets(rb, G, s));
       DS_CUDA(launch_pdl(tile_scatter_kernel, dim3(G), dim3(32 * kScatterWarps), sct_smem, s,
                          tile16,
                          rb.emit_splat, &sc->n_isects, T, rb.tile_hist, rb.ranges,
@@ -902,10 +785,7 @@ int raster_build_lists(RasterBuffers& rb, int n, cudaStream_t s, cudaEvent_t* ev
                        &sc->status));
   }
   DS_CUDA(cudaGetLastError());
-  if (rb.tile_order && rb.schedule == DS_SCHEDULE_LONGEST_FIRST) {
-    DS_CUDA(launch_pdl(tile_order_kernel, dim3(1), dim3(1024), 0, s, rb.ranges, rb.tiles,
-                       rb.tile_order));
-  }
+  DS_TRY(tile_order(rb, s));
   if (ev) DS_CUDA(cudaEventRecord(ev[2], s));
   return DS_OK;
 }

@@ -35,7 +35,8 @@ __device__ __forceinline__ uint32_t sort_chunk(uint32_t n, uint32_t G) {
 }
 
 __global__ void __launch_bounds__(kThreads)
-    radix_hist_kernel(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ n_dev,
+    radix_hist_kernel(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ vals,
+                      const uint16_t* __restrict__ group, const uint32_t* __restrict__ n_dev,
                       uint32_t cap, int shift, uint32_t* __restrict__ hist) {
   pdl_wait();
   __shared__ uint32_t h[256];
@@ -54,7 +55,8 @@ __global__ void __launch_bounds__(kThreads)
 #pragma unroll
     for (int it = 0; it < kItems; ++it) {
       const uint32_t i = t0 + it * kThreads + threadIdx.x;
-      d[it] = i < end ? ((keys[i] >> shift) & 255u) : 0x100u;
+      const uint32_t k = i < end ? (group ? (uint32_t)group[vals[i]] : keys[i]) : 0u;
+      d[it] = i < end ? ((k >> shift) & 255u) : 0x100u;
     }
 #pragma unroll
     for (int it = 0; it < kItems; ++it) {
@@ -109,12 +111,13 @@ __global__ void __launch_bounds__(kThreads) scan_hist_kernel(uint32_t* __restric
 // warp with __match_any_sync, turns the per-warp digit counts into tile-local
 // offsets, stages the tile in digit order in shared memory and writes it out
 // in that order, so items of one digit leave as contiguous runs.
+template <typename G>
 __global__ void __launch_bounds__(kThreads)
     radix_scatter_kernel(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin,
-                         int iota, uint32_t* __restrict__ kout, uint32_t* __restrict__ vout,
+                         const uint16_t* __restrict__ group, int iota, uint32_t* __restrict__ kout, uint32_t* __restrict__ vout,
                          const uint32_t* __restrict__ n_dev, uint32_t cap, int shift,
-                         const uint32_t* __restrict__ offs, const uint32_t* __restrict__ gsrc,
-                         uint32_t* __restrict__ gdst) {
+                         const uint32_t* __restrict__ offs, const G* __restrict__ gsrc,
+                         G* __restrict__ gdst) {
   pdl_wait();
   __shared__ uint32_t cnt[kWarps][256];  // per-warp digit counts, then per-warp offsets
   __shared__ uint32_t gbase[256];        // output position of the tile's first item of a digit
@@ -156,8 +159,8 @@ __global__ void __launch_bounds__(kThreads)
     for (int it = 0; it < kItems; ++it) {
       const uint32_t idx = t0 + w * 256 + it * 32 + lane;
       const bool ok = idx < end;
-      key[it] = ok ? kin[idx] : 0u;
       val[it] = ok ? (iota ? idx : vin[idx]) : 0u;
+      key[it] = ok ? (group ? (uint32_t)group[val[it]] : kin[idx]) : 0u;
     }
 #pragma unroll
     for (int it = 0; it < kItems; ++it) {
@@ -216,6 +219,15 @@ __global__ void __launch_bounds__(kThreads)
 // ---- permuted exclusive scan of counts -----------------------------------
 constexpr int kScanItems = 4;
 
+// Tiles of the p-th splat: its rectangle's area, or its count.
+__device__ __forceinline__ uint32_t tiles_of(const uint32_t* __restrict__ counts,
+                                             const uint32_t* __restrict__ perm,
+                                             const ushort4* __restrict__ rect_sorted, uint32_t p) {
+  if (!rect_sorted) return counts[perm[p]];
+  const ushort4 r = rect_sorted[p];
+  return (uint32_t)((int)r.y - (int)r.x + 1) * (uint32_t)((int)r.w - (int)r.z + 1);
+}
+
 __device__ __forceinline__ uint32_t scan_chunk(uint32_t n) {
   uint32_t per = (n + kSortBlocks - 1) / kSortBlocks;
   const uint32_t step = kThreads * kScanItems;
@@ -228,9 +240,11 @@ __device__ __forceinline__ uint32_t scan_chunk(uint32_t n) {
 // the long-segment gradient reduction walks.
 __global__ void __launch_bounds__(kThreads)
     scan_partial_kernel(const uint32_t* __restrict__ counts, const uint32_t* __restrict__ perm,
-                        uint32_t n, unsigned long long* __restrict__ partials,
-                        uint32_t* __restrict__ long_partials) {
+                        const ushort4* __restrict__ rect_sorted, uint32_t n,
+                        unsigned long long* __restrict__ partials,
+                        uint32_t* __restrict__ long_partials, DevScalars* __restrict__ sc) {
   pdl_wait();
+  if (sc && blockIdx.x == 0 && threadIdx.x == 0) sc->last_p = 0xffffffffu;
   __shared__ unsigned long long wsum[kWarps];
   __shared__ uint32_t wlong[kWarps];
   const uint32_t chunk = scan_chunk(n);
@@ -239,7 +253,7 @@ __global__ void __launch_bounds__(kThreads)
   unsigned long long s = 0;
   uint32_t l = 0;
   for (uint32_t p = begin + threadIdx.x; p < end; p += kThreads) {
-    const uint32_t c = counts[perm[p]];
+    const uint32_t c = tiles_of(counts, perm, rect_sorted, p);
     s += c;
     l += c > kSerialRecords ? 1u : 0u;
   }
@@ -267,8 +281,10 @@ __global__ void __launch_bounds__(kThreads)
 
 __global__ void __launch_bounds__(kThreads)
     scan_final_kernel(const uint32_t* __restrict__ counts, const uint32_t* __restrict__ perm,
-                      uint32_t n, const unsigned long long* __restrict__ partials,
+                      const ushort4* __restrict__ rect_sorted, uint32_t n,
+                      const unsigned long long* __restrict__ partials,
                       unsigned long long* __restrict__ offsets,
+                      uint32_t* __restrict__ seg_start, DevScalars* __restrict__ sc,
                       const uint32_t* __restrict__ long_partials,
                       uint4* __restrict__ long_list, uint32_t cap,
                       uint32_t* __restrict__ n_clamped, unsigned long long* __restrict__ raw,
@@ -332,7 +348,7 @@ __global__ void __launch_bounds__(kThreads)
     for (int k = 0; k < kScanItems; ++k) {
       uint32_t p = t0 + threadIdx.x * kScanItems + k;
       pi[k] = p < end ? perm[p] : 0u;
-      c[k] = p < end ? counts[pi[k]] : 0u;
+      c[k] = p < end ? tiles_of(counts, perm, rect_sorted, p) : 0u;
       s += c[k];
       lmask |= (c[k] > kSerialRecords ? 1u : 0u) << k;
     }
@@ -374,6 +390,13 @@ __global__ void __launch_bounds__(kThreads)
       const unsigned long long s0 = excl;
       if (p < end) offsets[p] = s0;
       excl += c[k];
+      if (seg_start && c[k]) {
+        seg_start[pi[k]] = (uint32_t)(s0 < cap ? s0 : cap);
+        if (s0 < cap && excl >= cap) {
+          sc->last_p = p;
+          sc->last_m = (uint32_t)(cap - s0);
+        }
+      }
       if (long_list && (lmask >> k & 1u)) {
         // {splat, first record, end of its records}, clamped to the capacity
         const unsigned long long cp = cap;
@@ -389,27 +412,31 @@ __global__ void __launch_bounds__(kThreads)
 
 }  // namespace
 
+template <typename G>
 int radix_sort_pairs(const uint32_t* kin, const uint32_t* vin, uint32_t* ka, uint32_t* va,
                      uint32_t* kb, uint32_t* vb, uint32_t** out_k, uint32_t** out_v,
-                     const uint32_t* n_dev, uint32_t cap, int bits, const uint32_t* gather_src,
-                     uint32_t* gather_dst, SortScratch& scratch, cudaStream_t s) {
-  const int passes = bits <= 0 ? 1 : (bits + 7) / 8;
+                     const uint32_t* n_dev, uint32_t cap, int bits, const G* gather_src,
+                     G* gather_dst, SortScratch& scratch, cudaStream_t s, const uint16_t* group,
+                     int group_bits) {
+  const int key_passes = bits <= 0 ? 1 : (bits + 7) / 8;
+  const int passes = key_passes + (group ? (group_bits + 7) / 8 : 0);
   // One CTA per 2048-item tile of the capacity, at most kSortBlocks.
   const uint64_t tiles = ((uint64_t)cap + kSortTileItems - 1) / kSortTileItems;
-  const int G = (int)(tiles < 1 ? 1 : (tiles > (uint64_t)kSortBlocks ? kSortBlocks : tiles));
+  const int blocks = (int)(tiles < 1 ? 1 : (tiles > (uint64_t)kSortBlocks ? kSortBlocks : tiles));
   const uint32_t* src_k = kin;
   const uint32_t* src_v = vin;
   uint32_t* dst_k = ka;
   uint32_t* dst_v = va;
   for (int p = 0; p < passes; ++p) {
-    const int shift = 8 * p;
+    const uint16_t* digits = p < key_passes ? nullptr : group;
+    const int shift = 8 * (p < key_passes ? p : p - key_passes);
     const bool last = p == passes - 1;
-    DS_CUDA(launch_pdl(radix_hist_kernel, dim3(G), dim3(kThreads), 0, s, src_k, n_dev, cap, shift,
-                       scratch.hist));
+    DS_CUDA(launch_pdl(radix_hist_kernel, dim3(blocks), dim3(kThreads), 0, s, src_k, src_v, digits,
+                       n_dev, cap, shift, scratch.hist));
     DS_CUDA(launch_pdl(scan_hist_kernel, dim3(256 / kWarps), dim3(kThreads), 0, s, scratch.hist,
-                       G));
-    DS_CUDA(launch_pdl(radix_scatter_kernel, dim3(G), dim3(kThreads), 0, s, src_k, src_v,
-                       src_v == nullptr ? 1 : 0, dst_k, dst_v, n_dev, cap, shift,
+                       blocks));
+    DS_CUDA(launch_pdl(radix_scatter_kernel<G>, dim3(blocks), dim3(kThreads), 0, s, src_k, src_v,
+                       digits, src_v == nullptr ? 1 : 0, dst_k, dst_v, n_dev, cap, shift,
                        (const uint32_t*)scratch.hist, last ? gather_src : nullptr,
                        last ? gather_dst : nullptr));
     *out_k = dst_k;
@@ -422,17 +449,29 @@ int radix_sort_pairs(const uint32_t* kin, const uint32_t* vin, uint32_t* ka, uin
   return cuda_status(cudaGetLastError());
 }
 
+template int radix_sort_pairs<uint32_t>(const uint32_t*, const uint32_t*, uint32_t*, uint32_t*,
+                                        uint32_t*, uint32_t*, uint32_t**, uint32_t**,
+                                        const uint32_t*, uint32_t, int, const uint32_t*,
+                                        uint32_t*, SortScratch&, cudaStream_t, const uint16_t*,
+                                        int);
+template int radix_sort_pairs<ushort4>(const uint32_t*, const uint32_t*, uint32_t*, uint32_t*,
+                                       uint32_t*, uint32_t*, uint32_t**, uint32_t**,
+                                       const uint32_t*, uint32_t, int, const ushort4*, ushort4*,
+                                       SortScratch&, cudaStream_t, const uint16_t*, int);
+
 int scan_counts_permuted(const uint32_t* counts, const uint32_t* perm, uint32_t n,
                          unsigned long long* offsets, uint32_t* n_clamped,
                          unsigned long long* raw_total, uint32_t cap, uint32_t* status,
                          ScanScratch& scratch, cudaStream_t s, uint4* long_list,
-                         uint32_t* n_long) {
+                         uint32_t* n_long, const ushort4* rect_sorted, uint32_t* seg_start,
+                         DevScalars* sc) {
   if (long_list && (!scratch.long_partials || !n_long)) return DS_ERR_ARG;
   uint32_t* lp = long_list ? scratch.long_partials : nullptr;
   DS_CUDA(launch_pdl(scan_partial_kernel, dim3(kSortBlocks), dim3(kThreads), 0, s, counts, perm,
-                     n, scratch.partials, lp));
-  DS_CUDA(launch_pdl(scan_final_kernel, dim3(kSortBlocks), dim3(kThreads), 0, s, counts, perm, n,
-                     (const unsigned long long*)scratch.partials, offsets, (const uint32_t*)lp,
+                     rect_sorted, n, scratch.partials, lp, seg_start ? sc : nullptr));
+  DS_CUDA(launch_pdl(scan_final_kernel, dim3(kSortBlocks), dim3(kThreads), 0, s, counts, perm,
+                     rect_sorted, n, (const unsigned long long*)scratch.partials, offsets,
+                     seg_start, sc, (const uint32_t*)lp,
                      long_list, cap, n_clamped, raw_total, long_list ? n_long : nullptr, status));
   return cuda_status(cudaGetLastError());
 }

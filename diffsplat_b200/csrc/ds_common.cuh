@@ -297,6 +297,9 @@ __device__ __forceinline__ uint32_t depth_bits(float depth) {
   uint32_t u = __float_as_uint(depth);
   return (u >> 31) ? ~u : (u ^ 0x80000000u);
 }
+// Depth key of a splat in no tile, which no list holds: that of depth 1, the farthest, so
+// that it adds no digit to the sort.
+constexpr uint32_t kInvisibleKey = 0xbf800000u;
 
 // ---------------------------------------------------------------------------
 // Per-splat compositing record.  Three float4 per splat, written once by the

@@ -117,11 +117,10 @@ struct SortScratch {
 // writes gather_dst[q] = gather_src[value[q]].  With group set, `group_bits` bits of
 // group[value] are the most significant digits (more passes; the sorted keys are then
 // the groups).
-template <typename G>
 int radix_sort_pairs(const uint32_t* kin, const uint32_t* vin, uint32_t* ka, uint32_t* va,
                      uint32_t* kb, uint32_t* vb, uint32_t** out_k, uint32_t** out_v,
-                     const uint32_t* n_dev, uint32_t cap, int bits, const G* gather_src,
-                     G* gather_dst, SortScratch& scratch, cudaStream_t s,
+                     const uint32_t* n_dev, uint32_t cap, int bits, const uint32_t* gather_src,
+                     uint32_t* gather_dst, SortScratch& scratch, cudaStream_t s,
                      const uint16_t* group = nullptr, int group_bits = 0);
 
 // Exclusive scan of counts gathered through a permutation:
@@ -141,8 +140,9 @@ struct ScanScratch {
 // offsets[p] = exclusive sum of counts[perm[q]], q < p.  With long_list set,
 // also long_list[0 .. *n_long) = {perm[p], offsets[p], offsets[p] +
 // counts[perm[p]]} (offsets clamped to cap) for the positions p with
-// counts[perm[p]] > kSerialRecords, ascending in p.  With rect_sorted set (the tile
-// rectangles in order of p), counts[perm[p]] is the rectangle's area, and also
+// counts[perm[p]] > kSerialRecords, ascending in p.  With rect set (the tile rectangles),
+// a splat's count is its rectangle's area, and also
+//   rect_sorted[p] = rect[perm[p]],
 //   seg_start[perm[p]] = min(offsets[p], cap) where it is not empty,
 //   sc->last_p, last_m: the last p of which any pair fits cap, and how many of its
 //   pairs do (last_p = 0xffffffff: all pairs fit).
@@ -151,8 +151,21 @@ int scan_counts_permuted(const uint32_t* counts, const uint32_t* perm, uint32_t 
                          unsigned long long* offsets, uint32_t* n_clamped,
                          unsigned long long* raw_total, uint32_t cap, uint32_t* status,
                          ScanScratch& scratch, cudaStream_t s, uint4* long_list = nullptr,
-                         uint32_t* n_long = nullptr, const ushort4* rect_sorted = nullptr,
-                         uint32_t* seg_start = nullptr, DevScalars* sc = nullptr);
+                         uint32_t* n_long = nullptr, const ushort4* rect = nullptr,
+                         ushort4* rect_sorted = nullptr, uint32_t* seg_start = nullptr,
+                         DevScalars* sc = nullptr);
+
+// Depth order of up to kSmallSort splats of a single instance (ds_sort_small.cu).
+// cluster_sort: depth_perm, in one launch.  rank_sort, of up to kRankSort splats where
+// rank_sort_fits: also rect_sorted and what scan_counts_permuted writes (the long list
+// in any order), in two.  small_sort_setup comes once before the first on a device.
+constexpr int kSmallSort = 65536;
+constexpr int kRankSort = 8192;
+struct RasterBuffers;
+int small_sort_setup();
+bool rank_sort_fits(const RasterBuffers& rb, int n);
+int rank_sort(RasterBuffers& rb, int n, bool with_long_list, cudaStream_t s);
+int cluster_sort(RasterBuffers& rb, int n, cudaStream_t s);
 
 // Device-resident scalars of one rasterizer / fitter.
 struct DevScalars {
@@ -210,7 +223,8 @@ struct RasterBuffers {
   uint32_t* counts = nullptr;  // tiles per splat (0 = invisible)
   uint32_t* seg_start = nullptr;  // first emission index of each splat
   uint4* long_list = nullptr;  // {splat, first record, record end} of splats with long segments
-  uint32_t* depth_keys = nullptr;  // depth key of each splat (0xffffffff when invisible)
+  uint32_t* depth_keys = nullptr;  // depth key of each splat (kInvisibleKey when invisible)
+  uint32_t* rank = nullptr;        // [2 kRankSort] of rank_sort, zero between calls
   uint32_t* depth_k0 = nullptr;    // ping-pong buffers of the depth sort
   uint32_t* depth_k1 = nullptr;
   uint32_t* depth_v0 = nullptr;

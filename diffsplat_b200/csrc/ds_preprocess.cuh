@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(kPreThreads)
     if (!vis) {
       rect[i] = make_ushort4(1, 0, 1, 0);
       counts[i] = 0u;
-      depth_keys[i] = 0xffffffffu;
+      depth_keys[i] = kInvisibleKey;
     }
   }
   unsigned m = __ballot_sync(0xffffffffu, vis);

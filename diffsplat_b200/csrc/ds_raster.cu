@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(kThreads)
     } else {
       rect[i] = make_ushort4(1, 0, 1, 0);
       counts[i] = 0u;
-      depth_keys[i] = 0xffffffffu;
+      depth_keys[i] = kInvisibleKey;
     }
   }
   count_visible(vis, &sc->visible);
@@ -568,6 +568,13 @@ static int alloc_tile_lists(RasterBuffers& rb, const InstGeom* inst = nullptr) {
   }();
   if (!radix_only && tile_bins_pay(rb, inst)) {
     if (!rb.rect_sorted) DS_TRY(alloc(&rb.rect_sorted, (size_t)rb.max_splats));
+    if (!inst) {
+      DS_TRY(small_sort_setup());
+      if (!rb.rank) {
+        DS_TRY(alloc(&rb.rank, 2 * (size_t)kRankSort));
+        DS_CUDA(cudaMemset(rb.rank, 0, 2 * sizeof(uint32_t) * kRankSort));
+      }
+    }
     return tile_bins_alloc(rb, inst);
   }
   release(rb.rect_sorted);
@@ -683,6 +690,7 @@ void raster_free(RasterBuffers& rb) {
   release(rb.last_ids);
   release(rb.loss_partials);
   release(rb.rect_sorted);
+  release(rb.rank);
   release(rb.tile_hist);
   release(rb.tile_totals);
   release(rb.bin_chunks);
@@ -707,20 +715,29 @@ int raster_build_lists(RasterBuffers& rb, int n, cudaStream_t s, cudaEvent_t* ev
   if (n > 0) {
     // 1) depth order of the splats: stable sort of (depth bits, id); batches that list
     //    their tiles by bins: within each instance
-    const bool bins = rb.rect_sorted != nullptr;
-    const bool by_instance = bins && rb.geom && rb.instances > 1;
-    DS_TRY(radix_sort_pairs(rb.depth_keys, nullptr, rb.depth_k0, rb.depth_v0, rb.depth_k1,
-                            rb.depth_v1, &rb.depth_sorted_keys, &rb.depth_perm, &sc->n_splats,
-                            (uint32_t)rb.max_splats, 32, bins ? rb.rect : nullptr, rb.rect_sorted,
-                            rb.sort, s, by_instance ? rb.inst_of_splat : nullptr,
-                            by_instance ? ceil_log2(rb.instances) : 0));
-    if (ev) DS_CUDA(cudaEventRecord(ev[0], s));
     // 2) offsets of the splats' pairs (and gradient records) in depth order
-    DS_TRY(scan_counts_permuted(rb.counts, rb.depth_perm, (uint32_t)n, rb.emit_offsets,
-                                &sc->n_isects, &sc->n_isects_raw, (uint32_t)rb.cap, &sc->status,
-                                rb.scan, s, with_long_list ? rb.long_list : nullptr, &sc->n_long,
-                                bins ? rb.rect_sorted : nullptr, bins ? rb.seg_start : nullptr,
-                                sc));
+    const bool bins = rb.rect_sorted != nullptr;
+    const bool small = bins && !rb.geom && n <= kSmallSort;
+    const bool ranked = small && rank_sort_fits(rb, n);
+    if (ranked) {
+      DS_TRY(rank_sort(rb, n, with_long_list, s));
+    } else if (small) {
+      DS_TRY(cluster_sort(rb, n, s));
+    } else {
+      const bool by_instance = bins && rb.geom && rb.instances > 1;
+      DS_TRY(radix_sort_pairs(rb.depth_keys, nullptr, rb.depth_k0, rb.depth_v0, rb.depth_k1,
+                              rb.depth_v1, &rb.depth_sorted_keys, &rb.depth_perm, &sc->n_splats,
+                              (uint32_t)rb.max_splats, 32, nullptr, nullptr, rb.sort, s,
+                              by_instance ? rb.inst_of_splat : nullptr,
+                              by_instance ? ceil_log2(rb.instances) : 0));
+    }
+    if (ev) DS_CUDA(cudaEventRecord(ev[0], s));
+    if (!ranked)
+      DS_TRY(scan_counts_permuted(rb.counts, rb.depth_perm, (uint32_t)n, rb.emit_offsets,
+                                  &sc->n_isects, &sc->n_isects_raw, (uint32_t)rb.cap, &sc->status,
+                                  rb.scan, s, with_long_list ? rb.long_list : nullptr, &sc->n_long,
+                                  bins ? rb.rect : nullptr, bins ? rb.rect_sorted : nullptr,
+                                  bins ? rb.seg_start : nullptr, sc));
     if (bins) {
       // 3) tile lists
       if (ev) DS_CUDA(cudaEventRecord(ev[1], s));

@@ -111,13 +111,12 @@ __global__ void __launch_bounds__(kThreads) scan_hist_kernel(uint32_t* __restric
 // warp with __match_any_sync, turns the per-warp digit counts into tile-local
 // offsets, stages the tile in digit order in shared memory and writes it out
 // in that order, so items of one digit leave as contiguous runs.
-template <typename G>
 __global__ void __launch_bounds__(kThreads)
     radix_scatter_kernel(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin,
                          const uint16_t* __restrict__ group, int iota, uint32_t* __restrict__ kout, uint32_t* __restrict__ vout,
                          const uint32_t* __restrict__ n_dev, uint32_t cap, int shift,
-                         const uint32_t* __restrict__ offs, const G* __restrict__ gsrc,
-                         G* __restrict__ gdst) {
+                         const uint32_t* __restrict__ offs, const uint32_t* __restrict__ gsrc,
+                         uint32_t* __restrict__ gdst) {
   pdl_wait();
   __shared__ uint32_t cnt[kWarps][256];  // per-warp digit counts, then per-warp offsets
   __shared__ uint32_t gbase[256];        // output position of the tile's first item of a digit
@@ -219,12 +218,7 @@ __global__ void __launch_bounds__(kThreads)
 // ---- permuted exclusive scan of counts -----------------------------------
 constexpr int kScanItems = 4;
 
-// Tiles of the p-th splat: its rectangle's area, or its count.
-__device__ __forceinline__ uint32_t tiles_of(const uint32_t* __restrict__ counts,
-                                             const uint32_t* __restrict__ perm,
-                                             const ushort4* __restrict__ rect_sorted, uint32_t p) {
-  if (!rect_sorted) return counts[perm[p]];
-  const ushort4 r = rect_sorted[p];
+__device__ __forceinline__ uint32_t area_of(const ushort4& r) {
   return (uint32_t)((int)r.y - (int)r.x + 1) * (uint32_t)((int)r.w - (int)r.z + 1);
 }
 
@@ -240,8 +234,8 @@ __device__ __forceinline__ uint32_t scan_chunk(uint32_t n) {
 // the long-segment gradient reduction walks.
 __global__ void __launch_bounds__(kThreads)
     scan_partial_kernel(const uint32_t* __restrict__ counts, const uint32_t* __restrict__ perm,
-                        const ushort4* __restrict__ rect_sorted, uint32_t n,
-                        unsigned long long* __restrict__ partials,
+                        const ushort4* __restrict__ rect, ushort4* __restrict__ rect_sorted,
+                        uint32_t n, unsigned long long* __restrict__ partials,
                         uint32_t* __restrict__ long_partials, DevScalars* __restrict__ sc) {
   pdl_wait();
   if (sc && blockIdx.x == 0 && threadIdx.x == 0) sc->last_p = 0xffffffffu;
@@ -253,7 +247,14 @@ __global__ void __launch_bounds__(kThreads)
   unsigned long long s = 0;
   uint32_t l = 0;
   for (uint32_t p = begin + threadIdx.x; p < end; p += kThreads) {
-    const uint32_t c = tiles_of(counts, perm, rect_sorted, p);
+    uint32_t c;
+    if (rect) {
+      const ushort4 r = rect[perm[p]];
+      rect_sorted[p] = r;
+      c = area_of(r);
+    } else {
+      c = counts[perm[p]];
+    }
     s += c;
     l += c > kSerialRecords ? 1u : 0u;
   }
@@ -348,7 +349,7 @@ __global__ void __launch_bounds__(kThreads)
     for (int k = 0; k < kScanItems; ++k) {
       uint32_t p = t0 + threadIdx.x * kScanItems + k;
       pi[k] = p < end ? perm[p] : 0u;
-      c[k] = p < end ? tiles_of(counts, perm, rect_sorted, p) : 0u;
+      c[k] = p < end ? (rect_sorted ? area_of(rect_sorted[p]) : counts[pi[k]]) : 0u;
       s += c[k];
       lmask |= (c[k] > kSerialRecords ? 1u : 0u) << k;
     }
@@ -412,11 +413,10 @@ __global__ void __launch_bounds__(kThreads)
 
 }  // namespace
 
-template <typename G>
 int radix_sort_pairs(const uint32_t* kin, const uint32_t* vin, uint32_t* ka, uint32_t* va,
                      uint32_t* kb, uint32_t* vb, uint32_t** out_k, uint32_t** out_v,
-                     const uint32_t* n_dev, uint32_t cap, int bits, const G* gather_src,
-                     G* gather_dst, SortScratch& scratch, cudaStream_t s, const uint16_t* group,
+                     const uint32_t* n_dev, uint32_t cap, int bits, const uint32_t* gather_src,
+                     uint32_t* gather_dst, SortScratch& scratch, cudaStream_t s, const uint16_t* group,
                      int group_bits) {
   const int key_passes = bits <= 0 ? 1 : (bits + 7) / 8;
   const int passes = key_passes + (group ? (group_bits + 7) / 8 : 0);
@@ -435,7 +435,7 @@ int radix_sort_pairs(const uint32_t* kin, const uint32_t* vin, uint32_t* ka, uin
                        n_dev, cap, shift, scratch.hist));
     DS_CUDA(launch_pdl(scan_hist_kernel, dim3(256 / kWarps), dim3(kThreads), 0, s, scratch.hist,
                        blocks));
-    DS_CUDA(launch_pdl(radix_scatter_kernel<G>, dim3(blocks), dim3(kThreads), 0, s, src_k, src_v,
+    DS_CUDA(launch_pdl(radix_scatter_kernel, dim3(blocks), dim3(kThreads), 0, s, src_k, src_v,
                        digits, src_v == nullptr ? 1 : 0, dst_k, dst_v, n_dev, cap, shift,
                        (const uint32_t*)scratch.hist, last ? gather_src : nullptr,
                        last ? gather_dst : nullptr));
@@ -449,28 +449,19 @@ int radix_sort_pairs(const uint32_t* kin, const uint32_t* vin, uint32_t* ka, uin
   return cuda_status(cudaGetLastError());
 }
 
-template int radix_sort_pairs<uint32_t>(const uint32_t*, const uint32_t*, uint32_t*, uint32_t*,
-                                        uint32_t*, uint32_t*, uint32_t**, uint32_t**,
-                                        const uint32_t*, uint32_t, int, const uint32_t*,
-                                        uint32_t*, SortScratch&, cudaStream_t, const uint16_t*,
-                                        int);
-template int radix_sort_pairs<ushort4>(const uint32_t*, const uint32_t*, uint32_t*, uint32_t*,
-                                       uint32_t*, uint32_t*, uint32_t**, uint32_t**,
-                                       const uint32_t*, uint32_t, int, const ushort4*, ushort4*,
-                                       SortScratch&, cudaStream_t, const uint16_t*, int);
-
 int scan_counts_permuted(const uint32_t* counts, const uint32_t* perm, uint32_t n,
                          unsigned long long* offsets, uint32_t* n_clamped,
                          unsigned long long* raw_total, uint32_t cap, uint32_t* status,
                          ScanScratch& scratch, cudaStream_t s, uint4* long_list,
-                         uint32_t* n_long, const ushort4* rect_sorted, uint32_t* seg_start,
+                         uint32_t* n_long, const ushort4* rect, ushort4* rect_sorted, uint32_t* seg_start,
                          DevScalars* sc) {
   if (long_list && (!scratch.long_partials || !n_long)) return DS_ERR_ARG;
   uint32_t* lp = long_list ? scratch.long_partials : nullptr;
   DS_CUDA(launch_pdl(scan_partial_kernel, dim3(kSortBlocks), dim3(kThreads), 0, s, counts, perm,
-                     rect_sorted, n, scratch.partials, lp, seg_start ? sc : nullptr));
+                     rect, rect_sorted, n, scratch.partials, lp, seg_start ? sc : nullptr));
   DS_CUDA(launch_pdl(scan_final_kernel, dim3(kSortBlocks), dim3(kThreads), 0, s, counts, perm,
-                     rect_sorted, n, (const unsigned long long*)scratch.partials, offsets,
+                     (const ushort4*)rect_sorted, n,
+                     (const unsigned long long*)scratch.partials, offsets,
                      seg_start, sc, (const uint32_t*)lp,
                      long_list, cap, n_clamped, raw_total, long_list ? n_long : nullptr, status));
   return cuda_status(cudaGetLastError());

@@ -56,3 +56,31 @@ def test_batch_lists_do_not_depend_on_the_company(cuda_lib):
     for k in (0, 131, 299):
         img, par = fit([k])[0]
         assert np.array_equal(img, many[k][0]) and np.array_equal(par, many[k][1])
+
+
+@pytest.mark.parametrize("n", [1, 31, 1024, 1025, 2049, 4096, 8192, 8193, 20000, 65535, 65536, 65537])
+@pytest.mark.parametrize("depths", [1, 7, 100_000])
+def test_order_is_by_depth_then_id(cuda_lib, n, depths):
+    """The sorts of up to 8192 splats (by counting), of up to 65536 (one cluster) and of
+    more: equal depths by id, depths that share all digits or few, splats in no tile
+    among them."""
+    import torch
+
+    from diffsplat_b200 import _lib as L, api
+    r = np.random.default_rng(n + depths)
+    S = np.zeros((10, n), np.float32)
+    S[0:2] = r.uniform(-1.2, 1.2, (2, n))  # some centres outside: culled
+    S[2] = -0.5 + r.integers(0, depths, n) / depths
+    S[3] = S[5] = r.uniform(1e-3, 4e-2, n) ** 2
+    S[6:10] = 0.5
+    S2 = torch.from_numpy(S).cuda()
+    ras = api.Rasterizer(200, 120, n, 1 << 22)
+    ras.forward(S2)
+    keys, ids = ras.download(L.DS_RASTER_KEYS), ras.download(L.DS_RASTER_IDS)
+    counts = ras.download(L.DS_RASTER_COUNTS, n)
+    assert len(keys) == counts.sum() and ras.status()[0] == 0
+    k, i = keys.astype(np.int64), ids.astype(np.int64)
+    assert np.all((k[1:] > k[:-1]) | ((k[1:] == k[:-1]) & (i[1:] > i[:-1])))
+    assert np.array_equal(np.bincount(i, minlength=n), counts)
+    ranges = ras.download(L.DS_RASTER_RANGES).reshape(-1, 2)
+    assert np.array_equal(np.bincount(k >> 32, minlength=len(ranges)), ranges[:, 1] - ranges[:, 0])

@@ -14,9 +14,9 @@
 // With stride 2 the input gradient splits into the four parities of (iy, ix),
 // each a dense sum over 4, 2, 2 or 1 taps of dz.
 //
-// One persistent CTA per SM, 6 warps: warp 0 issues the TMA loads of a ring of
+// One persistent CTA per SM, 10 warps: warp 0 issues the TMA loads of a ring of
 // stages, warp 1 issues tcgen05.mma into one of two TMEM accumulators, warps
-// 2-5 read the other one back, so a tile's epilogue runs beside the next
+// 2-9 read the other one back, so a tile's epilogue runs beside the next
 // tile's MMAs.  Operand layouts: what is contiguous along K in HBM is loaded
 // K-major, what is contiguous along M or N (the weights in dgrad, both operands
 // in wgrad) MN-major, so nothing is transposed.  The K order of the forward is
@@ -40,7 +40,8 @@ namespace {
 enum ConvMode : int { kConvFwd = 0, kConvDgrad = 1, kConvWgrad = 2 };
 enum ConvEpi : int { kConvGelu = 0, kConvF32 = 1 };  // forward only
 
-constexpr int kConvThreads = 192;
+constexpr int kEpiWarps = 8;  // two per 32 TMEM lanes, each with half of the columns
+constexpr int kConvThreads = 64 + 32 * kEpiWarps;
 constexpr int kWgradPixels = 64;  // K block of the weight gradient
 // Pixels summed by one accumulation chain of the weight gradient: the tensor
 // cores' FP32 sums lose precision with the chain's length (relative error
@@ -145,7 +146,8 @@ __device__ __forceinline__ void store_outputs(float* d, __nv_bfloat16* z, __nv_b
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       z2[k] = __floats2bfloat162_rn(v[2 * k], v[2 * k + 1]);
-      y2[k] = __floats2bfloat162_rn(gelu(v[2 * k]), gelu(v[2 * k + 1]));
+      const float2 g = gelu2(make_float2(v[2 * k], v[2 * k + 1]));
+      y2[k] = __floats2bfloat162_rn(g.x, g.y);
     }
     *reinterpret_cast<uint4*>(z + at) = *reinterpret_cast<uint4*>(z2);
     *reinterpret_cast<uint4*>(y + at) = *reinterpret_cast<uint4*>(y2);
@@ -183,7 +185,7 @@ __global__ void __launch_bounds__(kConvThreads, 1)
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&acc_full[a], 1);
-      mbar_init(&acc_empty[a], 4);
+      mbar_init(&acc_empty[a], kEpiWarps);
     }
     mbar_init(drained, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -342,7 +344,7 @@ __global__ void __launch_bounds__(kConvThreads, 1)
         }
       }
 #pragma unroll 1
-      for (int c0 = 0; c0 < BN; c0 += 32) {
+      for (int c0 = (warp - 2) / 4 * 32; c0 < BN; c0 += 32 * (kEpiWarps / 4)) {
         uint32_t r[32];
         tmem_ld32(ta + (uint32_t)c0, r);
         if (MODE == kConvWgrad) {
@@ -376,9 +378,9 @@ __global__ void __launch_bounds__(kConvThreads, 1)
                     *reinterpret_cast<const uint4*>(g.zprev + base + q);
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
-                  const float2 zf = __bfloat1622float2(z2[k]);
-                  v[2 * k] *= gelu_grad(zf.x);
-                  v[2 * k + 1] *= gelu_grad(zf.y);
+                  const float2 d = gelu_grad2(__bfloat1622float2(z2[k]));
+                  v[2 * k] *= d.x;
+                  v[2 * k + 1] *= d.y;
                 }
               }
               __align__(16) __nv_bfloat162 y2[4];
@@ -484,36 +486,67 @@ __global__ void __launch_bounds__(kRgbThreads) conv3x3_rgb_kernel(const RgbArgs 
   const uint32_t tmem = tmem_slot;
   const uint32_t tiles = (g.pixels + 127) / 128;
   const unsigned short* x = reinterpret_cast<const unsigned short*>(g.x);
+  const int64_t values = (int64_t)g.B * g.H * g.W * 3;
   uint32_t phase = 0;
   bool ok = true;
   for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x) {
     const uint32_t m = t * 128 + threadIdx.x;
-    uint32_t v[kK];
+    uint32_t v[kK / 2];  // pairs of products
 #pragma unroll
-    for (int k = 0; k < kK; ++k) v[k] = 0u;
+    for (int k = 0; k < kK / 2; ++k) v[k] = 0u;
     if (m < g.pixels) {
       const uint32_t row = m / (uint32_t)g.Wo;
       const int ox = (int)(m - row * (uint32_t)g.Wo);
       const uint32_t b = row / (uint32_t)g.Ho;
       const int oy = (int)(row - b * (uint32_t)g.Ho);
       const int iy0 = oy * g.stride - 1, ix0 = ox * g.stride - 1;
+      // nine neighbouring values per image row
+      const int64_t at = (((int64_t)b * g.H + iy0) * g.W + ix0) * 3, pitch = (int64_t)g.W * 3;
+      if (iy0 >= 0 && iy0 + 2 < g.H && ix0 >= 0 && ix0 + 2 < g.W && at + 2 * pitch + 9 < values) {
+        // inside: five aligned words cover a row, whichever half it starts in
+        uint32_t a[3][5];
 #pragma unroll
-      for (int ky = 0; ky < 3; ++ky) {
-        const int iy = iy0 + ky;
-        const unsigned short* line = x + (((int64_t)b * g.H + iy) * g.W + ix0) * 3;
+        for (int ky = 0; ky < 3; ++ky) {
+          const int64_t h = at + ky * pitch;
+          const uint32_t* word = reinterpret_cast<const uint32_t*>(x) + (h >> 1);
+          const uint32_t odd = 16u * (uint32_t)(h & 1);
+          uint32_t u[6];
 #pragma unroll
-        for (int kx = 0; kx < 3; ++kx)
-          if (iy >= 0 && iy < g.H && ix0 + kx >= 0 && ix0 + kx < g.W) {
+          for (int k = 0; k < 5; ++k) u[k] = word[k];
+          u[5] = 0u;
 #pragma unroll
-            for (int c = 0; c < 3; ++c) v[(ky * 3 + kx) * 3 + c] = line[kx * 3 + c];
-          }
+          for (int k = 0; k < 5; ++k) a[ky][k] = __funnelshift_r(u[k], u[k + 1], odd);
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          v[k] = a[0][k];
+          v[5 + k] = __funnelshift_r(a[1][k], a[1][k + 1], 16);
+          v[9 + k] = a[2][k];
+        }
+        v[4] = __byte_perm(a[0][4], a[1][0], 0x5410);
+        v[13] = a[2][4] & 0xffffu;
+      } else {
+        uint32_t e[kK];
+#pragma unroll
+        for (int k = 0; k < kK; ++k) e[k] = 0u;
+#pragma unroll
+        for (int ky = 0; ky < 3; ++ky) {
+          const int iy = iy0 + ky;
+#pragma unroll
+          for (int kx = 0; kx < 3; ++kx)
+            if (iy >= 0 && iy < g.H && ix0 + kx >= 0 && ix0 + kx < g.W) {
+#pragma unroll
+              for (int c = 0; c < 3; ++c)
+                e[(ky * 3 + kx) * 3 + c] = x[at + ky * pitch + kx * 3 + c];
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < kK / 2; ++k) v[k] = pack(e[2 * k], e[2 * k + 1]);
       }
     }
 #pragma unroll
     for (int q = 0; q < 4; ++q)
-      *chunk(sA, threadIdx.x, q) =
-          make_uint4(pack(v[8 * q], v[8 * q + 1]), pack(v[8 * q + 2], v[8 * q + 3]),
-                     pack(v[8 * q + 4], v[8 * q + 5]), pack(v[8 * q + 6], v[8 * q + 7]));
+      *chunk(sA, threadIdx.x, q) = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -767,6 +800,7 @@ int ds_conv3x3_forward(const void* x, int B, int H, int W, int C, int stride, co
   if (C == 3) {
     if (!conv_ok(B, H, W, 32, N, stride, 288) || Kp < 27) return DS_ERR_ARG;
     if (!aligned16(z) || !aligned16(y) || !aligned16(d)) return DS_ERR_ARG;
+    if ((uintptr_t)x & 3) return DS_ERR_ARG;
     RgbArgs g{};
     g.x = (const __nv_bfloat16*)x, g.w = (const __nv_bfloat16*)w;
     g.B = B, g.H = H, g.W = W, g.N = N, g.stride = stride, g.kp = Kp;

@@ -131,11 +131,29 @@ __device__ __forceinline__ float gelu(float x) {
   return 0.5f * x * (1.f + tanhf(u));
 }
 
+// gelu of two values with packed instructions, in gelu's rounding.
+__device__ __forceinline__ float2 gelu2(float2 x) {
+  const float2 cube = mul2(mul2(both(0.044715f), x), x);
+  const float2 u = mul2(both(0.7978845608f), fma2(cube, x, x));
+  const float2 t = make_float2(tanhf(u.x), tanhf(u.y));
+  return mul2(mul2(both(0.5f), x), add2(both(1.f), t));
+}
+
 __device__ __forceinline__ float gelu_grad(float x) {
   const float u = 0.7978845608f * (x + 0.044715f * x * x * x);
   const float t = tanhf(u);
   const float du = 0.7978845608f * (1.f + 3.f * 0.044715f * x * x);
   return 0.5f * (1.f + t) + 0.5f * x * (1.f - t * t) * du;
+}
+
+// gelu_grad of two values with packed instructions.
+__device__ __forceinline__ float2 gelu_grad2(float2 x) {
+  const float2 cube = mul2(mul2(both(0.044715f), x), x);
+  const float2 u = mul2(both(0.7978845608f), fma2(cube, x, x));
+  const float2 t = make_float2(tanhf(u.x), tanhf(u.y));
+  const float2 du = mul2(both(0.7978845608f), fma2(mul2(both(3.f * 0.044715f), x), x, both(1.f)));
+  const float2 slope = mul2(mul2(both(0.5f), x), fma2(mul2(t, both(-1.f)), t, both(1.f)));
+  return fma2(slope, du, mul2(both(0.5f), add2(both(1.f), t)));
 }
 
 using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,

@@ -78,9 +78,10 @@ struct ConvMaps {
   CUtensorMap x[9];  // the taps of x (forward, wgrad)
   CUtensorMap w;     // the weights (forward, dgrad)
   CUtensorMap dz;    // the output gradient (dgrad, wgrad)
+  CUtensorMap z, y;  // the outputs (forward with GELU)
 };
 
-template <int BN, int MODE, int G>
+template <int BN, int MODE, int G, int EPI>
 struct ConvShape {
   // forward: K block of G channels; dgrad: 64 output channels; wgrad: 64 pixels
   static constexpr int kBK = MODE == kConvFwd ? G : 64;
@@ -88,8 +89,17 @@ struct ConvShape {
   static constexpr uint32_t kBytesA = 128 * kBK * 2;
   static constexpr uint32_t kBytesB = kNB * kBK * 2;
   static constexpr uint32_t kStage = kBytesA + kBytesB;
-  static constexpr int kStages = 196608 / kStage < 8 ? 196608 / kStage : 8;
-  static constexpr size_t kSmem = 1024 + (size_t)kStages * kStage + 256;
+  // The forward's z and gelu(z) leave as TMA tiles of kSlab columns: stored by the lanes
+  // (a row each, 16 bytes at a time) every sector was written in two halves (64 -> 128
+  // channels, stride 2, 8 x 256 x 256: forward 0.047 -> 0.035 ms, B200).
+  static constexpr bool kStaged = MODE == kConvFwd && EPI == kConvGelu;
+  static constexpr int kSlab = BN < 64 ? 32 : 64;
+  static constexpr uint32_t kTile = 128 * kSlab * 2;
+  static constexpr int kBufs = BN == 256 ? 1 : 2;  // pairs of such tiles (256: four stages first)
+  static constexpr uint32_t kStaging = kStaged ? kBufs * 2 * kTile : 0;
+  static constexpr int kRoom = kStaged ? 230400 - (int)kStaging : 196608;
+  static constexpr int kStages = kRoom / (int)kStage < 8 ? kRoom / (int)kStage : 8;
+  static constexpr size_t kSmem = 1024 + (size_t)kStages * kStage + kStaging + 256;
   static constexpr uint32_t kCols = 2 * BN;  // two accumulators (32 .. 512 columns)
 };
 
@@ -159,14 +169,34 @@ __device__ __forceinline__ void store_outputs(float* d, __nv_bfloat16* z, __nv_b
 __device__ __forceinline__ int class_py(int cls) { return cls < 2 ? 1 : 0; }
 __device__ __forceinline__ int class_px(int cls) { return (cls & 1) ^ 1; }
 
+// Barrier of the epilogue's warps, and the same with a vote.
+__device__ __forceinline__ void epi_sync() {
+  __syncwarp();
+  asm volatile("barrier.cta.sync.aligned 1, %0;" ::"n"(32 * kEpiWarps) : "memory");
+}
+__device__ __forceinline__ bool epi_all(bool mine) {
+  __syncwarp();
+  uint32_t all;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 p, %1, 0;\n\t"
+      "barrier.cta.red.and.aligned.pred q, 1, %2, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(all)
+      : "r"(mine ? 1u : 0u), "n"(32 * kEpiWarps)
+      : "memory");
+  return all != 0u;
+}
+
 template <int BN, int MODE, int G, int EPI>
 __global__ void __launch_bounds__(kConvThreads, 1)
     conv3x3_kernel(const __grid_constant__ ConvMaps maps, const __grid_constant__ ConvArgs g) {
-  using S = ConvShape<BN, MODE, G>;
+  using S = ConvShape<BN, MODE, G, EPI>;
   constexpr int kStages = S::kStages;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  uint64_t* full = (uint64_t*)(smem + (size_t)kStages * S::kStage);
+  uint8_t* staging = smem + (size_t)kStages * S::kStage;
+  uint64_t* full = (uint64_t*)(staging + S::kStaging);
   uint64_t* empty = full + kStages;
   uint64_t* acc_full = empty + kStages;
   uint64_t* acc_empty = acc_full + 2;
@@ -313,12 +343,13 @@ __global__ void __launch_bounds__(kConvThreads, 1)
   } else if (warp >= 2) {
     const int quad = warp & 3;  // the TMEM lanes this warp may read: 32 quad ..
     const int row = quad * 32 + lane;
-    int li = 0;
+    int li = 0, slabs = 0;
     for (int it = blockIdx.x; it < items; it += gridDim.x, ++li) {
       const Item t = item_of<MODE>(g, it, BN);
       const int acc = li & 1;
-      if (!__all_sync(0xffffffffu,
-                      mbar_wait(&acc_full[acc], (uint32_t)(li >> 1) & 1u, g.spin))) {
+      const bool got = mbar_wait(&acc_full[acc], (uint32_t)(li >> 1) & 1u, g.spin);
+      // staged: the epilogue's warps meet at barriers, so they leave together
+      if (S::kStaged ? !epi_all(got) : !__all_sync(0xffffffffu, got)) {
         atomicExch(&failed, 1);
         break;
       }
@@ -343,50 +374,91 @@ __global__ void __launch_bounds__(kConvThreads, 1)
           pix = ((size_t)b * g.H + y) * g.W + x;
         }
       }
+      if (S::kStaged) {
+        const int half = (warp - 2) / 4;  // of the slab's columns
 #pragma unroll 1
-      for (int c0 = (warp - 2) / 4 * 32; c0 < BN; c0 += 32 * (kEpiWarps / 4)) {
-        uint32_t r[32];
-        tmem_ld32(ta + (uint32_t)c0, r);
-        if (MODE == kConvWgrad) {
-          // rows are columns of gw: the lanes write 128 contiguous bytes
-          const int j = t.x0 + row;
-          float* dst = g.d + ((size_t)t.split * g.N + t.n0 + c0) * g.kp + j;
-          if (j < g.kp) {
+        for (int n = 0; n < BN && t.n0 + n < g.N; n += S::kSlab, ++slabs) {
+          uint8_t* tz = staging + (size_t)(slabs % S::kBufs) * 2 * S::kTile;
+          uint8_t* ty = tz + S::kTile;
+          if (warp == 2 && lane == 0) bulk_wait_read<S::kBufs - 1>();
+          epi_sync();
+          if (half * 32 < S::kSlab) {
+            uint32_t r[32];
+            tmem_ld32(ta + (uint32_t)(n + 32 * half), r);
 #pragma unroll
-            for (int q = 0; q < 32; ++q)
-              if (t.n0 + c0 + q < g.N) dst[(size_t)q * g.kp] = __uint_as_float(r[q]);
-          }
-        } else if (valid) {
-          const int width = MODE == kConvFwd ? g.N : g.C;  // a multiple of 8
-          const size_t base = pix * width + t.n0 + c0;
+            for (int q = 0; q < 4; ++q) {
+              float v[8];
+              const int c = t.n0 + n + 32 * half + 8 * q;  // N is a multiple of 8
 #pragma unroll
-          for (int q = 0; q < 32; q += 8) {
-            if (t.n0 + c0 + q >= width) break;
-            float v[8];
-#pragma unroll
-            for (int k = 0; k < 8; ++k) v[k] = __uint_as_float(r[q + k]);
-            if (MODE == kConvFwd) {
-              const float4* bias = reinterpret_cast<const float4*>(g.bias + t.n0 + c0 + q);
-              const float4 b0 = bias[0], b1 = bias[1];
-              v[0] += b0.x, v[1] += b0.y, v[2] += b0.z, v[3] += b0.w;
-              v[4] += b1.x, v[5] += b1.y, v[6] += b1.z, v[7] += b1.w;
-              store_outputs<EPI>(g.d, g.z, g.y, base + q, v);
-            } else {
-              if (g.zprev) {
-                __align__(16) __nv_bfloat162 z2[4];
-                *reinterpret_cast<uint4*>(z2) =
-                    *reinterpret_cast<const uint4*>(g.zprev + base + q);
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                  const float2 d = gelu_grad2(__bfloat1622float2(z2[k]));
-                  v[2 * k] *= d.x;
-                  v[2 * k + 1] *= d.y;
-                }
+              for (int k = 0; k < 8; ++k) v[k] = __uint_as_float(r[8 * q + k]);
+              if (c < g.N) {
+                const float4* bias = reinterpret_cast<const float4*>(g.bias + c);
+                const float4 b0 = bias[0], b1 = bias[1];
+                v[0] += b0.x, v[1] += b0.y, v[2] += b0.z, v[3] += b0.w;
+                v[4] += b1.x, v[5] += b1.y, v[6] += b1.z, v[7] += b1.w;
               }
-              __align__(16) __nv_bfloat162 y2[4];
+              // the tensor maps' swizzle: 128-byte rows, or 64-byte ones
+              const int chunk = half * 4 + q;
+              const int at = S::kSlab == 64 ? row * 128 + ((chunk ^ (row & 7)) << 4)
+                                            : row * 64 + ((chunk ^ ((row >> 1) & 3)) << 4);
+              store_outputs<kConvGelu>(nullptr, reinterpret_cast<__nv_bfloat16*>(tz),
+                                       reinterpret_cast<__nv_bfloat16*>(ty), (size_t)(at / 2), v);
+            }
+          }
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          epi_sync();
+          if (warp == 2 && lane == 0) {
+            tma_store_4d(&maps.z, tz, t.n0 + n, t.x0, t.y0, t.b0);
+            tma_store_4d(&maps.y, ty, t.n0 + n, t.x0, t.y0, t.b0);
+            bulk_commit();
+          }
+        }
+      } else {
+#pragma unroll 1
+        for (int c0 = (warp - 2) / 4 * 32; c0 < BN; c0 += 32 * (kEpiWarps / 4)) {
+          uint32_t r[32];
+          tmem_ld32(ta + (uint32_t)c0, r);
+          if (MODE == kConvWgrad) {
+            // rows are columns of gw: the lanes write 128 contiguous bytes
+            const int j = t.x0 + row;
+            float* dst = g.d + ((size_t)t.split * g.N + t.n0 + c0) * g.kp + j;
+            if (j < g.kp) {
 #pragma unroll
-              for (int k = 0; k < 4; ++k) y2[k] = __floats2bfloat162_rn(v[2 * k], v[2 * k + 1]);
-              *reinterpret_cast<uint4*>(g.y + base + q) = *reinterpret_cast<uint4*>(y2);
+              for (int q = 0; q < 32; ++q)
+                if (t.n0 + c0 + q < g.N) dst[(size_t)q * g.kp] = __uint_as_float(r[q]);
+            }
+          } else if (valid) {
+            const int width = MODE == kConvFwd ? g.N : g.C;  // a multiple of 8
+            const size_t base = pix * width + t.n0 + c0;
+#pragma unroll
+            for (int q = 0; q < 32; q += 8) {
+              if (t.n0 + c0 + q >= width) break;
+              float v[8];
+#pragma unroll
+              for (int k = 0; k < 8; ++k) v[k] = __uint_as_float(r[q + k]);
+              if (MODE == kConvFwd) {
+                const float4* bias = reinterpret_cast<const float4*>(g.bias + t.n0 + c0 + q);
+                const float4 b0 = bias[0], b1 = bias[1];
+                v[0] += b0.x, v[1] += b0.y, v[2] += b0.z, v[3] += b0.w;
+                v[4] += b1.x, v[5] += b1.y, v[6] += b1.z, v[7] += b1.w;
+                store_outputs<EPI>(g.d, g.z, g.y, base + q, v);
+              } else {
+                if (g.zprev) {
+                  __align__(16) __nv_bfloat162 z2[4];
+                  *reinterpret_cast<uint4*>(z2) =
+                      *reinterpret_cast<const uint4*>(g.zprev + base + q);
+#pragma unroll
+                  for (int k = 0; k < 4; ++k) {
+                    const float2 d = gelu_grad2(__bfloat1622float2(z2[k]));
+                    v[2 * k] *= d.x;
+                    v[2 * k + 1] *= d.y;
+                  }
+                }
+                __align__(16) __nv_bfloat162 y2[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) y2[k] = __floats2bfloat162_rn(v[2 * k], v[2 * k + 1]);
+                *reinterpret_cast<uint4*>(g.y + base + q) = *reinterpret_cast<uint4*>(y2);
+              }
             }
           }
         }
@@ -397,6 +469,7 @@ __global__ void __launch_bounds__(kConvThreads, 1)
         asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[acc]))
                      : "memory");
     }
+    if (S::kStaged && warp == 2 && lane == 0) bulk_wait_all();
   }
   __syncwarp();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -426,9 +499,11 @@ __global__ void __launch_bounds__(kConvThreads, 1)
 // 128 x BN tile, and the same threads write z and gelu(z).  Bound by the output
 // (2 x 2 BN bytes a pixel): an im2col matrix of 64 columns would move 128 bytes
 // a pixel twice more.  Many small CTAs per SM (8 of 128 threads at BN = 32)
-// overlap one another's gather, MMA and epilogue, so no warp is specialised.
-// The initializer's forward on 16 images of 512 x 512 went from 2.92 ms with
-// im2col + GEMM in this layer to 0.81 ms (B200).
+// overlap one another's gather, MMA and epilogue, so no warp is specialised.  A row of
+// nine values is loaded as five aligned words, and the tiles of z and gelu(z) are
+// stored by TMA.  On 16 images of 512 x 512 (B200): 2.3 ms as im2col + GEMM, 0.231 with
+// two-byte loads and 16-byte stores a lane, 0.216 with word loads, 0.111 with TMA
+// stores; the 0.56 GB alone take 0.086.
 constexpr int kRgbThreads = 128;
 
 struct RgbArgs {
@@ -442,11 +517,18 @@ struct RgbArgs {
   uint32_t spin;
 };
 
+struct RgbMaps {
+  CUtensorMap z, y;  // [pixels][N], boxes of 128 x BN
+};
+
 template <int BN, int EPI>
-__global__ void __launch_bounds__(kRgbThreads) conv3x3_rgb_kernel(const RgbArgs g) {
+__global__ void __launch_bounds__(kRgbThreads)
+    conv3x3_rgb_kernel(const RgbArgs g, const __grid_constant__ RgbMaps maps) {
   constexpr int kK = 32;  // 27 products and five zeros
   __shared__ __align__(1024) uint8_t sA[128 * kK * 2];
   __shared__ __align__(1024) uint8_t sB[BN * kK * 2];
+  constexpr bool kStaged = EPI == kConvGelu;
+  __shared__ __align__(1024) uint8_t sOut[kStaged ? 2 : 1][kStaged ? 128 * BN * 2 : 16];
   __shared__ uint64_t done;
   __shared__ uint32_t tmem_slot;
   __shared__ __align__(16) float sBias[BN];
@@ -562,6 +644,7 @@ __global__ void __launch_bounds__(kRgbThreads) conv3x3_rgb_kernel(const RgbArgs 
     // Every thread polls to the same limit; a timeout is voted on, so that the
     // whole CTA leaves together.
     ok = mbar_wait(&done, phase, g.spin);
+    if (kStaged && threadIdx.x == 0) bulk_wait_read<0>();
     ok = __syncthreads_and(ok);
     if (!ok) break;
     phase ^= 1u;
@@ -570,7 +653,20 @@ __global__ void __launch_bounds__(kRgbThreads) conv3x3_rgb_kernel(const RgbArgs 
     for (int c0 = 0; c0 < BN; c0 += 32) {
       uint32_t r[32];
       tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, r);
-      if (m < g.pixels) {
+      if (kStaged) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          float f[8];
+#pragma unroll
+          for (int k = 0; k < 8; ++k) f[k] = __uint_as_float(r[8 * q + k]) + sBias[c0 + 8 * q + k];
+          const int row = threadIdx.x, chunk = c0 / 8 + q;
+          const int at = BN == 64 ? row * 128 + ((chunk ^ (row & 7)) << 4)
+                                  : row * 64 + ((chunk ^ ((row >> 1) & 3)) << 4);
+          store_outputs<kConvGelu>(nullptr, reinterpret_cast<__nv_bfloat16*>(sOut[0]),
+                                   reinterpret_cast<__nv_bfloat16*>(sOut[kStaged ? 1 : 0]),
+                                   (size_t)(at / 2), f);
+        }
+      } else if (m < g.pixels) {
         const size_t base = (size_t)m * g.N + n0 + c0;
 #pragma unroll
         for (int q = 0; q < 32; q += 8) {
@@ -584,8 +680,15 @@ __global__ void __launch_bounds__(kRgbThreads) conv3x3_rgb_kernel(const RgbArgs 
     }
     // the accumulator and the A tile are free again once every thread has read
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    if (kStaged) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
+    if (kStaged && threadIdx.x == 0) {
+      tma_store_2d(&maps.z, sOut[0], n0, (int)(t * 128));
+      tma_store_2d(&maps.y, sOut[kStaged ? 1 : 0], n0, (int)(t * 128));
+      bulk_commit();
+    }
   }
+  if (kStaged && threadIdx.x == 0) bulk_wait_all();
   if (!ok && threadIdx.x == 0) {
     mbar_wait(&done, phase, kSpinLimit);  // the MMAs land before TMEM is freed
     atomicOr(g.err, 1u);
@@ -700,7 +803,7 @@ int sm_count() {
 
 template <int BN, int MODE, int G, int EPI>
 int launch_conv(const ConvMaps& maps, const ConvArgs& g, cudaStream_t s) {
-  using S = ConvShape<BN, MODE, G>;
+  using S = ConvShape<BN, MODE, G, EPI>;
   static std::once_flag once;
   static cudaError_t attr = cudaSuccess;
   std::call_once(once, [] {
@@ -745,11 +848,17 @@ bool conv_ok(int B, int H, int W, int C, int N, int stride, int kp) {
 
 template <int BN, int EPI>
 int launch_rgb(const RgbArgs& g, cudaStream_t s) {
-  // TMEM holds 512 / BN accumulators per SM; 8 CTAs are what the registers allow
-  const int per_sm = std::min(8, 512 / BN);
+  // TMEM holds 512 / BN accumulators per SM; 8 CTAs (4 of 64 columns, with their tiles in
+  // shared memory) are what the SM holds
+  const int per_sm = BN == 32 ? 8 : EPI == kConvGelu ? 4 : 8;
+  RgbMaps maps{};
+  if (EPI == kConvGelu) {
+    DS_TRY(map_matrix(&maps.z, g.z, (int)g.pixels, g.N, g.N, BN, 128));
+    DS_TRY(map_matrix(&maps.y, g.y, (int)g.pixels, g.N, g.N, BN, 128));
+  }
   const int tiles = (int)((g.pixels + 127) / 128), ny = (g.N + BN - 1) / BN;
   const dim3 grid(std::max(1, std::min(tiles, sm_count() * per_sm / ny)), ny);
-  conv3x3_rgb_kernel<BN, EPI><<<grid, kRgbThreads, 0, s>>>(g);
+  conv3x3_rgb_kernel<BN, EPI><<<grid, kRgbThreads, 0, s>>>(g, maps);
   return cuda_status(cudaGetLastError());
 }
 
@@ -834,7 +943,11 @@ int ds_conv3x3_forward(const void* x, int B, int H, int W, int C, int stride, co
   ConvMaps maps;
   DS_TRY(map_taps(maps, g, (const __nv_bfloat16*)x, G, g.pt[0]));
   DS_TRY(map_matrix(&maps.w, w, N, Kp, Kp, G, bn));
-  maps.dz = maps.w;  // not read
+  maps.dz = maps.z = maps.y = maps.w;  // not read
+  if (!d)
+    for (int k = 0; k < 2; ++k)
+      DS_TRY(map_pixels(k ? &maps.y : &maps.z, k ? g.y : g.z, N, g.Wo, g.Ho, B, N, (int64_t)g.Wo * N,
+                        (int64_t)g.Ho * g.Wo * N, bn < 64 ? 32 : 64, g.pt[0]));
   cudaStream_t s = (cudaStream_t)stream;
   if (G == 32)
     return d ? dispatch_bn<kConvFwd, 32, kConvF32>(bn, maps, g, s)
@@ -877,6 +990,7 @@ int ds_conv3x3_dgrad(const void* dz, int B, int H, int W, int C, int stride, con
                     (int64_t)g.Ho * g.Wo * N, 64, p));
   DS_TRY(map_matrix(&maps.w, w, N, Kp, Kp, 64, 64));
   for (int t = 0; t < 9; ++t) maps.x[t] = maps.dz;  // not read
+  maps.z = maps.y = maps.dz;
   return dispatch_bn<kConvDgrad, 64, 0>(bn, maps, g, (cudaStream_t)stream);
 }
 
@@ -909,7 +1023,7 @@ int ds_conv3x3_wgrad(const void* x, const void* dz, int B, int H, int W, int C, 
   DS_TRY(map_taps(maps, g, (const __nv_bfloat16*)x, G, g.pt[0]));
   DS_TRY(map_pixels(&maps.dz, (const __nv_bfloat16*)dz, N, g.Wo, g.Ho, B, N, (int64_t)g.Wo * N,
                     (int64_t)g.Ho * g.Wo * N, 64, g.pt[0]));
-  maps.w = maps.dz;  // not read
+  maps.w = maps.z = maps.y = maps.dz;  // not read
   cudaStream_t s = (cudaStream_t)stream;
   if (G == 32) DS_TRY((dispatch_bn<kConvWgrad, 32, 0>(bn, maps, g, s)));
   else DS_TRY((dispatch_bn<kConvWgrad, 64, 0>(bn, maps, g, s)));

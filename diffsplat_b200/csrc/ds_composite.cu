@@ -618,8 +618,8 @@ __device__ __forceinline__ void reduce_hits(BwdShared<TS>& sm, int w, int lane, 
 //
 // The pixel loop was next: of some 70 issue slots a hit, half went to tests and
 // selects on the ALU pipe, which issues at half rate.  Splats that cannot reach alpha
-// 0.99, whose conic is not nearly singular and behind which every pixel's list has
-// begun ("plain", nearly all) need one test of alpha and no select.  With the moments
+// 0.99 and whose conic is not nearly singular ("plain", nearly all) need a test of alpha
+// and one of the pixel's last contributor, and no other select.  With the moments
 // of reduce_hits: step 4 of the 1280x720 fit 0.258 -> 0.214 ms, the million splats
 // 0.525 -> 0.511 (there the warps of a tile wait for one another at every batch).
 template <int TS, bool kFusedLoss, bool kExact, bool kBatch>
@@ -661,17 +661,9 @@ __global__ void __launch_bounds__(Lay<TS>::kThreads, Lay<TS>::kMinBlocksBwd)
   if (lane == 0) sm.box[w] = make_float4(m.wx_lo, m.wx_hi, m.wy_lo, m.wy_hi);
   // acc: over the splats behind (already visited), weight x (colour . dL/dpixel)
   float2 T, gr, gg, gb, acc = both(0.f);
-  // NaN outside the image: no splat reaches it there
-  const float nan = __int_as_float(0x7fffffff);
-  const float2 npx = both(-m.px);
-  const float2 npy = make_float2(m.inside[0] ? -m.py[0] : nan, m.inside[1] ? -m.py[1] : nan);
+  const float2 npx = both(-m.px), npy = make_float2(-m.py[0], -m.py[1]);
   int32_t fin[2];
   int32_t my_final = -1;
-  // The splats from which on no pixel's last contributor needs a look: behind the
-  // last contributor of a pixel that did not end opaque nothing passes the alpha
-  // test (the forward's arithmetic), so only opaque ones count.  1% above kTThres for
-  // the rounding of 1 - alpha.
-  int32_t first_plain = 0x7fffffff;
   bool finite = true;
 #pragma unroll
   for (int k = 0; k < 2; ++k) {
@@ -679,7 +671,6 @@ __global__ void __launch_bounds__(Lay<TS>::kThreads, Lay<TS>::kMinBlocksBwd)
     const float t = 1.f - alphas[pix];
     fin[k] = m.inside[k] ? last_ids[pix] : -1;
     my_final = max(my_final, fin[k]);
-    if (m.inside[k] && !(t > 1.01f * kTThres)) first_plain = min(first_plain, fin[k]);
     float r = 0.f, g = 0.f, b = 0.f;
     if (m.inside[k]) {
       if (kFusedLoss) {
@@ -703,7 +694,6 @@ __global__ void __launch_bounds__(Lay<TS>::kThreads, Lay<TS>::kMinBlocksBwd)
   reinterpret_cast<float2*>(sm.gg[w])[pixel_slot(lane) / 2] = gg;
   reinterpret_cast<float2*>(sm.gb[w])[pixel_slot(lane) / 2] = gb;
   const bool safe_pixels = __all_sync(0xffffffffu, finite);
-  first_plain = safe_pixels ? __reduce_min_sync(0xffffffffu, first_plain) : -1;
   {
     const float y1 = __shfl_sync(0xffffffffu, m.py[0], 8);
     const float y5 = __shfl_sync(0xffffffffu, m.py[1], 8);
@@ -839,23 +829,23 @@ __global__ void __launch_bounds__(Lay<TS>::kThreads, Lay<TS>::kMinBlocksBwd)
       const float2 nia = kExact ? make_float2(-1.f / T.x, -1.f / T.y) : both(-1.f);
       return fma2(acc, nia, lit);
     };
-    // from this slot on every pixel's list has begun
-    const int t_plain = max(0, batch_end - first_plain);
     // The hits two at a time: conic, exp and alpha of both first (independent of
     // T), then the recurrence back to front.
     for (int i = 0; i < hits; i += 2) {
       const int2 pair = sm.list[w][i >> 1];
       float2 oe[2], al[2];
       bool any[2];
-      if (pair.x >= t_plain && pair.y >= 0) {
+      if (safe_pixels && (pair.x | pair.y) >= 0) {
         // Plain splats: alpha = opacity exp() where it passes, 0 elsewhere, which
         // leaves T and acc as they are.
 #pragma unroll
         for (int g = 0; g < 2; ++g) {
-          const SplatRec& r = sm.splat[g ? pair.y : pair.x];
+          const int t = g ? pair.y : pair.x, id = batch_end - t;
+          const SplatRec& r = sm.splat[t];
           const float2 dx = add2(r.x(), npx);
           oe[g] = pair_opacity(pair_dist2(dx, mul2(dx, dx), add2(r.y(), npy), r), r);
-          const bool o0 = oe[g].x >= kAlphaThres, o1 = oe[g].y >= kAlphaThres;
+          const bool o0 = oe[g].x >= kAlphaThres && id <= fin[0];
+          const bool o1 = oe[g].y >= kAlphaThres && id <= fin[1];
           al[g] = make_float2(o0 ? oe[g].x : 0.f, o1 ? oe[g].y : 0.f);
           any[g] = o0 || o1;
         }

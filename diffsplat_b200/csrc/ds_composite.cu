@@ -756,8 +756,10 @@ __global__ void __launch_bounds__(Lay<TS>::kThreads, Lay<TS>::kMinBlocksBwd)
   for (int bi = 0; bi < nb; ++bi) {
     const int batch_end = end - 1 - B * bi;  // farthest splat of the batch
     const int bs = min(B, batch_end + 1 - start);
-    __syncthreads();
-    // stage the batch back to front: slot l holds sorted index batch_end - l
+    // Stage the batch back to front: slot l holds sorted index batch_end - l.  Every warp
+    // is past the previous batch's hits; its sums may still be read, but they lie
+    // elsewhere, and a slot's record index is this warp's own.
+    __syncwarp();
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       const int slot = threadIdx.x + r * NT, l = slot / kSplit, h = slot % kSplit;

@@ -37,7 +37,13 @@
 namespace ds {
 namespace {
 
-enum ConvMode : int { kConvFwd = 0, kConvDgrad = 1, kConvWgrad = 2 };
+// kConvPair: forward of 32 channels at stride 2.  TMA moves a row of a box in 2.4 (128
+// bytes) to 3.6 cycles (64 bytes), and a tile took 128 rows of A and 64 of weights for
+// each tap.  Two neighbouring pixels are one row of 64 channels here: the taps kx = 1
+// and 2 of an output pixel are the pair it starts at, kx = 0 the second half of the
+// pair before, so six boxes serve nine taps, and the weights stay in shared memory.
+// 16 x 512 x 512 x 32 -> 64 channels (B200): 0.190 -> 0.128 ms.
+enum ConvMode : int { kConvFwd = 0, kConvDgrad = 1, kConvWgrad = 2, kConvPair = 3 };
 enum ConvEpi : int { kConvGelu = 0, kConvF32 = 1 };  // forward only
 
 constexpr int kEpiWarps = 8;  // two per 32 TMEM lanes, each with half of the columns
@@ -83,23 +89,24 @@ struct ConvMaps {
 
 template <int BN, int MODE, int G, int EPI>
 struct ConvShape {
-  // forward: K block of G channels; dgrad: 64 output channels; wgrad: 64 pixels
+  // forward: K block of G channels (pairs: 64); dgrad: 64 output channels; wgrad: 64 pixels
   static constexpr int kBK = MODE == kConvFwd ? G : 64;
-  static constexpr int kNB = MODE == kConvFwd ? BN : (BN < 64 ? 64 : BN);  // columns staged of B
+  static constexpr int kNB = MODE == kConvFwd || MODE == kConvPair ? BN : (BN < 64 ? 64 : BN);  // columns staged of B
   static constexpr uint32_t kBytesA = 128 * kBK * 2;
-  static constexpr uint32_t kBytesB = kNB * kBK * 2;
+  static constexpr uint32_t kBytesB = MODE == kConvPair ? 0 : kNB * kBK * 2;
+  static constexpr uint32_t kWeights = MODE == kConvPair ? 9 * BN * 64 : 0;  // resident
   static constexpr uint32_t kStage = kBytesA + kBytesB;
   // The forward's z and gelu(z) leave as TMA tiles of kSlab columns: stored by the lanes
   // (a row each, 16 bytes at a time) every sector was written in two halves (64 -> 128
   // channels, stride 2, 8 x 256 x 256: forward 0.047 -> 0.035 ms, B200).
-  static constexpr bool kStaged = MODE == kConvFwd && EPI == kConvGelu;
+  static constexpr bool kStaged = (MODE == kConvFwd && EPI == kConvGelu) || MODE == kConvPair;
   static constexpr int kSlab = BN < 64 ? 32 : 64;
   static constexpr uint32_t kTile = 128 * kSlab * 2;
   static constexpr int kBufs = BN == 256 ? 1 : 2;  // pairs of such tiles (256: four stages first)
   static constexpr uint32_t kStaging = kStaged ? kBufs * 2 * kTile : 0;
-  static constexpr int kRoom = kStaged ? 230400 - (int)kStaging : 196608;
+  static constexpr int kRoom = kStaged ? 230400 - (int)(kStaging + kWeights) : 196608;
   static constexpr int kStages = kRoom / (int)kStage < 8 ? kRoom / (int)kStage : 8;
-  static constexpr size_t kSmem = 1024 + (size_t)kStages * kStage + kStaging + 256;
+  static constexpr size_t kSmem = 1024 + (size_t)kStages * kStage + kStaging + kWeights + 256;
   static constexpr uint32_t kCols = 2 * BN;  // two accumulators (32 .. 512 columns)
 };
 
@@ -196,12 +203,14 @@ __global__ void __launch_bounds__(kConvThreads, 1)
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* staging = smem + (size_t)kStages * S::kStage;
-  uint64_t* full = (uint64_t*)(staging + S::kStaging);
+  uint8_t* weights = staging + S::kStaging;
+  uint64_t* full = (uint64_t*)(weights + S::kWeights);
   uint64_t* empty = full + kStages;
   uint64_t* acc_full = empty + kStages;
   uint64_t* acc_empty = acc_full + 2;
   uint64_t* drained = acc_empty + 2;
-  uint32_t* tmem_slot = (uint32_t*)(drained + 1);
+  uint64_t* wfull = drained + 1;
+  uint32_t* tmem_slot = (uint32_t*)(wfull + 1);
   __shared__ int failed;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -218,6 +227,7 @@ __global__ void __launch_bounds__(kConvThreads, 1)
       mbar_init(&acc_empty[a], kEpiWarps);
     }
     mbar_init(drained, 1);
+    mbar_init(wfull, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) {
@@ -234,6 +244,7 @@ __global__ void __launch_bounds__(kConvThreads, 1)
   // K blocks of a work item
   auto blocks_of = [&](const Item& t) {
     if (MODE == kConvFwd) return 9 * (g.C / G);
+    if (MODE == kConvPair) return 6;
     if (MODE == kConvWgrad) return t.kb1 - t.kb0;
     const int nb = (g.N + 63) / 64;
     if (g.stride == 1) return 9 * nb;
@@ -243,6 +254,11 @@ __global__ void __launch_bounds__(kConvThreads, 1)
   int issued = 0;
   if (warp == 0 && lane == 0) {
     bool ok = true;
+    if (MODE == kConvPair) {
+      mbar_expect_tx(wfull, S::kWeights);
+      for (int tap = 0; tap < 9; ++tap)
+        tma_load_2d(weights + tap * BN * 64, &maps.w, wfull, tap * 32, 0);
+    }
     for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
       const Item t = item_of<MODE>(g, it, BN);
       const int nkb = blocks_of(t);
@@ -261,6 +277,10 @@ __global__ void __launch_bounds__(kConvThreads, 1)
           tma_load_4d(a, &maps.x[tap], &full[s], c, t.x0 + g.off_x[tap], t.y0 + g.off_y[tap],
                       t.b0);
           tma_load_2d(b, &maps.w, &full[s], tap * g.C + c, t.n0);
+        } else if (MODE == kConvPair) {
+          // even blocks: the pairs before, odd ones: the pairs themselves
+          const int ky = i >> 1;
+          tma_load_4d(a, &maps.x[ky], &full[s], 0, t.x0 - 1 + (i & 1), t.y0 + g.off_y[ky], t.b0);
         } else if (MODE == kConvDgrad) {
           const int nb = (g.N + 63) / 64, k = i / nb, n = (i - k * nb) * 64;
           int ky, kx, oy, ox;
@@ -301,8 +321,12 @@ __global__ void __launch_bounds__(kConvThreads, 1)
     }
   } else if (warp == 1 && lane == 0) {
     constexpr uint32_t idesc =
-        instr_desc_bf16(128, BN, MODE == kConvWgrad, MODE != kConvFwd);
+        instr_desc_bf16(128, BN, MODE == kConvWgrad, MODE != kConvFwd && MODE != kConvPair);
     bool ok = true;
+    if (MODE == kConvPair && !mbar_wait(wfull, 0, g.spin)) {
+      atomicExch(&failed, 1);
+      ok = false;
+    }
     int n = 0, li = 0;
     for (int it = blockIdx.x; it < items && ok; it += gridDim.x, ++li) {
       const Item t = item_of<MODE>(g, it, BN);
@@ -323,6 +347,7 @@ __global__ void __launch_bounds__(kConvThreads, 1)
         const uint32_t a = smem_u32(smem + (size_t)s * S::kStage), b = a + S::kBytesA;
 #pragma unroll
         for (int kk = 0; kk < S::kBK / 16; ++kk) {
+          if (MODE == kConvPair && !(i & 1) && kk < 2) continue;  // the second pixel only
           // K-major rows of G (64) channels: 16 channels further are 32 bytes.
           // MN-major: 8-row groups of 128 (64) bytes, 16 rows further two groups,
           // the next 64 (32) columns a whole K block further.
@@ -331,9 +356,15 @@ __global__ void __launch_bounds__(kConvThreads, 1)
                   ? smem_desc(a + kk * G * 32, G * 128, G * 16, G == 64 ? 2u : 4u)
                   : smem_desc(a + kk * 32, 16, S::kBK * 16, S::kBK == 64 ? 2u : 4u);
           const uint64_t db =
-              MODE == kConvFwd ? smem_desc(b + kk * 32, 16, G * 16, G == 64 ? 2u : 4u)
+              MODE == kConvPair
+                  ? smem_desc(smem_u32(weights) +
+                                  ((i >> 1) * 3 + (i & 1 ? 1 + (kk >> 1) : 0)) * BN * 64 +
+                                  (kk & 1) * 32,
+                              16, 512, 4u)
+              : MODE == kConvFwd ? smem_desc(b + kk * 32, 16, G * 16, G == 64 ? 2u : 4u)
                                : smem_desc(b + kk * 2048, 8192, 1024, 2u);
-          umma_bf16(tmem + (uint32_t)(acc * BN), da, db, idesc, (i > 0 || kk > 0) ? 1u : 0u);
+          umma_bf16(tmem + (uint32_t)(acc * BN), da, db, idesc,
+                    (i > 0 || kk > (MODE == kConvPair ? 2 : 0)) ? 1u : 0u);
         }
         umma_commit(&empty[s]);
       }
@@ -362,7 +393,7 @@ __global__ void __launch_bounds__(kConvThreads, 1)
         int x = t.x0 + (row & ((1 << p.lw) - 1));
         int y = t.y0 + ((row >> p.lw) & ((1 << p.lh) - 1));
         const int b = t.b0 + (row >> (p.lw + p.lh));
-        if (MODE == kConvFwd) {
+        if (MODE == kConvFwd || MODE == kConvPair) {
           valid = x < g.Wo && y < g.Ho && b < g.B;
           pix = ((size_t)b * g.Ho + y) * g.Wo + x;
         } else {
@@ -481,6 +512,7 @@ __global__ void __launch_bounds__(kConvThreads, 1)
     if (warp == 0 && lane == 0) {
       for (int i = max(0, issued - kStages); i < issued; ++i)
         mbar_wait(&full[i % kStages], (uint32_t)(i / kStages) & 1u, kSpinLimit);
+      if (MODE == kConvPair) mbar_wait(wfull, 0, kSpinLimit);
       mbar_wait(drained, 0, kSpinLimit);
       atomicOr(g.err, 1u);
     }
@@ -785,6 +817,20 @@ int map_taps(ConvMaps& maps, ConvArgs& g, const __nv_bfloat16* x, int group,
   return DS_OK;
 }
 
+// The image rows 2 oy - 1 + ky as rows of pixel pairs.
+int map_pairs(ConvMaps& maps, ConvArgs& g, const __nv_bfloat16* x, const PixelTiles& p) {
+  for (int ky = 0; ky < 3; ++ky) {
+    const int oy0 = ky == 0 ? 1 : 0, oy1 = std::min(g.Ho, (g.H - ky) / 2 + 1);
+    const bool none = oy1 <= oy0 || g.H < ky;
+    g.off_y[ky] = none ? 1 << 24 : -oy0;
+    DS_TRY(map_pixels(&maps.x[ky],
+                      none ? x : x + (int64_t)(oy0 * 2 - 1 + ky) * g.W * g.C, 64, g.W / 2,
+                      none ? 1 : oy1 - oy0, g.B, 64, 2 * (int64_t)g.W * g.C,
+                      (int64_t)g.H * g.W * g.C, 64, p));
+  }
+  return DS_OK;
+}
+
 int map_matrix(CUtensorMap* map, const void* base, int rows, int cols, int ld, int box_cols,
                int box_rows) {
   const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
@@ -941,14 +987,21 @@ int ds_conv3x3_forward(const void* x, int B, int H, int W, int C, int stride, co
   g.y = (__nv_bfloat16*)y;
   g.d = d;
   ConvMaps maps;
-  DS_TRY(map_taps(maps, g, (const __nv_bfloat16*)x, G, g.pt[0]));
+  const bool pairs = C == 32 && stride == 2 && W % 2 == 0 && !d && N > 32 && N <= 64;
   DS_TRY(map_matrix(&maps.w, w, N, Kp, Kp, G, bn));
+  if (pairs) {
+    for (int t = 3; t < 9; ++t) maps.x[t] = maps.w;  // not read
+    DS_TRY(map_pairs(maps, g, (const __nv_bfloat16*)x, g.pt[0]));
+  } else {
+    DS_TRY(map_taps(maps, g, (const __nv_bfloat16*)x, G, g.pt[0]));
+  }
   maps.dz = maps.z = maps.y = maps.w;  // not read
   if (!d)
     for (int k = 0; k < 2; ++k)
       DS_TRY(map_pixels(k ? &maps.y : &maps.z, k ? g.y : g.z, N, g.Wo, g.Ho, B, N, (int64_t)g.Wo * N,
                         (int64_t)g.Ho * g.Wo * N, bn < 64 ? 32 : 64, g.pt[0]));
   cudaStream_t s = (cudaStream_t)stream;
+  if (pairs) return launch_conv<64, kConvPair, 32, kConvGelu>(maps, g, s);
   if (G == 32)
     return d ? dispatch_bn<kConvFwd, 32, kConvF32>(bn, maps, g, s)
              : dispatch_bn<kConvFwd, 32, kConvGelu>(bn, maps, g, s);

@@ -116,3 +116,32 @@ def test_conv_timeout_is_reported_and_device_stays_usable(cuda_lib):
     torch.cuda.synchronize()
     gemm.check()
     assert torch.equal(z0, z1)
+
+
+@pytest.mark.parametrize("B,H,W,cout", [(1, 1, 2, 64), (2, 2, 4, 40), (3, 5, 6, 64), (1, 33, 258, 56),
+                                        (2, 130, 64, 64), (1, 16, 31, 64), (5, 40, 20, 64)])
+def test_pixel_pairs_of_32_channels_match_im2col(cuda_lib, B, H, W, cout):
+    """Stride 2 from 32 channels: rows of pixel pairs (an odd width takes the taps one by
+    one), bit for bit, and a wait that runs out is reported."""
+    import torch
+    from diffsplat_b200 import nn
+    gen = torch.Generator().manual_seed(H * W)
+    conv = nn.Conv3x3(32, cout, 2, gen=gen)
+    conv.b.copy_(torch.randn(cout, generator=gen))
+    x = torch.randn(B, H, W, 32, generator=gen).to(torch.bfloat16).cuda()
+    gemm = nn.Gemm()
+    nn.set_spin_limit(1)
+    try:
+        conv.forward(gemm, x)
+        torch.cuda.synchronize()
+    finally:
+        nn.set_spin_limit(0)
+    with pytest.raises(RuntimeError, match="timed out"):
+        gemm.check()
+    gemm.clear()
+    z, y = conv.forward(gemm, x)
+    col, _ = nn.im2col(x, 2, conv.kp)
+    torch.cuda.synchronize()
+    gemm.check()
+    want_z, want_y = gemm(col, conv.w16, nn.EPI_BIAS_GELU, bias=conv.b)
+    assert torch.equal(z.view(want_z.shape), want_z) and torch.equal(y.view(want_y.shape), want_y)

@@ -248,9 +248,8 @@ __global__ void __launch_bounds__(kThreads)
   const uint32_t total = sc->n_long;
   for (uint32_t w = (uint32_t)((blockIdx.x * (int64_t)kThreads + threadIdx.x) >> 5); w < total;
        w += (uint32_t)(gridDim.x * (kThreads / 32))) {
-    const uint4 seg = long_list[w];
+    const uint4 seg = long_list[w];  // {splat, first record, end}; record indices are 32-bit
     const uint32_t i = seg.x;
-    const unsigned long long s = seg.y, e = seg.z;
     float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     float a = 0.f;
     const ushort4 rc = sg.rect[i];
@@ -258,22 +257,20 @@ __global__ void __launch_bounds__(kThreads)
     uint32_t row0, pitch;
     seg_origin(sg, i, rc, row0, pitch);
     const unsigned long long key = seg_key(sg, i);
-    // record q is tile k = q - first of the row-major rectangle; lanes step by
-    // 32 = 32 / wd rows and 32 % wd columns
-    const uint32_t first = sg.start[i];
-    uint32_t ty = 0, tx = 0;
-    if (s + lane < e) {
-      const uint32_t k = (uint32_t)(s + lane - first);
-      ty = k / wd;
-      tx = k - ty * wd;
-    }
-    const uint32_t dy = 32u / wd, dx = 32u - dy * wd;
-    for (unsigned long long q = s + lane; q < e; q += 32) {
+    // Record q is tile q - first of the row-major rectangle; lanes step by 32 = 32 / wd rows
+    // and 32 % wd columns.  The quotients of numbers up to 32 come from the reciprocal:
+    // half a unit keeps them clear of its error.
+    const float inv = rcp((float)wd);
+    uint32_t ty = (uint32_t)((lane + 0.5f) * inv), tx = lane - ty * wd;
+    const uint32_t dy = (uint32_t)(32.5f * inv), dx = 32u - dy * wd;
+    bool any = false;
+    for (uint32_t q = seg.y + lane; q < seg.z; q += 32) {
       if (key < sg.tile_bound[row0 + ty * pitch + tx]) {
-        const float* r = isect_grad + q * 9;
+        const float* r = isect_grad + (size_t)q * 9;
 #pragma unroll
         for (int k = 0; k < 8; ++k) v[k] += r[k];
         a += r[8];
+        any = true;
       }
       ty += dy;
       tx += dx;
@@ -281,6 +278,10 @@ __global__ void __launch_bounds__(kThreads)
         tx -= wd;
         ++ty;
       }
+    }
+    if (!__any_sync(0xffffffffu, any)) {  // hidden in all its tiles, as most may be
+      if (lane < 9) store_g2<kAccumulate>(lane, i, n, 0.f, g2, gin);
+      continue;
     }
     const float s8 = warp_sum8_transposed(v, lane);
     const float sa = warp_sum(a);

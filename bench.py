@@ -143,13 +143,19 @@ NCU_DRAM_BYTES_PER_ISECT = {"composite_fwd": 22.396416e6 / 3085820,
                             "composite_bwd": (47.626240e6 + 11.928064e6) / 3085820}
 
 
-def kernels_per_step(tiles: int) -> int:
-    # step_begin, preprocess, 4 depth-sort passes x 3, count scan x 2, emission,
-    # tile sort (grids of up to 8192 tiles: count, offsets + ranges, scatter;
-    # larger: 3 kernels per radix pass over the tile id, then ranges and the
-    # tile schedule), composite forward, composite backward (two launches, one per
-    # pixel layout, each taking its own tiles), long-segment reduce,
-    # backward + Adam (which sums the short segments itself)
+def kernels_per_step(tiles: int, splats: int | None = None) -> int:
+    # Around the lists: step_begin, preprocess, composite forward, composite backward,
+    # long-segment reduce, backward + Adam (which sums the short segments itself).
+    # Lists by bins (bins, offsets, bins): after rank + place of up to 8192 splats, or the
+    # cluster sort and the two scans of up to 65536.
+    if splats is not None:
+        if splats <= 65536:
+            return 6 + 3 + (2 if splats <= 8192 else 3)
+        return kernels_per_step(tiles) - 1
+    # Without the splats an upper bound: 4 depth-sort passes x 3, count scan x 2,
+    # emission, tile sort (grids of up to 8192 tiles: count, offsets + ranges, scatter;
+    # larger: 3 kernels per radix pass over the tile id, then ranges and the tile
+    # schedule), and one spare launch of the backward.
     if tiles <= 8192:
         tile_sort = 3  # the offsets kernel also writes the tile schedule
     else:
@@ -803,7 +809,7 @@ def main():
         "mpix_per_s": value * pixels / 1e6,
         "e2e": {"value": steps_total / (r["e2e_ms"] / 1e3), "unit": "steps/s",
                 "h2d_bytes_per_step": 80, "d2h_bytes_per_step": 4},
-        "gpu_launches": kernels_per_step(tiles) * args.steps,
+        "gpu_launches": kernels_per_step(tiles, prob.params.shape[1]) * args.steps,
         "clocks": r["clocks"],
         "roofline": {"bound": "fp32", "kernel": dom, "achieved": tflops.get(dom),
                      "peak": fp32_peak, "unit": "TFLOP/s",

@@ -16,7 +16,7 @@
 // distributed shared memory (item by item they took twice the time).
 #include <cooperative_groups.h>
 
-#include <algorithm>
+#include <atomic>
 
 #include "ds_common.cuh"
 #include "ds_internal.h"
@@ -282,13 +282,13 @@ __global__ void __launch_bounds__(kThreads, 1)
 }  // namespace
 
 int small_sort_setup() {
-  static uint64_t set = 0;
+  static std::atomic<uint64_t> set{0};
   int dev = 0;
   DS_CUDA(cudaGetDevice(&dev));
-  if (dev < 64 && (set >> dev & 1u)) return DS_OK;
+  if (dev < 64 && (set.load() >> dev & 1u)) return DS_OK;
   DS_CUDA(cudaFuncSetAttribute(cluster_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)sizeof(SortShared)));
-  if (dev < 64) set |= 1ull << dev;
+  if (dev < 64) set.fetch_or(1ull << dev);
   return DS_OK;
 }
 

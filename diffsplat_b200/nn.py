@@ -1,7 +1,8 @@
 """Tensor-core building blocks of the learned initializer on the C ABI:
-BF16 GEMM (tcgen05), 3x3 convolutions as im2col + GEMM with fused bias/GELU,
-their backward (col2im with the producing layer's GELU derivative, weight
-gradients by split-K GEMM over pixels) and AdamW.  Activations are NHWC BF16;
+BF16 GEMM (tcgen05), 3x3 convolutions as implicit GEMMs with fused bias/GELU
+(im2col + GEMM for what the tensor maps do not take), their backward (with the
+producing layer's GELU derivative, weight gradients by split-K over pixels) and
+AdamW.  Activations are NHWC BF16;
 torch tensors are only the memory.
 """
 from __future__ import annotations
@@ -154,8 +155,8 @@ class Conv3x3:
         """Whether the convolution runs without an im2col matrix (ds_conv3x3_*):
         whole 64-channel blocks (or 32 channels; with `rgb` also 3), 16-byte
         rows and addresses, counts that fit 32 bits.  Measured against im2col +
-        GEMM (B200, forward + backward): 64 -> 128 channels, stride 2, 8 x 256 x 256: 2.03 -> 0.31 ms;
-        256 -> 256, 32 x 64 x 64: 6.16 -> 0.58 ms.  What it does not take (the
+        GEMM (B200, forward + backward): 64 -> 128 channels, stride 2, 8 x 256 x 256: 2.02 -> 0.24 ms;
+        256 -> 256, 32 x 64 x 64: 6.13 -> 0.54 ms.  What it does not take (the
         weight gradient of a 3-channel layer above all) goes through im2col."""
         x = tensors[0]
         return ((self.cin == 32 or self.cin % 64 == 0 or (rgb and self.cin == 3))

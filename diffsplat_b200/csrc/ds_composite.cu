@@ -198,9 +198,9 @@ __device__ __forceinline__ bool finite3(float r, float g, float b) {
   return fabsf(r) <= 3.0e38f && fabsf(g) <= 3.0e38f && fabsf(b) <= 3.0e38f;
 }
 
-// Mahalanobis distances (conic_dist2 in its rounding) of a splat at a pair of
-// pixels and opacity exp(-dist2 / 2) there, exp as 2^(dist2 (-log2(e) / 2)); dxx =
-// dx dx.
+// Mahalanobis distances dx^2 a + 2 dx dy b + dy^2 c of a splat at a pair of pixels, in
+// the reference's rounding (tile_rasterize_layer.cu:321, :341), and opacity
+// exp(-dist2 / 2) there, exp as 2^(dist2 (-log2(e) / 2)); dxx = dx dx.
 __device__ __forceinline__ float2 pair_dist2(float2 dx, float2 dxx, float2 dy,
                                              const SplatRec& r) {
   return fma2(mul2(dy, dy), r.conic_c(),

@@ -22,6 +22,13 @@
 // in wgrad) MN-major, so nothing is transposed.  The K order of the forward is
 // that of the im2col matrix, hence its results too, bit for bit.
 //
+// The input gradient sums as the GEMM dz . w with col2im does: the N products of a tap
+// are one accumulator of the tensor cores, the taps that reach a pixel are added in FP32
+// in their order, hence its results, bit for bit, and chains no longer than N (all nine
+// taps in one accumulator round 9 N products in a row).  Each tap's accumulator is
+// read back while the next one fills, so the epilogue warps hold a tile's sums in
+// registers.
+//
 // An RGB input (the first layer) has rows of 27 products, too short and too
 // unaligned for TMA: conv3x3_rgb_kernel gathers them into shared memory itself.
 //
@@ -46,8 +53,7 @@ namespace {
 enum ConvMode : int { kConvFwd = 0, kConvDgrad = 1, kConvWgrad = 2, kConvPair = 3 };
 enum ConvEpi : int { kConvGelu = 0, kConvF32 = 1 };  // forward only
 
-constexpr int kEpiWarps = 8;  // two per 32 TMEM lanes, each with half of the columns
-constexpr int kConvThreads = 64 + 32 * kEpiWarps;
+constexpr int kEpiWarps = 8;  // forward: two per 32 TMEM lanes, each with half of the columns
 constexpr int kWgradPixels = 64;  // K block of the weight gradient
 // Pixels summed by one accumulation chain of the weight gradient: the tensor
 // cores' FP32 sums lose precision with the chain's length (relative error
@@ -107,7 +113,19 @@ struct ConvShape {
   static constexpr int kRoom = kStaged ? 230400 - (int)(kStaging + kWeights) : 196608;
   static constexpr int kStages = kRoom / (int)kStage < 8 ? kRoom / (int)kStage : 8;
   static constexpr size_t kSmem = 1024 + (size_t)kStages * kStage + kStaging + kWeights + 256;
-  static constexpr uint32_t kCols = 2 * BN;  // two accumulators (32 .. 512 columns)
+  // dgrad: each tap has columns of its own, and as many taps as fit 256 columns are handed
+  // to the epilogue together (a hand-over takes it some 1100 cycles, a tap of 64 channels
+  // and columns 128 of the tensor cores).  From 128 columns on, four warps per 32 lanes hold the
+  // tile's sums.  With gelu'(z), B200: 64 -> 64 channels, 16 x 256 x 256: 0.245 ms (0.341 with a
+  // tap a hand-over); 64 -> 128, stride 2, 8 x 256 x 256: 0.091 (0.097); 256 -> 256, 32 x 64 x 64:
+  // 0.172.  All taps in one accumulator took 0.185, 0.084 and 0.137, and rounded 9 N products
+  // in a row.
+  static constexpr int kTogether = MODE == kConvDgrad ? 256 / BN : 1;
+  static constexpr uint32_t kAccCols = kTogether * BN;
+  static constexpr uint32_t kCols = 2 * kAccCols;  // two accumulators (64 .. 512 columns)
+  static constexpr int kEpi = MODE == kConvDgrad && BN >= 128 ? 16 : kEpiWarps;
+  static constexpr int kGroups = kEpi / 4;  // column groups: 32 of every 32 kGroups
+  static constexpr int kThreads = 64 + 32 * kEpi;
 };
 
 struct Item {
@@ -176,6 +194,28 @@ __device__ __forceinline__ void store_outputs(float* d, __nv_bfloat16* z, __nv_b
 __device__ __forceinline__ int class_py(int cls) { return cls < 2 ? 1 : 0; }
 __device__ __forceinline__ int class_px(int cls) { return (cls & 1) ^ 1; }
 
+// Tap k of the taps that reach the pixels of a class, in ascending (ky, kx): pixel (y, x)
+// of the class reads dz(y + oy, x + ox) through it.
+struct DgradTap {
+  int ky, kx, oy, ox;
+};
+__device__ __forceinline__ int dgrad_taps(int stride, int cls) {
+  return stride == 1 ? 9 : (class_py(cls) ? 2 : 1) * (class_px(cls) ? 2 : 1);
+}
+__device__ __forceinline__ DgradTap dgrad_tap(int stride, int cls, int k) {
+  DgradTap t;
+  if (stride == 1) {
+    t.ky = k / 3, t.kx = k - 3 * t.ky;
+    t.oy = 1 - t.ky, t.ox = 1 - t.kx;
+  } else {
+    // iy = 2 y + py reads oy = (iy + 1 - ky) / 2: ky = 1 for even rows, 0 and 2 for odd
+    const int py = class_py(cls), px = class_px(cls);
+    t.ky = py ? 2 * (px ? k >> 1 : k) : 1, t.kx = px ? 2 * (k & 1) : 1;
+    t.oy = py && t.ky == 0 ? 1 : 0, t.ox = px && t.kx == 0 ? 1 : 0;
+  }
+  return t;
+}
+
 // Barrier of the epilogue's warps, and the same with a vote.
 __device__ __forceinline__ void epi_sync() {
   __syncwarp();
@@ -196,7 +236,7 @@ __device__ __forceinline__ bool epi_all(bool mine) {
 }
 
 template <int BN, int MODE, int G, int EPI>
-__global__ void __launch_bounds__(kConvThreads, 1)
+__global__ void __launch_bounds__(ConvShape<BN, MODE, G, EPI>::kThreads, 1)
     conv3x3_kernel(const __grid_constant__ ConvMaps maps, const __grid_constant__ ConvArgs g) {
   using S = ConvShape<BN, MODE, G, EPI>;
   constexpr int kStages = S::kStages;
@@ -224,7 +264,7 @@ __global__ void __launch_bounds__(kConvThreads, 1)
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&acc_full[a], 1);
-      mbar_init(&acc_empty[a], kEpiWarps);
+      mbar_init(&acc_empty[a], S::kEpi);
     }
     mbar_init(drained, 1);
     mbar_init(wfull, 1);
@@ -241,14 +281,15 @@ __global__ void __launch_bounds__(kConvThreads, 1)
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
 
-  // K blocks of a work item
+  // A work item is sums_of sums of blocks_of K blocks each, kTogether sums at a time.
+  auto sums_of = [&](const Item& t) {
+    return MODE == kConvDgrad ? dgrad_taps(g.stride, t.cls) : 1;
+  };
   auto blocks_of = [&](const Item& t) {
     if (MODE == kConvFwd) return 9 * (g.C / G);
     if (MODE == kConvPair) return 6;
     if (MODE == kConvWgrad) return t.kb1 - t.kb0;
-    const int nb = (g.N + 63) / 64;
-    if (g.stride == 1) return 9 * nb;
-    return (class_py(t.cls) ? 2 : 1) * (class_px(t.cls) ? 2 : 1) * nb;
+    return (g.N + 63) / 64;
   };
 
   int issued = 0;
@@ -261,7 +302,7 @@ __global__ void __launch_bounds__(kConvThreads, 1)
     }
     for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
       const Item t = item_of<MODE>(g, it, BN);
-      const int nkb = blocks_of(t);
+      const int nkb = sums_of(t) * blocks_of(t);
       for (int i = 0; i < nkb; ++i) {
         const int s = issued % kStages;
         if (!mbar_wait(&empty[s], ((uint32_t)(issued / kStages) & 1u) ^ 1u, g.spin)) {
@@ -283,19 +324,9 @@ __global__ void __launch_bounds__(kConvThreads, 1)
           tma_load_4d(a, &maps.x[ky], &full[s], 0, t.x0 - 1 + (i & 1), t.y0 + g.off_y[ky], t.b0);
         } else if (MODE == kConvDgrad) {
           const int nb = (g.N + 63) / 64, k = i / nb, n = (i - k * nb) * 64;
-          int ky, kx, oy, ox;
-          if (g.stride == 1) {
-            ky = k / 3, kx = k - 3 * ky;
-            oy = t.y0 + 1 - ky, ox = t.x0 + 1 - kx;
-          } else {
-            // iy = 2 y + py reads oy = (iy + 1 - ky) / 2: ky = 1 for even rows, 0 and 2 for odd
-            const int py = class_py(t.cls), px = class_px(t.cls);
-            const int iy = px ? k >> 1 : k, ix = px ? k & 1 : 0;
-            ky = py ? 2 * iy : 1, kx = px ? 2 * ix : 1;
-            oy = t.y0 + (py && ky == 0 ? 1 : 0), ox = t.x0 + (px && kx == 0 ? 1 : 0);
-          }
-          tma_load_4d(a, &maps.dz, &full[s], n, ox, oy, t.b0);
-          const int c = (ky * 3 + kx) * g.C + t.n0;
+          const DgradTap tap = dgrad_tap(g.stride, t.cls, k);
+          tma_load_4d(a, &maps.dz, &full[s], n, t.x0 + tap.ox, t.y0 + tap.oy, t.b0);
+          const int c = (tap.ky * 3 + tap.kx) * g.C + t.n0;
 #pragma unroll
           for (int j = 0; j < S::kNB / 64; ++j)
             tma_load_2d(b + j * 8192, &maps.w, &full[s], c + 64 * j, n);
@@ -327,99 +358,186 @@ __global__ void __launch_bounds__(kConvThreads, 1)
       atomicExch(&failed, 1);
       ok = false;
     }
-    int n = 0, li = 0;
-    for (int it = blockIdx.x; it < items && ok; it += gridDim.x, ++li) {
+    int n = 0, turn = 0;  // K blocks and accumulators issued
+    for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
       const Item t = item_of<MODE>(g, it, BN);
-      const int nkb = blocks_of(t), acc = li & 1;
-      if (!mbar_wait(&acc_empty[acc], ((uint32_t)(li >> 1) & 1u) ^ 1u, g.spin)) {
-        atomicExch(&failed, 1);
-        break;
-      }
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      for (int i = 0; i < nkb; ++i, ++n) {
-        const int s = n % kStages;
-        if (!mbar_wait(&full[s], (uint32_t)(n / kStages) & 1u, g.spin)) {
+      const int nkb = blocks_of(t), sums = sums_of(t);
+      for (int j = 0; j < sums && ok; j += S::kTogether, ++turn) {
+        const int acc = turn & 1;
+        if (!mbar_wait(&acc_empty[acc], ((uint32_t)(turn >> 1) & 1u) ^ 1u, g.spin)) {
           atomicExch(&failed, 1);
           ok = false;
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t a = smem_u32(smem + (size_t)s * S::kStage), b = a + S::kBytesA;
+        const int blocks = min(S::kTogether, sums - j) * nkb;
+        uint32_t d = tmem + acc * S::kAccCols;
+        for (int k = 0, i = 0; k < blocks; ++k, ++n) {
+          const int s = n % kStages;
+          if (!mbar_wait(&full[s], (uint32_t)(n / kStages) & 1u, g.spin)) {
+            atomicExch(&failed, 1);
+            ok = false;
+            break;
+          }
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t a = smem_u32(smem + (size_t)s * S::kStage), b = a + S::kBytesA;
 #pragma unroll
-        for (int kk = 0; kk < S::kBK / 16; ++kk) {
-          if (MODE == kConvPair && !(i & 1) && kk < 2) continue;  // the second pixel only
-          // K-major rows of G (64) channels: 16 channels further are 32 bytes.
-          // MN-major: 8-row groups of 128 (64) bytes, 16 rows further two groups,
-          // the next 64 (32) columns a whole K block further.
-          const uint64_t da =
-              MODE == kConvWgrad
-                  ? smem_desc(a + kk * G * 32, G * 128, G * 16, G == 64 ? 2u : 4u)
-                  : smem_desc(a + kk * 32, 16, S::kBK * 16, S::kBK == 64 ? 2u : 4u);
-          const uint64_t db =
-              MODE == kConvPair
-                  ? smem_desc(smem_u32(weights) +
-                                  ((i >> 1) * 3 + (i & 1 ? 1 + (kk >> 1) : 0)) * BN * 64 +
-                                  (kk & 1) * 32,
-                              16, 512, 4u)
-              : MODE == kConvFwd ? smem_desc(b + kk * 32, 16, G * 16, G == 64 ? 2u : 4u)
-                               : smem_desc(b + kk * 2048, 8192, 1024, 2u);
-          umma_bf16(tmem + (uint32_t)(acc * BN), da, db, idesc,
-                    (i > 0 || kk > (MODE == kConvPair ? 2 : 0)) ? 1u : 0u);
+          for (int kk = 0; kk < S::kBK / 16; ++kk) {
+            if (MODE == kConvPair && !(i & 1) && kk < 2) continue;  // the second pixel only
+            // K-major rows of G (64) channels: 16 channels further are 32 bytes.
+            // MN-major: 8-row groups of 128 (64) bytes, 16 rows further two groups,
+            // the next 64 (32) columns a whole K block further.
+            const uint64_t da =
+                MODE == kConvWgrad
+                    ? smem_desc(a + kk * G * 32, G * 128, G * 16, G == 64 ? 2u : 4u)
+                    : smem_desc(a + kk * 32, 16, S::kBK * 16, S::kBK == 64 ? 2u : 4u);
+            const uint64_t db =
+                MODE == kConvPair
+                    ? smem_desc(smem_u32(weights) +
+                                    ((i >> 1) * 3 + (i & 1 ? 1 + (kk >> 1) : 0)) * BN * 64 +
+                                    (kk & 1) * 32,
+                                16, 512, 4u)
+                : MODE == kConvFwd ? smem_desc(b + kk * 32, 16, G * 16, G == 64 ? 2u : 4u)
+                                 : smem_desc(b + kk * 2048, 8192, 1024, 2u);
+            umma_bf16(d, da, db, idesc,
+                      (i > 0 || kk > (MODE == kConvPair ? 2 : 0)) ? 1u : 0u);
+          }
+          umma_commit(&empty[s]);
+          if (++i == nkb && MODE == kConvDgrad) i = 0, d += BN;  // the next tap
         }
-        umma_commit(&empty[s]);
+        umma_commit(&acc_full[acc]);
       }
-      umma_commit(&acc_full[acc]);
     }
     umma_commit(drained);
   } else if (warp >= 2) {
     const int quad = warp & 3;  // the TMEM lanes this warp may read: 32 quad ..
     const int row = quad * 32 + lane;
-    int li = 0, slabs = 0;
-    for (int it = blockIdx.x; it < items; it += gridDim.x, ++li) {
-      const Item t = item_of<MODE>(g, it, BN);
-      const int acc = li & 1;
-      const bool got = mbar_wait(&acc_full[acc], (uint32_t)(li >> 1) & 1u, g.spin);
-      // staged: the epilogue's warps meet at barriers, so they leave together
+    const int group = (warp - 2) / 4;  // of the columns (of a slab's)
+    // The accumulator of a turn in this warp's lanes, once it is complete: -1 if the wait
+    // ran out.  Staged: the epilogue's warps meet at barriers, so they leave together.
+    auto take = [&](int turn) {
+      const int acc = turn & 1;
+      const bool got = mbar_wait(&acc_full[acc], (uint32_t)(turn >> 1) & 1u, g.spin);
       if (S::kStaged ? !epi_all(got) : !__all_sync(0xffffffffu, got)) {
         atomicExch(&failed, 1);
-        break;
+        return -1;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t ta = tmem + (uint32_t)(acc * BN) + ((uint32_t)(quad * 32) << 16);
+      return (int)(tmem + acc * S::kAccCols + ((uint32_t)(quad * 32) << 16));
+    };
+    auto give_back = [&](int turn) {
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0)
+        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(
+                         smem_u32(&acc_empty[turn & 1]))
+                     : "memory");
+    };
+    int turn = 0, slabs = 0;
+    for (int it = blockIdx.x; it < items; it += gridDim.x) {
+      const Item t = item_of<MODE>(g, it, BN);
       bool valid = false;
       size_t pix = 0;
+      int x = 0, y = 0;
       if (MODE != kConvWgrad) {
         const PixelTiles& p = g.pt[MODE == kConvDgrad ? t.cls : 0];
-        int x = t.x0 + (row & ((1 << p.lw) - 1));
-        int y = t.y0 + ((row >> p.lw) & ((1 << p.lh) - 1));
+        x = t.x0 + (row & ((1 << p.lw) - 1));
+        y = t.y0 + ((row >> p.lw) & ((1 << p.lh) - 1));
         const int b = t.b0 + (row >> (p.lw + p.lh));
         if (MODE == kConvFwd || MODE == kConvPair) {
           valid = x < g.Wo && y < g.Ho && b < g.B;
           pix = ((size_t)b * g.Ho + y) * g.Wo + x;
         } else {
-          if (g.stride == 2) {
-            x = 2 * x + class_px(t.cls);
-            y = 2 * y + class_py(t.cls);
-          }
-          valid = x < g.W && y < g.H && b < g.B;
-          pix = ((size_t)b * g.H + y) * g.W + x;
+          const int s = g.stride, ix = s == 2 ? 2 * x + class_px(t.cls) : x;
+          const int iy = s == 2 ? 2 * y + class_py(t.cls) : y;
+          valid = ix < g.W && iy < g.H && b < g.B;
+          pix = ((size_t)b * g.H + iy) * g.W + ix;
         }
       }
+      if (MODE == kConvDgrad) {
+        constexpr int kWide = 32 * S::kGroups;
+        constexpr int kParts = (BN + kWide - 1) / kWide;  // of 32 columns: 32 group + kWide j
+        float sum[kParts][32];
+#pragma unroll
+        for (int j = 0; j < kParts; ++j)
+#pragma unroll
+          for (int q = 0; q < 32; ++q) sum[j][q] = 0.f;
+        const int taps = dgrad_taps(g.stride, t.cls);
+        int ta = 0;
+#pragma unroll 1
+        for (int k0 = 0; k0 < taps; k0 += S::kTogether, ++turn) {
+          ta = take(turn);
+          if (ta == -1) break;
+          const int k1 = min(taps, k0 + S::kTogether);
+#pragma unroll 1
+          for (int k = k0; k < k1; ++k) {
+            // a tap that reads past dz adds nothing (not 0 times its weight)
+            const DgradTap tap = dgrad_tap(g.stride, t.cls, k);
+            const bool reads = (unsigned)(y + tap.oy) < (unsigned)g.Ho &&
+                               (unsigned)(x + tap.ox) < (unsigned)g.Wo;
+#pragma unroll
+            for (int j = 0; j < kParts; ++j) {
+              if (32 * group + kWide * j >= BN) continue;
+              constexpr int kRead = kParts > 1 ? 16 : 32;  // (registers)
+#pragma unroll
+              for (int h = 0; h < 32; h += kRead) {
+                uint32_t r[kRead];
+                tmem_ld((uint32_t)ta + (uint32_t)((k - k0) * BN + 32 * group + kWide * j + h), r);
+                if (reads) {
+#pragma unroll
+                  for (int q = 0; q < kRead; ++q) sum[j][h + q] += __uint_as_float(r[q]);
+                }
+                __syncwarp();
+              }
+            }
+          }
+          give_back(turn);
+        }
+        if (ta == -1) break;
+#pragma unroll
+        for (int j = 0; j < kParts && valid; ++j) {
+          const int c0 = t.n0 + 32 * group + kWide * j;
+          const size_t base = pix * g.C + c0;
+#pragma unroll
+          for (int q = 0; q < 32; q += 8) {
+            if (32 * group + kWide * j >= BN || c0 + q >= g.C) break;  // C is a multiple of 8
+            if (g.zprev) {
+              __align__(16) __nv_bfloat162 z2[4];
+              *reinterpret_cast<uint4*>(z2) = *reinterpret_cast<const uint4*>(g.zprev + base + q);
+#pragma unroll
+              for (int k = 0; k < 4; ++k) {
+                const float2 slope = gelu_grad2(__bfloat1622float2(z2[k]));
+                sum[j][q + 2 * k] *= slope.x;
+                sum[j][q + 2 * k + 1] *= slope.y;
+              }
+            }
+            __align__(16) __nv_bfloat162 y2[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+              y2[k] = __floats2bfloat162_rn(sum[j][q + 2 * k], sum[j][q + 2 * k + 1]);
+            *reinterpret_cast<uint4*>(g.y + base + q) = *reinterpret_cast<uint4*>(y2);
+          }
+        }
+        __syncwarp();
+        continue;
+      }
+      const int got = take(turn);
+      if (got == -1) break;
+      const uint32_t ta = (uint32_t)got;
       if (S::kStaged) {
-        const int half = (warp - 2) / 4;  // of the slab's columns
 #pragma unroll 1
         for (int n = 0; n < BN && t.n0 + n < g.N; n += S::kSlab, ++slabs) {
           uint8_t* tz = staging + (size_t)(slabs % S::kBufs) * 2 * S::kTile;
           uint8_t* ty = tz + S::kTile;
           if (warp == 2 && lane == 0) bulk_wait_read<S::kBufs - 1>();
           epi_sync();
-          if (half * 32 < S::kSlab) {
+          if (group * 32 < S::kSlab) {
             uint32_t r[32];
-            tmem_ld32(ta + (uint32_t)(n + 32 * half), r);
+            tmem_ld(ta + (uint32_t)(n + 32 * group), r);
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
               float v[8];
-              const int c = t.n0 + n + 32 * half + 8 * q;  // N is a multiple of 8
+              const int c = t.n0 + n + 32 * group + 8 * q;  // N is a multiple of 8
 #pragma unroll
               for (int k = 0; k < 8; ++k) v[k] = __uint_as_float(r[8 * q + k]);
               if (c < g.N) {
@@ -429,7 +547,7 @@ __global__ void __launch_bounds__(kConvThreads, 1)
                 v[4] += b1.x, v[5] += b1.y, v[6] += b1.z, v[7] += b1.w;
               }
               // the tensor maps' swizzle: 128-byte rows, or 64-byte ones
-              const int chunk = half * 4 + q;
+              const int chunk = group * 4 + q;
               const int at = S::kSlab == 64 ? row * 128 + ((chunk ^ (row & 7)) << 4)
                                             : row * 64 + ((chunk ^ ((row >> 1) & 3)) << 4);
               store_outputs<kConvGelu>(nullptr, reinterpret_cast<__nv_bfloat16*>(tz),
@@ -446,9 +564,9 @@ __global__ void __launch_bounds__(kConvThreads, 1)
         }
       } else {
 #pragma unroll 1
-        for (int c0 = (warp - 2) / 4 * 32; c0 < BN; c0 += 32 * (kEpiWarps / 4)) {
+        for (int c0 = group * 32; c0 < BN; c0 += 32 * S::kGroups) {
           uint32_t r[32];
-          tmem_ld32(ta + (uint32_t)c0, r);
+          tmem_ld(ta + (uint32_t)c0, r);
           if (MODE == kConvWgrad) {
             // rows are columns of gw: the lanes write 128 contiguous bytes
             const int j = t.x0 + row;
@@ -459,46 +577,23 @@ __global__ void __launch_bounds__(kConvThreads, 1)
                 if (t.n0 + c0 + q < g.N) dst[(size_t)q * g.kp] = __uint_as_float(r[q]);
             }
           } else if (valid) {
-            const int width = MODE == kConvFwd ? g.N : g.C;  // a multiple of 8
-            const size_t base = pix * width + t.n0 + c0;
+            const size_t base = pix * g.N + t.n0 + c0;
 #pragma unroll
             for (int q = 0; q < 32; q += 8) {
-              if (t.n0 + c0 + q >= width) break;
+              if (t.n0 + c0 + q >= g.N) break;  // N is a multiple of 8
               float v[8];
+              const float4* bias = reinterpret_cast<const float4*>(g.bias + t.n0 + c0 + q);
+              const float4 b0 = bias[0], b1 = bias[1];
 #pragma unroll
               for (int k = 0; k < 8; ++k) v[k] = __uint_as_float(r[q + k]);
-              if (MODE == kConvFwd) {
-                const float4* bias = reinterpret_cast<const float4*>(g.bias + t.n0 + c0 + q);
-                const float4 b0 = bias[0], b1 = bias[1];
-                v[0] += b0.x, v[1] += b0.y, v[2] += b0.z, v[3] += b0.w;
-                v[4] += b1.x, v[5] += b1.y, v[6] += b1.z, v[7] += b1.w;
-                store_outputs<EPI>(g.d, g.z, g.y, base + q, v);
-              } else {
-                if (g.zprev) {
-                  __align__(16) __nv_bfloat162 z2[4];
-                  *reinterpret_cast<uint4*>(z2) =
-                      *reinterpret_cast<const uint4*>(g.zprev + base + q);
-#pragma unroll
-                  for (int k = 0; k < 4; ++k) {
-                    const float2 d = gelu_grad2(__bfloat1622float2(z2[k]));
-                    v[2 * k] *= d.x;
-                    v[2 * k + 1] *= d.y;
-                  }
-                }
-                __align__(16) __nv_bfloat162 y2[4];
-#pragma unroll
-                for (int k = 0; k < 4; ++k) y2[k] = __floats2bfloat162_rn(v[2 * k], v[2 * k + 1]);
-                *reinterpret_cast<uint4*>(g.y + base + q) = *reinterpret_cast<uint4*>(y2);
-              }
+              v[0] += b0.x, v[1] += b0.y, v[2] += b0.z, v[3] += b0.w;
+              v[4] += b1.x, v[5] += b1.y, v[6] += b1.z, v[7] += b1.w;
+              store_outputs<EPI>(g.d, g.z, g.y, base + q, v);
             }
           }
         }
       }
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      __syncwarp();
-      if (lane == 0)
-        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[acc]))
-                     : "memory");
+      give_back(turn++);
     }
     if (S::kStaged && warp == 2 && lane == 0) bulk_wait_all();
   }
@@ -684,7 +779,7 @@ __global__ void __launch_bounds__(kRgbThreads)
 #pragma unroll 1
     for (int c0 = 0; c0 < BN; c0 += 32) {
       uint32_t r[32];
-      tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, r);
+      tmem_ld(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, r);
       if (kStaged) {
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -858,7 +953,7 @@ int launch_conv(const ConvMaps& maps, const ConvArgs& g, cudaStream_t s) {
   });
   DS_CUDA(attr);
   const int grid = std::min(g.first[g.classes], sm_count());
-  conv3x3_kernel<BN, MODE, G, EPI><<<grid, kConvThreads, S::kSmem, s>>>(maps, g);
+  conv3x3_kernel<BN, MODE, G, EPI><<<grid, S::kThreads, S::kSmem, s>>>(maps, g);
   return cuda_status(cudaGetLastError());
 }
 

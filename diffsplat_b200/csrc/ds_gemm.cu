@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 #pragma unroll 1
     for (int c0 = 0; c0 < BN; c0 += 32) {
       uint32_t r[32];
-      tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, r);
+      tmem_ld(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, r);
       if (row < g.M) {
         if (EPI == kEpiBiasGeluBf16) {
           __nv_bfloat16* yrow = g.Y + (size_t)row * g.ldy;

@@ -155,8 +155,8 @@ class Conv3x3:
         """Whether the convolution runs without an im2col matrix (ds_conv3x3_*):
         whole 64-channel blocks (or 32 channels; with `rgb` also 3), 16-byte
         rows and addresses, counts that fit 32 bits.  Measured against im2col +
-        GEMM (B200, forward + backward): 64 -> 128 channels, stride 2, 8 x 256 x 256: 2.02 -> 0.24 ms;
-        256 -> 256, 32 x 64 x 64: 6.13 -> 0.54 ms.  What it does not take (the
+        GEMM (B200, forward + backward): 64 -> 128 channels, stride 2, 8 x 256 x 256: 2.02 -> 0.25 ms;
+        256 -> 256, 32 x 64 x 64: 6.13 -> 0.57 ms.  What it does not take (the
         weight gradient of a 3-channel layer above all) goes through im2col."""
         x = tensors[0]
         return ((self.cin == 32 or self.cin % 64 == 0 or (rgb and self.cin == 3))

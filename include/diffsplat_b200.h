@@ -402,7 +402,7 @@ int ds_col2im_bf16(const float *dcol, int B, int H, int W, int C, int stride, in
  * order.  Forward: z = BF16(conv + bias) and y = BF16(gelu(conv + bias))
  * [B*Ho*Wo][N], or FP32 d = conv + bias when d is given; equal to im2col +
  * ds_gemm_bf16_tn bit for bit.  dgrad: dx [B][H][W][C] BF16, times gelu'(zprev)
- * when given.  wgrad: gw [N][Kp] FP32 (B*Ho*Wo a multiple of 8); workspace holds
+ * when given; equal to ds_gemm_bf16_tn (dz . w) + ds_col2im_bf16 bit for bit.  wgrad: gw [N][Kp] FP32 (B*Ho*Wo a multiple of 8); workspace holds
  * the floats that ds_conv3x3_wgrad_workspace returns (0: none; negative: a
  * shape it does not take).  *err as for ds_gemm_bf16_tn. */
 int ds_conv3x3_forward(const void *x, int B, int H, int W, int C, int stride, const void *w,

@@ -24,6 +24,7 @@
 
 #include "ds_common.cuh"
 #include "ds_internal.h"
+#include "ds_warp_gather.cuh"
 
 namespace ds {
 
@@ -216,17 +217,7 @@ __global__ void __launch_bounds__(kBinThreads) tile_bins_kernel(const BinArgs g)
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         if (!word[u]) continue;
-        if (word[u] >> lane & 1u)
-          sbuf[w][pend + __popc(word[u] & lt)] = (uint16_t)(k + 32 * u + lane);
-        pend += __popc(word[u]);
-        if (pend >= 32) {
-          __syncwarp();
-          place(32);
-          const uint16_t rest = sbuf[w][32 + lane];
-          __syncwarp();
-          sbuf[w][lane] = rest;
-          pend -= 32;
-        }
+        pend = warp_gather(sbuf[w], pend, word[u], k + 32 * u, lane, place);
       }
     }
     __syncwarp();

@@ -471,8 +471,7 @@ struct BwdShared {
   float4 box[NW];
   float4 gr[NW][16], gg[NW][16], gb[NW][16];  // per pixel of a warp: dL/dpixel
   float2 nx[NW][4];    // -x (NDC) of a warp's columns 2q and 2q + 1
-  float2 ny[NW];       // -y of its rows 1 and 5,
-  float2 row[NW][4];   // and what rows r and r + 4 add to that
+  float2 ny[NW][4];    // -y of its rows r and r + 4
   float4 s[NW][kBwdHits * kPitch / 4];    // per (hit, pixel): opacity exp() dL/dalpha
   float4 fac[NW][kBwdHits * kPitch / 4];  // per (hit, pixel): alpha T
   float part[NW][B * 9];       // per-warp gradient of each batch splat
@@ -498,11 +497,12 @@ __device__ __forceinline__ int pixel_slot(int lane) {
 //   d dist2 / d(ndc x, ndc y) = (2u, 2w)
 //   d dist2 / d(cov xx, xy, yy) = -u^2, -2uw, -w^2
 // (uw = b dist2 + dx dy / det written without the cancelling difference), and s
-// = -2 dL/d(dist2).  In a column u and w are linear in y, so the sums of s u, s w,
-// s u^2, s u w and s w^2 over four rows follow from three moments of s about one of
-// them (from the rows' own y, which are not quite evenly spaced in FP32).  kSafe
-// forms them pixel by pixel instead and leaves out what s = 0 or fac = 0 multiplies,
-// as it may be infinite or NaN.
+// = -2 dL/d(dist2).  u and w are formed at every pixel, from its own dx and dy: sums of s u^2,
+// s u w and s w^2 rebuilt from moments of s about a row cancel for splats thinner than a
+// pixel, to a relative error of 3e-6 at sigma = 0.1 pixels and 1e-3 at 0.003, where this
+// form stays at 1e-7, and saved little (1280x720 fit, step 4, 0.218 -> 0.214 ms; a million
+// splats at 1920x1080 0.491 -> 0.484, B200).  kSafe also leaves out what s = 0 or fac = 0
+// multiplies, as it may be infinite or NaN.
 template <bool kSafe, int TS>
 __device__ __forceinline__ void reduce_hits(BwdShared<TS>& sm, int w, int lane, int count,
                                             int slot) {
@@ -510,7 +510,6 @@ __device__ __forceinline__ void reduce_hits(BwdShared<TS>& sm, int w, int lane, 
   const int h = lane >> 2, q = lane & 3;
   const SplatRec& hit = sm.splat[slot];
   const float2 ca = hit.conic_a(), cb = mul2(hit.conic_2b(), both(0.5f)), cc = hit.conic_c();
-  const float2 dyc = add2(hit.y(), sm.ny[w]);  // dy in rows 1 and 5
   const float2 nx = sm.nx[w][q];
   float2 v[9];
 #pragma unroll
@@ -542,39 +541,23 @@ __device__ __forceinline__ void reduce_hits(BwdShared<TS>& sm, int w, int lane, 
 #pragma unroll
   for (int e = 0; e < 2; ++e) {
     const float2 dx = add2(hit.x(), both(e ? nx.y : nx.x));
-    if (kSafe) {
 #pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const float2 dy = add2(dyc, sm.row[w][r]);
-        float2 u = fma2(dx, ca, mul2(dy, cb));
-        float2 t = fma2(dx, cb, mul2(dy, cc));
-        const float2 z = s[r][e];
+    for (int r = 0; r < 4; ++r) {
+      const float2 dy = add2(hit.y(), sm.ny[w][r]);
+      float2 u = fma2(dx, ca, mul2(dy, cb));
+      float2 t = fma2(dx, cb, mul2(dy, cc));
+      const float2 z = s[r][e];
+      if (kSafe) {
         u.x = z.x != 0.f ? u.x : 0.f, u.y = z.y != 0.f ? u.y : 0.f;
         t.x = z.x != 0.f ? t.x : 0.f, t.y = z.y != 0.f ? t.y : 0.f;
-        const float2 su = mul2(z, u), st = mul2(z, t);
-        v[3] = add2(v[3], su);
-        v[4] = add2(v[4], st);
-        v[5] = fma2(su, u, v[5]);
-        v[6] = fma2(su, t, v[6]);
-        v[7] = fma2(st, t, v[7]);
-        v[8] = add2(v[8], z);
       }
-    } else {
-      const float2 d0 = sm.row[w][0], d2 = sm.row[w][2], d3 = sm.row[w][3];
-      const float2 z0 = mul2(s[0][e], d0), z2 = mul2(s[2][e], d2), z3 = mul2(s[3][e], d3);
-      const float2 m0 = add2(add2(s[0][e], s[1][e]), add2(s[2][e], s[3][e]));
-      const float2 m1 = add2(add2(z0, z2), z3);
-      const float2 m2 = fma2(z3, d3, fma2(z2, d2, mul2(z0, d0)));
-      // in row 1 (5): u and t
-      const float2 u = fma2(dx, ca, mul2(dyc, cb)), t = fma2(dx, cb, mul2(dyc, cc));
-      const float2 su = fma2(u, m0, mul2(cb, m1)), ru = fma2(u, m1, mul2(cb, m2));
-      const float2 st = fma2(t, m0, mul2(cc, m1)), rt = fma2(t, m1, mul2(cc, m2));
+      const float2 su = mul2(z, u), st = mul2(z, t);
       v[3] = add2(v[3], su);
       v[4] = add2(v[4], st);
-      v[5] = fma2(u, su, fma2(cb, ru, v[5]));
-      v[6] = fma2(t, su, fma2(cc, ru, v[6]));
-      v[7] = fma2(t, st, fma2(cc, rt, v[7]));
-      v[8] = add2(v[8], m0);
+      v[5] = fma2(su, u, v[5]);
+      v[6] = fma2(su, t, v[6]);
+      v[7] = fma2(st, t, v[7]);
+      v[8] = add2(v[8], z);
     }
   }
   float r[9];
@@ -611,7 +594,7 @@ __device__ __forceinline__ void reduce_hits(BwdShared<TS>& sm, int w, int lane, 
 // (lane = pixel) only stores s and fac to shared memory, and for every
 // kBwdHits hits (or one fewer, so that the loop has a single place to do it) the
 // lanes regroup, four to a hit, and form the sums over the pixels (reduce_hits),
-// which costs about 18 issue slots a hit where the nine-value butterfly over the
+// which costs about 22 issue slots a hit where the nine-value butterfly over the
 // warp took about 60.  Against the butterfly (B200): 1280x720 fit of 60000 splats at
 // step 25 0.366 -> 0.301 ms, at step 400 0.828 -> 0.504; a million splats at
 // 1920x1080 0.656 -> 0.600.
@@ -619,9 +602,9 @@ __device__ __forceinline__ void reduce_hits(BwdShared<TS>& sm, int w, int lane, 
 // The pixel loop was next: of some 70 issue slots a hit, half went to tests and
 // selects on the ALU pipe, which issues at half rate.  Splats that cannot reach alpha
 // 0.99 and whose conic is not nearly singular ("plain", nearly all) need a test of alpha
-// and one of the pixel's last contributor, and no other select.  With the moments
-// of reduce_hits: step 4 of the 1280x720 fit 0.258 -> 0.214 ms, the million splats
-// 0.525 -> 0.511 (there the warps of a tile wait for one another at every batch).
+// and one of the pixel's last contributor, and no other select.
+// Step 4 of the 1280x720 fit 0.258 -> 0.218 ms; the million splats 0.525 -> 0.491, with
+// batches staged ahead (there the warps of a tile wait for one another at every batch).
 template <int TS, bool kFusedLoss, bool kExact, bool kBatch>
 __global__ void __launch_bounds__(Lay<TS>::kThreads, Lay<TS>::kMinBlocksBwd)
     composite_bwd_kernel(const float4* __restrict__ ra, const float4* __restrict__ rb,
@@ -694,13 +677,8 @@ __global__ void __launch_bounds__(Lay<TS>::kThreads, Lay<TS>::kMinBlocksBwd)
   reinterpret_cast<float2*>(sm.gg[w])[pixel_slot(lane) / 2] = gg;
   reinterpret_cast<float2*>(sm.gb[w])[pixel_slot(lane) / 2] = gb;
   const bool safe_pixels = __all_sync(0xffffffffu, finite);
-  {
-    const float y1 = __shfl_sync(0xffffffffu, m.py[0], 8);
-    const float y5 = __shfl_sync(0xffffffffu, m.py[1], 8);
-    if (lane < 8) reinterpret_cast<float*>(sm.nx[w])[lane] = -m.px;
-    if ((lane & 7) == 0) sm.row[w][lane >> 3] = make_float2(y1 - m.py[0], y5 - m.py[1]);
-    if (lane == 0) sm.ny[w] = make_float2(-y1, -y5);
-  }
+  if (lane < 8) reinterpret_cast<float*>(sm.nx[w])[lane] = -m.px;
+  if ((lane & 7) == 0) sm.ny[w][lane >> 3] = make_float2(-m.py[0], -m.py[1]);
   const int32_t warp_final = warp_max(my_final);
   // Pairs after the tile's last contributing splat reach no pixel: the list
   // ends there for the backward, and no record is written for them (their

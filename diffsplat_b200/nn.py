@@ -157,12 +157,24 @@ class Conv3x3:
         rows and addresses, counts that fit 32 bits.  Measured against im2col +
         GEMM (B200, forward + backward): 64 -> 128 channels, stride 2, 8 x 256 x 256: 2.02 -> 0.25 ms;
         256 -> 256, 32 x 64 x 64: 6.13 -> 0.57 ms.  What it does not take (the
-        weight gradient of a 3-channel layer above all) goes through im2col."""
+        weight gradient of a 3-channel layer above all) goes through im2col, and so
+        does what does not fit the layer (other channel counts, types or numbers of
+        pixels): the kernels get bare pointers, the GEMM checks its shapes."""
         x = tensors[0]
         return ((self.cin == 32 or self.cin % 64 == 0 or (rgb and self.cin == 3))
-                and self.cout % 8 == 0 and max(self.cin, self.cout) <= 1 << 16 and x[..., 0].numel() < 1 << 30
+                and self.cout % 8 == 0 and max(self.cin, self.cout) <= 1 << 16
+                and x.shape[-1] == self.cin and x[..., 0].numel() < 1 << 30
+                and all(t is None or t.dtype == torch.bfloat16 for t in tensors)
                 and all(t is None or (t.data_ptr() % 16 == 0 and t.is_contiguous())
                         for t in (self.w16, self.b, self.gw, *tensors)))
+
+    def _implicit_backward(self, dz2, z_prev):
+        """The same for the backward of the last forward with gradient rows dz2."""
+        if self.col is not None:
+            return False
+        B, H, W, _ = self.in_shape
+        pixels = B * ((H - 1) // self.stride + 1) * ((W - 1) // self.stride + 1)
+        return dz2.shape[0] == pixels and self._implicit(self.x, dz2, z_prev)
 
     def forward(self, gemm, x, keep=False):
         """x [B, H, W, Cin] BF16 -> (z, y) [B, Ho, Wo, Cout] (y = gelu(z) BF16, or
@@ -199,7 +211,7 @@ class Conv3x3:
         M = dz.numel() // self.cout
         dz2 = dz.reshape(M, self.cout)
         self.gb.copy_(colsum(dz2))
-        if self.col is None and self._implicit(self.x, dz2, z_prev):
+        if self._implicit_backward(dz2, z_prev):
             shape = (*self.in_shape, self.stride)
             ws = None
             need = L.lib().ds_conv3x3_wgrad_workspace(*shape, self.kp, self.cout)
@@ -214,7 +226,7 @@ class Conv3x3:
                    self.cout, _p(z_prev), dx.data_ptr(), gemm.err.data_ptr(), _s())
             return dx
         col = self.col
-        if col is None:  # three channels, or an address the tensor maps do not take
+        if col is None:  # three channels, or gradients that ds_conv3x3_* do not take
             col, _ = im2col(self.x, self.stride, self.kp)
         dzt = transpose(dz2)              # [Cout, M]
         colt = transpose(col)             # [Kp, M]

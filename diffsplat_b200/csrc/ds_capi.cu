@@ -180,6 +180,7 @@ int ds_raster_set_grad_mode(ds_raster* r, int mode) {
 
 int ds_raster_forward(ds_raster* r, const ds_splat2d* in, float* out_rgb, ds_stream stream) {
   if (!r || !s2_ok(in) || !out_rgb || in->count > r->rb.max_splats) return DS_ERR_ARG;
+  if (r->rb.tiles <= 0) return DS_ERR_STATE;  // a resize failed
   cudaStream_t s = (cudaStream_t)stream;
   DS_TRY(ds::raster_prepare_from_splat2d(r->rb, *in, s));
   DS_TRY(ds::raster_build_lists(r->rb, in->count, s, nullptr, true));
@@ -192,6 +193,7 @@ int ds_raster_backward(ds_raster* r, const ds_splat2d* in, const float* grad_rgb
                        const ds_splat2d* grad_in, ds_stream stream) {
   if (!r || !s2_ok(in) || !grad_rgb || !s2_ok(grad_in) || in->count != r->last_count)
     return DS_ERR_ARG;
+  if (r->rb.tiles <= 0) return DS_ERR_STATE;
   cudaStream_t s = (cudaStream_t)stream;
   DS_TRY(ds::raster_composite_backward(r->rb, nullptr, grad_rgb, nullptr, s));
   DS_TRY(ds::raster_reduce_grads(r->rb, *grad_in, in->count, s));

@@ -579,14 +579,8 @@ static int alloc_tile_lists(RasterBuffers& rb, const InstGeom* inst = nullptr) {
     return tile_bins_alloc(rb, inst);
   }
   release(rb.rect_sorted);
-  if (!rb.tile_k0) {
-    const size_t c = (size_t)rb.cap;
-    DS_TRY(alloc(&rb.tile_k0, c));
-    DS_TRY(alloc(&rb.tile_k1, c));
-    DS_TRY(alloc(&rb.tile_v0, c));
-    DS_TRY(alloc(&rb.tile_v1, c));
-    DS_TRY(alloc(&rb.emit_splat, c));
-  }
+  for (uint32_t** p : {&rb.tile_k0, &rb.tile_k1, &rb.tile_v0, &rb.tile_v1, &rb.emit_splat})
+    if (!*p) DS_TRY(alloc(p, (size_t)rb.cap));
   if (radix_only || rb.tiles <= 0 || rb.tiles > kCountSortMaxTiles) return DS_OK;
   // one chunk per 2 x 148 SMs, at least 512 pairs each
   rb.count_chunks = (int)std::max<int64_t>(1, std::min<int64_t>(kSortBlocks, (rb.cap + 511) / 512));
@@ -632,21 +626,26 @@ int raster_alloc_batch(RasterBuffers& rb, int64_t pixels, int tiles, int tile_si
   return alloc_tile_lists(rb, inst);
 }
 
-int raster_resize(RasterBuffers& rb, int width, int height) {
-  if (width <= 0 || height <= 0) return DS_ERR_ARG;
-  if (width == rb.width && height == rb.height) return DS_OK;
+// Everything that depends on the grid.
+static void release_grid(RasterBuffers& rb) {
   release(rb.ranges);
   release(rb.tile_bound);
   release(rb.tile_order);
   release(rb.alphas);
   release(rb.last_ids);
   release(rb.loss_partials);
+  release(rb.rect_sorted);
+  release(rb.tile_hist);
+  release(rb.tile_totals);
+  rb.width = rb.height = rb.ntx = rb.nty = rb.tiles = 0;
+}
+
+static int alloc_grid(RasterBuffers& rb, int width, int height) {
   rb.width = width;
   rb.height = height;
   rb.ntx = (width + kTile - 1) / kTile;
   rb.nty = (height + kTile - 1) / kTile;
   rb.tiles = rb.ntx * rb.nty;
-  if (rb.ntx > 65535 || rb.nty > 65535) return DS_ERR_ARG;
   const size_t px = (size_t)width * height;
   DS_TRY(alloc(&rb.ranges, (size_t)rb.tiles));
   DS_TRY(alloc(&rb.tile_bound, (size_t)rb.tiles));
@@ -656,6 +655,17 @@ int raster_resize(RasterBuffers& rb, int width, int height) {
   DS_TRY(alloc(&rb.loss_partials, (size_t)rb.tiles));
   DS_CUDA(cudaMemset(rb.ranges, 0, rb.tiles * sizeof(int2)));
   return alloc_tile_lists(rb);
+}
+
+int raster_resize(RasterBuffers& rb, int width, int height) {
+  if (width <= 0 || height <= 0) return DS_ERR_ARG;
+  if (width == rb.width && height == rb.height) return DS_OK;
+  if ((width - 1) / kTile >= 65535 || (height - 1) / kTile >= 65535) return DS_ERR_ARG;
+  release_grid(rb);
+  const int st = alloc_grid(rb, width, height);
+  // no half of a grid stays: until a resize succeeds there are no tiles (DS_ERR_STATE)
+  if (st != DS_OK) release_grid(rb);
+  return st;
 }
 
 void raster_free(RasterBuffers& rb) {
@@ -684,19 +694,10 @@ void raster_free(RasterBuffers& rb) {
   release(rb.scan.partials);
   release(rb.scan.long_partials);
   release(rb.scalars);
-  release(rb.ranges);
-  release(rb.tile_bound);
-  release(rb.tile_order);
-  release(rb.alphas);
-  release(rb.last_ids);
-  release(rb.loss_partials);
-  release(rb.rect_sorted);
   release(rb.rank);
-  release(rb.tile_hist);
-  release(rb.tile_totals);
   release(rb.bin_chunks);
   release(rb.inst_hist);
-  rb.width = rb.height = 0;
+  release_grid(rb);
 }
 
 int raster_prepare_from_splat2d(RasterBuffers& rb, const ds_splat2d& in, cudaStream_t s) {

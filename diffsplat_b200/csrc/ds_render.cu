@@ -116,7 +116,7 @@ int ds_renderer_set_sh_degree(ds_renderer* r, int degree) {
 int ds_renderer_render(ds_renderer* r, const float pv[16], const float cam_pos[3],
                        ds_stream stream) {
   if (!r || !pv || !cam_pos) return DS_ERR_ARG;
-  if (!r->have_params) return DS_ERR_STATE;
+  if (!r->have_params || r->rb.tiles <= 0 || !r->image) return DS_ERR_STATE;
   cudaStream_t s = (cudaStream_t)stream;
   ds::Camera c;
   for (int k = 0; k < 16; ++k) c.pv[k] = pv[k];
@@ -155,7 +155,7 @@ int ds_renderer_resize(ds_renderer* r, int width, int height) {
   DS_CUDA(cudaDeviceSynchronize());
   DS_TRY(ds::raster_resize(r->rb, width, height));
   cudaFree(r->image);
-  r->image = nullptr;
+  r->image = nullptr;  // renders are refused until there is one again
   DS_CUDA(ds::device_alloc(&r->image, image_floats(width, height) * 4));
   DS_CUDA(cudaMemset(r->image, 0, image_floats(width, height) * 4));
   return DS_OK;

@@ -114,14 +114,13 @@ struct SortScratch {
 // kb may alias kin (the input is consumed by pass 0); ka may not.  *out_k /
 // *out_v receive the buffers holding the result.  vin == nullptr means the
 // input values are 0..n-1.  When gather_src != nullptr, the last pass also
-// writes gather_dst[q] = gather_src[value[q]].  With group set, `group_bits` bits of
-// group[value] are the most significant digits (more passes; the sorted keys are then
-// the groups).
+// writes gather_dst[q] = gather_src[value[q]].  With group set the keys are group[value]
+// (kin is not read).
 int radix_sort_pairs(const uint32_t* kin, const uint32_t* vin, uint32_t* ka, uint32_t* va,
                      uint32_t* kb, uint32_t* vb, uint32_t** out_k, uint32_t** out_v,
                      const uint32_t* n_dev, uint32_t cap, int bits, const uint32_t* gather_src,
                      uint32_t* gather_dst, SortScratch& scratch, cudaStream_t s,
-                     const uint16_t* group = nullptr, int group_bits = 0);
+                     const uint16_t* group = nullptr);
 
 // Exclusive scan of counts gathered through a permutation:
 //   offsets[p] = sum_{q < p} counts[perm[q]]   (64-bit),
@@ -140,10 +139,10 @@ struct ScanScratch {
 // offsets[p] = exclusive sum of counts[perm[q]], q < p.  With long_list set,
 // also long_list[0 .. *n_long) = {perm[p], offsets[p], offsets[p] +
 // counts[perm[p]]} (offsets clamped to cap) for the positions p with
-// counts[perm[p]] > kSerialRecords, ascending in p.  With rect set (the tile rectangles),
-// a splat's count is its rectangle's area, and also
+// counts[perm[p]] > kSerialRecords, ascending in p.  With seg_start set, also
+//   seg_start[perm[p]] = min(offsets[p], cap) where the count is not 0.
+// With rect set too (the tile rectangles), a splat's count is its rectangle's area, and
 //   rect_sorted[p] = rect[perm[p]],
-//   seg_start[perm[p]] = min(offsets[p], cap) where it is not empty,
 //   sc->last_p, last_m: the last p of which any pair fits cap, and how many of its
 //   pairs do (last_p = 0xffffffff: all pairs fit).
 struct DevScalars;
@@ -337,6 +336,9 @@ int raster_build_lists(RasterBuffers& rb, int n, cudaStream_t s, cudaEvent_t* ev
 // from rect_sorted and depth_perm.  tile_bins_pay: whether they are the faster way
 // for this grid and max_splats; inst: the instances of a batch.
 bool tile_bins_pay(const RasterBuffers& rb, const InstGeom* inst);
+// Batches: rect_sorted in the order of depth_perm (by instance, then depth), from
+// seg_start; a splat none of whose pairs fit the capacity gets an empty one.
+int gather_rects(RasterBuffers& rb, int n, cudaStream_t s);
 int tile_bins_alloc(RasterBuffers& rb, const InstGeom* inst);
 int tile_bins(RasterBuffers& rb, int n, cudaStream_t s);
 // Column prefix of the per-chunk counts, ranges and schedule (single instance).

@@ -715,8 +715,7 @@ int raster_build_lists(RasterBuffers& rb, int n, cudaStream_t s, cudaEvent_t* ev
                        bool with_long_list) {
   DevScalars* sc = rb.scalars;
   if (n > 0) {
-    // 1) depth order of the splats: stable sort of (depth bits, id); batches that list
-    //    their tiles by bins: within each instance
+    // 1) depth order of the splats: stable sort of (depth bits, id)
     // 2) offsets of the splats' pairs (and gradient records) in depth order
     const bool bins = rb.rect_sorted != nullptr;
     const bool small = bins && !rb.geom && n <= kSmallSort;
@@ -726,21 +725,33 @@ int raster_build_lists(RasterBuffers& rb, int n, cudaStream_t s, cudaEvent_t* ev
     } else if (small) {
       DS_TRY(cluster_sort(rb, n, s));
     } else {
-      const bool by_instance = bins && rb.geom && rb.instances > 1;
       DS_TRY(radix_sort_pairs(rb.depth_keys, nullptr, rb.depth_k0, rb.depth_v0, rb.depth_k1,
                               rb.depth_v1, &rb.depth_sorted_keys, &rb.depth_perm, &sc->n_splats,
-                              (uint32_t)rb.max_splats, 32, nullptr, nullptr, rb.sort, s,
-                              by_instance ? rb.inst_of_splat : nullptr,
-                              by_instance ? ceil_log2(rb.instances) : 0));
+                              (uint32_t)rb.max_splats, 32, nullptr, nullptr, rb.sort, s));
     }
     if (ev) DS_CUDA(cudaEventRecord(ev[0], s));
+    const bool in_order = bins && !rb.geom;  // of the bins' chunks
     if (!ranked)
       DS_TRY(scan_counts_permuted(rb.counts, rb.depth_perm, (uint32_t)n, rb.emit_offsets,
                                   &sc->n_isects, &sc->n_isects_raw, (uint32_t)rb.cap, &sc->status,
                                   rb.scan, s, with_long_list ? rb.long_list : nullptr, &sc->n_long,
-                                  bins ? rb.rect : nullptr, bins ? rb.rect_sorted : nullptr,
+                                  in_order ? rb.rect : nullptr,
+                                  in_order ? rb.rect_sorted : nullptr,
                                   bins ? rb.seg_start : nullptr, sc));
     if (bins) {
+      if (rb.geom) {
+        // Batches: the pairs past the capacity are the deepest of all instances', as in
+        // the order above; the chunks hold one instance's splats each.
+        if (rb.instances > 1) {
+          uint32_t* other = rb.depth_perm == rb.depth_v0 ? rb.depth_v1 : rb.depth_v0;
+          DS_TRY(radix_sort_pairs(nullptr, rb.depth_perm, rb.depth_k0, other, rb.depth_k1,
+                                  rb.depth_perm, &rb.depth_sorted_keys, &rb.depth_perm,
+                                  &sc->n_splats, (uint32_t)rb.max_splats,
+                                  ceil_log2(rb.instances), nullptr, nullptr, rb.sort, s,
+                                  rb.inst_of_splat));
+        }
+        DS_TRY(gather_rects(rb, n, s));
+      }
       // 3) tile lists
       if (ev) DS_CUDA(cudaEventRecord(ev[1], s));
       DS_TRY(tile_bins(rb, n, s));

@@ -401,7 +401,7 @@ __global__ void __launch_bounds__(kThreads)
       excl += c[k];
       if (seg_start && c[k]) {
         seg_start[pi[k]] = (uint32_t)(s0 < cap ? s0 : cap);
-        if (s0 < cap && excl >= cap) {
+        if (rect_sorted && s0 < cap && excl >= cap) {
           sc->last_p = p;
           sc->last_m = (uint32_t)(cap - s0);
         }
@@ -424,10 +424,9 @@ __global__ void __launch_bounds__(kThreads)
 int radix_sort_pairs(const uint32_t* kin, const uint32_t* vin, uint32_t* ka, uint32_t* va,
                      uint32_t* kb, uint32_t* vb, uint32_t** out_k, uint32_t** out_v,
                      const uint32_t* n_dev, uint32_t cap, int bits, const uint32_t* gather_src,
-                     uint32_t* gather_dst, SortScratch& scratch, cudaStream_t s, const uint16_t* group,
-                     int group_bits) {
-  const int key_passes = bits <= 0 ? 1 : (bits + 7) / 8;
-  const int passes = key_passes + (group ? (group_bits + 7) / 8 : 0);
+                     uint32_t* gather_dst, SortScratch& scratch, cudaStream_t s,
+                     const uint16_t* group) {
+  const int passes = bits <= 0 ? 1 : (bits + 7) / 8;
   // One CTA per 2048-item tile of the capacity, at most kSortBlocks.
   const uint64_t tiles = ((uint64_t)cap + kSortTileItems - 1) / kSortTileItems;
   const int blocks = (int)(tiles < 1 ? 1 : (tiles > (uint64_t)kSortBlocks ? kSortBlocks : tiles));
@@ -436,15 +435,14 @@ int radix_sort_pairs(const uint32_t* kin, const uint32_t* vin, uint32_t* ka, uin
   uint32_t* dst_k = ka;
   uint32_t* dst_v = va;
   for (int p = 0; p < passes; ++p) {
-    const uint16_t* digits = p < key_passes ? nullptr : group;
-    const int shift = 8 * (p < key_passes ? p : p - key_passes);
+    const int shift = 8 * p;
     const bool last = p == passes - 1;
-    DS_CUDA(launch_pdl(radix_hist_kernel, dim3(blocks), dim3(kThreads), 0, s, src_k, src_v, digits,
+    DS_CUDA(launch_pdl(radix_hist_kernel, dim3(blocks), dim3(kThreads), 0, s, src_k, src_v, group,
                        n_dev, cap, shift, scratch.hist));
     DS_CUDA(launch_pdl(scan_hist_kernel, dim3(256 / kWarps), dim3(kThreads), 0, s, scratch.hist,
                        blocks));
     DS_CUDA(launch_pdl(radix_scatter_kernel, dim3(blocks), dim3(kThreads), 0, s, src_k, src_v,
-                       digits, src_v == nullptr ? 1 : 0, dst_k, dst_v, n_dev, cap, shift,
+                       group, src_v == nullptr ? 1 : 0, dst_k, dst_v, n_dev, cap, shift,
                        (const uint32_t*)scratch.hist, last ? gather_src : nullptr,
                        last ? gather_dst : nullptr));
     *out_k = dst_k;

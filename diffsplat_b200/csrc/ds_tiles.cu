@@ -16,8 +16,8 @@
 // Counting is a popcount, a splat's rank in a tile the bits below it.  No (tile,
 // splat) pair exists before it is written to its place.
 //
-// Batches: a chunk holds splats of one instance (the depth order is by instance
-// first) and only that instance's bins are walked.
+// Batches: the splats are ordered by instance first, a chunk holds splats of one
+// instance, and only that instance's bins are walked.
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -128,14 +128,15 @@ __global__ void __launch_bounds__(kBinThreads) tile_bins_kernel(const BinArgs g)
   if ((int)blockIdx.y * kBinWarps >= bins) return;  // uniform
   const int count = hi - lo;
   // Pairs past the capacity are dropped in depth order: last_p is the splat whose
-  // pairs fill it, with last_m of them kept.
+  // pairs fill it, with last_m of them kept.  (Batches: its position in their order; what
+  // is behind it has an empty rectangle.)
   const uint32_t last_p = g.sc->last_p, last_m = g.sc->last_m;
   for (int k = threadIdx.x; k < ((count + 127) & ~127); k += kBinThreads) {
     uint32_t b = 0x7f7f7f7fu;  // reaches no bin
     if (k < count) {
       const ushort4 r = g.rect[lo + k];
       srect[k] = r;
-      if (r.x <= r.y && (uint32_t)(lo + k) <= last_p)
+      if (r.x <= r.y && (g.chunks || (uint32_t)(lo + k) <= last_p))
         b = bin_bytes(r.x / kBin, r.z / kBin, r.y / kBin, r.w / kBin);
       if (kWrite) sid[k] = g.perm[lo + k];
     }
@@ -228,6 +229,28 @@ __global__ void __launch_bounds__(kBinThreads) tile_bins_kernel(const BinArgs g)
       if (in1) g.hist[row + t1] = at1;
     }
   }
+}
+
+__global__ void __launch_bounds__(kBinThreads)
+    gather_rects_kernel(const ushort4* __restrict__ rect, const uint32_t* __restrict__ perm,
+                        const uint32_t* __restrict__ seg_start, int n, uint32_t cap,
+                        ushort4* __restrict__ rect_sorted, DevScalars* __restrict__ sc) {
+  pdl_wait();
+  const int p = blockIdx.x * kBinThreads + threadIdx.x;
+  if (p >= n) return;
+  const uint32_t id = perm[p];
+  ushort4 r = rect[id];
+  const uint32_t area = (uint32_t)((int)r.y - (int)r.x + 1) * (uint32_t)((int)r.w - (int)r.z + 1);
+  const uint32_t room = area ? cap - seg_start[id] : 0u;  // (seg_start stops at cap)
+  if (area > room) {
+    if (room == 0u) {
+      r = make_ushort4(1, 0, 1, 0);
+    } else {  // at most one splat
+      sc->last_p = (uint32_t)p;
+      sc->last_m = room;
+    }
+  }
+  rect_sorted[p] = r;
 }
 
 // Longest-first schedule of the composite CTAs: tiles bucketed by their list
@@ -467,6 +490,13 @@ int tile_bins_alloc(RasterBuffers& rb, const InstGeom* inst) {
   }
   DS_CUDA(device_alloc(&rb.tile_hist, std::max<size_t>(1, values) * 4));
   DS_CUDA(device_alloc(&rb.tile_totals, (size_t)std::max(1, rb.tiles) * 4));
+  return DS_OK;
+}
+
+int gather_rects(RasterBuffers& rb, int n, cudaStream_t s) {
+  DS_CUDA(launch_pdl(gather_rects_kernel, dim3((n + kBinThreads - 1) / kBinThreads),
+                     dim3(kBinThreads), 0, s, rb.rect, rb.depth_perm, rb.seg_start, n,
+                     (uint32_t)rb.cap, rb.rect_sorted, rb.scalars));
   return DS_OK;
 }
 

@@ -343,7 +343,8 @@ typedef struct ds_batch_instance {
 typedef struct ds_batch_config {
   int32_t instances;
   int32_t sh_degree;
-  int64_t max_isects; /* all instances together; <= 0: 2^25 */
+  int64_t max_isects; /* all instances together (<= 0: 2^25); beyond it the deepest pairs of
+                         all instances are dropped and ds_batch_status says so */
   float lr_pos, lr_scale, lr_rot, lr_sh_dc, lr_sh_rest, lr_opacity;
   float beta1, beta2, epsilon;
   int32_t storage;

@@ -21,7 +21,6 @@
 #include <stdlib.h>
 #include <string.h>
 
-#include <atomic>
 #include <type_traits>
 
 #include "ds_common.cuh"
@@ -894,17 +893,6 @@ __global__ void __launch_bounds__(Lay<TS>::kThreads, Lay<TS>::kMinBlocksBwd)
       for (int q = h; q < 9; q += kSplit) dst[q] = v[q / kSplit];
     }
   }
-}
-
-// Lets a kernel use `bytes` of dynamic shared memory, once per device (`set`: the
-// devices done).
-template <class K>
-void allow_smem(K kernel, int bytes, std::atomic<uint64_t>& set) {
-  int dev = 0;
-  if (bytes <= 48 * 1024 || cudaGetDevice(&dev) != cudaSuccess) return;
-  if (dev < 64 && (set.load() >> dev & 1u)) return;
-  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  if (dev < 64) set.fetch_or(1ull << dev);
 }
 
 const int32_t* schedule(const RasterBuffers& rb) {

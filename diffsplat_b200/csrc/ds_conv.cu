@@ -35,7 +35,6 @@
 // Every mbarrier wait is bounded as in ds_gemm.cu: on a timeout the CTA sets the
 // error word, lets what it issued land, frees its TMEM and returns.
 #include <algorithm>
-#include <mutex>
 
 #include "ds_common.cuh"
 #include "ds_internal.h"
@@ -945,13 +944,8 @@ int sm_count() {
 template <int BN, int MODE, int G, int EPI>
 int launch_conv(const ConvMaps& maps, const ConvArgs& g, cudaStream_t s) {
   using S = ConvShape<BN, MODE, G, EPI>;
-  static std::once_flag once;
-  static cudaError_t attr = cudaSuccess;
-  std::call_once(once, [] {
-    attr = cudaFuncSetAttribute(conv3x3_kernel<BN, MODE, G, EPI>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::kSmem);
-  });
-  DS_CUDA(attr);
+  static std::atomic<uint64_t> set{0};
+  DS_CUDA(allow_smem(conv3x3_kernel<BN, MODE, G, EPI>, S::kSmem, set));
   const int grid = std::min(g.first[g.classes], sm_count());
   conv3x3_kernel<BN, MODE, G, EPI><<<grid, S::kThreads, S::kSmem, s>>>(maps, g);
   return cuda_status(cudaGetLastError());

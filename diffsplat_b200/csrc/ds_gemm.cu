@@ -25,7 +25,6 @@
 #include <stdint.h>
 
 #include <algorithm>
-#include <mutex>
 
 #include "ds_common.cuh"
 #include "ds_internal.h"
@@ -236,13 +235,8 @@ template <int BN, int EPI>
 int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, const GemmArgs& g, int splits,
                 cudaStream_t s) {
   constexpr size_t smem = 1024 + kStages * (kBM * kBK * 2 + BN * kBK * 2) + 256;
-  static std::once_flag once;
-  static cudaError_t attr = cudaSuccess;
-  std::call_once(once, [] {
-    attr = cudaFuncSetAttribute(gemm_bf16_tn_kernel<BN, EPI>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  });
-  DS_CUDA(attr);
+  static std::atomic<uint64_t> set{0};
+  DS_CUDA(allow_smem(gemm_bf16_tn_kernel<BN, EPI>, smem, set));
   dim3 grid((g.M + kBM - 1) / kBM, (g.N + BN - 1) / BN, splits);
   gemm_bf16_tn_kernel<BN, EPI><<<grid, kGemmThreads, smem, s>>>(ma, mb, g);
   return cuda_status(cudaGetLastError());

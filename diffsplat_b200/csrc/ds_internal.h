@@ -6,6 +6,7 @@
 #include <utility>
 
 #include "../../include/diffsplat_b200.h"
+#include "ds_smem.h"
 
 namespace ds {
 

@@ -587,15 +587,8 @@ static int alloc_tile_lists(RasterBuffers& rb, const InstGeom* inst = nullptr) {
   DS_TRY(alloc(&rb.tile_hist, (size_t)rb.count_chunks * rb.tiles));
   DS_TRY(alloc(&rb.tile_totals, (size_t)rb.tiles));
   // the scatter's shared memory (up to 160 KB) is opted into once per device
-  static uint64_t smem_set = 0;
-  int dev = 0;
-  DS_CUDA(cudaGetDevice(&dev));
-  if (dev >= 64 || !(smem_set >> dev & 1u)) {
-    const int most = kCountSortMaxTiles * (4 + 2 * kScatterWarps) + 64;
-    DS_CUDA(cudaFuncSetAttribute(tile_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 most));
-    if (dev < 64) smem_set |= 1ull << dev;
-  }
+  static std::atomic<uint64_t> set{0};
+  DS_CUDA(allow_smem(tile_scatter_kernel, kCountSortMaxTiles * (4 + 2 * kScatterWarps) + 64, set));
   return DS_OK;
 }
 

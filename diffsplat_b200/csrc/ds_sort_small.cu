@@ -16,8 +16,6 @@
 // distributed shared memory (item by item they took twice the time).
 #include <cooperative_groups.h>
 
-#include <atomic>
-
 #include "ds_common.cuh"
 #include "ds_internal.h"
 
@@ -283,13 +281,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 
 int small_sort_setup() {
   static std::atomic<uint64_t> set{0};
-  int dev = 0;
-  DS_CUDA(cudaGetDevice(&dev));
-  if (dev < 64 && (set.load() >> dev & 1u)) return DS_OK;
-  DS_CUDA(cudaFuncSetAttribute(cluster_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)sizeof(SortShared)));
-  if (dev < 64) set.fetch_or(1ull << dev);
-  return DS_OK;
+  return cuda_status(allow_smem(cluster_sort_kernel, sizeof(SortShared), set));
 }
 
 bool rank_sort_fits(const RasterBuffers& rb, int n) {

@@ -502,7 +502,8 @@ def normalize_scene(rec: np.ndarray, scene_scale: float = 1.0) -> np.ndarray:
 class Batch:
     """Owns a ds_batch: many independent fitting instances stepped together.
 
-    sizes: [(width, height, splat count)] per instance."""
+    sizes: [(width, height, splat count)] per instance.  ppt (pixels per thread, 1 or 2)
+    is accepted and has no effect: the composite kernels have one layout."""
 
     def __init__(self, sizes, sh_degree: int = 0, lrs=None, max_isects: int = 0,
                  storage: int = L.DS_STORAGE_BF16, tile_size: int = 16, ppt: int = 1,

@@ -1,7 +1,6 @@
 """Autotuner of the batched fitter: picks the composite tile size (8, 16 or 32
-pixels), pixels per thread (1 or 2) and CTA schedule (longest tile list first
-or raster order) for a given batch by timing a few steps of each candidate on
-the batch's own inputs with CUDA events.
+pixels) and CTA schedule (longest tile list first or raster order) for a given batch by
+timing a few steps of each candidate on the batch's own inputs with CUDA events.
 
     best, table = tune_batch(sizes, setup, sh_degree=0)
     batch = api.Batch(sizes, **best)
@@ -17,7 +16,7 @@ from . import _lib as L
 from . import api
 
 TILE_SIZES = (8, 16, 32)
-PPTS = (1, 2)
+PPTS = (1,)  # accepted values 1 and 2 run the same kernels: one is timed
 SCHEDULES = (L.DS_SCHEDULE_LONGEST_FIRST, L.DS_SCHEDULE_RASTER)
 
 

@@ -332,10 +332,9 @@ int ds_fitter_density_stats(ds_fitter *f, float **grad_accum, uint32_t **visible
  * step is captured once into a CUDA graph.  Splats of all instances share one
  * parameter SoA (ds_batch_params, count = all splats; instance k owns columns
  * [first, first + count) of ds_batch_instance_range); each instance has its
- * own target, camera, image and loss.  tile_size 8, 16 or 32 and
- * pixels_per_thread 1 or 2 select the composite kernels (16 is the
- * reference's tile; other sizes change which splats a tile lists, not the
- * compositing rule).  Default storage is BF16 (FP32 masters). */
+ * own target, camera, image and loss.  tile_size 8, 16 or 32 selects the
+ * composite kernels (16 is the reference's tile; other sizes change which
+ * splats a tile lists, not the compositing rule).  Default storage is BF16 (FP32 masters). */
 typedef struct ds_batch ds_batch;
 typedef struct ds_batch_instance {
   int32_t width, height, count, reserved;
@@ -352,7 +351,7 @@ typedef struct ds_batch_config {
   int32_t grad_mode;
   int32_t schedule;
   int32_t tile_size;         /* 8, 16 or 32 */
-  int32_t pixels_per_thread; /* 1 or 2 */
+  int32_t pixels_per_thread; /* 1 or 2; without effect (one composite layout) */
 } ds_batch_config;
 int ds_batch_default_config(ds_batch_config *cfg);
 int ds_batch_create(const ds_batch_config *cfg, const ds_batch_instance *instances,

@@ -210,18 +210,32 @@ __device__ __forceinline__ float2 pair_opacity(float2 dist2, const SplatRec& r) 
   return mul2(make_float2(r.co.z, r.co.w), make_float2(exp2f(p.x), exp2f(p.y)));
 }
 
+// Mask bits of a staged splat above the warps': its colour may be infinite, NaN or near
+// overflow; it is not plain (the sign bit).
+constexpr uint32_t kWild = 0x40000000u, kNotPlain = 0x80000000u;
+
 // A warp's hits of a staged batch, listed in order: the splats l of [from, n)
 // whose mask has the warp's bit, with the mask's sign bit.  Padded with `none` to an
-// even count; returns the count before padding.
+// even count; returns the count before padding.  A wild splat may leave an infinite or
+// NaN sum in the pixels that it covers, which the hits after it that do not cover them must
+// not see: it sets *spoilt, and they too get the sign bit.
 __device__ __forceinline__ int list_hits(const uint32_t* mask, int w, int lane, int from, int n,
-                                         int none, int* list) {
+                                         int none, int* list, uint32_t* spoilt) {
   int count = 0;
+  const uint32_t lt = (1u << lane) - 1u;
   for (int k = 0; k < n; k += 32) {
     const int l = k + lane;
     const uint32_t mk = l >= from && l < n ? mask[l] : 0u;
     const bool hit = (mk >> w) & 1u;
     const uint32_t word = __ballot_sync(0xffffffffu, hit);
-    if (hit) list[count + __popc(word & ((1u << lane) - 1u))] = l | (int)(mk & 0x80000000u);
+    const uint32_t wild = __ballot_sync(0xffffffffu, hit && (mk & kWild));
+    const bool odd = (mk & kNotPlain) || *spoilt || (wild & lt);
+    if (hit) list[count + __popc(word & lt)] = odd ? l | (int)kNotPlain : l;
+    if (wild) {
+      __syncwarp();
+      if (lane == 0) *spoilt = 1u;
+      __syncwarp();
+    }
     count += __popc(word);
   }
   if (lane == 0) list[count] = none;
@@ -475,10 +489,11 @@ struct BwdShared {
   float4 fac[NW][kBwdHits * kPitch / 4];  // per (hit, pixel): alpha T
   float part[NW][B * 9];       // per-warp gradient of each batch splat
   uint32_t rec[B];             // record index of each batch splat
-  uint32_t mask[B];            // warps whose block the splat can reach; bit 31: not plain
+  uint32_t mask[B];            // warps whose block the splat can reach, kWild, kNotPlain
   uint32_t got[NW][B / 32];    // batch splats with a partial from the warp
   int2 list[NW][B / 2 + 1];    // the warp's hits of the batch
   int32_t final_id[NW];
+  uint32_t spoilt[NW];         // a wild splat was among the warp's hits
 };
 
 // Slot of lane l's pixel pair (column l % 8, rows l / 8 and l / 8 + 4) in a hit's row
@@ -682,7 +697,7 @@ __global__ void __launch_bounds__(Lay<TS>::kThreads, Lay<TS>::kMinBlocksBwd)
   // Pairs after the tile's last contributing splat reach no pixel: the list
   // ends there for the backward, and no record is written for them (their
   // consumers skip them by tile_bound).
-  if (lane == 0) sm.final_id[w] = warp_final;
+  if (lane == 0) sm.final_id[w] = warp_final, sm.spoilt[w] = 0u;
   __syncthreads();
   int32_t tile_final = sm.final_id[0];
 #pragma unroll
@@ -757,9 +772,9 @@ __global__ void __launch_bounds__(Lay<TS>::kThreads, Lay<TS>::kMinBlocksBwd)
           sm.splat[l].set(a, b, c, 0);
           sm.rec[l] = pf_rec[r];
           // plain: cannot reach alpha 0.99, and nothing about it overflows
-          const bool plain = definite(b) && b.w <= kMaxAlpha && fabsf(c.x) <= 1e15f &&
-                             fabsf(c.y) <= 1e15f && fabsf(c.z) <= 1e15f;
-          if (!plain) mk |= 0x80000000u;
+          const bool wild = !(fabsf(c.x) <= 1e15f && fabsf(c.y) <= 1e15f && fabsf(c.z) <= 1e15f);
+          if (wild) mk |= kWild;
+          if (wild || !(definite(b) && b.w <= kMaxAlpha)) mk |= kNotPlain;
         }
       }
       if (kSplit == 2) mk |= __shfl_xor_sync(0xffffffffu, mk, 1);  // pairs are adjacent lanes
@@ -769,7 +784,7 @@ __global__ void __launch_bounds__(Lay<TS>::kThreads, Lay<TS>::kMinBlocksBwd)
     __syncthreads();
     const int t_start = max(0, batch_end - warp_final);
     int* const list = reinterpret_cast<int*>(sm.list[w]);
-    const int hits = list_hits(sm.mask, w, lane, t_start, bs, B, list);
+    const int hits = list_hits(sm.mask, w, lane, t_start, bs, B, list, &sm.spoilt[w]);
     if (lane < B / 32) sm.got[w][lane] = 0u;
     __syncwarp();
     int count = 0, slot = 0;  // hits stored; the slot of this lane's hit (lane / 4)
@@ -816,7 +831,7 @@ __global__ void __launch_bounds__(Lay<TS>::kThreads, Lay<TS>::kMinBlocksBwd)
       bool any[2];
       if (safe_pixels && (pair.x | pair.y) >= 0) {
         // Plain splats: alpha = opacity exp() where it passes, 0 elsewhere, which
-        // leaves T and acc as they are.
+        // leaves T and acc as they are, and s at 0 while acc is finite.
 #pragma unroll
         for (int g = 0; g < 2; ++g) {
           const int t = g ? pair.y : pair.x, id = batch_end - t;

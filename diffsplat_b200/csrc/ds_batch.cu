@@ -89,7 +89,7 @@ static void launch_batch_preprocess(ds_batch* b, const Soa<T>& R, cudaStream_t s
   const unsigned blocks = (unsigned)((b->total_splats + kPreThreads - 1) / kPreThreads);
   fit_preprocess_kernel<T, TS, true><<<blocks, kPreThreads, 0, s>>>(
       b->P, R, b->cfg.sh_degree, b->cams, 0, 0, 0, 0, rb.rec_a, rb.rec_b, rb.rec_c,
-      rb.rect, rb.counts, rb.depth_keys, rb.scalars, b->inst_of_splat, b->geom_dev);
+      rb.rec_idet, rb.rect, rb.counts, rb.depth_keys, rb.scalars, b->inst_of_splat, b->geom_dev);
 }
 
 template <typename T>

@@ -301,6 +301,7 @@ constexpr uint32_t kInvisibleKey = 0xbf800000u;
 //   A = {ndc x, ndc y, cull half-width x, cull half-width y}
 //   B = {conic xx, conic xy, conic yy, opacity}
 //   C = {r, g, b, sigma cut}
+// plus idet (1/det of Cov2D) used only by the backward.
 // The conic is computed with the reference's formula (tile_rasterize_layer.cu:
 // 260-272) so the per-pixel Gaussian value is bit-identical.  The culling box
 // and sigma cut are conservative bounds of the region where the reference's
@@ -309,6 +310,7 @@ constexpr uint32_t kInvisibleKey = 0xbf800000u;
 // ---------------------------------------------------------------------------
 struct Record {
   float4 a, b, c;
+  float idet;
 };
 
 __device__ __forceinline__ Record make_record(float x, float y, float cxx, float cxy, float cyy,
@@ -319,6 +321,7 @@ __device__ __forceinline__ Record make_record(float x, float y, float cxx, float
   float icxx = cyy * idet;
   float icxy = -cxy * idet;
   float icyy = cxx * idet;
+  rec.idet = idet;
   // alpha = min(0.99, o*exp(-sigma)) >= 1/255 needs sigma <= ln(255 o); 0.01 of slack
   // in sigma covers the approximate exp and every rounding step.
   float cut = logf(255.f * opac) + 0.01f;

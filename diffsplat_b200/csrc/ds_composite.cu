@@ -150,6 +150,7 @@ __device__ __forceinline__ bool ellipse_hits(const float4& a, const float4& b, f
 // gathers overlap the current batch's compositing.
 struct Staged {
   float4 a, b, c;
+  float idet;  // backward
   bool ok;
 };
 
@@ -161,14 +162,14 @@ struct SplatRec {
   float4 ab;      // conic a, a, 2b, 2b
   float4 co;      // conic c, c, opacity, opacity
   float4 rg;      // r, r, g, g
-  float4 blue;    // b, b, -, - (forward: the splat's sorted index as bits)
+  float4 blue;    // b, b, extra, -: the splat's sorted index as bits; backward: 1 / det of Cov2D
   __device__ __forceinline__ void set(const float4& a, const float4& b, const float4& c,
-                                      int index) {
+                                      float extra) {
     pos = make_float4(a.x, a.x, a.y, a.y);
     ab = make_float4(b.x, b.x, 2.f * b.y, 2.f * b.y);
     co = make_float4(b.z, b.z, b.w, b.w);
     rg = make_float4(c.x, c.x, c.y, c.y);
-    blue = make_float4(c.z, c.z, __int_as_float(index), 0.f);
+    blue = make_float4(c.z, c.z, extra, 0.f);
   }
   // opacity 0: skipped at every pixel
   __device__ __forceinline__ void set_none() {
@@ -382,7 +383,7 @@ __global__ void __launch_bounds__(32 * kFwdWarps, DS_FWD_MIN_BLOCKS)
     const int n = __popc(word);
     bool odd = false;  // a colour that is not finite, a conic that may go negative
     if (mine) {
-      hit[__popc(word & ((1u << lane) - 1u))].set(pf.a, pf.b, pf.c, b0 + lane);
+      hit[__popc(word & ((1u << lane) - 1u))].set(pf.a, pf.b, pf.c, __int_as_float(b0 + lane));
       odd = !(finite3(pf.c.x, pf.c.y, pf.c.z) && definite(pf.b));
     }
     // the last group is filled with splats of opacity 0
@@ -510,32 +511,31 @@ __device__ __forceinline__ int pixel_slot(int lane) {
 // w = b dx + c dy,
 //   d dist2 / d(ndc x, ndc y) = (2u, 2w)
 //   d dist2 / d(cov xx, xy, yy) = -u^2, -2uw, -w^2
-// (uw = b dist2 + dx dy / det written without the cancelling difference), and s
-// = -2 dL/d(dist2).  u and w are formed at every pixel, from its own dx and dy: sums of s u^2,
-// s u w and s w^2 rebuilt from moments of s about a row cancel for splats thinner than a
-// pixel, to a relative error of 3e-6 at sigma = 0.1 pixels and 1e-3 at 0.003, where this
+// and s = -2 dL/d(dist2).  u and w are formed at every pixel, from its own dx and dy: sums of
+// s u^2, s u w and s w^2 rebuilt from moments of s about a row cancel for splats thinner than
+// a pixel, to a relative error of 3e-6 at sigma = 0.1 pixels and 1e-3 at 0.003, where this
 // form stays at 1e-7, and saved little (1280x720 fit, step 4, 0.218 -> 0.214 ms; a million
 // splats at 1920x1080 0.491 -> 0.484, B200).  kSafe also leaves out what s = 0 or fac = 0
 // multiplies, as it may be infinite or NaN.
-template <bool kSafe, int TS>
-__device__ __forceinline__ void reduce_hits(BwdShared<TS>& sm, int w, int lane, int count,
+// The sum for cov xy takes u w as b dist2 + dx dy / det, the form that this gradient has always
+// had: for long tilted splats either cancels, to as much as 1e-4 of a sum, and only the
+// same products give the same values (u w would save 0.03 of 0.79 ms of that fit's step).
+template <bool kSafe, class Sh>
+__device__ __forceinline__ void reduce_hits(Sh& sm, int w, int lane, int count,
                                             int slot) {
-  using Sh = BwdShared<TS>;
   const int h = lane >> 2, q = lane & 3;
   const SplatRec& hit = sm.splat[slot];
   const float2 ca = hit.conic_a(), cb = mul2(hit.conic_2b(), both(0.5f)), cc = hit.conic_c();
-  const float2 nx = sm.nx[w][q];
+  const float2 idet = both(hit.blue.z);
+  const float2 dxs[2] = {add2(hit.x(), both(sm.nx[w][q].x)), add2(hit.x(), both(sm.nx[w][q].y))};
   float2 v[9];
 #pragma unroll
   for (int k = 0; k < 9; ++k) v[k] = make_float2(0.f, 0.f);
-  float2 s[4][2];
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
     const int at = at_word(r, q);
-    const float4 s4 = sm.s[w][h * (Sh::kPitch / 4) + at];
     const float4 f4 = sm.fac[w][h * (Sh::kPitch / 4) + at];
     const float4 r4 = sm.gr[w][at], g4 = sm.gg[w][at], b4 = sm.gb[w][at];
-    s[r][0] = make_float2(s4.x, s4.y), s[r][1] = make_float2(s4.z, s4.w);
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
       const float2 f = e ? make_float2(f4.z, f4.w) : make_float2(f4.x, f4.y);
@@ -551,25 +551,26 @@ __device__ __forceinline__ void reduce_hits(BwdShared<TS>& sm, int w, int lane, 
       v[1] = fma2(f, gg, v[1]);
       v[2] = fma2(f, gb, v[2]);
     }
-  }
+    const float4 s4 = sm.s[w][h * (Sh::kPitch / 4) + at];
+    const float2 dy = add2(hit.y(), sm.ny[w][r]);
+    const float2 dyb = mul2(dy, cb), dyc = mul2(dy, cc), dyy = mul2(dy, dy);
 #pragma unroll
-  for (int e = 0; e < 2; ++e) {
-    const float2 dx = add2(hit.x(), both(e ? nx.y : nx.x));
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const float2 dy = add2(hit.y(), sm.ny[w][r]);
-      float2 u = fma2(dx, ca, mul2(dy, cb));
-      float2 t = fma2(dx, cb, mul2(dy, cc));
-      const float2 z = s[r][e];
+    for (int e = 0; e < 2; ++e) {
+      const float2 z = e ? make_float2(s4.z, s4.w) : make_float2(s4.x, s4.y);
+      const float2 dx = dxs[e], xy = mul2(dx, dy);
+      float2 u = fma2(dx, ca, dyb), t = fma2(dx, cb, dyc);
+      const float2 dist2 = fma2(dyy, cc, fma2(mul2(dx, dx), ca, mul2(xy, hit.conic_2b())));
+      float2 x = fma2(cb, dist2, mul2(xy, idet));
       if (kSafe) {
         u.x = z.x != 0.f ? u.x : 0.f, u.y = z.y != 0.f ? u.y : 0.f;
         t.x = z.x != 0.f ? t.x : 0.f, t.y = z.y != 0.f ? t.y : 0.f;
+        x.x = z.x != 0.f ? x.x : 0.f, x.y = z.y != 0.f ? x.y : 0.f;
       }
       const float2 su = mul2(z, u), st = mul2(z, t);
       v[3] = add2(v[3], su);
       v[4] = add2(v[4], st);
       v[5] = fma2(su, u, v[5]);
-      v[6] = fma2(su, t, v[6]);
+      v[6] = fma2(z, x, v[6]);
       v[7] = fma2(st, t, v[7]);
       v[8] = add2(v[8], z);
     }
@@ -622,7 +623,7 @@ __device__ __forceinline__ void reduce_hits(BwdShared<TS>& sm, int w, int lane, 
 template <int TS, bool kFusedLoss, bool kExact, bool kBatch>
 __global__ void __launch_bounds__(Lay<TS>::kThreads, Lay<TS>::kMinBlocksBwd)
     composite_bwd_kernel(const float4* __restrict__ ra, const float4* __restrict__ rb,
-                         const float4* __restrict__ rc,
+                         const float4* __restrict__ rc, const float* __restrict__ ridet,
                          const uint32_t* __restrict__ sorted_splat,
                          const uint32_t* __restrict__ seg_start,
                          const ushort4* __restrict__ rect, const int2* __restrict__ ranges,
@@ -731,6 +732,7 @@ __global__ void __launch_bounds__(Lay<TS>::kThreads, Lay<TS>::kMinBlocksBwd)
         pf[r].a = ra[g];
         pf[r].b = rb[g];
         pf[r].c = rc[g];
+        pf[r].idet = ridet[g];
         if ((threadIdx.x + r * NT) % kSplit == 0) {
           // the pair's emission index: the splat's first one plus the tile's
           // row-major index in the splat's tile rectangle
@@ -769,7 +771,7 @@ __global__ void __launch_bounds__(Lay<TS>::kThreads, Lay<TS>::kMinBlocksBwd)
           }
         }
         if (h == 0) {
-          sm.splat[l].set(a, b, c, 0);
+          sm.splat[l].set(a, b, c, pf[r].idet);
           sm.rec[l] = pf_rec[r];
           // plain: cannot reach alpha 0.99, and nothing about it overflows
           const bool wild = !(fabsf(c.x) <= 1e15f && fabsf(c.y) <= 1e15f && fabsf(c.z) <= 1e15f);
@@ -798,9 +800,9 @@ __global__ void __launch_bounds__(Lay<TS>::kThreads, Lay<TS>::kMinBlocksBwd)
         if ((lane & 3) == 0) atomicOr(&sm.got[w][slot >> 5], 1u << (slot & 31));
       }
       if (safe_pixels && __all_sync(0xffffffffu, tame))
-        reduce_hits<false, TS>(sm, w, lane, count, slot);
+        reduce_hits<false>(sm, w, lane, count, slot);
       else
-        reduce_hits<true, TS>(sm, w, lane, count, slot);
+        reduce_hits<true>(sm, w, lane, count, slot);
       count = 0;
       __syncwarp();
     };
@@ -879,7 +881,7 @@ __global__ void __launch_bounds__(Lay<TS>::kThreads, Lay<TS>::kMinBlocksBwd)
           const float2 Tb = mul2(T, make_float2(rcp(om.x), rcp(om.y)));
           const float2 fac = mul2(al[g], Tb);
           const float2 lit = lit_of(sm.splat[t]);
-          const float2 s2 = mul2(oe[g], mul2(Tb, weigh(lit)));
+          const float2 s2 = mul2(fac, weigh(lit));  // (fac as for a plain splat where it counts)
           const float2 next = fma2(lit, fac, acc);
           float2 s;
           s.x = o0 && oe[g].x <= kMaxAlpha ? s2.x : 0.f;
@@ -946,8 +948,8 @@ void launch_bwd(RasterBuffers& rb, const float* image, const float* grad_rgb, co
     static std::atomic<uint64_t> set{0};                                                     \
     allow_smem(composite_bwd_kernel<TS, F, E, kBatch>, smem, set);                           \
     launch_pdl(composite_bwd_kernel<TS, F, E, kBatch>, dim3(rb.tiles), dim3(NT), smem, s,    \
-               rb.rec_a, rb.rec_b, rb.rec_c, rb.sorted_splat, rb.seg_start, rb.rect,         \
-               rb.ranges, order, rb.alphas, rb.last_ids, g, t, rb.isect_grad, rb.width,      \
+               rb.rec_a, rb.rec_b, rb.rec_c, rb.rec_idet, rb.sorted_splat, rb.seg_start,     \
+               rb.rect, rb.ranges, order, rb.alphas, rb.last_ids, g, t, rb.isect_grad, rb.width,      \
                rb.height, rb.ntx, rb.tile_inst, rb.geom, rb.depth_keys, rb.tile_bound);      \
   } while (0)
   if (grad_rgb) {

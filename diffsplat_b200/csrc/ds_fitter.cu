@@ -79,12 +79,12 @@ static int fitter_enqueue(ds_fitter* f, cudaStream_t s, cudaEvent_t* ev = nullpt
   if (bf16)
     DS_CUDA(launch_pdl(fit_preprocess_kernel<__nv_bfloat16>, dim3(blocks), dim3(kThreads), 0, s,
                        f->P, f->R16, f->cfg.sh_degree, f->cam_dev, rb.width, rb.height, rb.ntx,
-                       rb.nty, rb.rec_a, rb.rec_b, rb.rec_c, rb.rect, rb.counts,
+                       rb.nty, rb.rec_a, rb.rec_b, rb.rec_c, rb.rec_idet, rb.rect, rb.counts,
                        rb.depth_keys, rb.scalars, nullptr, nullptr));
   else
     DS_CUDA(launch_pdl(fit_preprocess_kernel<float>, dim3(blocks), dim3(kThreads), 0, s, f->P,
                        soa_of(f->P), f->cfg.sh_degree, f->cam_dev, rb.width, rb.height, rb.ntx,
-                       rb.nty, rb.rec_a, rb.rec_b, rb.rec_c, rb.rect, rb.counts,
+                       rb.nty, rb.rec_a, rb.rec_b, rb.rec_c, rb.rec_idet, rb.rect, rb.counts,
                        rb.depth_keys, rb.scalars, nullptr, nullptr));
   if (ev) DS_CUDA(cudaEventRecord(ev[1], s));
   DS_TRY(raster_build_lists(rb, n, s, ev ? ev + 2 : nullptr, true));

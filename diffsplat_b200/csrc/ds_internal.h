@@ -218,6 +218,7 @@ struct RasterBuffers {
   float4* rec_a = nullptr;
   float4* rec_b = nullptr;
   float4* rec_c = nullptr;
+  float* rec_idet = nullptr;   // null: no backward follows
   ushort4* rect = nullptr;     // tile rectangle {x0, x1, y0, y1}; {1, 0, 1, 0} when invisible
   ushort4* rect_sorted = nullptr;  // in depth order (tile lists by bins; else null)
   uint32_t* counts = nullptr;  // tiles per splat (0 = invisible)

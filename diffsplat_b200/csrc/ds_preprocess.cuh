@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(kPreThreads)
     fit_preprocess_kernel(ds_gaussian3d P, Soa<T> R, int degree, const Camera* __restrict__ camp,
                           int W, int H, int ntx, int nty, float4* __restrict__ ra,
                           float4* __restrict__ rb, float4* __restrict__ rc,
-                          ushort4* __restrict__ rect,
+                          float* __restrict__ ridet, ushort4* __restrict__ rect,
                           uint32_t* __restrict__ counts, uint32_t* __restrict__ depth_keys,
                           DevScalars* __restrict__ sc,
                           const uint16_t* __restrict__ inst_of_splat = nullptr,
@@ -119,6 +119,7 @@ __global__ void __launch_bounds__(kPreThreads)
         ra[i] = rec.a;
         rb[i] = rec.b;
         rc[i] = rec.c;
+        if (ridet) ridet[i] = rec.idet;
         rect[i] = make_ushort4(r.x0, r.x1, r.y0, r.y1);
         counts[i] = (uint32_t)((r.x1 - r.x0 + 1) * (r.y1 - r.y0 + 1));
         depth_keys[i] = depth_bits(ndc_z);

@@ -38,7 +38,7 @@ __device__ __forceinline__ void count_visible(bool vis, uint32_t* visible) {
 // Splat2D SoA -> records / rectangles / counts / depth keys (layer-API path).
 __global__ void __launch_bounds__(kThreads)
     prep_splat2d_kernel(ds_splat2d in, int n, int W, int H, int ntx, int nty, float4* ra,
-                        float4* rb, float4* rc, ushort4* rect, uint32_t* counts,
+                        float4* rb, float4* rc, float* ridet, ushort4* rect, uint32_t* counts,
                         uint32_t* depth_keys, DevScalars* sc) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i == 0) sc->n_splats = (uint32_t)n;
@@ -54,6 +54,7 @@ __global__ void __launch_bounds__(kThreads)
       ra[i] = rec.a;
       rb[i] = rec.b;
       rc[i] = rec.c;
+      if (ridet) ridet[i] = rec.idet;
       rect[i] = make_ushort4(r.x0, r.x1, r.y0, r.y1);
       counts[i] = (uint32_t)((r.x1 - r.x0 + 1) * (r.y1 - r.y0 + 1));
       depth_keys[i] = depth_bits(z);
@@ -533,6 +534,7 @@ static int raster_alloc_splats(RasterBuffers& rb, int max_splats, int64_t cap) {
   DS_TRY(alloc(&rb.rec_a, n));
   DS_TRY(alloc(&rb.rec_b, n));
   DS_TRY(alloc(&rb.rec_c, n));
+  if (!rb.image_only) DS_TRY(alloc(&rb.rec_idet, n));
   DS_TRY(alloc(&rb.rect, n));
   DS_TRY(alloc(&rb.counts, n));
   DS_TRY(alloc(&rb.seg_start, n));
@@ -665,6 +667,7 @@ void raster_free(RasterBuffers& rb) {
   release(rb.rec_a);
   release(rb.rec_b);
   release(rb.rec_c);
+  release(rb.rec_idet);
   release(rb.rect);
   release(rb.counts);
   release(rb.seg_start);
@@ -699,7 +702,7 @@ int raster_prepare_from_splat2d(RasterBuffers& rb, const ds_splat2d& in, cudaStr
   DS_CUDA(cudaMemsetAsync(&rb.scalars->visible, 0, sizeof(uint32_t), s));
   const int blocks = n > 0 ? (n + kThreads - 1) / kThreads : 1;
   prep_splat2d_kernel<<<blocks, kThreads, 0, s>>>(in, n, rb.width, rb.height, rb.ntx, rb.nty,
-                                                  rb.rec_a, rb.rec_b, rb.rec_c,
+                                                  rb.rec_a, rb.rec_b, rb.rec_c, rb.rec_idet,
                                                   rb.rect, rb.counts, rb.depth_keys, rb.scalars);
   return cuda_status(cudaGetLastError());
 }

@@ -55,8 +55,8 @@ int ds_renderer_create(int width, int height, int max_splats, int sh_degree, int
   r->max_splats = max_splats;
   r->bands = ds::sh_bands(sh_degree);
   int st;
-  if ((st = ds::raster_alloc(r->rb, width, height, max_splats, max_isects))) return fail(st);
   r->rb.image_only = true;
+  if ((st = ds::raster_alloc(r->rb, width, height, max_splats, max_isects))) return fail(st);
   if ((st = ds::cuda_status(ds::device_alloc(&r->cam_dev, sizeof(ds::Camera))))) return fail(st);
   cudaMemset(r->cam_dev, 0, sizeof(ds::Camera));
   if ((st = ds::cuda_status(ds::device_alloc(&r->image, image_floats(width, height) * 4))))
@@ -131,12 +131,12 @@ int ds_renderer_render(ds_renderer* r, const float pv[16], const float cam_pos[3
     if (r->storage == DS_STORAGE_BF16)
       ds::fit_preprocess_kernel<<<blocks, ds::kPreThreads, 0, s>>>(
           r->P, r->R16, r->active_degree, r->cam_dev, rb.width, rb.height, rb.ntx, rb.nty,
-          rb.rec_a, rb.rec_b, rb.rec_c, rb.rect, rb.counts, rb.depth_keys,
+          rb.rec_a, rb.rec_b, rb.rec_c, rb.rec_idet, rb.rect, rb.counts, rb.depth_keys,
           rb.scalars);
     else
       ds::fit_preprocess_kernel<<<blocks, ds::kPreThreads, 0, s>>>(
           r->P, ds::soa_of(r->P), r->active_degree, r->cam_dev, rb.width, rb.height, rb.ntx,
-          rb.nty, rb.rec_a, rb.rec_b, rb.rec_c, rb.rect, rb.counts, rb.depth_keys,
+          rb.nty, rb.rec_a, rb.rec_b, rb.rec_c, rb.rec_idet, rb.rect, rb.counts, rb.depth_keys,
           rb.scalars);
     DS_CUDA(cudaGetLastError());
   }

@@ -42,17 +42,18 @@ namespace {
 constexpr int kFwdGroup = DS_FWD_GROUP;  // forward hits whose alphas are computed together
 constexpr int kBwdHits = 8;  // hits whose gradients a warp sums at once, four lanes each
 
-// Backward CTA of one tile: a warp per 8x8 block.
-template <int TS>
+// Backward CTA of one tile: a warp per 8x8 block.  kLong: batches of 256 splats for
+// grids where the longest lists decide (long_batches).
+template <int TS, bool kLong>
 struct Lay {
   static constexpr int kWarps = (TS / 8) * (TS / 8);
   static constexpr int kThreads = 32 * kWarps;
   // backward batch: the per-warp partials (kWarps x kBwdBatch x 36 B) stay within
-  // 9 KB up to 16-pixel tiles, 18 KB at 32
-  static constexpr int kBwdBatch = kWarps <= 1 ? 128 : kWarps <= 4 ? 64 : 32;
+  // 9 KB up to 16-pixel tiles (37 KB with kLong), 18 KB at 32
+  static constexpr int kBwdBatch = kWarps <= 1 ? 128 : kWarps <= 4 ? (kLong ? 256 : 64) : 32;
   // 16-pixel tiles: 5 CTAs per SM (96 registers); 4 and 6 measured 0.307 and
   // 0.326 ms against 0.301 on the 1280x720 fit at step 25 (B200)
-  static constexpr int kMinBlocksBwd = kWarps == 4 ? DS_BWD_MIN_BLOCKS : 1;
+  static constexpr int kMinBlocksBwd = kWarps != 4 ? 1 : kLong ? 2 : DS_BWD_MIN_BLOCKS;
 };
 
 // Where a tile lies: its image size, its tile grid, its index in that grid and
@@ -473,9 +474,9 @@ __global__ void __launch_bounds__(32 * kFwdWarps, DS_FWD_MIN_BLOCKS)
 }
 
 // Shared memory of one backward CTA (dynamic: up to 120 KB for 32-pixel tiles).
-template <int TS>
+template <int TS, bool kLong>
 struct BwdShared {
-  using Lc = Lay<TS>;
+  using Lc = Lay<TS, kLong>;
   static constexpr int B = Lc::kBwdBatch, NW = Lc::kWarps;
   // Row of a hit's per-pixel values: 4 floats past the pixels of a warp, so
   // that the eight lanes of a 16-byte shared-memory phase (two hits, four
@@ -620,8 +621,8 @@ __device__ __forceinline__ void reduce_hits(Sh& sm, int w, int lane, int count,
 // and one of the pixel's last contributor, and no other select.
 // Step 4 of the 1280x720 fit 0.258 -> 0.218 ms; the million splats 0.525 -> 0.491, with
 // batches staged ahead (there the warps of a tile wait for one another at every batch).
-template <int TS, bool kFusedLoss, bool kExact, bool kBatch>
-__global__ void __launch_bounds__(Lay<TS>::kThreads, Lay<TS>::kMinBlocksBwd)
+template <int TS, bool kFusedLoss, bool kExact, bool kBatch, bool kLong>
+__global__ void __launch_bounds__(Lay<TS, kLong>::kThreads, Lay<TS, kLong>::kMinBlocksBwd)
     composite_bwd_kernel(const float4* __restrict__ ra, const float4* __restrict__ rb,
                          const float4* __restrict__ rc, const float* __restrict__ ridet,
                          const uint32_t* __restrict__ sorted_splat,
@@ -636,8 +637,8 @@ __global__ void __launch_bounds__(Lay<TS>::kThreads, Lay<TS>::kMinBlocksBwd)
                          const uint32_t* __restrict__ depth_keys,
                          unsigned long long* __restrict__ tile_bound) {
   pdl_wait();
-  using Lc = Lay<TS>;
-  using Sh = BwdShared<TS>;
+  using Lc = Lay<TS, kLong>;
+  using Sh = BwdShared<TS, kLong>;
   constexpr int NT = Lc::kThreads;
   constexpr int NW = Lc::kWarps;
   constexpr int B = Lc::kBwdBatch;
@@ -934,20 +935,21 @@ void launch_fwd(RasterBuffers& rb, float* out_rgb, const float* target, bool cou
 #undef DS_FWD
 }
 
-template <int TS, bool kBatch>
+template <int TS, bool kBatch, bool kLong = false>
 void launch_bwd(RasterBuffers& rb, const float* image, const float* grad_rgb, const float* target,
                 cudaStream_t s) {
-  constexpr int NT = Lay<TS>::kThreads;
+  constexpr int NT = Lay<TS, kLong>::kThreads;
   const float* g = grad_rgb ? grad_rgb : image;
   const float* t = grad_rgb ? nullptr : target;
   const bool exact = rb.grad_mode == DS_GRAD_EXACT;
   const int32_t* order = schedule(rb);
-  constexpr int smem = (int)sizeof(BwdShared<TS>);
+  constexpr int smem = (int)sizeof(BwdShared<TS, kLong>);
 #define DS_BWD(F, E)                                                                         \
   do {                                                                                       \
     static std::atomic<uint64_t> set{0};                                                     \
-    allow_smem(composite_bwd_kernel<TS, F, E, kBatch>, smem, set);                           \
-    launch_pdl(composite_bwd_kernel<TS, F, E, kBatch>, dim3(rb.tiles), dim3(NT), smem, s,    \
+    allow_smem(composite_bwd_kernel<TS, F, E, kBatch, kLong>, smem, set);                     \
+    launch_pdl(composite_bwd_kernel<TS, F, E, kBatch, kLong>, dim3(rb.tiles), dim3(NT), smem, \
+               s,                                                                            \
                rb.rec_a, rb.rec_b, rb.rec_c, rb.rec_idet, rb.sorted_splat, rb.seg_start,     \
                rb.rect, rb.ranges, order, rb.alphas, rb.last_ids, g, t, rb.isect_grad, rb.width,      \
                rb.height, rb.ntx, rb.tile_inst, rb.geom, rb.depth_keys, rb.tile_bound);      \
@@ -960,6 +962,18 @@ void launch_bwd(RasterBuffers& rb, const float* image, const float* grad_rgb, co
     else DS_BWD(true, false);
   }
 #undef DS_BWD
+}
+
+// Whether the backward takes its lists in batches of 256 splats, 2 CTAs per SM, not of 64,
+// 5 CTAs.  The warps of a tile meet twice a batch, which counts where few warps
+// share an SM: in grids whose tiles are all on the chip at once, and where most splats
+// lie in few tiles, as with more than 65536 of them (surfaces).  Elsewhere the other CTAs
+// are worth more.  Kernel in ms, 64 / 256 (B200): random splats, 60000 at 256x256 (256 tiles)
+// 0.073 / 0.066, 433x341 (616) 0.070 / 0.094, 1280x720 (3600) 0.221 / 0.333; surfaces, 94000 at
+// 184x144 0.501 / 0.435, 433x341 0.549 / 0.463, 1280x720 0.201 / 0.164, 500000 at 1280x720 0.569 /
+// 0.490.  128 splats and 4 CTAs lie between (94000 at 433x341 0.502).
+bool long_batches(const RasterBuffers& rb) {
+  return rb.tiles <= (rb.max_splats > kSmallSort ? 4096 : 2 * 148);
 }
 
 // Single instance: 16-pixel tiles.  Batch: tiles of 8, 16 or 32 pixels.
@@ -995,7 +1009,9 @@ int raster_composite_count(RasterBuffers& rb, float* out_rgb, cudaStream_t s) {
 
 int raster_composite_backward(RasterBuffers& rb, const float* image, const float* grad_rgb,
                               const float* target, cudaStream_t s) {
-  if (!rb.geom) launch_bwd<16, false>(rb, image, grad_rgb, target, s);
+  if (!rb.geom && long_batches(rb))
+    launch_bwd<16, false, true>(rb, image, grad_rgb, target, s);
+  else if (!rb.geom) launch_bwd<16, false>(rb, image, grad_rgb, target, s);
   else if (rb.tile_size == 8) launch_bwd<8, true>(rb, image, grad_rgb, target, s);
   else if (rb.tile_size == 32) launch_bwd<32, true>(rb, image, grad_rgb, target, s);
   else launch_bwd<16, true>(rb, image, grad_rgb, target, s);

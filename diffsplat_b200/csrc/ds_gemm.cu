@@ -329,67 +329,102 @@ __global__ void transpose_bf16_kernel(const __nv_bfloat16* __restrict__ in, int 
   }
 }
 
-// Column sums of a [M][C] BF16 matrix in two fixed-order passes.  Bound by reading the
-// matrix: a thread takes eight columns of a row (16 bytes) where rows are whole
-// 16-byte groups, the CTA's threads several rows side by side, four of them in
-// flight.  One column per thread, a row at a time, and a second pass of one thread per
-// column took 49 us on 131072 x 128 (33 MB) and 54 on 131072 x 256; now 19 and 28 (B200,
+// Column sums of a [M][C] BF16 matrix in two fixed-order passes: the rows of a chunk one
+// after another, then the chunks.  Bound by reading the matrix: where rows are whole
+// 16-byte groups, the CTA of a chunk brings 16 KB of rows at a time into shared memory, the
+// next ones in flight, and a thread per column adds them in order; the second pass does the
+// same with the partials.  One column per thread straight from memory, and a second pass of one
+// thread per column, took 49 us on 131072 x 128 (33 MB) and 54 on 131072 x 256; now 16 and 23 (B200,
 // cold caches).
 constexpr int kColThreads = 256;
+constexpr int kColTile = 16384;  // bytes of rows in shared memory
+constexpr int kColMost = 256;    // columns of a CTA
 
-// VEC columns per thread: 8, or 1 for rows that are not whole 16-byte groups.
-template <int VEC>
 __global__ void __launch_bounds__(kColThreads)
-    colsum_partial_kernel(const __nv_bfloat16* __restrict__ a, int64_t M, int C, int chunk,
-                          float* __restrict__ part) {
-  __shared__ float sum[kColThreads][VEC + (VEC > 1 ? 1 : 0)];
-  const int groups = (C + VEC - 1) / VEC;           // of columns
-  const int wide = min(groups, kColThreads);        // of them side by side in this CTA
-  const int lines = kColThreads / wide;             // rows side by side
-  const int g = blockIdx.x * wide + threadIdx.x % wide, line = threadIdx.x / wide;
-  const int64_t r0 = (int64_t)blockIdx.y * chunk, r1 = min(M, r0 + chunk);
-  float s[VEC];
+    colsum_rows_kernel(const __nv_bfloat16* __restrict__ a, int64_t M, int C, int chunk,
+                       float* __restrict__ part) {
+  __shared__ __align__(16) unsigned char tile[2][kColTile];
+  constexpr int kLoads = kColTile / 16 / kColThreads;
+  const int c0 = blockIdx.y * kColMost, wide = min(kColMost, C - c0), groups = wide / 8;
+  const int rows = kColTile / (2 * wide);  // of a tile
+  const int64_t r0 = (int64_t)blockIdx.x * chunk, r1 = min(M, r0 + chunk);
+  uint4 v[kLoads];
+  auto load = [&](int64_t r) {
 #pragma unroll
-  for (int k = 0; k < VEC; ++k) s[k] = 0.f;
-  if (g < groups && line < lines) {
-#pragma unroll 4
-    for (int64_t r = r0 + line; r < r1; r += lines) {
-      if constexpr (VEC == 8) {
-        const uint4 v = *reinterpret_cast<const uint4*>(a + r * C + 8 * g);
-        const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+    for (int q = 0; q < kLoads; ++q) {
+      const int i = q * kColThreads + threadIdx.x, y = i / groups;
+      if (y < rows && r + y < r1)
+        v[q] = *reinterpret_cast<const uint4*>(a + (r + y) * C + c0 + 8 * (i - y * groups));
+    }
+  };
+  float s = 0.f;
+  load(r0);
+  int buf = 0;
+  for (int64_t r = r0; r < r1; r += rows, buf ^= 1) {
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          s[2 * k] += __uint_as_float(u[k] << 16);
-          s[2 * k + 1] += __uint_as_float(u[k] & 0xffff0000u);
-        }
-      } else {
-        s[0] += __bfloat162float(a[r * C + g]);
-      }
+    for (int q = 0; q < kLoads; ++q) {
+      const int i = q * kColThreads + threadIdx.x;
+      if (i / groups < rows) reinterpret_cast<uint4*>(tile[buf])[i] = v[q];
+    }
+    __syncthreads();  // and everyone is past the other tile
+    load(r + rows);
+    if ((int)threadIdx.x < wide) {
+      const int n = (int)min((int64_t)rows, r1 - r);
+      const unsigned short* t = reinterpret_cast<const unsigned short*>(tile[buf]) + threadIdx.x;
+#pragma unroll 16
+      for (int y = 0; y < n; ++y) s += __uint_as_float((uint32_t)t[y * wide] << 16);
     }
   }
-#pragma unroll
-  for (int k = 0; k < VEC; ++k) sum[threadIdx.x][k] = s[k];
-  __syncthreads();
-  if (line != 0 || g >= groups) return;
-#pragma unroll
-  for (int k = 0; k < VEC; ++k) {
-    float t = 0.f;
-    for (int l = 0; l < lines; ++l) t += sum[l * wide + threadIdx.x][k];
-    part[(int64_t)blockIdx.y * C + VEC * g + k] = t;
-  }
+  if ((int)threadIdx.x < wide) part[(int64_t)blockIdx.x * C + c0 + threadIdx.x] = s;
 }
 
-// One warp per column.
+// Any C and alignment: a thread per column and chunk, sixteen rows in flight.
 __global__ void __launch_bounds__(kColThreads)
+    colsum_any_kernel(const __nv_bfloat16* __restrict__ a, int64_t M, int C, int chunk, int parts,
+                      float* __restrict__ part) {
+  const int64_t id = (int64_t)blockIdx.x * kColThreads + threadIdx.x;
+  const int k = (int)(id / C), c = (int)(id - (int64_t)k * C);
+  if (k >= parts) return;
+  const int64_t r1 = min(M, (int64_t)(k + 1) * chunk);
+  float s = 0.f;
+#pragma unroll 16
+  for (int64_t r = (int64_t)k * chunk; r < r1; ++r) s += __bfloat162float(a[r * C + c]);
+  part[(int64_t)k * C + c] = s;
+}
+
+// 16 columns per CTA: the partials of up to 592 chunks at once into shared memory, added in
+// order by a thread per column.
+constexpr int kFinalThreads = 1024, kFinalCols = 16, kFinalRows = 592;
+__global__ void __launch_bounds__(kFinalThreads)
     colsum_final_kernel(const float* __restrict__ part, int parts, int C,
                         float* __restrict__ out) {
-  const int c = blockIdx.x * (kColThreads / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (c >= C) return;
+  __shared__ float tile[kFinalRows][kFinalCols + 1];
+  constexpr int kStep = kFinalThreads / kFinalCols;
+  const int x = threadIdx.x % kFinalCols, y = threadIdx.x / kFinalCols;
+  const int c = blockIdx.x * kFinalCols + x;
   float s = 0.f;
-#pragma unroll 4
-  for (int k = lane; k < parts; k += 32) s += part[(int64_t)k * C + c];
-  s = warp_sum(s);
-  if (lane == 0) out[c] = s;
+  for (int k0 = 0; k0 < parts; k0 += kFinalRows) {
+    const int n = min(kFinalRows, parts - k0);
+#pragma unroll
+    for (int q = 0; q < (kFinalRows + kStep - 1) / kStep; ++q) {
+      const int k = q * kStep + y;
+      if (k < n && c < C) tile[k][x] = part[(int64_t)(k0 + k) * C + c];
+    }
+    __syncthreads();
+    if (y == 0) {
+      int k = 0;
+      for (; k + 16 <= n; k += 16) {
+        float v[16];
+#pragma unroll
+        for (int q = 0; q < 16; ++q) v[q] = tile[k + q][x];
+#pragma unroll
+        for (int q = 0; q < 16; ++q) s += v[q];
+      }
+      for (; k < n; ++k) s += tile[k][x];
+    }
+    __syncthreads();
+  }
+  if (y == 0 && c < C) out[c] = s;
 }
 
 // AdamW (decoupled weight decay) on FP32 master weights; writes the BF16
@@ -590,17 +625,17 @@ int ds_colsum_bf16(const void* a, int64_t M, int C, float* workspace, int max_pa
   const int parts = (int)((M + chunk - 1) / chunk);
   cudaStream_t s = (cudaStream_t)stream;
   const bool vec = C % 8 == 0 && ((uintptr_t)a & 15) == 0;
-  const int groups = vec ? C / 8 : C;
-  const dim3 grid((groups + ds::kColThreads - 1) / ds::kColThreads, parts);
-  if (vec)
-    ds::colsum_partial_kernel<8><<<grid, ds::kColThreads, 0, s>>>((const __nv_bfloat16*)a, M, C,
-                                                                  chunk, workspace);
-  else
-    ds::colsum_partial_kernel<1><<<grid, ds::kColThreads, 0, s>>>((const __nv_bfloat16*)a, M, C,
-                                                                  chunk, workspace);
-  const int warps = ds::kColThreads / 32;
-  ds::colsum_final_kernel<<<(C + warps - 1) / warps, ds::kColThreads, 0, s>>>(workspace, parts, C,
-                                                                              out);
+  if (vec) {
+    ds::colsum_rows_kernel<<<dim3(parts, (C + ds::kColMost - 1) / ds::kColMost), ds::kColThreads, 0,
+                             s>>>((const __nv_bfloat16*)a, M, C, chunk, workspace);
+  } else {
+    const int64_t blocks = ((int64_t)parts * C + ds::kColThreads - 1) / ds::kColThreads;
+    if (blocks > INT32_MAX) return DS_ERR_ARG;
+    ds::colsum_any_kernel<<<(unsigned)blocks, ds::kColThreads, 0, s>>>(
+        (const __nv_bfloat16*)a, M, C, chunk, parts, workspace);
+  }
+  ds::colsum_final_kernel<<<(C + ds::kFinalCols - 1) / ds::kFinalCols, ds::kFinalThreads, 0, s>>>(
+      workspace, parts, C, out);
   return ds::cuda_status(cudaGetLastError());
 }
 

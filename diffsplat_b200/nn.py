@@ -170,7 +170,7 @@ class Conv3x3:
 
     def _implicit_backward(self, dz2, z_prev):
         """The same for the backward of the last forward with gradient rows dz2."""
-        if self.col is not None:
+        if self.col is not None or self.cin == 3:
             return False
         B, H, W, _ = self.in_shape
         pixels = B * ((H - 1) // self.stride + 1) * ((W - 1) // self.stride + 1)
@@ -184,7 +184,15 @@ class Conv3x3:
         if self._implicit(x, rgb=True):
             B, H, W, _ = self.in_shape = tuple(x.shape)
             Ho, Wo = (H - 1) // self.stride + 1, (W - 1) // self.stride + 1
-            self.x, self.col = x if keep else x.clone(), None
+            self.x = self.col = self.x_col = None
+            if keep:
+                self.x = x
+            elif self.cin == 3 and B * Ho * Wo < 1 << 16:
+                # the backward wants the im2col matrix of x, and at these sizes each call
+                # counts (B200, forward + backward of 8 x 39 x 97: 110 us with a copy, 96 so)
+                self.x_col, _ = im2col(x, self.stride, self.kp)
+            else:
+                self.x = x.clone()
             shape = B, Ho, Wo, self.cout
             z = y = d = None
             if self.gelu:
@@ -197,7 +205,7 @@ class Conv3x3:
                    _p(d), gemm.err.data_ptr(), _s())
             return (z, y) if self.gelu else (d, None)
         col, (B, Ho, Wo) = im2col(x, self.stride, self.kp)
-        self.col, self.x, self.in_shape = col, None, tuple(x.shape)
+        self.col, self.x, self.x_col, self.in_shape = col, None, None, tuple(x.shape)
         if self.gelu:
             z, y = gemm(col, self.w16, EPI_BIAS_GELU, bias=self.b)
             return z.view(B, Ho, Wo, self.cout), y.view(B, Ho, Wo, self.cout)
@@ -225,7 +233,7 @@ class Conv3x3:
             L.call("ds_conv3x3_dgrad", dz2.data_ptr(), *shape, self.w16.data_ptr(), self.kp,
                    self.cout, _p(z_prev), dx.data_ptr(), gemm.err.data_ptr(), _s())
             return dx
-        col = self.col
+        col = self.col if self.col is not None else self.x_col
         if col is None:  # three channels, or gradients that ds_conv3x3_* do not take
             col, _ = im2col(self.x, self.stride, self.kp)
         dzt = transpose(dz2)              # [Cout, M]

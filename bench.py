@@ -137,10 +137,10 @@ FLOPS_PER_PAIR = {"composite_fwd": 24, "composite_bwd": 70}
 
 # DRAM bytes (read + write) per (tile, splat) pair of one composite launch, from
 # one ncu capture of the same 1280x720 / 60000-splat workload (profile run,
-# step 21, 3,085,820 pairs: forward 22.40 MB, backward 59.55 MB), scaled by
+# step 21, 3,085,838 pairs: forward 18.83 MB, backward 56.99 MB), scaled by
 # the bench's own pair count.
-NCU_DRAM_BYTES_PER_ISECT = {"composite_fwd": 22.396416e6 / 3085820,
-                            "composite_bwd": (47.626240e6 + 11.928064e6) / 3085820}
+NCU_DRAM_BYTES_PER_ISECT = {"composite_fwd": (18.820096e6 + 0.005120e6) / 3085838,
+                            "composite_bwd": (46.428672e6 + 10.566144e6) / 3085838}
 
 
 def kernels_per_step(tiles: int, splats: int | None = None) -> int:
@@ -155,7 +155,7 @@ def kernels_per_step(tiles: int, splats: int | None = None) -> int:
     # Without the splats an upper bound: 4 depth-sort passes x 3, count scan x 2,
     # emission, tile sort (grids of up to 8192 tiles: count, offsets + ranges, scatter;
     # larger: 3 kernels per radix pass over the tile id, then ranges and the tile
-    # schedule), and one spare launch of the backward.
+    # schedule), and one more than the single launch of the backward.
     if tiles <= 8192:
         tile_sort = 3  # the offsets kernel also writes the tile schedule
     else:

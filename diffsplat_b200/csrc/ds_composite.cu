@@ -610,8 +610,8 @@ __device__ __forceinline__ void reduce_hits(Sh& sm, int w, int lane, int count,
 // (lane = pixel) only stores s and fac to shared memory, and for every
 // kBwdHits hits (or one fewer, so that the loop has a single place to do it) the
 // lanes regroup, four to a hit, and form the sums over the pixels (reduce_hits),
-// which costs about 22 issue slots a hit where the nine-value butterfly over the
-// warp took about 60.  Against the butterfly (B200): 1280x720 fit of 60000 splats at
+// which cost about 22 issue slots a hit where the nine-value butterfly over the
+// warp took about 60 (counted before the sum for cov xy had its own products).  Against the butterfly (B200): 1280x720 fit of 60000 splats at
 // step 25 0.366 -> 0.301 ms, at step 400 0.828 -> 0.504; a million splats at
 // 1920x1080 0.656 -> 0.600.
 //
@@ -621,6 +621,7 @@ __device__ __forceinline__ void reduce_hits(Sh& sm, int w, int lane, int count,
 // and one of the pixel's last contributor, and no other select.
 // Step 4 of the 1280x720 fit 0.258 -> 0.218 ms; the million splats 0.525 -> 0.491, with
 // batches staged ahead (there the warps of a tile wait for one another at every batch).
+// With the sum for cov xy as it is now: 0.243 and 0.540.
 template <int TS, bool kFusedLoss, bool kExact, bool kBatch, bool kLong>
 __global__ void __launch_bounds__(Lay<TS, kLong>::kThreads, Lay<TS, kLong>::kMinBlocksBwd)
     composite_bwd_kernel(const float4* __restrict__ ra, const float4* __restrict__ rb,

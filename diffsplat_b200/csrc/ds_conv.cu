@@ -52,12 +52,13 @@ namespace {
 enum ConvMode : int { kConvFwd = 0, kConvDgrad = 1, kConvWgrad = 2, kConvPair = 3 };
 enum ConvEpi : int { kConvGelu = 0, kConvF32 = 1 };  // forward only
 
-constexpr int kEpiWarps = 8;  // forward: two per 32 TMEM lanes, each with half of the columns
+constexpr int kEpiWarps = 8;  // two per 32 TMEM lanes; kEpi has the exception
 constexpr int kWgradPixels = 64;  // K block of the weight gradient
 // Pixels summed by one accumulation chain of the weight gradient: the tensor
 // cores' FP32 sums lose precision with the chain's length (relative error
 // 4.6e-6 at 4096 products, the length the im2col path used), so longer
-// reductions are split and their partials added in order.
+// reductions are split and their partials added in order.  There are at most 512
+// partials (64 on the im2col path): beyond 2.1 million pixels the chains grow again.
 constexpr int kWgradChain = 4096;
 
 // A rectangle of pixels per tile: bw x bh of each of bb images (powers of two),

@@ -435,8 +435,11 @@ int offsets(RasterBuffers& rb, int chunks, const int2* inst_hist, cudaStream_t s
 //   surfaces seen from a distance (2 tiles each, most in few bins): 5000 at 512x512
 //   0.071 / 0.073, 60000 at 1280x720 0.100 / 0.083, 300000 0.144 / 0.098, a million at
 //   1920x1080 0.327 / 0.206
-// A fit of many splats comes with small ones, so those sort pairs; batches are of
-// many small fits.
+// What decides is the splats per bin, which the host does not know; their number stands
+// in for it.  A fit of many splats comes with small ones, so those sort pairs, and batches
+// are of many small fits.  It is a guess either way: surfaces of 60000 splats would be
+// 0.02 ms faster by pairs, and 300000 splats over a whole image (29 million pairs) 1.9 ms
+// faster by bins.
 bool tile_bins_pay(const RasterBuffers& rb, const InstGeom* inst) {
   const int k = inst ? rb.instances : 1;
   double hist = 0;

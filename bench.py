@@ -752,8 +752,8 @@ def main():
               "l2": "256 MiB flush between timed steps", "parallelism": f"replicas x{world}",
               "steps_before_timed": args.warmup,
               "fit_state": f"timed steps {args.warmup + 1}-{args.warmup + args.steps} of the fit "
-                           "from its initial state (the composite's cost falls as the fit "
-                           "proceeds)"}
+                           "from its initial state (the composite's cost depends on the "
+                           "state)"}
     line = {"metric": METRIC, "unit": "steps/s", "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "higher_is_better": True, "scaling": "weak",
             "vs_baseline": None, "dtype": "f32", "data": "synthetic (seeded procedural)",
